@@ -585,19 +585,20 @@ int mvg_set_band_whole_fraction(mvg_handle h, double fraction);
  * the strip kernel.  Results are identical either way. */
 int mvg_set_band_ring(mvg_handle h, int on);
 
-/* Watchdog of the gap DP's whole-CTA mode: each wait of a warp for the
- * previous strip's warp polls at most `polls` times (default 2^26, about a
- * second) before it gives up; the kernel then stops that problem, the other
- * warps of the CTA stop at their next wait, and the call returns
- * MVG_ERR_DEVICE instead of hanging.  The handle stays usable.  A very small
+/* Watchdog of the gap DP's pipelined strips: each wait of a warp for the
+ * previous strip's warp polls at most `polls` times (default 2^26, a second
+ * or so; the full DP's slower polls of the L2 cache count as 32) before it
+ * gives up; the other warps then stop at their next wait, and the call
+ * returns MVG_ERR_DEVICE instead of hanging.  The handle stays usable.  A very small
  * limit makes the waits give up on purpose (a test of the watchdog).  No
  * counterpart in the reference (single-threaded). */
 int mvg_set_dp_spin_limit(mvg_handle h, long long polls);
 
 /* Full gap DP: problems of at least `strips` strips (of 32 * rows-per-lane
- * rows) are solved by a whole CTA whose 8 warps pipeline the strips, smaller
- * ones by one warp each (default 16; the Python binding applies the tuned
- * choice in mauve-py_gb300/dp_tuning.json).  Results do not depend on it. */
+ * rows) are solved by a warp per strip, each following its predecessor,
+ * smaller ones by one warp each (default 16; the Python binding applies the
+ * tuned choice in mauve-py_gb300/dp_tuning.json).  Results do not depend on
+ * it. */
 int mvg_set_dp_coop_strips(mvg_handle h, int strips);
 
 /* mvg_gapdp_banded: the tallest group height (rows per lane) a band may use
@@ -613,19 +614,21 @@ int mvg_set_ring_max_rows(mvg_handle h, int rows);
 int mvg_set_band_whole_full_rows(mvg_handle h, int64_t rows);
 
 /* Full gap-DP passes checkpointed (on = 1, the default): the forward pass
- * keeps every strip's bottom row and, every 128 columns, every strip's
- * column of cell states instead of traceback bits (about 0.19 instead of
- * 0.5 bytes per cell), and the traceback recomputes the bits of only the
- * blocks of the matrix its path crosses, with the same recurrence and tie
- * order.  on = 0 stores the bits.  Scores and paths are identical either
+ * keeps every strip's bottom row and, every 128 steps, the strip's state
+ * instead of traceback bits (about 0.1 instead of 0.5 bytes per cell), and
+ * the traceback recomputes the bits of only the blocks of the matrix its
+ * path crosses, with the same recurrence and tie order; problems of up to
+ * 700 columns store the bits all the same.  on = 0 stores the bits (except
+ * for pairs of which both sequences are longer than 400,000).  Scores and paths are identical either
  * way; banded passes always store bits.  No counterpart in the reference. */
 int mvg_set_dp_checkpoint(mvg_handle h, int on);
 
 /* Gap-DP passes as one CUDA graph (on = 1, the default): the launches of a
- * call's waves (claim counters, the persistent DP kernel, both traceback
- * walkers, path compaction) are recorded into one graph and launched at
- * once; the handle keeps the executable graph per DP lane and updates it in
- * place from the next call's recording when its shape is the same.  on = 0
+ * call's waves (claim counters, the persistent DP kernels, the traceback
+ * walkers) are recorded into one graph and launched at once; the handle
+ * keeps the executable graph per DP lane and updates it in place from the
+ * next call's recording when its shape is the same.  A full-DP pass of a
+ * single wave is three launches and is not recorded.  on = 0
  * launches them one by one.  Results are identical either way.  No
  * counterpart in the reference. */
 int mvg_set_dp_graph(mvg_handle h, int on);

@@ -27,12 +27,13 @@
 #include <functional>
 #include <numeric>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "gapdp_kernel.cuh"
 #include "traceback_win.cuh"
-#include "traceback_ck.cuh"
 #include "gapdp_ring.cuh"
+#include "gapdp_strips.cuh"
 #include "mvg_internal.h"
 
 namespace mvg {
@@ -70,20 +71,10 @@ int upload_score_table() {
   return 0;
 }
 
-template __global__ void k_gapdp_t<false, 4>(DpJob);
-template __global__ void k_gapdp_t<true, 4>(DpJob);
-template __global__ void k_gapdp_t<false, 8>(DpJob);
-template __global__ void k_gapdp_t<true, 8>(DpJob);
-template __global__ void k_gapdp_t<true, 2>(DpJob);
-template __global__ void k_gapdp_t<true, 1>(DpJob);
-template __global__ void k_gapdp_t<false, 4, true>(DpJob);
-template __global__ void k_gapdp_t<false, 8, true>(DpJob);
-template __global__ void k_tb_ck<4>(const uint8_t*, const uint64_t*, const uint8_t*, const uint64_t*, const uint32_t*,
-                                    const uint64_t*, int, const uint32_t*, const uint8_t*, const uint64_t*, char*,
-                                    int64_t*, uint32_t*, int32_t*, unsigned*);
-template __global__ void k_tb_ck<8>(const uint8_t*, const uint64_t*, const uint8_t*, const uint64_t*, const uint32_t*,
-                                    const uint64_t*, int, const uint32_t*, const uint8_t*, const uint64_t*, char*,
-                                    int64_t*, uint32_t*, int32_t*, unsigned*);
+template __global__ void k_gapdp_t<1>(DpJob);
+template __global__ void k_gapdp_t<2>(DpJob);
+template __global__ void k_gapdp_t<4>(DpJob);
+template __global__ void k_gapdp_t<8>(DpJob);
 template __global__ void k_gapdp_ring<4>(RingJob);
 template __global__ void k_gapdp_ring<6>(RingJob);
 template __global__ void k_gapdp_ring<8>(RingJob);
@@ -147,16 +138,17 @@ static void (*ring_kernel(int R))(RingJob) {
   }
 }
 
-// BitTraceBack from (LA, LB); writes the path reversed at the end of the
-// problem's path slot and its length.  Banded problems index their strips
-// through the band geometry (only accepted ones are traced).
+// BitTraceBack of the banded strip kernel's problems from (LA, LB); writes the
+// path reversed at the end of the problem's path slot and its length.  The
+// strips are indexed through the band geometry (only accepted problems are
+// traced).
 __global__ void k_traceback(const uint64_t* __restrict__ oa, const uint64_t* __restrict__ ob,
                             const uint32_t* __restrict__ order, const uint64_t* __restrict__ tb_off, int nwork,
                             const uint32_t* __restrict__ tb, const uint8_t* __restrict__ end_edge,
                             const int32_t* __restrict__ band_delta, const int32_t* __restrict__ band_half,
                             const uint8_t* __restrict__ accept, const uint64_t* __restrict__ path_off,
                             char* __restrict__ paths, int64_t* __restrict__ path_len, uint32_t* err,
-                            int rows, int32_t* __restrict__ env, int long_path) {
+                            int rows, int long_path) {
   const int srows = 32 * rows;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nwork; w += gridDim.x * blockDim.x) {
     const uint32_t p = order[w];
@@ -164,8 +156,7 @@ __global__ void k_traceback(const uint64_t* __restrict__ oa, const uint64_t* __r
     const int LA = (int)(oa[p + 1] - oa[p]), LB = (int)(ob[p + 1] - ob[p]);
     if (LA + LB >= long_path) continue;  // k_traceback_win walks it
     const uint32_t* T = tb + tb_off[w] / 4;
-    const bool banded = band_delta != nullptr;
-    const Band band = banded ? make_band(LA, LB, band_delta[p], band_half[p], srows) : make_full(LA, LB, srows);
+    const Band band = make_band(LA, LB, band_delta[p], band_half[p], srows);
     // strip k's word base and first column; strips are walked bottom-up
     int cur_k = (LA - 1) / srows;
     int64_t base = 0;
@@ -177,9 +168,6 @@ __global__ void k_traceback(const uint64_t* __restrict__ oa, const uint64_t* __r
     char cur = (char)end_edge[p];
     int64_t n = 0;
     const int64_t limit = (int64_t)LA + LB;
-    // path envelope: extreme deviations of the visited cells (rows >= 1) from
-    // the diagonal j = i*LB/LA, the quantity a band must cover
-    int32_t dev_lo = INT32_MAX, dev_hi = INT32_MIN;
     for (;;) {
       if (n >= limit) {
         set_error(err, kDevCapacity);
@@ -187,11 +175,6 @@ __global__ void k_traceback(const uint64_t* __restrict__ oa, const uint64_t* __r
       }
       *(--out) = cur;
       ++n;
-      if (env && pa >= 1) {
-        const int32_t dv = pb - (int32_t)((int64_t)pa * LB / LA);
-        dev_lo = min(dev_lo, dv);
-        dev_hi = max(dev_hi, dv);
-      }
       uint32_t bits = 0;
       if (pa >= 1 && pb >= 1) {
         const int i0 = pa - 1;
@@ -243,10 +226,6 @@ __global__ void k_traceback(const uint64_t* __restrict__ oa, const uint64_t* __r
       cur = next;
     }
     path_len[p] = n;
-    if (env) {
-      env[2 * p] = dev_lo;
-      env[2 * p + 1] = dev_hi;
-    }
   }
 }
 
@@ -283,7 +262,7 @@ struct DpInputs {
   char* paths;
   const uint64_t* path_off;
   int64_t* path_len;
-  int32_t* env = nullptr;  // optional path envelope output [2 * nprob]
+  int32_t* env = nullptr;  // optional path envelope output [2 * nprob], full DP only
 };
 
 // Starts the long-path walker for one wave on the aux stream (joined by
@@ -299,8 +278,6 @@ struct TbLanes {
   cudaEvent_t fork, join;
   int slot_list, slot_ctr;
 };
-
-static TbLanes main_lanes(Ctx* c) { return TbLanes{c->stream, c->aux, c->fork, c->join, 62, 63}; }
 
 // Host side of the long-path walker: the slots (of this wave's order) whose
 // paths go to warps, longest first, and the length from which they do.
@@ -356,7 +333,7 @@ static int tb_long_launch(Ctx* c, const TbLanes& L, const DpInputs& in, const ui
   MVG_CUDA_TRY(cudaStreamWaitEvent(L.side, L.fork, 0));
   k_traceback_win<<<grid, kTbWarps * 32, kTbSmem, L.side>>>(in.oa, in.ob, d_order, d_tboff, d_slots, n, tb, d_edge,
                                                             d_delta, d_half, d_accept, in.path_off, in.paths,
-                                                            in.path_len, c->d_err, rows, d_rows, in.env, d_ctr);
+                                                            in.path_len, c->d_err, rows, d_rows, d_ctr);
   MVG_CUDA_TRY(cudaEventRecord(L.join, L.side));
   c->launches++;
   return 0;
@@ -461,44 +438,248 @@ class GraphRecorder {
   bool active_ = false;
 };
 
-// Runs the DP for the problems in `ids` (full, or banded with per-problem
-// delta/half on the device): LPT order, size-mixed waves that fit the
-// traceback arena, then traceback and path compaction per wave.
-// Workspace slots of one run_dp lane: row buffers, order, traceback
-// offsets, claim counter, traceback arena.
+// Indices of the problems, largest first (by cells), ties in input order.
+static std::vector<uint32_t> largest_first(const std::vector<uint64_t>& cells) {
+  const size_t n = cells.size();
+  if (n < 2048) {  // the radix passes' 2,048 counters cost more than sorting a few
+    std::vector<uint32_t> idx(n);
+    std::iota(idx.begin(), idx.end(), 0u);
+    std::stable_sort(idx.begin(), idx.end(), [&](uint32_t x, uint32_t y) { return cells[x] > cells[y]; });
+    return idx;
+  }
+  constexpr uint64_t kMax = (1ull << 40) - 1;  // at most 1e6 x 1e6 cells
+  std::vector<uint64_t> key(n);
+  for (size_t w = 0; w < n; ++w) key[w] = kMax - std::min(cells[w], kMax);
+  return radix_order(key);
+}
+
+// Waves of a pass: the size-sorted problems idx are dealt round-robin, so
+// every wave holds the same mix of sizes, and a wave's slots fit `arena`
+// bytes.  Inside a wave the `big` problems come first, each part largest
+// first.
+struct DpWaves {
+  std::vector<uint32_t> item;      // per slot: index into the pass's problems
+  std::vector<uint64_t> off;       // per slot: byte offset in the arena
+  std::vector<int64_t> begin, nbig;  // per wave (begin has one entry more)
+  uint64_t need = 0;
+};
+static DpWaves deal_waves(const std::vector<uint32_t>& idx, const std::vector<char>& big,
+                          const std::vector<uint64_t>& bytes, uint64_t arena) {
+  const int64_t n = (int64_t)idx.size();
+  uint64_t total = 0;
+  for (uint64_t b : bytes) total += b;
+  DpWaves W;
+  W.item.resize(n);
+  W.off.resize(n);
+  for (int64_t nwaves = std::max<int64_t>(1, (int64_t)((total + arena - 1) / std::max<uint64_t>(arena, 1)));; ++nwaves) {
+    W.begin.clear();
+    W.nbig.clear();
+    W.need = 0;
+    int64_t at = 0;
+    bool fits = true;
+    for (int64_t v = 0; v < nwaves && fits; ++v) {
+      W.begin.push_back(at);
+      uint64_t acc = 0;
+      int64_t nb = 0;
+      for (int pass = 0; pass < 2; ++pass)
+        for (int64_t q = v; q < n; q += nwaves) {
+          if ((big[idx[q]] != 0) != (pass == 0)) continue;
+          W.item[at] = idx[q];
+          W.off[at++] = acc;
+          acc += bytes[idx[q]];
+          nb += pass == 0;
+        }
+      W.nbig.push_back(nb);
+      fits = acc <= arena;
+      W.need = std::max(W.need, acc);
+    }
+    if (fits) break;
+  }
+  W.begin.push_back(n);
+  return W;
+}
+
+// The arena bound of a pass: at most 60% of what is free, counting what the
+// slot already holds.
+static uint64_t arena_bound(Ctx* c, int slot, uint64_t total) {
+  if (total <= c->ws.size[slot]) return std::min<uint64_t>(c->tb_arena, total);  // held already: nothing to ask for
+  uint64_t arena = c->tb_arena;
+  size_t free_b = 0, total_b = 0;
+  HostSpan mem_span(c, "meminfo");
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    const size_t have = c->ws.size[slot] + free_b;  // the arena slot itself may be re-allocated
+    arena = std::min(arena, (uint64_t)(have * 0.6));
+  }
+  return arena;
+}
+
+// Workspace slots of one DP lane: row buffers (full DP: units), order,
+// traceback offsets, claim counter, traceback arena.
 struct DpSlots {
   int rowbuf, order, tboff, counter, arena;
 };
 constexpr DpSlots kDpSlots{10, 11, 12, 14, 18};
-constexpr DpSlots kDpSlotsLane2{49, 50, 51, 52, 53};
+constexpr DpSlots kDpSlotsBand{49, 50, 51, 52, 53};
 
-static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, const std::vector<int64_t>& la,
-                  const std::vector<int64_t>& lb, const int32_t* d_delta, const int32_t* d_half,
-                  const std::vector<int32_t>* h_delta, const std::vector<int32_t>* h_half, uint8_t* d_accept,
-                  const TbLanes* lanes = nullptr, const DpSlots& sl = kDpSlots) {
-  const TbLanes L = lanes ? *lanes : main_lanes(c);
+// The full DP of the problems in `ids` on the handle's stream
+// (gapdp_strips.cuh): size-mixed waves that fit the arena, per wave the
+// units of the pipelined problems, the strips kernel and the walk.
+static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, const std::vector<int64_t>& la,
+                    const std::vector<int64_t>& lb) {
   const int64_t nwork = (int64_t)ids.size();
   if (nwork == 0) return 0;
   std::unique_ptr<HostSpan> span(new HostSpan(c, "dp_plan"));
-  const bool banded = d_delta != nullptr;
-  // banded passes may use shorter strips: the staircase of a narrow band
-  // widens by the diagonal's drift over one strip
-  const int rows = banded ? c->band_rows : c->dp_rows;
-  // full passes keep checkpoints instead of traceback bits (traceback_ck.cuh)
-  const bool ckpt = !banded && c->dp_ckpt && (rows == 4 || rows == 8);
   std::unique_ptr<HostSpan> sub(new HostSpan(c, "dp_sizes"));
+  const bool ckpt = c->dp_ckpt != 0;
   std::vector<uint64_t> bytes(nwork), cells(nwork);
-  int64_t maxlb = 0;
+  std::vector<char> piped(nwork), direct(nwork);
+  std::vector<uint32_t> strips(nwork);
+  uint64_t total = 0, most = 0, most_least = 0;
   for (int64_t w = 0; w < nwork; ++w) {
     const uint32_t p = ids[w];
-    const Band b = banded ? make_band((int)la[p], (int)lb[p], (*h_delta)[p], (*h_half)[p], 32 * rows)
-                          : make_full((int)la[p], (int)lb[p], 32 * rows);
-    const uint64_t slot = ckpt ? (uint64_t)ck_entries((int)la[p], (int)lb[p], rows) * sizeof(int4)
-                               : band_tb_words(b, rows) * 4;
-    cells[w] = banded ? band_cells(b) : (uint64_t)la[p] * (uint64_t)lb[p];
-    bytes[w] = (slot + 255) & ~255ull;
-    maxlb = std::max(maxlb, lb[p]);
+    const StripShape h = strip_shape((int)la[p], (int)lb[p], c->dp_rows, ckpt);
+    bytes[w] = strip_slot_bytes(h);
+    cells[w] = (uint64_t)la[p] * (uint64_t)lb[p];
+    strips[w] = (uint32_t)h.n;
+    piped[w] = h.n >= c->dp_coop_strips;
+    direct[w] = h.direct;
+    total += bytes[w];
+    most = std::max(most, bytes[w]);
+    most_least = std::max(most_least, std::min(bytes[w], strip_least_bytes(h, c->dp_rows, ckpt)));
   }
+  uint64_t arena = arena_bound(c, kDpSlots.arena, total);
+  if (most_least > arena) return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
+  arena = std::max(arena, most);
+  sub.reset(new HostSpan(c, "dp_sort"));
+  const std::vector<uint32_t> idx = largest_first(cells);
+  sub.reset(new HostSpan(c, "dp_waves"));
+  const DpWaves W = deal_waves(idx, piped, bytes, arena);
+  const size_t nwaves = W.begin.size() - 1;
+  // one upload: the slots' problems, then per wave the pipelined slots' first
+  // units and the walk's slots (checkpointed, then direct)
+  std::vector<uint32_t> order(nwork);
+  for (int64_t q = 0; q < nwork; ++q) order[q] = ids[W.item[q]];
+  std::vector<size_t> first_at(nwaves), todo_at(nwaves);
+  std::vector<uint32_t> nunits(nwaves);
+  std::vector<int> nck(nwaves);
+  uint32_t max_units = 0;
+  for (size_t wv = 0; wv < nwaves; ++wv) {
+    first_at[wv] = order.size();
+    uint32_t u = 0;
+    for (int64_t q = W.begin[wv]; q < W.begin[wv] + W.nbig[wv]; ++q) {
+      order.push_back(u);
+      u += strips[W.item[q]];
+    }
+    order.push_back(u);
+    nunits[wv] = u;
+    todo_at[wv] = order.size();
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int64_t q = W.begin[wv]; q < W.begin[wv + 1]; ++q)
+        if ((direct[W.item[q]] != 0) == (pass == 1)) order.push_back((uint32_t)(q - W.begin[wv]));
+      if (pass == 0) nck[wv] = (int)(order.size() - todo_at[wv]);
+    }
+    max_units = std::max(max_units, u);
+  }
+  sub.reset(new HostSpan(c, "dp_copy"));
+  Workspace& ws = c->ws;
+  uint32_t* d_units = (uint32_t*)ws.get(c, kDpSlots.rowbuf, (size_t)max_units * 4 + 16);
+  uint32_t* d_order = (uint32_t*)ws.get(c, kDpSlots.order, order.size() * 4);
+  uint64_t* d_off = (uint64_t*)ws.get(c, kDpSlots.tboff, (size_t)nwork * 8);
+  uint8_t* d_edge = (uint8_t*)ws.get(c, 13, la.size() + 16);  // per problem, shared by all lanes
+  unsigned* d_counter = (unsigned*)ws.get(c, kDpSlots.counter, nwaves * 16);
+  uint8_t* arena_p = (uint8_t*)ws.get(c, kDpSlots.arena, std::max<uint64_t>(W.need, 256));
+  if (!d_units || !d_order || !d_off || !d_edge || !d_counter || !arena_p)
+    return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  if (int e = h2d_async(c, d_order, order.data(), order.size() * 4, c->stream)) return e;
+  if (int e = h2d_async(c, d_off, W.off.data(), (size_t)nwork * 8, c->stream)) return e;
+  if (!c->strip_grid) {
+    int sms = 0, bps = 0;
+    MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_strip_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_strip_walk, kWalkWarps * 32, kWalkSmem));
+    c->walk_grid = sms * std::max(1, bps);
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_strips, kStWarps * 32, 0));
+    c->strip_grid = sms * std::max(1, bps);
+  }
+  sub.reset();
+  span.reset();
+  GraphRecorder rec(c, c->stream, c->dp_graph != 0 && nwaves > 1);
+  if (int e = rec.begin()) return e;
+  if (int e = rec.check(cudaMemsetAsync(d_counter, 0, nwaves * 16, c->stream), "cudaMemsetAsync")) return e;
+  for (size_t wv = 0; wv < nwaves; ++wv) {
+    const int64_t w0 = W.begin[wv], n = W.begin[wv + 1] - w0;
+    StripJob J;
+    J.sa = in.sa;
+    J.oa = in.oa;
+    J.sb = in.sb;
+    J.ob = in.ob;
+    J.order = d_order + w0;
+    J.slot_off = d_off + w0;
+    J.unit_first = d_order + first_at[wv];
+    J.unit_slot = d_units;
+    J.nwork = (int)n;
+    J.npipe = (int)W.nbig[wv];
+    J.nunits = (int)nunits[wv];
+    J.max_rows = c->dp_rows;
+    J.ckpt = ckpt;
+    J.arena = arena_p;
+    J.scores = in.scores;
+    J.end_edge = d_edge;
+    J.counter = d_counter + 4 * wv;
+    J.err = c->d_err;
+    J.spin_limit = c->dp_spin_limit;
+    stage_mark(c, "dp");
+    if (J.npipe) {
+      k_strip_units<<<dim3(std::min(J.npipe, 4096), 8), 256, 0, c->stream>>>(J);
+      c->launches++;
+    }
+    const int64_t units = J.nunits + (n - J.npipe);
+    k_gapdp_strips<<<(int)std::min<int64_t>(c->strip_grid, (units + kStWarps - 1) / kStWarps), kStWarps * 32, 0,
+                     c->stream>>>(J);
+    stage_mark(c, "traceback");
+    WalkJob K;
+    K.sa = in.sa;
+    K.oa = in.oa;
+    K.sb = in.sb;
+    K.ob = in.ob;
+    K.order = J.order;
+    K.slot_off = J.slot_off;
+    K.todo = d_order + todo_at[wv];
+    K.nwork = J.nwork;
+    K.nck = nck[wv];
+    K.max_rows = J.max_rows;
+    K.ckpt = ckpt;
+    K.arena = arena_p;
+    K.end_edge = d_edge;
+    K.path_off = in.path_off;
+    K.paths = in.paths;
+    K.path_len = in.path_len;
+    K.err = c->d_err;
+    K.env = in.env;
+    K.counter = J.counter + 2;
+    const int64_t walkers = std::max<int64_t>(K.nck, (n - K.nck + kWalkWarps - 1) / kWalkWarps);
+    k_strip_walk<<<(int)std::min<int64_t>(c->walk_grid, walkers), kWalkWarps * 32, kWalkSmem, c->stream>>>(K);
+    c->launches += 2;
+    if (int e = rec.check(cudaGetLastError(), "kernel launch")) return e;
+  }
+  return rec.launch(&c->dp_exec[0]);
+}
+
+// Banded problems on the strip kernel (bands no ring height fits, and short
+// whole-matrix problems) with per-problem delta/half on the device.
+static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids,
+                           const std::vector<int64_t>& la, const std::vector<int64_t>& lb, const int32_t* d_delta,
+                           const int32_t* d_half, const std::vector<int32_t>& h_delta,
+                           const std::vector<int32_t>& h_half, uint8_t* d_accept, const TbLanes& L) {
+  const int64_t nwork = (int64_t)ids.size();
+  if (nwork == 0) return 0;
+  std::unique_ptr<HostSpan> span(new HostSpan(c, "dp_plan"));
+  // short strips: the staircase of a narrow band widens by the diagonal's drift over one strip
+  const int rows = c->band_rows;
+  std::unique_ptr<HostSpan> sub(new HostSpan(c, "dp_sizes"));
+  std::vector<uint64_t> bytes(nwork), cells(nwork);
+  uint64_t total = 0, most = 0;
+  int64_t maxlb = 0;
   // Whole-CTA (pipelined) mode for problems with many strips.  A banded
   // strip can only start once the previous one has passed the next strip's
   // first column (about one strip height of drift plus the 64-column
@@ -506,83 +687,29 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
   // stay on one warp unless their strips are at least 8 strip heights wide.
   std::vector<char> is_big(nwork);
   for (int64_t w = 0; w < nwork; ++w) {
-    const int64_t a = la[ids[w]];
-    const bool many = (a + 32 * rows - 1) / (32 * rows) >= (banded ? kCoopMinStrips : c->dp_coop_strips);
-    is_big[w] = many && (!banded || cells[w] >= (uint64_t)a * 8 * 32 * rows);
+    const uint32_t p = ids[w];
+    const Band b = make_band((int)la[p], (int)lb[p], h_delta[p], h_half[p], 32 * rows);
+    cells[w] = band_cells(b);
+    bytes[w] = (band_tb_words(b, rows) * 4 + 255) & ~255ull;
+    is_big[w] = b.nstrips >= kCoopMinStrips && cells[w] >= (uint64_t)la[p] * 8 * 32 * rows;
+    maxlb = std::max(maxlb, lb[p]);
+    total += bytes[w];
+    most = std::max(most, bytes[w]);
   }
-  // largest first, ties in input order: one sort of packed (cells, index) keys
+  const uint64_t arena = arena_bound(c, kDpSlotsBand.arena, total);
+  if (most > arena) return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
   sub.reset(new HostSpan(c, "dp_sort"));
-  std::vector<uint32_t> idx;
-  {
-    constexpr uint64_t kMax = (1ull << 40) - 1;  // at most 1e6 x 1e6 cells
-    std::vector<uint64_t> key(nwork);
-    for (int64_t w = 0; w < nwork; ++w) key[w] = kMax - std::min(cells[w], kMax);
-    idx = radix_order(key);
-  }
-
-  uint64_t arena = c->tb_arena;
-  {
-    size_t free_b = 0, total_b = 0;
-    HostSpan mem_span(c, "meminfo");
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-      const size_t have = c->ws.size[sl.arena] + free_b;  // the arena slot itself may be re-allocated
-      const uint64_t cap = (uint64_t)(have * 0.6);
-      if (arena > cap) arena = cap;
-    }
-  }
-  uint64_t total_tb = 0, max_tb = 0;
-  for (int64_t w = 0; w < nwork; ++w) {
-    total_tb += bytes[w];
-    max_tb = std::max(max_tb, bytes[w]);
-  }
-  if (max_tb > arena) return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
+  const std::vector<uint32_t> idx = largest_first(cells);
   sub.reset(new HostSpan(c, "dp_waves"));
-  // Waves: deal the size-sorted problems round-robin, so every wave holds the
-  // same mix of sizes and stays largest-first inside.
-  // at least one wave: checkpointed slots of problems within one block hold nothing
-  int64_t nwaves = std::max<int64_t>(1, (int64_t)((total_tb + arena - 1) / arena));
-  std::vector<uint32_t> order;
-  std::vector<uint64_t> tboff;
-  std::vector<int64_t> wave_begin, wave_nbig;
-  uint64_t arena_need = 0;
-  for (;;) {
-    order.clear();
-    tboff.clear();
-    wave_begin.clear();
-    wave_nbig.clear();
-    arena_need = 0;
-    bool fits = true;
-    for (int64_t v = 0; v < nwaves && fits; ++v) {
-      wave_begin.push_back((int64_t)order.size());
-      uint64_t acc = 0;
-      // large problems (solved by a whole CTA) first, then the rest; each part largest first
-      int64_t nb = 0;
-      for (int pass = 0; pass < 2; ++pass)
-        for (int64_t q = v; q < nwork; q += nwaves) {
-          const bool big = is_big[idx[q]];
-          if (big != (pass == 0)) continue;
-          order.push_back(ids[idx[q]]);
-          tboff.push_back(acc);
-          acc += bytes[idx[q]];
-          nb += big;
-        }
-      wave_nbig.push_back(nb);
-      if (acc > arena) fits = false;
-      arena_need = std::max(arena_need, acc);
-    }
-    if (fits) break;
-    ++nwaves;
-  }
-  wave_begin.push_back(nwork);
+  const DpWaves W = deal_waves(idx, is_big, bytes, arena);
+  const size_t nwaves = W.begin.size() - 1;
+  std::vector<uint32_t> order(nwork);
+  for (int64_t q = 0; q < nwork; ++q) order[q] = ids[W.item[q]];
 
   sub.reset(new HostSpan(c, "dp_copy"));
   int dev_sms = 0;
   MVG_CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
-  void (*kern)(DpJob) = ckpt        ? (rows == 8 ? k_gapdp_t<false, 8, true> : k_gapdp_t<false, 4, true>)
-                        : rows == 8 ? (banded ? k_gapdp_t<true, 8> : k_gapdp_t<false, 8>)
-                        : rows == 4 ? (banded ? k_gapdp_t<true, 4> : k_gapdp_t<false, 4>)
-                        : rows == 2 ? k_gapdp_t<true, 2>
-                                    : k_gapdp_t<true, 1>;
+  void (*kern)(DpJob) = rows == 8 ? k_gapdp_t<8> : rows == 4 ? k_gapdp_t<4> : rows == 2 ? k_gapdp_t<2> : k_gapdp_t<1>;
   int bps = 0;
   MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kDpThreads, 0));
   if (bps < 1) bps = 1;
@@ -590,47 +717,32 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
   const int64_t nwarps = (int64_t)grid * (kDpThreads / 32);
   Workspace& ws = c->ws;
   const int64_t rb_stride = maxlb + 2;
+  const DpSlots& sl = kDpSlotsBand;
   int4* rowbuf = (int4*)ws.get(c, sl.rowbuf, (size_t)nwarps * rb_stride * sizeof(int4));
   uint32_t* d_order = (uint32_t*)ws.get(c, sl.order, (size_t)nwork * 4);
   uint64_t* d_tboff = (uint64_t*)ws.get(c, sl.tboff, (size_t)nwork * 8);
   uint8_t* d_edge = (uint8_t*)ws.get(c, 13, (size_t)(la.size()) + 16);  // per problem, shared by all lanes
   unsigned* d_counter = (unsigned*)ws.get(c, sl.counter, 64);
-  uint32_t* tb = (uint32_t*)ws.get(c, sl.arena, std::max<uint64_t>(arena_need, 256));
+  uint32_t* tb = (uint32_t*)ws.get(c, sl.arena, std::max<uint64_t>(W.need, 256));
   if (!rowbuf || !d_order || !d_tboff || !d_edge || !d_counter || !tb)
     return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   if (int e = h2d_async(c, d_order, order.data(), (size_t)nwork * 4, L.st)) return e;
-  if (int e = h2d_async(c, d_tboff, tboff.data(), (size_t)nwork * 8, L.st)) return e;
+  if (int e = h2d_async(c, d_tboff, W.off.data(), (size_t)nwork * 8, L.st)) return e;
   // the long-path walkers of all waves: slot lists concatenated, one counter each
-  const size_t nwaves_run = wave_begin.size() - 1;
-  std::vector<int> long_path(nwaves_run, INT_MAX), long_n(nwaves_run, 0), long_grid(nwaves_run, 0);
-  std::vector<size_t> long_at(nwaves_run, 0);
+  std::vector<int> long_path(nwaves, INT_MAX), long_n(nwaves, 0), long_grid(nwaves, 0);
+  std::vector<size_t> long_at(nwaves, 0);
   std::vector<uint32_t> all_long;
-  for (size_t wv = 0; wv < nwaves_run; ++wv) {
-    const int64_t w0 = wave_begin[wv], w1 = wave_begin[wv + 1];
+  for (size_t wv = 0; wv < nwaves; ++wv) {
+    const int64_t w0 = W.begin[wv], w1 = W.begin[wv + 1];
     std::vector<uint32_t> slot_len(w1 - w0), ls;
     for (int64_t q = w0; q < w1; ++q) slot_len[q - w0] = (uint32_t)(la[order[q]] + lb[order[q]]);
-    if (!ckpt)  // checkpointed passes walk every path on a warp
-      if (int e = tb_long_plan(c, slot_len, &ls, &long_path[wv], &long_grid[wv])) return e;
+    if (int e = tb_long_plan(c, slot_len, &ls, &long_path[wv], &long_grid[wv])) return e;
     long_at[wv] = all_long.size();
     long_n[wv] = (int)ls.size();
     all_long.insert(all_long.end(), ls.begin(), ls.end());
   }
-  int ck_grid = 0;
-  if (ckpt) {
-    static bool ck_attr[2] = {false, false};  // once per process and kernel: more than 48 KB of shared memory
-    void (*tbk)(const uint8_t*, const uint64_t*, const uint8_t*, const uint64_t*, const uint32_t*, const uint64_t*,
-                int, const uint32_t*, const uint8_t*, const uint64_t*, char*, int64_t*, uint32_t*, int32_t*,
-                unsigned*) = rows == 8 ? k_tb_ck<8> : k_tb_ck<4>;
-    if (!ck_attr[rows == 8]) {
-      MVG_CUDA_TRY(cudaFuncSetAttribute(tbk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCkSmem));
-      ck_attr[rows == 8] = true;
-    }
-    int cbps = 0;
-    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cbps, tbk, kCkWarps * 32, kCkSmem));
-    ck_grid = dev_sms * std::max(1, cbps);
-  }
   uint32_t* d_long = (uint32_t*)ws.get(c, L.slot_list, all_long.size() * 4 + 16);
-  unsigned* d_long_ctr = (unsigned*)ws.get(c, L.slot_ctr, nwaves_run * 4 + 64);
+  unsigned* d_long_ctr = (unsigned*)ws.get(c, L.slot_ctr, nwaves * 4 + 64);
   if (!d_long || !d_long_ctr) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   if (!all_long.empty())
     if (int e = h2d_async(c, d_long, all_long.data(), all_long.size() * 4, L.st)) return e;
@@ -638,13 +750,12 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
   span.reset();
   // Every wave's launches (claim counters, the persistent DP kernel, the two
   // traceback walkers, path compaction) are recorded into one CUDA graph and
-  // launched at once; the executable graph is kept per lane and updated in
-  // place when the next call has the same shape.
-  const int lane_id = sl.arena == kDpSlots.arena ? 0 : 1;
+  // launched at once; the executable graph is kept and updated in place when
+  // the next call has the same shape.
   GraphRecorder rec(c, L.st, c->dp_graph != 0);
   if (int e = rec.begin()) return e;
-  for (size_t wv = 0; wv < nwaves_run; ++wv) {
-    const int64_t w0 = wave_begin[wv], w1 = wave_begin[wv + 1];
+  for (size_t wv = 0; wv < nwaves; ++wv) {
+    const int64_t w0 = W.begin[wv], w1 = W.begin[wv + 1];
     DpJob J;
     J.sa = in.sa;
     J.oa = in.oa;
@@ -653,7 +764,7 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
     J.order = d_order + w0;
     J.tb_off = d_tboff + w0;
     J.nwork = (int)(w1 - w0);
-    J.nbig = (int)wave_nbig[wv];
+    J.nbig = (int)W.nbig[wv];
     J.tb = tb;
     J.rowbuf = rowbuf;
     J.rowbuf_stride = rb_stride;
@@ -667,27 +778,9 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
     J.err = c->d_err;
     J.spin_limit = c->dp_spin_limit;
     if (int e = rec.check(cudaMemsetAsync(d_counter, 0, 8, L.st), "cudaMemsetAsync")) return e;
-    stage_mark(c, banded ? "dp_banded" : "dp");
+    stage_mark(c, "dp_banded");
     kern<<<grid, kDpThreads, 0, L.st>>>(J);
     stage_mark(c, "traceback");
-    if (ckpt) {
-      unsigned* ctr = d_long_ctr + wv;
-      if (int e = rec.check(cudaMemsetAsync(ctr, 0, 4, L.st), "cudaMemsetAsync")) return e;
-      if (rows == 8)
-        k_tb_ck<8><<<ck_grid, kCkWarps * 32, kCkSmem, L.st>>>(in.sa, in.oa, in.sb, in.ob, J.order, J.tb_off, J.nwork,
-                                                               tb, d_edge, in.path_off, in.paths, in.path_len,
-                                                               c->d_err, in.env, ctr);
-      else
-        k_tb_ck<4><<<ck_grid, kCkWarps * 32, kCkSmem, L.st>>>(in.sa, in.oa, in.sb, in.ob, J.order, J.tb_off, J.nwork,
-                                                               tb, d_edge, in.path_off, in.paths, in.path_len,
-                                                               c->d_err, in.env, ctr);
-      stage_mark(c, "path_compact");
-      k_path_compact<<<grid_for((int64_t)J.nwork * 32, 256), 256, 0, L.st>>>(
-          in.oa, in.ob, J.order, J.nwork, d_accept, in.path_off, in.paths, in.path_len);
-      c->launches += 3;
-      if (int e = rec.check(cudaGetLastError(), "kernel launch")) return e;
-      continue;
-    }
     const bool forked = long_n[wv] > 0;
     if (forked)
       if (int e = rec.check(tb_long_launch(c, L, in, J.order, J.tb_off, tb, d_edge, d_delta, d_half, d_accept, rows,
@@ -696,7 +789,7 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
         return e;
     k_traceback<<<grid_for(J.nwork, 128), 128, 0, L.st>>>(in.oa, in.ob, J.order, J.tb_off, J.nwork, tb, d_edge,
                                                                 d_delta, d_half, d_accept, in.path_off, in.paths,
-                                                                in.path_len, c->d_err, rows, in.env, long_path[wv]);
+                                                                in.path_len, c->d_err, rows, long_path[wv]);
     if (int e = rec.check(tb_long_join(L, forked))) return e;
     stage_mark(c, "path_compact");
     k_path_compact<<<grid_for((int64_t)J.nwork * 32, 256), 256, 0, L.st>>>(
@@ -704,7 +797,7 @@ static int run_dp(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, 
     c->launches += 3;
     if (int e = rec.check(cudaGetLastError(), "kernel launch")) return e;
   }
-  return rec.launch(&c->dp_exec[lane_id]);
+  return rec.launch(&c->dp_exec[1]);
 }
 
 // Ring-scheduled banded problems (gapdp_ring.cuh): rsel[w] is the group
@@ -911,7 +1004,7 @@ int gapdp_batch_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const uin
   std::vector<int64_t> la, lb;
   int rc = check_lengths(nprob, h_oa, h_ob, la, lb);
   if (rc) return rc;
-  if ((rc = stage_reserve(c, (size_t)nprob * 40 + (1 << 20)))) return rc;
+  if ((rc = stage_reserve(c, (size_t)nprob * 48 + (1 << 20)))) return rc;
   DpInputs in{d_sa, d_oa, d_sb, d_ob, d_scores, d_paths, d_path_off, d_path_len, d_env};
   if (!d_paths && (rc = scratch_paths(c, nprob, la, lb, in))) return rc;
   std::vector<uint32_t> ids(nprob);
@@ -919,7 +1012,7 @@ int gapdp_batch_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const uin
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
   if ((rc = check_codes(c, d_sa, h_oa[nprob], d_sb, h_ob[nprob]))) return rc;
   stage_begin_call(c);
-  rc = run_dp(c, in, ids, la, lb, nullptr, nullptr, nullptr, nullptr, nullptr);
+  rc = run_full(c, in, ids, la, lb);
   if (rc) return rc;
   stage_end(c);
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1039,7 +1132,6 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
   // the ring-scheduled bands on the aux stream beside the strip kernel's
   // problems on the main stream (their launches have separate tails)
   const TbLanes ring_lanes{c->aux, c->aux2, c->fork2, c->join2, 68, 69};
-  const TbLanes strip_lanes{c->stream, c->aux3, c->fork3, c->join3, 57, 58};
   const TbLanes band_lanes{c->aux4, c->aux5, c->fork5, c->join5, 54, 55};
   if (!rids.empty()) {
     MVG_CUDA_TRY(cudaEventRecord(c->fork, c->stream));
@@ -1053,12 +1145,12 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
   if (!ids.empty()) {
     MVG_CUDA_TRY(cudaEventRecord(c->fork4, c->stream));
     MVG_CUDA_TRY(cudaStreamWaitEvent(c->aux4, c->fork4, 0));
-    rc = run_dp(c, in, ids, la, lb, d_delta, d_half, &dv, &hv, d_accept, &band_lanes, kDpSlotsLane2);
+    rc = run_band_strips(c, in, ids, la, lb, d_delta, d_half, dv, hv, d_accept, band_lanes);
     if (rc) return rc;
     MVG_CUDA_TRY(cudaEventRecord(c->join4, c->aux4));
   }
   if (!wids.empty()) {
-    rc = run_dp(c, in, wids, la, lb, nullptr, nullptr, nullptr, nullptr, nullptr, &strip_lanes);
+    rc = run_full(c, in, wids, la, lb);
     if (rc) return rc;
   }
   if (!ids.empty()) MVG_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->join4, 0));
@@ -1083,7 +1175,7 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
   }
   tail.reset();
   // rejected bands: the full DP is both the fallback and the exact result
-  rc = run_dp(c, in, fallback, la, lb, nullptr, nullptr, nullptr, nullptr, nullptr);
+  rc = run_full(c, in, fallback, la, lb);
   if (rc) return rc;
   stage_end(c);
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));

@@ -33,8 +33,8 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t aux = nullptr;       // second stream for work that runs beside the main stream's
   cudaEvent_t fork = nullptr, join = nullptr;
-  cudaStream_t aux2 = nullptr, aux3 = nullptr;  // side streams of work already on two streams
-  cudaEvent_t fork2 = nullptr, join2 = nullptr, fork3 = nullptr, join3 = nullptr;
+  cudaStream_t aux2 = nullptr;  // side stream of work already on two streams
+  cudaEvent_t fork2 = nullptr, join2 = nullptr;
   cudaStream_t aux4 = nullptr, aux5 = nullptr;  // a third lane of banded work and its side stream
   cudaEvent_t fork4 = nullptr, join4 = nullptr, fork5 = nullptr, join5 = nullptr;
   uint32_t* d_err = nullptr;     // device error word
@@ -57,7 +57,8 @@ struct Ctx {
   int dp_ckpt = 1;                       // full-DP passes keep checkpoints, the traceback recomputes blocks
   int64_t whole_full_rows = 512;         // banded calls: whole-matrix problems from this many rows go to the full DP
   int ring_max_rows = 32;                // banded calls: tallest ring group height used
-  int dp_coop_strips = 16;               // full-DP problems of at least this many strips use a whole CTA
+  int dp_coop_strips = 16;               // full-DP problems of at least this many strips run on a warp per strip
+  int strip_grid = 0, walk_grid = 0;     // full DP: resident CTAs of the strips and walk kernels (0: not asked yet)
   cudaGraphExec_t dp_exec[2] = {};       // the executable graph of each DP lane, updated per call
   uint64_t graph_launches = 0;
   int mlp_tc = 1;              // MLP forward hidden layers on tcgen05 (else mma.sync)

@@ -28,7 +28,7 @@ struct StripMap {
   __device__ void init(int LA, int LB, const int32_t* delta, const int32_t* half, uint32_t p, int rows_) {
     rows = rows_;
     srows = 32 * rows;
-    band = delta ? make_band(LA, LB, delta[p], half[p], srows) : make_full(LA, LB, srows);
+    band = make_band(LA, LB, delta[p], half[p], srows);
     cur_k = (LA - 1) / srows;
     base = 0;
     for (int k = 0; k < cur_k; ++k)
@@ -97,7 +97,7 @@ __device__ __forceinline__ void tb_wait_copies() {
 // One warp walks problem slot w; Map gives (row, lane, shift) per cell.
 template <class Map>
 __device__ void tb_walk_warp(Map& map, const uint32_t* T, uint32_t* win0, uint32_t* win1, int LA, int LB, char cur,
-                             char* out_end, int64_t* len_out, uint32_t* err, int32_t* env_out) {
+                             char* out_end, int64_t* len_out, uint32_t* err) {
   const int lane = threadIdx.x & 31;
   uint32_t* bc = win0;  // window the walk reads
   uint32_t* bo = win1;  // the other window (prefetch target)
@@ -107,7 +107,6 @@ __device__ void tb_walk_warp(Map& map, const uint32_t* T, uint32_t* win0, uint32
   int pa = LA, pb = LB;
   int64_t n = 0;
   const int64_t limit = (int64_t)LA + LB;
-  int32_t dev_lo = INT32_MAX, dev_hi = INT32_MIN;
   for (;;) {
     if (n >= limit) {
       if (lane == 0) set_error(err, kDevCapacity);
@@ -116,11 +115,6 @@ __device__ void tb_walk_warp(Map& map, const uint32_t* T, uint32_t* win0, uint32
     --out;
     if (lane == 0) *out = cur;
     ++n;
-    if (env_out && pa >= 1) {
-      const int32_t dv = pb - (int32_t)((int64_t)pa * LB / LA);
-      dev_lo = min(dev_lo, dv);
-      dev_hi = max(dev_hi, dv);
-    }
     uint32_t bits = 0;
     if (pa >= 1 && pb >= 1) {
       int64_t X;
@@ -177,13 +171,7 @@ __device__ void tb_walk_warp(Map& map, const uint32_t* T, uint32_t* win0, uint32
     cur = next;
   }
   if (pending) tb_wait_copies();
-  if (lane == 0) {
-    *len_out = n;
-    if (env_out) {
-      env_out[0] = dev_lo;
-      env_out[1] = dev_hi;
-    }
-  }
+  if (lane == 0) *len_out = n;
 }
 
 // The long paths of a wave, one warp each: slots[0..nslots) index the
@@ -196,7 +184,7 @@ __global__ void __launch_bounds__(kTbWarps * 32) k_traceback_win(
     const uint32_t* __restrict__ tb, const uint8_t* __restrict__ end_edge, const int32_t* __restrict__ band_delta,
     const int32_t* __restrict__ band_half, const uint8_t* __restrict__ accept, const uint64_t* __restrict__ path_off,
     char* __restrict__ paths, int64_t* __restrict__ path_len, uint32_t* err, int rows,
-    const uint8_t* __restrict__ rows_of, int32_t* __restrict__ env, unsigned* counter) {
+    const uint8_t* __restrict__ rows_of, unsigned* counter) {
   extern __shared__ __align__(16) uint32_t tb_smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   uint32_t* win0 = tb_smem + (size_t)wib * 2 * kTbRows * 32;
@@ -212,15 +200,14 @@ __global__ void __launch_bounds__(kTbWarps * 32) k_traceback_win(
     const int LA = (int)(oa[p + 1] - oa[p]), LB = (int)(ob[p + 1] - ob[p]);
     const uint32_t* T = tb + tb_off[w] / 4;
     char* out_end = paths + path_off[p] + (LA + LB);
-    int32_t* e = env ? env + 2 * p : nullptr;
     if (rows_of) {
       RingMap m;
       m.init(LA, LB, band_delta, band_half, p, rows_of[w]);
-      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err, e);
+      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err);
     } else {
       StripMap m;
       m.init(LA, LB, band_delta, band_half, p, rows);
-      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err, e);
+      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err);
     }
   }
 }
