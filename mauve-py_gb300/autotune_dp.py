@@ -6,8 +6,9 @@
 Knobs: rows per lane of the full-DP kernel (4 or 8: the tile is a strip of
 128 or 256 rows swept column by column) and of the banded kernel (1, 2, 4
 or 8); warps per problem of the full DP, i.e. the bucket edge between the
-problems a whole CTA (8 warps) pipelines and those one warp solves (at
-least S strips: S in 8, 12, 16, 24, 32, 48); and, for the record, the
+problems pipelined by a warp per strip and those one warp solves (at least
+S strips: S in 2, 3, 4, 6, 8, 12, 16), timed on the full batch and on the
+banded call, whose fallbacks and whole-matrix problems it also cuts; and, for the record, the
 batch launched as one CUDA graph or launch by launch.  The full DP is timed on a
 sample of the gap-DP distribution (lengths log-uniform 10-20,000,
 divergence U(0,30%)); the banded DP on gaps drawn like the recoded-genome
@@ -52,13 +53,6 @@ def run(args):
     best_full = max(res["full"], key=lambda r: res["full"][r]["gcups"])
     ctx.set_dp_rows(best_full, 4)
     res["coop_min_strips"] = {}
-    for strips in (8, 12, 16, 24, 32, 48):
-        ctx.set_dp_coop_strips(strips)
-        timed_full(ctx, full)  # warm
-        secs = min(timed_full(ctx, full)[0] for _ in range(2))
-        res["coop_min_strips"][strips] = {"seconds": secs, "gcups": full.cells / secs / 1e9}
-    best_coop = max(res["coop_min_strips"], key=lambda r: res["coop_min_strips"][r]["gcups"])
-    ctx.set_dp_coop_strips(best_coop)
     res["graph"] = {}
     for on in (True, False):
         ctx.set_dp_graph(on)
@@ -79,6 +73,17 @@ def run(args):
     else:
         d, h = bandnet.heuristic_band(band.la, band.lb)
         src = "network-free band"
+    ctx.set_dp_rows(best_full, 8)
+    for strips in (2, 3, 4, 6, 8, 12, 16):
+        ctx.set_dp_coop_strips(strips)
+        timed_full(ctx, full)  # warm
+        timed_banded(ctx, band, d, h)
+        secs = min(timed_full(ctx, full)[0] for _ in range(2))
+        bsecs = min(timed_banded(ctx, band, d, h)[0] for _ in range(3))
+        res["coop_min_strips"][strips] = {"seconds": secs, "gcups": full.cells / secs / 1e9, "banded_seconds": bsecs}
+    best_coop = min(res["coop_min_strips"], key=lambda r: res["coop_min_strips"][r]["seconds"] *
+                    res["coop_min_strips"][r]["banded_seconds"])
+    ctx.set_dp_coop_strips(best_coop)
     for rows in (1, 2, 4, 8):
         ctx.set_dp_rows(best_full, rows)
         timed_banded(ctx, band, d, h)  # warm

@@ -513,17 +513,17 @@ static uint64_t arena_bound(Ctx* c, int slot, uint64_t total) {
   return arena;
 }
 
-// Workspace slots of one DP lane: row buffers (full DP: units), order,
-// traceback offsets, claim counter, traceback arena.
+// Workspace slots of one DP lane: row buffers (banded only), order, traceback
+// offsets, claim counter, traceback arena.
 struct DpSlots {
   int rowbuf, order, tboff, counter, arena;
 };
-constexpr DpSlots kDpSlots{10, 11, 12, 14, 18};
+constexpr DpSlots kDpSlots{-1, 11, 12, 14, 18};
 constexpr DpSlots kDpSlotsBand{49, 50, 51, 52, 53};
 
 // The full DP of the problems in `ids` on the handle's stream
 // (gapdp_strips.cuh): size-mixed waves that fit the arena, per wave the
-// units of the pipelined problems, the strips kernel and the walk.
+// strips kernel and the walk.
 static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids, const std::vector<int64_t>& la,
                     const std::vector<int64_t>& lb) {
   const int64_t nwork = (int64_t)ids.size();
@@ -531,17 +531,35 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   std::unique_ptr<HostSpan> span(new HostSpan(c, "dp_plan"));
   std::unique_ptr<HostSpan> sub(new HostSpan(c, "dp_sizes"));
   const bool ckpt = c->dp_ckpt != 0;
+  if (!c->strip_grid) {
+    int bps = 0;
+    MVG_CUDA_TRY(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_strip_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_strip_walk, kWalkWarps * 32, kWalkSmem));
+    c->walk_grid = c->sms * std::max(1, bps);
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_strips, kStWarps * 32, 0));
+    c->strip_grid = c->sms * std::max(1, bps);
+  }
+  // A pass of fewer strips than the chip has warp schedulers is bound by the
+  // chain of steps of its longest problem: half-height strips, all of them
+  // pipelined, shorten it (one 310 bp gap: 80 -> 54 us).
+  int64_t strips_all = 0;
+  for (int64_t w = 0; w < nwork && strips_all <= 4 * c->sms; ++w)
+    strips_all += strip_shape((int)la[ids[w]], (int)lb[ids[w]], c->dp_rows, ckpt).n;
+  const bool few = strips_all <= 4 * c->sms;
+  const int max_rows = few ? 4 : c->dp_rows;
+  const int min_piped = few ? 2 : c->dp_coop_strips;
   std::vector<uint64_t> bytes(nwork), cells(nwork);
   std::vector<char> piped(nwork), direct(nwork);
   std::vector<uint32_t> strips(nwork);
   uint64_t total = 0, most = 0, most_least = 0;
   for (int64_t w = 0; w < nwork; ++w) {
     const uint32_t p = ids[w];
-    const StripShape h = strip_shape((int)la[p], (int)lb[p], c->dp_rows, ckpt);
+    const StripShape h = strip_shape((int)la[p], (int)lb[p], max_rows, ckpt);
     bytes[w] = strip_slot_bytes(h);
     cells[w] = (uint64_t)la[p] * (uint64_t)lb[p];
     strips[w] = (uint32_t)h.n;
-    piped[w] = h.n >= c->dp_coop_strips;
+    piped[w] = h.n >= min_piped;
     direct[w] = h.direct;
     total += bytes[w];
     most = std::max(most, bytes[w]);
@@ -555,52 +573,48 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   sub.reset(new HostSpan(c, "dp_waves"));
   const DpWaves W = deal_waves(idx, piped, bytes, arena);
   const size_t nwaves = W.begin.size() - 1;
-  // one upload: the slots' problems, then per wave the pipelined slots' first
-  // units and the walk's slots (checkpointed, then direct)
+  // one upload: the slots' problems, then per wave the pipelined strips in
+  // claim order (pairs) and the walk's slots (checkpointed, then direct)
   std::vector<uint32_t> order(nwork);
   for (int64_t q = 0; q < nwork; ++q) order[q] = ids[W.item[q]];
-  std::vector<size_t> first_at(nwaves), todo_at(nwaves);
-  std::vector<uint32_t> nunits(nwaves);
-  std::vector<int> nck(nwaves);
-  uint32_t max_units = 0;
+  std::vector<size_t> units_at(nwaves), todo_at(nwaves);
+  std::vector<int> nck(nwaves), nunits(nwaves);
   for (size_t wv = 0; wv < nwaves; ++wv) {
-    first_at[wv] = order.size();
-    uint32_t u = 0;
-    for (int64_t q = W.begin[wv]; q < W.begin[wv] + W.nbig[wv]; ++q) {
-      order.push_back(u);
-      u += strips[W.item[q]];
+    order.resize((order.size() + 1) & ~(size_t)1);
+    units_at[wv] = order.size();
+    for (int64_t g = 0; g < W.nbig[wv]; g += kStGroup) {
+      const int64_t end = std::min<int64_t>(g + kStGroup, W.nbig[wv]);
+      std::vector<uint32_t> live;  // slots with a strip k
+      for (int64_t q = g; q < end; ++q) live.push_back((uint32_t)q);
+      for (uint32_t k = 0; !live.empty(); ++k) {
+        size_t keep = 0;
+        for (uint32_t q : live) {
+          order.push_back(q);
+          order.push_back(k);
+          if (strips[W.item[W.begin[wv] + q]] > k + 1) live[keep++] = q;
+        }
+        live.resize(keep);
+      }
     }
-    order.push_back(u);
-    nunits[wv] = u;
+    nunits[wv] = (int)((order.size() - units_at[wv]) / 2);
     todo_at[wv] = order.size();
     for (int pass = 0; pass < 2; ++pass) {
       for (int64_t q = W.begin[wv]; q < W.begin[wv + 1]; ++q)
         if ((direct[W.item[q]] != 0) == (pass == 1)) order.push_back((uint32_t)(q - W.begin[wv]));
       if (pass == 0) nck[wv] = (int)(order.size() - todo_at[wv]);
     }
-    max_units = std::max(max_units, u);
   }
   sub.reset(new HostSpan(c, "dp_copy"));
   Workspace& ws = c->ws;
-  uint32_t* d_units = (uint32_t*)ws.get(c, kDpSlots.rowbuf, (size_t)max_units * 4 + 16);
   uint32_t* d_order = (uint32_t*)ws.get(c, kDpSlots.order, order.size() * 4);
   uint64_t* d_off = (uint64_t*)ws.get(c, kDpSlots.tboff, (size_t)nwork * 8);
   uint8_t* d_edge = (uint8_t*)ws.get(c, 13, la.size() + 16);  // per problem, shared by all lanes
   unsigned* d_counter = (unsigned*)ws.get(c, kDpSlots.counter, nwaves * 16);
   uint8_t* arena_p = (uint8_t*)ws.get(c, kDpSlots.arena, std::max<uint64_t>(W.need, 256));
-  if (!d_units || !d_order || !d_off || !d_edge || !d_counter || !arena_p)
+  if (!d_order || !d_off || !d_edge || !d_counter || !arena_p)
     return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   if (int e = h2d_async(c, d_order, order.data(), order.size() * 4, c->stream)) return e;
   if (int e = h2d_async(c, d_off, W.off.data(), (size_t)nwork * 8, c->stream)) return e;
-  if (!c->strip_grid) {
-    int sms = 0, bps = 0;
-    MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_strip_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
-    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_strip_walk, kWalkWarps * 32, kWalkSmem));
-    c->walk_grid = sms * std::max(1, bps);
-    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_strips, kStWarps * 32, 0));
-    c->strip_grid = sms * std::max(1, bps);
-  }
   sub.reset();
   span.reset();
   GraphRecorder rec(c, c->stream, c->dp_graph != 0 && nwaves > 1);
@@ -615,12 +629,11 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     J.ob = in.ob;
     J.order = d_order + w0;
     J.slot_off = d_off + w0;
-    J.unit_first = d_order + first_at[wv];
-    J.unit_slot = d_units;
+    J.units = reinterpret_cast<const uint2*>(d_order + units_at[wv]);
     J.nwork = (int)n;
     J.npipe = (int)W.nbig[wv];
-    J.nunits = (int)nunits[wv];
-    J.max_rows = c->dp_rows;
+    J.nunits = nunits[wv];
+    J.max_rows = max_rows;
     J.ckpt = ckpt;
     J.arena = arena_p;
     J.scores = in.scores;
@@ -630,7 +643,7 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     J.spin_limit = c->dp_spin_limit;
     stage_mark(c, "dp");
     if (J.npipe) {
-      k_strip_units<<<dim3(std::min(J.npipe, 4096), 8), 256, 0, c->stream>>>(J);
+      k_strip_unwritten<<<dim3(std::min(J.npipe, 4096), 8), 256, 0, c->stream>>>(J);
       c->launches++;
     }
     const int64_t units = J.nunits + (n - J.npipe);

@@ -13,7 +13,11 @@
 // 32 columns, warps spent 40% of their time on the fence and on the two L2
 // round trips before each chunk).  A unit is claimed only after its
 // predecessor was, by a warp that is running, so every wait ends; a bounded
-// spin turns a fault of that reasoning into an error.
+// spin turns a fault of that reasoning into an error.  Problems are claimed in
+// groups of kStGroup, strip by strip: first all their first strips, then all
+// their second ones, and so on.  A strip claimed right after its predecessor
+// would hold a warp for as long as the strips above it take to get going.
+//
 // Before, a CTA's 8 warps shared a problem, and a batch took as long as one
 // CTA needed for its 20 kbp pairs.  Measured on 4,000 pairs of 10-20,000 bp
 // (1.05e11 cells): forward pass 70.3 -> 27.5 ms, traceback 20.8 -> 3.3 ms.
@@ -57,8 +61,9 @@
 namespace mvg {
 
 constexpr int kStWarps = 4;
+constexpr int kStGroup = 1024;             // problems whose strips are claimed level by level
 constexpr unsigned long long kStUnwritten = 0x8080808080808080ull;  // V far below any score
-constexpr int kStBlock = 128;              // steps between stored states
+constexpr int kStBlock = 64;               // steps between stored states
 constexpr int kStDirectCols = 700;         // direct bits up to this LB ...
 constexpr int64_t kStDirectCells = 4 << 20;  // ... and this many cells
 constexpr int kStScaledMax = 400000;       // min(LA, LB) up to which scaled scores fit 32 bits
@@ -107,8 +112,7 @@ struct StripJob {
   const uint64_t* ob;
   const uint32_t* order;       // slot -> problem: pipelined problems first, each part largest first
   const uint64_t* slot_off;    // byte offset of each slot in the arena
-  const uint32_t* unit_first;  // per pipelined slot (one more at the end): its first unit
-  uint32_t* unit_slot;         // per unit: its slot
+  const uint2* units;          // pipelined strips in claim order: slot, strip
   int nwork, npipe, nunits;
   int max_rows;
   bool ckpt;
@@ -120,14 +124,12 @@ struct StripJob {
   long long spin_limit;
 };
 
-// Before a pass: the units of the pipelined slots, and their rows unwritten.
-// Slots along grid.x, shares of a slot's rows along grid.y.
-__global__ void k_strip_units(StripJob J) {
+// Before a pass: the pipelined slots' rows unwritten.  Slots along grid.x,
+// shares of a slot's rows along grid.y.
+__global__ void k_strip_unwritten(StripJob J) {
   for (int w = blockIdx.x; w < J.npipe; w += gridDim.x) {
     const uint32_t p = J.order[w];
     const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
-    if (blockIdx.y == 0)
-      for (uint32_t u = J.unit_first[w] + threadIdx.x; u < J.unit_first[w + 1]; u += blockDim.x) J.unit_slot[u] = (uint32_t)w;
     ulonglong2* rows = reinterpret_cast<ulonglong2*>(J.arena + J.slot_off[w]);
     const int64_t n = (int64_t)(strip_rows_bytes(h) / 16);
     for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.y * blockDim.x)
@@ -343,7 +345,7 @@ __device__ bool strip_run(const StripJob& J, StripSmem& sm, const StripShape& h,
       st[R * 32] = make_int2(dg, D);
     }
     if (s0 >= 32 && s0 + 32 < LB) {
-#pragma unroll 4
+#pragma unroll 16
       for (int q = 0; q < 32; ++q) step(s0 + q, std::false_type{});
     } else {
       const int end = S - s0 < 32 ? S - s0 : 32;
@@ -374,7 +376,10 @@ __device__ bool strip_run(const StripJob& J, StripSmem& sm, const StripShape& h,
   return true;
 }
 
-__global__ void __launch_bounds__(kStWarps * 32) k_gapdp_strips(StripJob J) {
+// 5 CTAs of 4 warps per SM and 16 steps unrolled (96 registers): on the
+// 4,000-pair batch 22.7 ms against 23.8 at 4 steps, 24.5 at 7 CTAs and 4 steps
+// (72 registers) and 32.5 at 9 CTAs; 2 or 8 warps per CTA measure the same.
+__global__ void __launch_bounds__(kStWarps * 32, 5) k_gapdp_strips(StripJob J) {
   __shared__ StripSmem smem[kStWarps];
   const int lane = threadIdx.x & 31;
   StripSmem& sm = smem[threadIdx.x >> 5];
@@ -383,16 +388,14 @@ __global__ void __launch_bounds__(kStWarps * 32) k_gapdp_strips(StripJob J) {
     if (lane == 0) u = (int)atomicAdd(&J.counter[0], 1u);
     u = __shfl_sync(0xffffffffu, u, 0);
     const bool piped = u < J.nunits;
-    const int w = piped ? (int)J.unit_slot[u] : J.npipe + (u - J.nunits);
+    const uint2 unit = piped ? J.units[u] : make_uint2((uint32_t)(J.npipe + (u - J.nunits)), 0u);
+    const int w = (int)unit.x;
     if (w >= J.nwork) break;
     const uint32_t p = J.order[w];
     const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
     uint8_t* slot = J.arena + J.slot_off[w];
-    int k = 0, end = h.n;
-    if (piped) {
-      k = u - (int)J.unit_first[w];
-      end = k + 1;
-    }
+    int k = (int)unit.y;
+    const int end = piped ? k + 1 : h.n;
     bool ok = true;
     for (; k < end && ok; ++k) {
       if (h.R == 8)
@@ -420,7 +423,7 @@ __global__ void __launch_bounds__(kStWarps * 32) k_gapdp_strips(StripJob J) {
 // computed at once, one per warp, and the first warp walks them: a block is a
 // serial chain of 128 steps, and the longest paths, which end the pass, took
 // one such chain per block when one warp did everything.
-constexpr int kWalkWarps = 4;
+constexpr int kWalkWarps = 512 / kStBlock;
 struct WalkJob {
   const uint8_t* sa;
   const uint64_t* oa;
@@ -444,7 +447,7 @@ struct WalkJob {
 struct WalkSmem {
   StripSmem strip[kWalkWarps];
   uint32_t nib[kWalkWarps * kStBlock * 32];  // [step][lane] (uint16_t for R = 4); direct: a block per warp
-  int claim, want_k, want_s;                 // a CTA's problem; the strip and step it walks at
+  int claim, want_k, want_s, want_n;         // a CTA's problem; the strip, the step and the blocks it walks
   int64_t path_n;
 };
 constexpr size_t kWalkSmem = sizeof(WalkSmem);
@@ -614,14 +617,18 @@ __device__ int64_t walk_path(const WalkJob& J, WalkSmem& sm, const StripShape& h
       s1 = pb - 1 + (pa - 1 - row0) / R;
       s0 = s1 & ~(kStBlock - 1);
       if (COOP) {
+        // the steps a path along the problem's slope takes to leave the strip
+        const int64_t steps = (int64_t)SR * LB / LA + 31 + 16;
+        const int nblk = (int)min((int64_t)kWalkWarps, (int64_t)(s1 / kStBlock) - (s1 - steps < 0 ? 0 : (s1 - steps) / kStBlock) + 1);
         if (lane == 0) {
           sm.want_k = k;
           sm.want_s = s1;
+          sm.want_n = nblk;
         }
         __syncthreads();
         walk_block<R>(J, sm.strip[0], sm.nib, kMask, h, slot, p, k, s0, s1);
         __syncthreads();
-        s0 = max(0, s0 - (kWalkWarps - 1) * kStBlock);
+        s0 -= (nblk - 1) * kStBlock;
       } else {
         __syncwarp();
         const int4* src = reinterpret_cast<const int4*>(slot + strip_rows_bytes(h) + ((int64_t)k * h.S + s0) * (16 * R));
@@ -660,7 +667,7 @@ __device__ void walk_help(const WalkJob& J, WalkSmem& sm, const StripShape& h, c
     __syncthreads();
     const int k = sm.want_k, s0 = (sm.want_s & ~(kStBlock - 1)) - w * kStBlock;
     if (k < 0) return;
-    if (s0 >= 0)
+    if (w < sm.want_n)
       walk_block<R>(J, sm.strip[w], sm.nib, kWalkWarps * kStBlock - 1, h, slot, p, k, s0, s0 + kStBlock - 1);
     __syncthreads();
   }

@@ -58,7 +58,7 @@ struct Ctx {
   int64_t whole_full_rows = 512;         // banded calls: whole-matrix problems from this many rows go to the full DP
   int ring_max_rows = 32;                // banded calls: tallest ring group height used
   int dp_coop_strips = 16;               // full-DP problems of at least this many strips run on a warp per strip
-  int strip_grid = 0, walk_grid = 0;     // full DP: resident CTAs of the strips and walk kernels (0: not asked yet)
+  int strip_grid = 0, walk_grid = 0, sms = 0;  // full DP: resident CTAs of the strips and walk kernels, SMs (0: not asked yet)
   cudaGraphExec_t dp_exec[2] = {};       // the executable graph of each DP lane, updated per call
   uint64_t graph_launches = 0;
   int mlp_tc = 1;              // MLP forward hidden layers on tcgen05 (else mma.sync)
