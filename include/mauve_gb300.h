@@ -573,7 +573,7 @@ int mvg_set_dp_rows(mvg_handle h, int full_rows, int band_rows);
 
 /* Banded passes: a proposed band that covers at least `fraction` of its
  * matrix (0 < fraction <= 1, default 0.5) is not banded; the problem runs
- * over the whole matrix in the strip kernel's launch (status 2).  With the
+ * over the whole matrix (status 2).  With the
  * ring schedule on, the share is that of the columns a row keeps
  * (2*half + 2 + ceil(LB/LA)) in LB; otherwise that of the strips' cells. */
 int mvg_set_band_whole_fraction(mvg_handle h, double fraction);
@@ -581,7 +581,8 @@ int mvg_set_band_whole_fraction(mvg_handle h, double fraction);
 /* Banded passes on the ring schedule (on = 1, the default): one warp per
  * problem, groups of 4, 6, 8, 12, 16, 24 or 32 rows per lane chained lane to lane along
  * the band, the smallest group height whose schedule is valid for the band;
- * bands no height fits run in the strip kernel.  on = 0 runs every band in
+ * bands no height fits, and pairs of which both sequences are longer than
+ * 200,000, run in the strip kernel.  on = 0 runs every band in
  * the strip kernel.  Results are identical either way. */
 int mvg_set_band_ring(mvg_handle h, int on);
 
@@ -609,8 +610,8 @@ int mvg_set_ring_max_rows(mvg_handle h, int rows);
 /* mvg_gapdp_banded: problems whose band covers so much of the matrix that
  * they run whole (see mvg_set_band_whole_fraction) go to the full DP when A
  * has at least `rows` rows, else into the strip kernel's launch with a band
- * covering the matrix (default 512, measured on 200,000 gaps drawn like the
- * recoded pair's).  Results do not depend on it. */
+ * covering the matrix (default 0: all of them to the full DP).  Results do
+ * not depend on it. */
 int mvg_set_band_whole_full_rows(mvg_handle h, int64_t rows);
 
 /* Full gap-DP passes checkpointed (on = 1, the default): the forward pass

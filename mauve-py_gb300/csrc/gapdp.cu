@@ -32,8 +32,8 @@
 
 #include "gapdp_kernel.cuh"
 #include "traceback_win.cuh"
-#include "gapdp_ring.cuh"
 #include "gapdp_strips.cuh"
+#include "gapdp_ring.cuh"
 #include "mvg_internal.h"
 
 namespace mvg {
@@ -75,14 +75,6 @@ template __global__ void k_gapdp_t<1>(DpJob);
 template __global__ void k_gapdp_t<2>(DpJob);
 template __global__ void k_gapdp_t<4>(DpJob);
 template __global__ void k_gapdp_t<8>(DpJob);
-template __global__ void k_gapdp_ring<4>(RingJob);
-template __global__ void k_gapdp_ring<6>(RingJob);
-template __global__ void k_gapdp_ring<8>(RingJob);
-template __global__ void k_gapdp_ring<12>(RingJob);
-template __global__ void k_gapdp_ring<16>(RingJob);
-template __global__ void k_gapdp_ring<24>(RingJob);
-template __global__ void k_gapdp_ring<32>(RingJob);
-
 // The group heights the ring schedule offers, smallest first.
 static const int kRingRows[] = {4, 6, 8, 12, 16, 24, 32};
 constexpr int kRingHeights = (int)(sizeof(kRingRows) / sizeof(kRingRows[0]));
@@ -124,18 +116,6 @@ static int host_chunks(int64_t n, F f) {
   for (int t = 0; t < nt; ++t) th.emplace_back(f, n * t / nt, n * (t + 1) / nt, t);
   for (auto& x : th) x.join();
   return nt;
-}
-
-static void (*ring_kernel(int R))(RingJob) {
-  switch (R) {
-    case 4: return k_gapdp_ring<4>;
-    case 6: return k_gapdp_ring<6>;
-    case 8: return k_gapdp_ring<8>;
-    case 12: return k_gapdp_ring<12>;
-    case 16: return k_gapdp_ring<16>;
-    case 24: return k_gapdp_ring<24>;
-    default: return k_gapdp_ring<32>;
-  }
 }
 
 // BitTraceBack of the banded strip kernel's problems from (LA, LB); writes the
@@ -326,37 +306,15 @@ static int tb_long_plan(Ctx* c, const std::vector<uint32_t>& slot_len, std::vect
 // so a pass's launches can be recorded into a CUDA graph.
 static int tb_long_launch(Ctx* c, const TbLanes& L, const DpInputs& in, const uint32_t* d_order,
                           const uint64_t* d_tboff, const uint32_t* tb, const uint8_t* d_edge, const int32_t* d_delta,
-                          const int32_t* d_half, const uint8_t* d_accept, int rows, const uint8_t* d_rows,
-                          const uint32_t* d_slots, int n, int grid, unsigned* d_ctr) {
+                          const int32_t* d_half, const uint8_t* d_accept, int rows, const uint32_t* d_slots, int n, int grid, unsigned* d_ctr) {
   MVG_CUDA_TRY(cudaMemsetAsync(d_ctr, 0, 4, L.st));
   MVG_CUDA_TRY(cudaEventRecord(L.fork, L.st));
   MVG_CUDA_TRY(cudaStreamWaitEvent(L.side, L.fork, 0));
   k_traceback_win<<<grid, kTbWarps * 32, kTbSmem, L.side>>>(in.oa, in.ob, d_order, d_tboff, d_slots, n, tb, d_edge,
                                                             d_delta, d_half, d_accept, in.path_off, in.paths,
-                                                            in.path_len, c->d_err, rows, d_rows, d_ctr);
+                                                            in.path_len, c->d_err, rows, d_ctr);
   MVG_CUDA_TRY(cudaEventRecord(L.join, L.side));
   c->launches++;
-  return 0;
-}
-
-static int tb_long_fork(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vector<uint32_t>& slot_len,
-                        const uint32_t* d_order, const uint64_t* d_tboff, const uint32_t* tb, const uint8_t* d_edge,
-                        const int32_t* d_delta, const int32_t* d_half, const uint8_t* d_accept, int rows,
-                        const uint8_t* d_rows, int* long_path, bool* forked) {
-  *forked = false;
-  std::vector<uint32_t> long_slots;
-  int grid = 0;
-  if (int e = tb_long_plan(c, slot_len, &long_slots, long_path, &grid)) return e;
-  if (long_slots.empty()) return 0;
-  const int n = (int)long_slots.size();
-  uint32_t* d_slots = (uint32_t*)c->ws.get(c, L.slot_list, (size_t)n * 4 + 16);
-  unsigned* d_ctr = (unsigned*)c->ws.get(c, L.slot_ctr, 64);
-  if (!d_slots || !d_ctr) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-  if (int e = h2d_async(c, d_slots, long_slots.data(), (size_t)n * 4, L.st)) return e;
-  if (int e = tb_long_launch(c, L, in, d_order, d_tboff, tb, d_edge, d_delta, d_half, d_accept, rows, d_rows,
-                             d_slots, n, grid, d_ctr))
-    return e;
-  *forked = true;
   return 0;
 }
 
@@ -697,14 +655,16 @@ static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_
   // strip can only start once the previous one has passed the next strip's
   // first column (about one strip height of drift plus the 64-column
   // prefetch), so narrow bands would leave the pipeline nearly serial: they
-  // stay on one warp unless their strips are at least 8 strip heights wide.
+  // stay on one warp unless their strips are at least 4 strip heights wide
+  // (bands of 1,100 columns on 5,000 rows, which no ring height takes: at 8
+  // they were one warp's chain of 28,000 steps, 6.6 ms; at 4 STRIPMS ms).
   std::vector<char> is_big(nwork);
   for (int64_t w = 0; w < nwork; ++w) {
     const uint32_t p = ids[w];
     const Band b = make_band((int)la[p], (int)lb[p], h_delta[p], h_half[p], 32 * rows);
     cells[w] = band_cells(b);
     bytes[w] = (band_tb_words(b, rows) * 4 + 255) & ~255ull;
-    is_big[w] = b.nstrips >= kCoopMinStrips && cells[w] >= (uint64_t)la[p] * 8 * 32 * rows;
+    is_big[w] = b.nstrips >= kCoopMinStrips && cells[w] >= (uint64_t)la[p] * 4 * 32 * rows;
     maxlb = std::max(maxlb, lb[p]);
     total += bytes[w];
     most = std::max(most, bytes[w]);
@@ -797,7 +757,7 @@ static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_
     const bool forked = long_n[wv] > 0;
     if (forked)
       if (int e = rec.check(tb_long_launch(c, L, in, J.order, J.tb_off, tb, d_edge, d_delta, d_half, d_accept, rows,
-                                           nullptr, d_long + long_at[wv], long_n[wv], long_grid[wv],
+                                           d_long + long_at[wv], long_n[wv], long_grid[wv],
                                            d_long_ctr + wv)))
         return e;
     k_traceback<<<grid_for(J.nwork, 128), 128, 0, L.st>>>(in.oa, in.ob, J.order, J.tb_off, J.nwork, tb, d_edge,
@@ -814,9 +774,10 @@ static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_
 }
 
 // Ring-scheduled banded problems (gapdp_ring.cuh): rsel[w] is the group
-// height R of ids[w].  Slots are ordered by R, each class most expensive
-// first, and cut into waves that fit the traceback arena; per wave one
-// k_gapdp_ring<R> launch per class, then traceback and path compaction.
+// height R of ids[w].  Slots are cut into waves that fit the traceback arena;
+// per wave one launch for the heights up to 12 and, beside it on the side
+// stream, one for the taller ones (they need twice the registers), each
+// longest first, then the walks.
 static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vector<uint32_t>& ids,
                     const std::vector<uint8_t>& rsel, const std::vector<int64_t>& la, const std::vector<int64_t>& lb,
                     const std::vector<int32_t>& dv, const std::vector<int32_t>& hv, const int32_t* d_delta,
@@ -824,36 +785,22 @@ static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vec
   const int64_t nwork = (int64_t)ids.size();
   if (nwork == 0) return 0;
   std::unique_ptr<HostSpan> span(new HostSpan(c, "ring_plan"));
-  std::vector<uint64_t> bytes(nwork), cost(nwork);
+  std::vector<uint64_t> bytes(nwork), key(nwork);
+  constexpr uint64_t kMax = (1ull << 40) - 1;
   host_chunks(nwork, [&](int64_t w0, int64_t w1, int) {
     for (int64_t w = w0; w < w1; ++w) {
       const uint32_t p = ids[w];
       const RingBand b = make_ring_band((int)la[p], (int)lb[p], dv[p], hv[p], rsel[w]);
       bytes[w] = (ring_tb_words(b) * 4 + 255) & ~255ull;
-      cost[w] = (uint64_t)b.steps * (uint64_t)(rsel[w] * 18 + 50);
+      // tallest first, each height longest first (ties in input order): the
+      // warps of an SM then run mostly one height's code at a time
+      key[w] = ((uint64_t)(32 - rsel[w]) << 40) | (kMax - std::min((uint64_t)b.steps, kMax));
     }
   });
-  // by group height, each class most expensive first, ties in input order
-  std::vector<uint32_t> idx;
-  {
-    constexpr uint64_t kMax = (1ull << 40) - 1;
-    std::vector<uint64_t> key(nwork);
-    for (int64_t w = 0; w < nwork; ++w) {
-      int q = 0;
-      while (q + 1 < kRingHeights && kRingRows[q] != rsel[w]) ++q;
-      key[w] = ((uint64_t)q << 40) | (kMax - std::min(cost[w], kMax));
-    }
-    idx = radix_order(key);
-  }
-  uint64_t arena = c->tb_arena;
-  {
-    size_t free_b = 0, total_b = 0;
-    HostSpan mem_span(c, "meminfo");
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-      const uint64_t cap = (uint64_t)((c->ws.size[67] + free_b) * 0.6);
-      if (arena > cap) arena = cap;
-    }
-  }
+  const std::vector<uint32_t> idx = radix_order(key);
+  uint64_t total = 0;
+  for (uint64_t b : bytes) total += b;
+  const uint64_t arena = arena_bound(c, 67, total);
   std::vector<uint32_t> order(nwork);
   std::vector<uint8_t> rows_of(nwork);
   std::vector<uint64_t> tboff(nwork);
@@ -873,11 +820,12 @@ static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vec
     arena_need = std::max(arena_need, acc);
   }
   wave_begin.push_back(nwork);
+  const size_t nwaves = wave_begin.size() - 1;
   Workspace& ws = c->ws;
   uint32_t* d_order = (uint32_t*)ws.get(c, 64, (size_t)nwork * 4);
   uint64_t* d_tboff = (uint64_t*)ws.get(c, 65, (size_t)nwork * 8);
   uint8_t* d_edge = (uint8_t*)ws.get(c, 13, la.size() + 16);
-  unsigned* d_counter = (unsigned*)ws.get(c, 66, 64 * kRingHeights);  // one claim counter per height
+  unsigned* d_counter = (unsigned*)ws.get(c, 66, 64);  // one claim counter per class
   uint8_t* d_rows = (uint8_t*)ws.get(c, 60, (size_t)nwork + 16);
   uint32_t* tb = (uint32_t*)ws.get(c, 67, arena_need);
   if (!d_order || !d_tboff || !d_edge || !d_counter || !d_rows || !tb)
@@ -885,76 +833,64 @@ static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vec
   if (int e = h2d_async(c, d_order, order.data(), (size_t)nwork * 4, L.st)) return e;
   if (int e = h2d_async(c, d_tboff, tboff.data(), (size_t)nwork * 8, L.st)) return e;
   if (int e = h2d_async(c, d_rows, rows_of.data(), (size_t)nwork, L.st)) return e;
-  int dev_sms = 0;
-  MVG_CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
+  constexpr size_t kSmem[2] = {sizeof(RingSmem<32>) * (kRingThreads / 32), sizeof(RingSmem<12>) * (kRingThreads / 32)};
+  if (!c->ring_grid[0]) {
+    int sms = 0, bps = 0;
+    MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gapdp_ring<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem[0]));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gapdp_ring<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem[1]));
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_ring<12>, kRingThreads, kSmem[1]));
+    c->ring_grid[1] = sms * std::max(1, bps);
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_ring<32>, kRingThreads, kSmem[0]));
+    c->ring_grid[0] = sms * std::max(1, bps);
+  }
   span.reset();
-  for (size_t wv = 0; wv + 1 < wave_begin.size(); ++wv) {
+  for (size_t wv = 0; wv < nwaves; ++wv) {
     const int64_t w0 = wave_begin[wv], w1 = wave_begin[wv + 1];
-    // heights of 16 rows and more run on the side stream beside the smaller
-    // ones: their few long problems end in a latency-bound tail (one warp,
-    // one problem) that would otherwise hold up the next launch
-    bool side_used = false;
-    for (int64_t a = w0; a < w1 && !side_used; ++a) side_used = rows_of[a] >= 16;
-    if (side_used) {  // the side stream starts with the wave, not after the smaller heights
-      MVG_CUDA_TRY(cudaEventRecord(L.fork, L.st));
-      MVG_CUDA_TRY(cudaStreamWaitEvent(L.side, L.fork, 0));
-    }
-    for (int64_t a = w0; a < w1;) {
-      int64_t e = a;
-      while (e < w1 && rows_of[e] == rows_of[a]) ++e;
-      const int R = rows_of[a];
-      int hq = 0;
-      while (hq + 1 < kRingHeights && kRingRows[hq] != R) ++hq;
-      const bool side = R >= 16;
-      const cudaStream_t ks = side ? L.side : L.st;
-      unsigned* ctr = d_counter + 16 * hq;
-      void (*kern)(RingJob) = ring_kernel(R);
-      int bps = 0;
-      MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kRingThreads, 0));
-      if (bps < 1) bps = 1;
-      const int64_t need_blocks = (e - a + kRingThreads / 32 - 1) / (kRingThreads / 32);
-      const int grid = (int)std::min<int64_t>((int64_t)dev_sms * bps, need_blocks);
-      RingJob J;
-      J.sa = in.sa;
-      J.oa = in.oa;
-      J.sb = in.sb;
-      J.ob = in.ob;
+    int64_t cut = w0;
+    while (cut < w1 && rows_of[cut] > 12) ++cut;
+    RingJob J;
+    J.sa = in.sa;
+    J.oa = in.oa;
+    J.sb = in.sb;
+    J.ob = in.ob;
+    J.tb = tb;
+    J.scores = in.scores;
+    J.end_edge = d_edge;
+    J.band_delta = d_delta;
+    J.band_half = d_half;
+    J.accept = d_accept;
+    J.base_max = g_base_max;
+    J.cells = d_cells;
+    auto slots = [&](int64_t a, int64_t e, unsigned* counter) {
       J.order = d_order + a;
+      J.rows_of = d_rows + a;
       J.tb_off = d_tboff + a;
       J.nwork = (int)(e - a);
-      J.tb = tb;
-      J.scores = in.scores;
-      J.end_edge = d_edge;
-      J.band_delta = d_delta;
-      J.band_half = d_half;
-      J.accept = d_accept;
-      J.base_max = g_base_max;
-      J.counter = ctr;
-      J.cells = d_cells;
-      MVG_CUDA_TRY(cudaMemsetAsync(ctr, 0, 4, ks));
-      kern<<<grid, kRingThreads, 0, ks>>>(J);
+      J.counter = counter;
+      return (int)((e - a + kRingThreads / 32 - 1) / (kRingThreads / 32));
+    };
+    MVG_CUDA_TRY(cudaMemsetAsync(d_counter, 0, 64, L.st));
+    const bool tall = cut > w0, low = cut < w1;
+    if (tall) {
+      MVG_CUDA_TRY(cudaEventRecord(L.fork, L.st));
+      MVG_CUDA_TRY(cudaStreamWaitEvent(L.side, L.fork, 0));
+      const int need = slots(w0, cut, d_counter);
+      k_gapdp_ring<32><<<std::min(need, c->ring_grid[0]), kRingThreads, kSmem[0], L.side>>>(J);
       c->launches++;
-      a = e;
     }
-    if (side_used) {
+    if (low) {
+      const int need = slots(cut, w1, d_counter + 1);
+      k_gapdp_ring<12><<<std::min(need, c->ring_grid[1]), kRingThreads, kSmem[1], L.st>>>(J);
+      c->launches++;
+    }
+    if (tall) {
       MVG_CUDA_TRY(cudaEventRecord(L.join, L.side));
       MVG_CUDA_TRY(cudaStreamWaitEvent(L.st, L.join, 0));
     }
-    const int nw = (int)(w1 - w0);
-    std::vector<uint32_t> slot_len(w1 - w0);
-    for (int64_t q = w0; q < w1; ++q) slot_len[q - w0] = (uint32_t)(la[order[q]] + lb[order[q]]);
-    bool forked = false;
-    int long_path = INT_MAX;
-    int trc = tb_long_fork(c, L, in, slot_len, d_order + w0, d_tboff + w0, tb, d_edge, d_delta, d_half, d_accept, 0,
-                           d_rows + w0, &long_path, &forked);
-    if (trc) return trc;
-    k_traceback_ring<<<grid_for(nw, 128), 128, 0, L.st>>>(
-        in.oa, in.ob, d_order + w0, d_rows + w0, d_tboff + w0, nw, tb, d_edge, d_delta, d_half, d_accept,
-        in.path_off, in.paths, in.path_len, c->d_err, long_path);
-    if ((trc = tb_long_join(L, forked))) return trc;
-    k_path_compact<<<grid_for((int64_t)nw * 32, 256), 256, 0, L.st>>>(in.oa, in.ob, d_order + w0, nw, d_accept,
-                                                                            in.path_off, in.paths, in.path_len);
-    c->launches += 2;
+    const int blocks = slots(w0, w1, nullptr);
+    k_ring_walk<<<blocks, kRingThreads, 0, L.st>>>(J, in.path_off, in.paths, in.path_len, c->d_err);
+    c->launches++;
     MVG_CUDA_TRY(cudaGetLastError());
   }
   return 0;
@@ -1105,7 +1041,7 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
         const double slope = (double)lb[p] / (double)la[p];
         for (int q = 0; q < kRingHeights && !rr; ++q) {
           const int R = kRingRows[q];
-          if (R > c->ring_max_rows) break;  // taller groups go to the strip kernel
+          if (R > c->ring_max_rows || std::min(la[p], lb[p]) > kRingScaledMax) break;  // go to the strip kernel
           const bool many = (la[p] + R - 1) / R > 32;
           if (many && 2.0 * hv[p] + 2.0 + (R - 1) * slope > 32.0 + 32.0 * R * slope + 2.0) continue;
           if (ring_eligible(make_ring_band((int)la[p], (int)lb[p], dv[p], hv[p], R))) rr = R;

@@ -1,5 +1,6 @@
 // The banded NWSmall kernel on a ring schedule (included by gapdp.cu after
-// gapdp_kernel.cuh, whose recurrences and bound it shares).
+// gapdp_strips.cuh, whose recurrence, profile and nibbles it shares; the bound
+// is gapdp_kernel.cuh's).
 //
 // One warp solves one problem.  Rows are cut into groups of R (RingBand,
 // band.h); lane g mod 32 runs group g, and the 32 lanes form a ring: lane t
@@ -13,18 +14,21 @@
 // picks the smallest R whose schedule is valid (ring_eligible), which keeps
 // lanes busy most of the time.
 //
+// Values are scaled by 16 with the strips' tags.  Cells outside the band are
+// kRingNeg; scores added along the band's edge let such a value drift by at
+// most 2,560 a row, and kRingScaledMax keeps it below every real score.
+//
 // Exactness: the kept region is a union of group rectangles.  A banded score
 // is accepted only when it is strictly above an upper bound on every path
 // that leaves the region, as in the strip kernel: each cell a path can leave
 // from (the bottom row of a group left of the next group's first column, the
 // right-most column of a group short of LB, row 0 right of group 0, column 0
 // below the last group that reaches it) contributes its score plus
-// min(sum of A's best-base scores below it, sum of B's right of it).  The
-// prefix sums travel along the ring with each group start.
+// min(sum of A's best-base scores below it, sum of B's right of it).  Prefix
+// sums of both are staged in shared memory with the sequences.
 //
-// Traceback words: each lane writes its R nibbles per step as one stream;
-// nibble s*R + r of lane t is in word ((s*R + r) / 8) * 32 + t, so every
-// store is one coalesced 128-byte row.
+// Traceback words: each lane writes its R nibbles per step as one stream
+// (ring_tb_at), so every store is one coalesced 128-byte row.
 #pragma once
 #include <limits.h>
 
@@ -37,7 +41,8 @@ struct RingJob {
   const uint64_t* oa;
   const uint8_t* sb;
   const uint64_t* ob;
-  const uint32_t* order;   // problem ids of this launch, largest first
+  const uint32_t* order;   // problem ids of this launch, longest first
+  const uint8_t* rows_of;  // group height of each
   const uint64_t* tb_off;  // byte offset of each slot's traceback words
   int nwork;
   uint32_t* tb;
@@ -53,44 +58,34 @@ struct RingJob {
 
 constexpr int kRingThreads = 128;
 constexpr int kRingA = 256;  // rows of A staged per warp (codes of the next groups to start)
+constexpr int32_t kRingNeg = -(1 << 30);
+constexpr int kRingScaledMax = 200000;  // min(LA, LB) up to which scaled scores and drift fit
 
-// One column segment of R rows, as dp_column, with the R traceback nibbles
-// returned in (R + 7) / 8 words (nibble r in word r / 8).
-template <int R>
-__device__ __forceinline__ void ring_column(DpLane<R>& L, int32_t upM, int32_t upD, int32_t dgM, int32_t dgD,
-                                            int32_t dgI, uint32_t bsel, int32_t goB, int32_t goA0,
-                                            uint32_t (&nw)[(R + 7) / 8]) {
-  int32_t cuM = upM, cuD = upD;
-  int32_t cdM = dgM, cdD = dgD, cdI = dgI;
+// Shared memory of one warp of a launch whose tallest groups have RMAX rows.
+template <int RMAX>
+struct RingSmem {
+  int4 prof[RMAX][32];  // [4 * (row / 4) + base][lane]: the scores of four rows of the lane's group
+  int2 colB[128];       // per staged column: 512 times the base's code, best scores of B up to it
+  int32_t prefA[kRingA];  // per staged row: best scores of A up to it
+  __align__(16) uint8_t codeA[kRingA];
+  int32_t score[16];    // [4 * a + b], scaled and tagged
+};
+
+// Inclusive sum over the warp's lanes.
+__device__ __forceinline__ int32_t ring_scan(int32_t v) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int q = 0; q < (R + 7) / 8; ++q) nw[q] = 0;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int32_t goA = r == 0 ? goA0 : kGap;
-    bool dm;
-    const int32_t D = __vibmax_s32(cuM + goA, cuD, &dm);
-    bool mi;
-    const int32_t I = __vibmax_s32(L.lM[r] + goB, L.lI[r], &mi);
-    bool dge, mge;
-    const int32_t DI = __vibmax_s32(cdD, cdI, &dge) + kGap;
-    const int32_t best = __vibmax_s32(cdM, DI, &mge);
-    const int32_t M = best + (int32_t)__byte_perm(L.arow[r], 0u, bsel) - kScoreBias;
-    const uint32_t tm = mge ? TB_MM : (dge ? TB_DM : TB_IM);
-    nw[r >> 3] |= (tm | (dm ? TB_MD : 0u) | (mi ? TB_MI : 0u)) << (4 * (r & 7));
-    cdM = L.lM[r];
-    cdD = L.lD[r];
-    cdI = L.lI[r];
-    cuM = M;
-    cuD = D;
-    L.lM[r] = M;
-    L.lD[r] = D;
-    L.lI[r] = I;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t t = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += t;
   }
+  return v;
 }
 
-template <int R>
-__device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int w) {
-  constexpr int NW = (R + 7) / 8;
+template <int R, int RMAX>
+__device__ void ring_solve(const RingJob& J, RingSmem<RMAX>& sm, int w) {
+  constexpr int NW = (R + 7) / 8, NQ = (R + 3) / 4;
+  constexpr int32_t kOpenD = kOpen2 * 16 + 3, kOpenI = kOpen2 * 16 + 6, kFree = kOpen2 * 16;
   const int lane = threadIdx.x & 31;
   const int src = (lane + 31) & 31;  // the ring's previous lane
   const uint32_t p = J.order[w];
@@ -112,23 +107,24 @@ __device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int
   const int shift = b.delta - b.half;
   int lo_next = f + shift;  // == lo0
   int lo_started = lo0;     // first column of the last group started
-  int filled = lo0 - 1;     // ringB holds the B codes of columns (filled-128, filled]
-  int filledA = 0;          // ringA holds rows [filledA - kRingA, filledA) of A
+  int filled = lo0 - 1;     // colB holds columns (filled - 128, filled]
+  int filledA = 0;          // codeA and prefA hold rows [filledA - kRingA, filledA) of A
+  int32_t sumA = 0, sumB = filled > 0 ? warp_best_sum(B, 0, filled, J.base_max) : 0;
 
   // this lane's group
-  int my_g = -1, my_end = INT_MIN, prev_hi = INT_MIN, next_lo = INT_MIN, end_col = INT_MIN, rexit_col = INT_MIN;
-  int32_t goA0 = kGap, topI = kNeg, pa_end = 0, pb = 0;
-  DpLane<R> L;
+  int my_g = -1, j = INT_MIN / 2, my_end = INT_MIN, j_end = INT_MIN, prev_hi = INT_MIN, next_lo = INT_MIN;
+  int exit_col = INT_MIN, end_col = INT_MIN;  // right-edge exits; the end cell
+  int32_t topV = kRingNeg, left_a = 0;
+  uint32_t codes[(R + 15) / 16];  // the group's rows of A, two bits each
+  int32_t V[R], I[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    L.arow[r] = 0;
-    L.lM[r] = kNeg;
-    L.lD[r] = kNeg;
-    L.lI[r] = kNeg;
+    V[r] = kRingNeg;
+    I[r] = kRingNeg;
   }
-  int32_t pubM = kNeg, pubD = kNeg, pubI = kNeg;     // this lane's bottom row, last column
-  int32_t dgM = kNeg, dgD = kNeg, dgI = kNeg;        // cell above-left of the next column
-  int32_t rawM = kNeg, rawD = kNeg, rawI = kNeg;     // what the previous lane published one step ago
+  int32_t pubV = kRingNeg, pubD = kRingNeg | 1;  // this lane's bottom row, last column
+  int32_t dg = kRingNeg;                         // V above-left of the next column
+  int32_t raw = kRingNeg;                        // V the previous lane published one step ago
   int32_t bound = kNeg, endsc = kNeg;
   int end_lane_edge = 0;
   uint32_t kept = 0;
@@ -136,26 +132,35 @@ __device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int
   uint32_t* tbp = J.tb + J.tb_off[w] / 4 + lane;
 
   for (int s = 0; s < S; ++s) {
-    const int32_t rM = __shfl_sync(0xffffffffu, pubM, src);
+    const int32_t rV = __shfl_sync(0xffffffffu, pubV, src);
     const int32_t rD = __shfl_sync(0xffffffffu, pubD, src);
-    const int32_t rI = __shfl_sync(0xffffffffu, pubI, src);
+    ++j;
     if (gnext < G && s - gnext == lo_next - lo0) {
-      // A codes of the rows about to start, staged 128 rows at a time
-      if (filledA < (gnext + 1) * R) {
-        __syncwarp();
+      const int g = gnext;
+      __syncwarp();
+      if (filledA < (g + 1) * R) {  // rows of A about to start, staged 128 at a time
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const int i = filledA + k * 32 + lane;
-          ringA[i & (kRingA - 1)] = i < LA ? A[i] : 0;
+          const uint32_t code = i < LA ? A[i] & 3u : 0u;
+          const int32_t incl = sumA + ring_scan(i < LA ? best_of(J.base_max, code) : 0);
+          sm.codeA[i & (kRingA - 1)] = (uint8_t)code;
+          sm.prefA[i & (kRingA - 1)] = incl;
+          sumA = __shfl_sync(0xffffffffu, incl, 31);
         }
         __syncwarp();
         filledA += 128;
       }
-      // group gnext starts on lane gnext % 32; its predecessor (previous
-      // lane) passes the prefix sums it carries
-      const int32_t chain_pb = __shfl_sync(0xffffffffu, pb, src);
-      const int32_t chain_pa = __shfl_sync(0xffffffffu, pa_end, src);
-      const int g = gnext;
+      // the group's profile: lane x writes base x / 8 of rows x mod 8, 8 + x mod 8, ...
+#pragma unroll
+      for (int k = 0; k < (R + 7) / 8; ++k) {
+        const int r = 8 * k + (lane & 7), base = lane >> 3;
+        if (R % 8 == 0 || r < R) {
+          const int32_t sc = sm.score[4 * sm.codeA[(g * R + r) & (kRingA - 1)] + base];
+          reinterpret_cast<int32_t*>(&sm.prof[4 * (r >> 2) + base][g & 31])[r & 3] = sc;
+        }
+      }
+      __syncwarp();
       const int lo_prev = lo_started;
       f += qR;
       m += rR;
@@ -167,172 +172,147 @@ __device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int
       if (lane == (g & 31)) {
         const int my_lo = lo_next;
         my_g = g;
+        j = my_lo;
         my_end = my_lo + W - 1;
+        j_end = my_end < LB ? my_end : LB;
         prev_hi = g == 0 ? INT_MIN : lo_prev + W - 1;
         next_lo = g + 1 < G ? lo_after : INT_MIN;
+        exit_col = my_end < LB ? my_end : INT_MIN;
         end_col = g == G - 1 ? LB : INT_MIN;
-        rexit_col = my_end < LB ? my_end : INT_MIN;
-        const int rows_here = LA - g * R < R ? LA - g * R : R;
-        // cells of this group inside the matrix
-        const int c0 = my_lo < 1 ? 1 : my_lo, c1 = my_end < LB ? my_end : LB;
-        if (c1 >= c0) kept += (uint32_t)rows_here * (uint32_t)(c1 - c0 + 1);
-        goA0 = g == 0 ? 0 : kGap;
-        topI = g == 0 ? 0 : kNeg;
-        int32_t pa = g == 0 ? 0 : chain_pa;
-        if constexpr (R % 4 == 0) {  // the group's codes as whole words
-          const uint32_t* ra = reinterpret_cast<const uint32_t*>(ringA);
 #pragma unroll
-          for (int q = 0; q < R / 4; ++q) {
-            const uint32_t c4 = ra[((g * R) >> 2) + q & (kRingA / 4 - 1)];
+        for (int q = 0; q < (R + 15) / 16; ++q) codes[q] = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int r = 4 * q + k;
-              const uint32_t code = (c4 >> (8 * k)) & 3u;
-              L.arow[r] = c_score_rows[code];
-              if (r < rows_here) pa += best_of(J.base_max, code);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const uint32_t code = ringA[(g * R + r) & (kRingA - 1)] & 3u;
-            L.arow[r] = c_score_rows[code];
-            if (r < rows_here) pa += best_of(J.base_max, code);
-          }
+        for (int r = 0; r < R; r += 2) {  // R is even and groups start at even rows
+          const uint32_t two = *reinterpret_cast<const uint16_t*>(&sm.codeA[(g * R + r) & (kRingA - 1)]);
+          codes[r >> 4] |= ((two & 3u) | ((two >> 6) & 12u)) << (2 * (r & 15));
         }
-        pa_end = pa;
-        // prefix of B's best scores before column my_lo: the predecessor
-        // has just added column my_lo
-        pb = (g == 0 || my_lo <= 0) ? 0 : chain_pb - best_of(J.base_max, ringB[my_lo & 127]);
-        const int32_t leftD = my_lo - 1 == 0 ? 0 : kNeg;  // column 0 is (-inf, 0, -inf) below row 0
+        const int rows_here = LA - g * R < R ? LA - g * R : R;
+        left_a = totA - sm.prefA[(g * R + rows_here - 1) & (kRingA - 1)];
+        // cells of this group inside the matrix
+        const int c0 = my_lo < 1 ? 1 : my_lo;
+        if (j_end >= c0) kept += (uint32_t)rows_here * (uint32_t)(j_end - c0 + 1);
+        topV = g == 0 ? kFree : kRingNeg;
+        // column 0 is (-inf, 0, -inf) below row 0
+        const int32_t left = my_lo == 1 ? kFree : kRingNeg;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          L.lM[r] = kNeg;
-          L.lD[r] = leftD;
-          L.lI[r] = kNeg;
+          V[r] = left;
+          I[r] = kRingNeg;
         }
         // cell above-left of the first column: (gR, my_lo - 1)
         const int x = my_lo - 1;
-        if (g == 0) {  // row 0: M(0,0) = 0, I(0,j) = 0 for j >= 1
-          dgM = x == 0 ? 0 : kNeg;
-          dgD = kNeg;
-          dgI = x >= 1 ? 0 : kNeg;
-        } else if (x <= 0) {
-          dgM = kNeg;
-          dgD = x == 0 ? 0 : kNeg;
-          dgI = kNeg;
-        } else if (x >= lo_prev) {  // the predecessor computed it two steps ago
-          dgM = rawM;
-          dgD = rawD;
-          dgI = rawI;
-        } else {
-          dgM = kNeg;
-          dgD = kNeg;
-          dgI = kNeg;
-        }
+        if (g == 0)  // row 0: M(0,0) = 0, I(0,j) = 0 for j >= 1
+          dg = x == 0 ? (LA > 1 ? kGap * 16 : kFree) : x >= 1 ? kFree : kRingNeg;
+        else if (x <= 0)
+          dg = x == 0 ? kFree : kRingNeg;
+        else
+          dg = x >= lo_prev ? raw : kRingNeg;  // the predecessor computed it two steps ago
       }
       lo_started = lo_next;
       lo_next = lo_after;
       ++gnext;
     }
-    // B codes of the running groups' columns: up to s - (gnext - 32) + lo0
+    // B of the running groups' columns: up to s - (gnext - 32) + lo0
     if (filled < s + 32 - gnext + lo0) {
       const int x = filled + 1 + lane;
+      const bool in = x >= 1 && x <= LB;
+      const uint32_t code = in ? B[x - 1] & 3u : 0u;
+      const int32_t incl = sumB + ring_scan(in ? best_of(J.base_max, code) : 0);
       __syncwarp();
-      ringB[x & 127] = (x >= 1 && x <= LB) ? B[x - 1] : 0;
+      sm.colB[x & 127] = make_int2((int)(code * 512u), incl);
       __syncwarp();
+      sumB = __shfl_sync(0xffffffffu, incl, 31);
       filled += 32;
     }
-    const int j = s - my_g + lo0;
     // the cell above: the predecessor's bottom row while inside its range;
     // for group 0 row 0 (I = 0 right of column 0; M(0,0) is set below)
     const bool from_ring = j <= prev_hi;
-    int32_t aM = from_ring ? rM : kNeg;
-    const int32_t aD = from_ring ? rD : kNeg;
-    int32_t aI = from_ring ? rI : topI;
+    int32_t uV = from_ring ? rV : topV;
+    const int32_t uD = from_ring ? rD : kRingNeg | 1;
     uint32_t nw[NW];
 #pragma unroll
     for (int q = 0; q < NW; ++q) nw[q] = 0;
-    if (j <= my_end && j >= 1 && j <= LB && my_g >= 0) {
-      const uint32_t bsel = (uint32_t)ringB[j & 127] | 0x4440u;
-      ring_column<R>(L, aM, aD, dgM, dgD, dgI, bsel, j == 1 ? 0 : kGap, goA0, nw);
-      if (LA == 1 && j == 1) {
-        // NWSmall's last-row special case (MU/nwsmall.cpp:616-624) with
-        // LA == 1: M(1,1) adds the open and close of position 0
-        L.lM[0] = (int32_t)__byte_perm(L.arow[0], 0u, bsel) - kScoreBias + kGap;
-        nw[0] = (nw[0] & ~3u) | TB_DM;
+    pubV = kRingNeg;
+    pubD = kRingNeg | 1;
+    if (j <= j_end && j >= 1) {
+      const int2 col = sm.colB[j & 127];
+      const char* prof = reinterpret_cast<const char*>(&sm.prof[0][lane]) + col.x;
+      int32_t sc[4 * NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int4 v = *reinterpret_cast<const int4*>(prof + q * 2048);
+        sc[4 * q] = v.x;
+        sc[4 * q + 1] = v.y;
+        sc[4 * q + 2] = v.z;
+        sc[4 * q + 3] = v.w;
       }
-      pubM = L.lM[R - 1];
-      pubD = L.lD[R - 1];
-      pubI = L.lI[R - 1];
-      pb += (int32_t)__byte_perm(J.base_max, 0u, bsel) - kScoreBias;  // prefix over B[0..j)
-      if (j < next_lo) {  // bottom-row exit
-        const int32_t best = max(pubM, max(pubD, pubI));
-        bound = max(bound, best + min(totA - pa_end, totB - pb));
-      }
-      if (j == end_col) {  // the end cell (LA, LB)
-        const int er = LA - 1 - my_g * R;
-        int32_t eM = kNeg, eD = kNeg, eI = kNeg;
+      if (j == exit_col) {  // every row's best state may leave the band to the right
+        const int rows_here = LA - my_g * R < R ? LA - my_g * R : R;
+        const int32_t leftB = totB - col.y;
+        int32_t up = dg, D = uD, left = left_a;
 #pragma unroll
         for (int r = 0; r < R; ++r)
-          if (r == er) {
-            eM = L.lM[r];
-            eD = L.lD[r];
-            eI = L.lI[r];
-          }
-        int32_t sc = eM;
-        int e = 'M';
-        if (eD > sc) {
-          sc = eD;
-          e = 'D';
+          if (r < rows_here) left += best_of(J.base_max, codes[r >> 4] >> (2 * (r & 15)));
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int32_t M = up + sc[r];
+          const int32_t best = (__viaddmax_s32(M, kGap * 16, max(D, I[r])) >> 4) - kOpen2;
+          left -= best_of(J.base_max, codes[r >> 4] >> (2 * (r & 15)));
+          if (r < rows_here) bound = __viaddmax_s32(best, min(left, leftB), bound);
+          D = __viaddmax_s32(M, kOpenD, D) & ~4;
+          up = V[r];
         }
-        if (eI > sc) {
-          sc = eI;
-          e = 'I';
-        }
-        endsc = sc;
-        end_lane_edge = e;
       }
-      if (j == rexit_col) {  // right-edge exits of every row
-        // the rows' best scores are the largest bytes of their score rows;
-        // A's prefix before the group is pa_end minus their sum
-        const int rows_here = LA - my_g * R < R ? LA - my_g * R : R;
-        int32_t run = pa_end;
+      if (j == end_col) {  // the end cell (LA, LB)
+        const int last = LA - 1 - my_g * R;
+        int32_t up = dg, D = uD;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const uint32_t h = __vmaxu4(L.arow[r], L.arow[r] >> 16);
-          if (r < rows_here) run -= (int32_t)max(h & 0xffu, (h >> 8) & 0xffu) - kScoreBias;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (r < rows_here) {
-            const uint32_t h = __vmaxu4(L.arow[r], L.arow[r] >> 16);
-            run += (int32_t)max(h & 0xffu, (h >> 8) & 0xffu) - kScoreBias;
-            const int32_t best = max(L.lM[r], max(L.lD[r], L.lI[r]));
-            bound = max(bound, best + min(totA - run, totB - pb));
+          const int32_t M = up + sc[r];
+          if (r == last) {
+            const int32_t eM = (M >> 4) - kGap, eD = (D >> 4) - kOpen2, eI = (I[r] >> 4) - kOpen2;
+            endsc = max(eM, max(eD, eI));
+            end_lane_edge = eM == endsc ? 'M' : eD == endsc ? 'D' : 'I';
           }
+          D = __viaddmax_s32(M, kOpenD, D) & ~4;
+          up = V[r];
         }
+      }
+      int32_t up = dg, D = uD;
+      int32_t lastM = 0, lastDI = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int32_t M = up + sc[r];
+        const int32_t v = __vimax3_s32(M, D, I[r]);
+        if (r == R - 1) {
+          lastM = M;
+          lastDI = max(D, I[r]);
+        }
+        const int32_t nd = __viaddmax_s32(M, kOpenD, D);
+        const int32_t ni = __viaddmax_s32(M, kOpenI, I[r]);
+        up = V[r];
+        nw[r >> 3] = __funnelshift_r(nw[r >> 3], (uint32_t)(v ^ nd ^ ni), 4);
+        V[r] = v & ~3;
+        D = nd & ~4;
+        I[r] = ni & ~8;
+      }
+      if constexpr (R % 8 != 0) nw[NW - 1] >>= 32 - 4 * (R % 8);
+      pubV = V[R - 1];
+      pubD = D;
+      if (j < next_lo) {  // bottom-row exit: max(M, D, I)
+        const int32_t best = (__viaddmax_s32(lastM, kGap * 16, lastDI) >> 4) - kOpen2;
+        bound = max(bound, best + min(left_a, totB - col.y));
       }
     } else if (j <= my_end && j <= 0 && my_g >= 0) {
       // the left boundary column (D = 0 below row 0) or outside the matrix
-      const int32_t d0 = j == 0 ? 0 : kNeg;
+      const int32_t left = j == 0 ? kFree : kRingNeg;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        L.lM[r] = kNeg;
-        L.lD[r] = d0;
-        L.lI[r] = kNeg;
+        V[r] = left;
+        I[r] = kRingNeg;
       }
-      pubM = kNeg;
-      pubD = d0;
-      pubI = kNeg;
-      if (my_g == 0 && j == 0) {  // cell (0, 0)
-        aM = 0;
-        aI = kNeg;
-      }
-    } else {
-      pubM = kNeg;
-      pubD = kNeg;
-      pubI = kNeg;
+      pubV = left;
+      if (my_g == 0 && j == 0) uV = LA > 1 ? kGap * 16 : kFree;  // cell (0, 0)
     }
     if constexpr (R < 8 && 8 % R == 0) {
       constexpr int kPer = 8 / R;
@@ -347,12 +327,8 @@ __device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int
       for (int q = 0; q < NW; ++q) tbp[q * 32] = nw[q];
       tbp += NW * 32;
     }
-    dgM = aM;
-    dgD = aD;
-    dgI = aI;
-    rawM = rM;
-    rawD = rD;
-    rawI = rI;
+    dg = uV;
+    raw = rV;
   }
   // paths along row 0 past group 0, and down column 0 past the last group
   // that reaches it (both score 0 up to the exit)
@@ -384,106 +360,144 @@ __device__ void ring_solve(const RingJob& J, uint8_t* ringB, uint8_t* ringA, int
   }
 }
 
-template <int R>
+// Problems of all heights up to RMAX (above the previous launch's), claimed
+// longest first.  One launch for several heights: a launch per height ends in
+// the chain of steps of its longest problem, and those tails added up.
+template <int RMAX>
 __global__ void __launch_bounds__(kRingThreads) k_gapdp_ring(RingJob J) {
-  __shared__ uint8_t ringB[kRingThreads / 32][128];
-  __shared__ __align__(16) uint8_t ringA[kRingThreads / 32][kRingA];
+  extern __shared__ __align__(16) uint8_t ring_smem[];
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
+  RingSmem<RMAX>& sm = reinterpret_cast<RingSmem<RMAX>*>(ring_smem)[threadIdx.x >> 5];
+  if (lane < 16)
+    sm.score[lane] = ((int32_t)((c_score_rows[lane >> 2] >> (8 * (lane & 3))) & 255u) - kScoreBias) * 16 + 2;
+  __syncwarp();
   for (;;) {
     int w = 0;
     if (lane == 0) w = (int)atomicAdd(J.counter, 1u);
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= J.nwork) break;
-    ring_solve<R>(J, ringB[wib], ringA[wib], w);
+    const int R = J.rows_of[w];
+    if constexpr (RMAX == 12) {
+      if (R == 4)
+        ring_solve<4>(J, sm, w);
+      else if (R == 6)
+        ring_solve<6>(J, sm, w);
+      else if (R == 8)
+        ring_solve<8>(J, sm, w);
+      else
+        ring_solve<12>(J, sm, w);
+    } else {
+      if (R == 16)
+        ring_solve<16>(J, sm, w);
+      else if (R == 24)
+        ring_solve<24>(J, sm, w);
+      else
+        ring_solve<32>(J, sm, w);
+    }
   }
 }
 
-// BitTraceBack (MU/bittraceback.cpp:138-210) over the ring layout, one
-// thread per accepted problem; the path is written reversed at the end of
-// the problem's slot, as k_traceback does.
-__global__ void k_traceback_ring(const uint64_t* __restrict__ oa, const uint64_t* __restrict__ ob,
-                                 const uint32_t* __restrict__ order, const uint8_t* __restrict__ rows_of,
-                                 const uint64_t* __restrict__ tb_off, int nwork, const uint32_t* __restrict__ tb,
-                                 const uint8_t* __restrict__ end_edge, const int32_t* __restrict__ band_delta,
-                                 const int32_t* __restrict__ band_half, const uint8_t* __restrict__ accept,
-                                 const uint64_t* __restrict__ path_off, char* __restrict__ paths,
-                                 int64_t* __restrict__ path_len, uint32_t* err, int long_path) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nwork; w += gridDim.x * blockDim.x) {
-    const uint32_t p = order[w];
-    if (!accept[p]) continue;
-    const int LA = (int)(oa[p + 1] - oa[p]), LB = (int)(ob[p + 1] - ob[p]);
-    if (LA + LB >= long_path) continue;  // k_traceback_win walks it
-    const int R = rows_of[w];
-    const RingBand b = make_ring_band(LA, LB, band_delta[p], band_half[p], R);
-    const uint32_t* T = tb + tb_off[w] / 4;
-    char* out = paths + path_off[p] + (LA + LB);
-    int pa = LA, pb = LB;
-    char cur = (char)end_edge[p];
-    int64_t n = 0;
-    const int64_t limit = (int64_t)LA + LB;
-    int gc = -1, loc = 0, gc8 = -1, loc8 = 0;  // first column of the last group looked up (and 8 cells back)
-    for (;;) {
-      if (n >= limit) {
-        set_error(err, kDevCapacity);
-        break;
+// BitTraceBack (MU/bittraceback.cpp:138-210) over the ring layout, one warp
+// per accepted problem, by runs of equal moves as walk_path finds them (lane l
+// reads the nibble l + 1 moves on; the words a window further along are
+// prefetched to L2).  The path is written from the end of its slot and moved
+// to the head.
+template <int R>
+__device__ void ring_walk(const uint32_t* T, const RingBand& b, char* path, char X, uint32_t* err, int64_t* path_len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t limit = (int64_t)b.LA + b.LB;
+  int pa = b.LA, pb = b.LB;
+  int64_t n = 0;
+  bool fail = false;
+  for (;;) {
+    const int di = X != 'I', dj = X != 'D';
+    const int i = pa - di * (lane + 1), j = pb - dj * (lane + 1);
+    bool valid = false, more = false;
+    uint32_t bits = 0;
+    auto word_of = [&](int ci, int cj, int& sh) -> const uint32_t* {
+      const int g = (ci - 1) / R, r = (ci - 1) % R;
+      const int64_t s = (int64_t)cj + g - b.lo0;
+      if (s < 0 || s >= b.steps) return nullptr;
+      int64_t word;
+      ring_tb_at(R, s, r, word, sh);
+      return T + word * 32 + (g & 31);
+    };
+    if (i >= 1 && j >= 1) {
+      int sh = 0;
+      if (const uint32_t* at = word_of(i, j, sh)) {
+        valid = true;
+        bits = (*at >> sh) & 15u;
+        more = X == 'M' ? (bits & 3u) == 3u : X == 'D' ? !(bits & 4u) : !(bits & 8u);
       }
-      *(--out) = cur;
-      ++n;
-      uint32_t bits = 0;
-      if (pa >= 1 && pb >= 1) {
-        const int g = (pa - 1) / R, r = (pa - 1) - g * R;
-        if (g != gc) {
-          gc = g;
-          loc = ring_lo(b, g);
-        }
-        if (pb < loc || pb > loc + b.W - 1) {  // outside an accepted band cannot happen
-          set_error(err, kDevCapacity);
-          break;
-        }
-        int64_t word;
-        int sh;
-        ring_tb_at(R, (int64_t)(pb + g - b.lo0), r, word, sh);
-        bits = (T[word * 32 + (g & 31)] >> sh) & 15u;
-        // start fetching the word of the cell 8 steps further along the
-        // diagonal (most steps are matches), which may lie in another group
-        // and column: each step's word is otherwise a dependent miss
-        if (pa > 8 && pb > 8) {
-          const int pa8 = pa - 8, pb8 = pb - 8;
-          const int g8 = (pa8 - 1) / R, r8 = (pa8 - 1) - g8 * R;
-          if (g8 != gc8) {
-            gc8 = g8;
-            loc8 = ring_lo(b, g8);
-          }
-          if (pb8 >= loc8 && pb8 <= loc8 + b.W - 1) {
-            int64_t w8;
-            int sh8;
-            ring_tb_at(R, (int64_t)(pb8 + g8 - b.lo0), r8, w8, sh8);
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(T + w8 * 32 + (g8 & 31)));
-          }
-        }
-      }
-      char next;
-      if (cur == 'M') {
-        const uint32_t x = bits & 3u;
-        next = x == TB_MM ? 'M' : (x == TB_DM ? 'D' : 'I');
-        --pa;
-        --pb;
-      } else if (cur == 'D') {
-        next = (bits & TB_MD) ? 'M' : 'D';
-        --pa;
-      } else {
-        next = (bits & TB_MI) ? 'M' : 'I';
-        --pb;
-      }
-      if (pa == 0 && pb == 0) break;
-      if (pa < 0 || pb < 0) {
-        set_error(err, kDevCapacity);
-        break;
-      }
-      cur = next;
+      if (i > 32 && j > 32)
+        if (const uint32_t* at = word_of(i - 32, j - 32, sh)) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
     }
-    path_len[p] = n;
+    const uint32_t stop = ~__ballot_sync(0xffffffffu, more);
+    const int run = stop ? __ffs(stop) - 1 : 32;
+    const int count = run < 32 ? run + 1 : 32;
+    if (n + count > limit) {
+      fail = true;
+      break;
+    }
+    if (lane < count) path[limit - n - 1 - lane] = X;
+    n += count;
+    pa -= di * count;
+    pb -= dj * count;
+    if (run == 32) continue;  // X also at the new cell
+    bits = __shfl_sync(0xffffffffu, bits, run);
+    valid = __shfl_sync(0xffffffffu, valid ? 1 : 0, run) != 0;
+    if (pa < 0 || pb < 0) {
+      fail = true;
+      break;
+    }
+    if (pa == 0 || pb == 0) {  // along row 0 or column 0 to the origin
+      X = pa == 0 ? 'I' : 'D';
+      const int rest = pa + pb;
+      if (n + rest > limit) {
+        fail = true;
+        break;
+      }
+      for (int l = lane; l < rest; l += 32) path[limit - n - 1 - l] = X;
+      n += rest;
+      break;
+    }
+    if (!valid) {  // outside an accepted band cannot happen
+      fail = true;
+      break;
+    }
+    if (X == 'M')
+      X = (bits & 3u) == 3u ? 'M' : (bits & 3u) == 0u ? 'D' : 'I';
+    else
+      X = (bits & (X == 'D' ? 4u : 8u)) ? 'M' : X;
+  }
+  if (fail && lane == 0) set_error(err, kDevCapacity);
+  if (lane == 0) *path_len = n;
+  __syncwarp();
+  walk_compact(path, limit, n, lane, 32, [] { __syncwarp(); });
+}
+
+__global__ void __launch_bounds__(128) k_ring_walk(RingJob J, const uint64_t* __restrict__ path_off,
+                                                   char* __restrict__ paths, int64_t* __restrict__ path_len,
+                                                   uint32_t* err) {
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (w >= J.nwork) return;
+  const uint32_t p = J.order[w];
+  if (!J.accept[p]) return;
+  const int LA = (int)(J.oa[p + 1] - J.oa[p]), LB = (int)(J.ob[p + 1] - J.ob[p]);
+  const int R = J.rows_of[w];
+  const RingBand b = make_ring_band(LA, LB, J.band_delta[p], J.band_half[p], R);
+  const uint32_t* T = J.tb + J.tb_off[w] / 4;
+  char* path = paths + path_off[p];
+  const char X = (char)J.end_edge[p];
+  int64_t* len = path_len + p;
+  switch (R) {
+    case 4: ring_walk<4>(T, b, path, X, err, len); break;
+    case 6: ring_walk<6>(T, b, path, X, err, len); break;
+    case 8: ring_walk<8>(T, b, path, X, err, len); break;
+    case 12: ring_walk<12>(T, b, path, X, err, len); break;
+    case 16: ring_walk<16>(T, b, path, X, err, len); break;
+    case 24: ring_walk<24>(T, b, path, X, err, len); break;
+    default: ring_walk<32>(T, b, path, X, err, len); break;
   }
 }
 

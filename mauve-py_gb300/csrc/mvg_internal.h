@@ -55,10 +55,11 @@ struct Ctx {
   long long dp_spin_limit = 1ll << 26;  // polls before a whole-CTA gap-DP wait gives up (about a second)
   int dp_graph = 1;                      // gap-DP passes launched as one recorded CUDA graph
   int dp_ckpt = 1;                       // full-DP passes keep checkpoints, the traceback recomputes blocks
-  int64_t whole_full_rows = 512;         // banded calls: whole-matrix problems from this many rows go to the full DP
+  int64_t whole_full_rows = 0;           // banded calls: whole-matrix problems from this many rows go to the full DP
   int ring_max_rows = 32;                // banded calls: tallest ring group height used
   int dp_coop_strips = 16;               // full-DP problems of at least this many strips run on a warp per strip
   int strip_grid = 0, walk_grid = 0, sms = 0;  // full DP: resident CTAs of the strips and walk kernels, SMs (0: not asked yet)
+  int ring_grid[2] = {};                 // resident CTAs of the tall and the low ring launch (0: not asked yet)
   cudaGraphExec_t dp_exec[2] = {};       // the executable graph of each DP lane, updated per call
   uint64_t graph_launches = 0;
   int mlp_tc = 1;              // MLP forward hidden layers on tcgen05 (else mma.sync)

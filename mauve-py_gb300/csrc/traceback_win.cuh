@@ -55,29 +55,6 @@ struct StripMap {
   }
 };
 
-// Ring layout: group g = (i-1)/R computes column j at step j + g - lo_0;
-// row r of the group is nibble r of that step in lane g mod 32 (ring_tb_at).
-struct RingMap {
-  RingBand b;
-  int gc, loc;
-  __device__ void init(int LA, int LB, const int32_t* delta, const int32_t* half, uint32_t p, int R) {
-    b = make_ring_band(LA, LB, delta[p], half[p], R);
-    gc = -1;
-    loc = 0;
-  }
-  __device__ bool map(int pa, int pb, int64_t& X, int& t, int& sh) {
-    const int g = (pa - 1) / b.R, r = (pa - 1) - g * b.R;
-    if (g != gc) {
-      gc = g;
-      loc = ring_lo(b, g);
-    }
-    if (pb < loc || pb > loc + b.W - 1) return false;
-    ring_tb_at(b.R, (int64_t)(pb + g - b.lo0), r, X, sh);
-    t = g & 31;
-    return true;
-  }
-};
-
 __device__ __forceinline__ void tb_copy_rows(uint32_t* dst, const uint32_t* T, int64_t row0, int nrows) {
   // nrows rows of 128 bytes as 16-byte cp.async chunks, spread over the lanes
   const int lane = threadIdx.x & 31;
@@ -176,15 +153,13 @@ __device__ void tb_walk_warp(Map& map, const uint32_t* T, uint32_t* win0, uint32
 
 // The long paths of a wave, one warp each: slots[0..nslots) index the
 // wave's arrays and are claimed through a counter, largest first.
-// rows_of == nullptr: strip layout with `rows` rows per lane, else the ring
-// layout with rows_of[w] rows per group.
 __global__ void __launch_bounds__(kTbWarps * 32) k_traceback_win(
     const uint64_t* __restrict__ oa, const uint64_t* __restrict__ ob, const uint32_t* __restrict__ order,
     const uint64_t* __restrict__ tb_off, const uint32_t* __restrict__ slots, int nslots,
     const uint32_t* __restrict__ tb, const uint8_t* __restrict__ end_edge, const int32_t* __restrict__ band_delta,
     const int32_t* __restrict__ band_half, const uint8_t* __restrict__ accept, const uint64_t* __restrict__ path_off,
     char* __restrict__ paths, int64_t* __restrict__ path_len, uint32_t* err, int rows,
-    const uint8_t* __restrict__ rows_of, unsigned* counter) {
+    unsigned* counter) {
   extern __shared__ __align__(16) uint32_t tb_smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   uint32_t* win0 = tb_smem + (size_t)wib * 2 * kTbRows * 32;
@@ -200,15 +175,9 @@ __global__ void __launch_bounds__(kTbWarps * 32) k_traceback_win(
     const int LA = (int)(oa[p + 1] - oa[p]), LB = (int)(ob[p + 1] - ob[p]);
     const uint32_t* T = tb + tb_off[w] / 4;
     char* out_end = paths + path_off[p] + (LA + LB);
-    if (rows_of) {
-      RingMap m;
-      m.init(LA, LB, band_delta, band_half, p, rows_of[w]);
-      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err);
-    } else {
-      StripMap m;
-      m.init(LA, LB, band_delta, band_half, p, rows);
-      tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err);
-    }
+    StripMap m;
+    m.init(LA, LB, band_delta, band_half, p, rows);
+    tb_walk_warp(m, T, win0, win1, LA, LB, (char)end_edge[p], out_end, path_len + p, err);
   }
 }
 
