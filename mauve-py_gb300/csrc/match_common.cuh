@@ -183,80 +183,74 @@ __device__ __forceinline__ uint64_t top64(uint64_t hi, uint64_t lo, int s) {
   return lo << (s - 64);
 }
 
-// One warp's fill: match bits of displacements u0 .. u0 + 32 * nlanes - 1
-// into ring words (u0 / 32 + lane) mod RING, lanes below nlanes (no
-// synchronisation).
-template <int RING>
-__device__ __forceinline__ void ext_fill_ring(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t u0,
-                                              uint64_t pmask, uint32_t* ring, int nlanes = 32) {
-  if ((int)(threadIdx.x & 31) >= nlanes) return;
-  const int lane = threadIdx.x & 31;
+// The even bits of x, packed (bit 2k to bit k).
+__device__ __forceinline__ uint32_t even_bits(uint64_t x) {
+  x &= 0x5555555555555555ull;
+  x = (x | (x >> 1)) & 0x3333333333333333ull;
+  x = (x | (x >> 2)) & 0x0f0f0f0f0f0f0f0full;
+  x = (x | (x >> 4)) & 0x00ff00ff00ff00ffull;
+  x = (x | (x >> 8)) & 0x0000ffff0000ffffull;
+  return (uint32_t)(x | (x >> 16));
+}
+
+// Match bits of displacements U .. U + 31.  Same-strand windows, and with a
+// symmetric pattern opposite-strand ones, are read as one 64-base stretch of
+// each genome: one exclusive or gives the differing bases, and an or of that
+// mask shifted by each selected base of the pattern tells for 32 windows at
+// once whether a selected base differs (about 150 instructions; 32 masked
+// 64-bit comparisons took 400).
+__device__ __forceinline__ uint32_t ext_word(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t U,
+                                             uint64_t pmask) {
   const int L = c.s.L;
   const bool same = (st0 > 0) == (st1 > 0);
   uint32_t word = 0;
-  bool done = false;
-  // Same-strand pairs: the lane's 32 windows lie in one 64-base stretch of
-  // each genome (both move the same way with u), so one XOR of the two
-  // stretches gives all 32 window tests.
-  if (same) {
-    const int64_t U = u0 + lane * 32;
-    const int64_t a0 = ext_start(st0, len, U, L, c.n[0]), a31 = ext_start(st0, len, U + 31, L, c.n[0]);
-    const int64_t b0 = ext_start(st1, len, U, L, c.n[1]), b31 = ext_start(st1, len, U + 31, L, c.n[1]);
-    const bool down = st0 > 0;  // window starts decrease with u
-    const int64_t amin = down ? a31 : a0, bmin = down ? b31 : b0;
-    if (a0 >= 0 && a31 >= 0 && b0 >= 0 && b31 >= 0 && amin + 80 <= c.n[0] && bmin + 80 <= c.n[1]) {
-      uint64_t ah, al, bh, bl;
-      window128(c.g[0], (uint64_t)amin, ah, al);
-      window128(c.g[1], (uint64_t)bmin, bh, bl);
-      const uint64_t dh = ah ^ bh, dl = al ^ bl;
-#pragma unroll 4
-      for (int t = 0; t < 32; ++t) {
-        const int j = down ? 31 - t : t;  // window start amin + j
-        const uint64_t w = j == 0 ? dh : ((dh << (2 * j)) | (dl >> (64 - 2 * j)));
-        word |= (uint32_t)((w & pmask) == 0) << t;
-      }
-      if (U == 0) word &= ~1u;  // displacement 0 is not a step
-      done = true;
-    }
-  } else if (c.s.sym) {
-    // Opposite strands with a symmetric pattern.  Per window the reference's
-    // test is "canonical mers equal and strands opposite", which for a mer
-    // set {f, rc(f)} means: B's forward mer is the reverse complement of A's,
-    // and A's mer is not its own reverse complement (then both canonical
-    // forms are the forward one).  With a symmetric pattern rc(mer(x)) =
+  if (same || c.s.sym) {
+    // Opposite strands with a symmetric pattern: the reference's test is
+    // "canonical mers equal and strands opposite", which for a mer set
+    // {f, rc(f)} means: B's forward mer is the reverse complement of A's, and
+    // A's mer is not its own reverse complement (then both canonical forms
+    // are the forward one).  With a symmetric pattern rc(mer(x)) =
     // mer(rc(x)), so both are masked window comparisons: A's window against
     // the reverse complement of B's (which moves the same way as A's, at a
     // fixed offset), and, where that holds, A's window against its own
     // reverse complement.
-    const int64_t U = u0 + lane * 32;
     const int64_t a0 = ext_start(st0, len, U, L, c.n[0]), a31 = ext_start(st0, len, U + 31, L, c.n[0]);
     const int64_t b0 = ext_start(st1, len, U, L, c.n[1]), b31 = ext_start(st1, len, U + 31, L, c.n[1]);
-    const bool adown = st0 > 0;  // A's window starts decrease with u, B's increase (and vice versa)
-    const int64_t amin = adown ? a31 : a0, bmin = adown ? b0 : b31;
+    const bool adown = st0 > 0, bdown = st1 > 0;  // window starts decrease with u
+    const int64_t amin = adown ? a31 : a0, bmin = bdown ? b31 : b0;
     if (a0 >= 0 && a31 >= 0 && b0 >= 0 && b31 >= 0 && amin + 80 <= c.n[0] && bmin + 80 <= c.n[1]) {
       uint64_t ah, al, bh, bl;
       window128(c.g[0], (uint64_t)amin, ah, al);
       window128(c.g[1], (uint64_t)bmin, bh, bl);
-      // reverse complements of the two 64-base stretches: base k is the
-      // complement of base 63 - k
-      const uint64_t rah = revcomp64(al), ral = revcomp64(ah);
-      const uint64_t rbh = revcomp64(bl), rbl = revcomp64(bh);
-#pragma unroll 4
-      for (int t = 0; t < 32; ++t) {
-        const int ja = adown ? 31 - t : t;  // A's window start amin + ja
-        const int jb = adown ? t : 31 - t;  // B's window start bmin + jb
-        // rc of the window at stretch offset j is the reverse stretch's window at 64 - L - j
-        const uint64_t aw = top64(ah, al, 2 * ja);
-        bool b = ((aw ^ top64(rbh, rbl, 2 * (64 - L - jb))) & pmask) == 0;
-        if (b) b = ((aw ^ top64(rah, ral, 2 * (64 - L - ja))) & pmask) != 0;
-        word |= (uint32_t)b << t;
+      uint64_t oh = bh, ol = bl;  // what A's bases are compared with
+      if (!same) {
+        // reverse complement of B's stretch; A's window at j meets its window at j + 33 - L
+        const uint64_t rh = revcomp64(bl), rl = revcomp64(bh);
+        const int sh = 2 * (33 - L);
+        oh = top64(rh, rl, sh);
+        ol = sh < 64 ? rl << sh : 0ull;
+      }
+      const uint64_t dh = ah ^ oh, dl = al ^ ol;
+      // bit 63 - k: base k differs
+      const uint64_t diff = (uint64_t)even_bits(dh | dh >> 1) << 32 | even_bits(dl | dl >> 1);
+      const uint32_t d1 = (uint32_t)(diff >> 32), d0 = (uint32_t)diff;
+      uint32_t bad = 0;  // bit 31 - j: window j has a selected base that differs
+      for (uint32_t p = __brev((uint32_t)c.s.pattern) >> (32 - L); p; p &= p - 1)
+        bad |= __funnelshift_l(d0, d1, __ffs(p) - 1);
+      word = adown ? ~bad : __brev(~bad);
+      if (!same) {
+        const uint64_t rah = revcomp64(al), ral = revcomp64(ah);
+        for (uint32_t todo = word; todo; todo &= todo - 1) {
+          const int t = __ffs(todo) - 1, ja = adown ? 31 - t : t;
+          if (((top64(ah, al, 2 * ja) ^ top64(rah, ral, 2 * (64 - L - ja))) & pmask) == 0) word &= ~(1u << t);
+        }
       }
       if (U == 0) word &= ~1u;  // displacement 0 is not a step
-      done = true;
+      return word;
     }
   }
-  for (int t = 0; t < 32 && !done; ++t) {
-    const int64_t u = u0 + lane * 32 + t;
+  for (int t = 0; t < 32; ++t) {
+    const int64_t u = U + t;
     const int64_t xa = ext_start(st0, len, u, L, c.n[0]);
     const int64_t xb = ext_start(st1, len, u, L, c.n[1]);
     bool b = false;
@@ -273,13 +267,18 @@ __device__ __forceinline__ void ext_fill_ring(const MatchCtx& c, int64_t st0, in
     }
     word |= (uint32_t)b << t;
   }
-  ring[((u0 >> 5) + lane) & (RING - 1)] = word;
+  return word;
 }
 
-static __device__ void ext_fill(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t u0, uint64_t pmask,
-                                uint32_t* ring) {
-  ext_fill_ring<kExtRing>(c, st0, st1, len, u0, pmask, ring);
-  __syncwarp();
+// One warp's fill: match bits of displacements u0 .. u0 + 32 * nlanes - 1
+// into ring words (u0 / 32 + lane) mod RING, lanes below nlanes (no
+// synchronisation).
+template <int RING>
+__device__ __forceinline__ void ext_fill_ring(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t u0,
+                                              uint64_t pmask, uint32_t* ring, int nlanes = 32) {
+  const int lane = threadIdx.x & 31;
+  if (lane >= nlanes) return;
+  ring[((u0 >> 5) + lane) & (RING - 1)] = ext_word(c, st0, st1, len, u0 + lane * 32, pmask);
 }
 
 // Where a side's walk stops.  On one side of the entry the walk starts at
@@ -347,87 +346,6 @@ static __device__ void warp_extend(const MatchCtx& c, Mhe& m, ExtRing& R) {
   m.len = elen + moved[0] + moved[1];
   m.s0 = e0 > 0 ? e0 - moved[0] : e0 + moved[1];
   m.s1 = e1 > 0 ? e1 - moved[0] : e1 + moved[1];
-}
-
-// ExtendMatch by a whole CTA (every thread calls it with the same entry and
-// gets the same result): per side the match bits are filled in chunks of
-// 1024, 2048, 4096, then 8192 displacements (one warp per 1024), and after
-// each chunk every thread checks one word of it for the walk's stopping
-// point (stop_in_word); the first one wins.  The ring keeps the last 16,384
-// displacements, so the previous chunk's last word is still there.
-constexpr int kCtaRing = 512;  // words per side
-struct CtaExtRing {
-  uint32_t w[2][kCtaRing];
-  uint32_t red[32];
-};
-
-static __device__ void cta_extend(const MatchCtx& c, Mhe& m, CtaExtRing& R) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;  // at most 8: a chunk fits half the ring
-  const int L = c.s.L;
-  const uint64_t pmask = pattern_mask64(c.s);
-  const int64_t e0 = m.s0, e1 = m.s1, elen = m.len;
-  int64_t moved[2] = {0, 0};
-#pragma unroll 1
-  for (int sd = 0; sd < 2; ++sd) {
-    const int64_t sg = sd == 0 ? 1 : -1;
-    const int64_t s0 = sg * e0, s1 = sg * e1;
-    uint32_t* ring = R.w[sd];
-    // room: the nearer genome end; every bit beyond it is clear, so the stop
-    // is found once the fills pass it by L (the bound below is never reached)
-    const int64_t r0 = s0 > 0 ? s0 - 1 : (s0 < 0 ? c.n[0] - elen + s0 + 1 : -1);
-    const int64_t r1 = s1 > 0 ? s1 - 1 : (s1 < 0 ? c.n[1] - elen + s1 + 1 : -1);
-    const int64_t room = r0 < r1 ? r0 : r1;
-    int64_t filled = 0, checked = 0;  // displacements filled, words checked
-    for (int k = 0;; ++k) {
-      // 256 displacements first (most matches stop there), then 1, 2, 4 and 8 warps' worth
-      const int nw = k == 0 ? 1 : (k < 4 ? min(nwarps, 1 << (k - 1)) : nwarps);
-      const int nlanes = k == 0 ? 8 : 32;
-      __syncthreads();  // every thread is past its reads of the words refilled now
-      if (wid < nw)
-        ext_fill_ring<kCtaRing>(c, s0, s1, elen, filled + (int64_t)wid * kExtChunk, pmask, ring, nlanes);
-      __syncthreads();
-      filled += (int64_t)nw * 32 * nlanes;
-      const int64_t last = filled / 32 - 1;  // words below it have their successor filled
-      uint32_t q = 0xffffffffu;
-      const int64_t i = checked + threadIdx.x;
-      if (i < last) {
-        const uint32_t hit = stop_in_word(ring[i & (kCtaRing - 1)], ring[(i + 1) & (kCtaRing - 1)], i == 0, L);
-        if (hit) q = (uint32_t)(32 * i) + (uint32_t)(__ffs(hit) - 1);
-      }
-      q = __reduce_min_sync(0xffffffffu, q);
-      if (lane == 0) R.red[wid] = q;
-      __syncthreads();
-      q = 0xffffffffu;
-      for (int w = 0; w < nwarps; ++w) q = min(q, R.red[w]);
-      checked = last;
-      if (q != 0xffffffffu || filled > room + 2 * kExtChunk * 8 + 64) {
-        moved[sd] = q != 0xffffffffu ? q : (room > 0 ? room : 0);
-        break;
-      }
-    }
-    __syncthreads();  // the ring and the reduction words are reused
-  }
-  m.len = elen + moved[0] + moved[1];
-  m.s0 = e0 > 0 ? e0 - moved[0] : e0 + moved[1];
-  m.s1 = e1 > 0 ? e1 - moved[0] : e1 + moved[1];
-}
-
-// lower_bound_mhe over the sorted order given by a map (logical position ->
-// slot in E): the same probes on the same logical array.
-__device__ __forceinline__ int64_t lower_bound_mapped(const Mhe* __restrict__ E, const uint32_t* __restrict__ M,
-                                                      int64_t n, const Mhe& x, int L) {
-  int64_t first = 0, len = n;
-  while (len > 0) {
-    int64_t half = len >> 1, mid = first + half;
-    if (mhe_less(E[M[mid]], x, L)) {
-      first = mid + 1;
-      len = len - half - 1;
-    } else {
-      len = half;
-    }
-  }
-  return first;
 }
 
 }  // namespace mvg
