@@ -122,9 +122,9 @@ int pairwise_matches_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t*
   const uint64_t ca = na >= (uint64_t)s.L ? na - s.L + 1 : 0;
   const uint64_t cb = nb >= (uint64_t)s.L ? nb - s.L + 1 : 0;
   if (ca == 0 || cb == 0) return check_device_error(c);
-  // 32-bit keys up to 2^25 of them: the bucketed join; otherwise one sort
-  // of both genomes' keys and a join over its runs
-  const bool bucketed = 2 * s.w + 2 <= 32 && ca + cb <= kPairBucketMaxKeys;
+  // weights up to 22 and up to 2^25 seeds: the bucketed join; otherwise one
+  // sort of both genomes' keys and a join over its runs
+  const bool bucketed = s.w <= kPairBucketMaxWeight && ca + cb <= kPairBucketMaxKeys;
   const int64_t ntiles = div_up((int64_t)na, kSegTile);
   uint32_t* tab = (uint32_t*)ws.get(c, 38, na * 4);
   uint32_t* masks = (uint32_t*)ws.get(c, 39, (size_t)ntiles * (kSegTile / 32) * 2 * 4);
@@ -138,10 +138,7 @@ int pairwise_matches_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t*
   MVG_CUDA_TRY(cudaMemsetAsync(scal, 0, 64, c->stream));
   stage_mark(c, "sml_sort");
   if (bucketed) {
-    PairStage ps;
-    if ((rc = pair_buckets(c, ga, ca, gb, cb, s, &ps))) return rc;
-    stage_mark(c, "unique_join");
-    k_tab_stage<<<(unsigned)ps.nbuckets, 256, 0, c->stream>>>(ps.stage, ps.bstart, ps.pcount, tab);
+    if ((rc = pair_buckets(c, ga, ca, gb, cb, s, tab))) return rc;
   } else {
     SmlKeys sk;
     if ((rc = pair_sort(c, ga, ca, gb, cb, s, &sk))) return rc;
@@ -151,10 +148,11 @@ int pairwise_matches_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t*
       k_tab_runs<uint64_t><<<div_up(nk, 256), 256, 0, c->stream>>>((const uint64_t*)sk.keys, sk.pos, nk, tab);
     else
       k_tab_runs<uint32_t><<<div_up(nk, 256), 256, 0, c->stream>>>((const uint32_t*)sk.keys, sk.pos, nk, tab);
+    c->launches++;
   }
   stage_mark(c, "segments");
   k_seg_bits<<<(unsigned)ntiles, 256, 0, c->stream>>>(tab, (int64_t)na, s.L, headw, tailw, tcount, ntiles, scal + 1);
-  c->launches += 2;
+  c->launches++;
   scan_counts(tcount, 2 * ntiles, toff, tscr, scal, c->stream, &c->launches);
   MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal, 8, cudaMemcpyDeviceToHost, c->stream));
   if ((rc = check_device_error(c))) return rc;

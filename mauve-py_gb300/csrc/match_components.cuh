@@ -74,17 +74,8 @@ __device__ __forceinline__ Mhe diag_entry(uint64_t d, uint32_t lo, uint32_t hi, 
 
 // ------------------------------------------------------------ pair table
 
-// From the seed join's buckets (pair_buckets.cu).
-__global__ void k_tab_stage(const uint2* __restrict__ stage, const uint32_t* __restrict__ bstart,
-                            const uint32_t* __restrict__ pcount, uint32_t* __restrict__ tab) {
-  const uint32_t np = pcount[blockIdx.x], s0 = bstart[blockIdx.x];
-  for (uint32_t q = threadIdx.x; q < np; q += blockDim.x) {
-    const uint2 e = stage[s0 + q];
-    tab[e.x] = e.y;
-  }
-}
-
-// From the joint sort: runs of exactly one key per genome.
+// From the joint sort (the bucketed join of pair_buckets.cu writes the table
+// itself): runs of exactly one key per genome.
 template <typename K>
 __global__ void k_tab_runs(const K* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n,
                            uint32_t* __restrict__ tab) {

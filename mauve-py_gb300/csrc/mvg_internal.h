@@ -136,23 +136,19 @@ int pack_sequence(Ctx* c, const uint8_t* d_seq, uint64_t n, uint32_t* d_packed);
 int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
              uint64_t* d_mer_out, SmlKeys* keep, int slot_base);
 // Both genomes' keys ((seed bits, strand, genome) with A = 0) sorted in one array.
-// The bucketed seed join (pair_buckets.cu) for 32-bit keys and at most
-// kPairBucketMaxKeys keys: pairs staged per bucket in mer order.
+// The bucketed seed join (pair_buckets.cu) for at most kPairBucketMaxKeys
+// keys: tab[position in A] = position in B | reverse << 31 for every seed
+// unique in both genomes (tab holds ~0 elsewhere).
 constexpr uint64_t kPairBucketMaxKeys = 1ull << 25;
+constexpr int kPairRestBits = 30;                      // mer bits below the bucket's
+constexpr int kPairBucketMaxWeight = (14 + kPairRestBits) / 2;  // with 2^14 buckets
 struct PairBucketGeom {
-  int bbits, nbuckets, npass, dbits, lbits, spass, sbits;
+  int bbits, nbuckets, npass, dbits, lbits;
   int64_t tile, ntiles, nchunks;
 };
 PairBucketGeom pair_bucket_geom(uint64_t n, int w);
-struct PairStage {
-  const uint2* stage = nullptr;   // bucket b's pairs at stage[bstart[b] ..]: (pos A, pos B | reverse << 31)
-  const uint32_t* bstart = nullptr;
-  uint32_t* pcount = nullptr;     // pairs per bucket
-  uint32_t* pbase = nullptr;      // room for their exclusive scan
-  int nbuckets = 0;
-};
 int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
-                 PairStage* out);
+                 uint32_t* tab);
 // Exclusive scan of n <= 16384 counts in one launch; *total gets the sum.
 void pair_scan_small(const uint32_t* in, int n, uint32_t* out, uint32_t* total, cudaStream_t st);
 int pair_sort(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,

@@ -1,31 +1,36 @@
 // The pairwise matcher's seed join by buckets: the seeds unique in each of
-// the two genomes, in mer order, without sorting the whole key array.
+// the two genomes, without sorting the keys.
 //
 // The SearchRange merge of the two sorted mer lists (LM/MatchFinder.cpp:
 // 172-340, driven by LM/PairwiseMatchFinder.cpp:37-71) hashes every mer that
-// occurs exactly once in each genome, in increasing mer order.  Only that
-// order and the run structure (how often a mer occurs in each genome) matter,
-// so the keys need not be sorted as one array:
+// occurs exactly once in each genome.  The matcher needs the set of these
+// pairs, by their position in A (match_components.cuh), not their mer order,
+// so mers are dealt to buckets by a bijective mix of their bits: buckets come
+// out even whatever the genomes' composition (by the mer's own top bits the
+// buckets of a genome at GC 0.38 differ ten times in size).
 //
-//   k_pb_keys     keys of both genomes (mer << 2 | strand << 1 | genome,
-//                 2w + 2 <= 32 bits) and positions, plus every tile's bucket
-//                 counts (bucket = the mer's top BB bits), one row per tile
+//   k_pb_keys     each position's bucket (the mixed mer's top BB bits),
+//                 counted: one row of counts per tile
 //   k_pb_csum     per-chunk sums of the count rows
 //   k_pb_scan     every bucket's start and size; chunk starts
 //   k_pb_offsets  count rows -> each tile's first slot in each bucket
-//   k_pb_scatter  (key, position) pairs into their buckets; the order
-//                 inside a bucket is arbitrary (shared-memory atomics)
-//   k_pb_local    one block per bucket: a stable LSD sort by the rest of the
-//                 mer and the genome bit (in shared memory, or through global
-//                 memory in chunks when the bucket is larger), then the runs:
-//                 a mer with one position in each genome is a pair, staged
-//                 as (position in A, position in B | reverse << 31) at the
-//                 bucket's start, and counted
+//   k_pb_scatter  the mers computed again (a few instructions a base; storing
+//                 and reading them back moved 16 bytes a base) and (rest of
+//                 the mixed mer, strand, genome; position) put into their
+//                 buckets; the order inside a bucket is arbitrary
+//                 (shared-memory atomics)
+//   k_pb_local    one block per bucket: grouped by the next 9 bits in shared
+//                 memory, then a thread per key looks for its mer in its
+//                 group; larger buckets are sorted in chunks through global
+//                 memory and their runs taken.  A mer with one position in
+//                 each genome goes to the table: position in B, the strand
+//                 relation in bit 31, at the position in A.
 //
-// Buckets are in mer order and each is sorted by mer, so the staged pairs
-// taken bucket by bucket are in the order the merge hashes them.  Positions
-// are below 2^25 on this path (the host takes the full sort beyond that), so
-// bit 31 of the B position is free for the strand relation.
+// With in-bucket keys of 32 bits this takes seeds of weight up to 22 (24 M
+// seeds of weight 17 in 1.06 ms, against 1.38 ms of a 64-bit radix sort
+// and its runs; 9.2 M of weight 15 in 0.27 ms against 0.39 ms with stored
+// keys, buckets in mer order and pairs staged in that order).  Positions are
+// below 2^25 on this path (the host takes the full sort beyond that).
 #include <algorithm>
 
 #include "mvg_internal.h"
@@ -40,9 +45,8 @@ constexpr int kLocWarps = kLocThreads / 32;
 constexpr int kCap = 3072;      // bucket elements sorted in shared memory
 constexpr int kLocItems = kCap / kLocThreads;
 constexpr int kMaxDigit = 64;   // chunked in-bucket passes: digits of at most 6 bits
-constexpr int kSmemDigit = 512; // shared-memory in-bucket passes: digits of at most 9 bits
-constexpr int kGroups = 512;    // groups of a bucket split by its top 9 in-bucket bits
-constexpr int kGroupMax = 256;  // larger groups: radix passes for the bucket instead
+constexpr int kGroups = 512;    // groups of a bucket: its top 9 in-bucket bits
+constexpr int kGroupMax = 256;  // larger groups: the bucket is sorted instead
 constexpr int kChunkTiles = 32;
 }  // namespace pb
 
@@ -50,81 +54,99 @@ PairBucketGeom pair_bucket_geom(uint64_t n, int w) {
   PairBucketGeom g;
   int bb = 4;
   while (bb < 14 && ((uint64_t)2048 << bb) < n) ++bb;  // about 2048 keys per bucket at most
+  if (bb < 2 * w - kPairRestBits) bb = 2 * w - kPairRestBits;
   if (bb > 2 * w) bb = 2 * w;
   g.bbits = bb;
   g.nbuckets = 1 << bb;
   g.tile = std::max<int64_t>(16384, 4ll * g.nbuckets);
   g.ntiles = (int64_t)((n + g.tile - 1) / g.tile);
   g.nchunks = (g.ntiles + pb::kChunkTiles - 1) / pb::kChunkTiles;
-  // in-bucket key: the mer bits below the bucket, then the genome bit; an
-  // odd number of passes leaves a chunked sort's result in the scratch copy
+  // in-bucket key: the rest of the mixed mer, then the genome bit; an odd
+  // number of passes leaves a sort's result in the scratch copy
   const int lbits = 2 * w - bb + 1;
   int np = (lbits + 5) / 6;
   if ((np & 1) == 0) ++np;
   g.npass = np;
   g.dbits = (lbits + np - 1) / np;
   g.lbits = lbits;
-  g.spass = (lbits + 8) / 9;
-  g.sbits = (lbits + g.spass - 1) / g.spass;
   return g;
 }
 
 // ------------------------------------------------------------------ keys
 
-__global__ void __launch_bounds__(pb::kKeyThreads) k_pb_keys(const uint32_t* __restrict__ ga, uint64_t ca,
-                                                             const uint32_t* __restrict__ gb, uint64_t cb, SeedDesc s,
-                                                             uint32_t* __restrict__ keys, uint32_t* __restrict__ pos,
-                                                             uint32_t* __restrict__ counts, int bbits, int64_t tile) {
-  extern __shared__ uint32_t h[];  // nbuckets counts
-  __shared__ uint32_t lut[8][256];
-  const int tid = threadIdx.x;
-  const int nbk = 1 << bbits;
-  seed_lut_build32(s, lut);
-  for (int d = tid; d < nbk; d += pb::kKeyThreads) h[d] = 0;
-  __syncthreads();
+// A bijection of 2w-bit mers whose top bits depend on all of the mer's.
+template <typename K>
+__device__ __forceinline__ K mix_mer(K m, int w) {
+  m ^= m >> w;
+  m *= (K)0x9E3779B97F4A7C15ull;
+  return m & ((((K)1 << (2 * w - 1)) << 1) - 1);
+}
+
+// Calls f(global index, mixed mer, strand, in B, position) for every position
+// of this block's tile.  K = uint32_t: w <= 15, four positions from one
+// 32-base window where they fit.
+template <typename K, class F>
+__device__ __forceinline__ void pb_tile(const uint32_t* __restrict__ ga, uint64_t ca, const uint32_t* __restrict__ gb,
+                                        uint64_t cb, const SeedDesc& s, const K (*lut)[256], int64_t tile, F f) {
   const int nb = seed_bytes(s);
-  const bool quad = nb <= 7;  // four positions from one 32-base window
-  const int sh = 32 - 2 * s.w, bsh = 2 * s.w + 2 - bbits;  // keys have 2w + 2 bits
   const uint64_t n = ca + cb;
   const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)tile;
-  for (int64_t o = 4 * tid; o < tile; o += 4 * pb::kKeyThreads) {
-    const uint64_t p0 = base + (uint64_t)o;
-    if (p0 >= n) break;
-    if (quad && p0 + 4 <= n && (p0 + 4 <= ca || p0 >= ca)) {
-      const bool in_b = p0 >= ca;
-      const uint64_t q0 = in_b ? p0 - ca : p0;
-      const uint64_t win = window64(in_b ? gb : ga, q0);
-      uint32_t kk[4];
+  if constexpr (sizeof(K) == 4) {
+    const bool quad = nb <= 7;
+    const int sh = 32 - 2 * s.w;
+    for (int64_t o = 4 * threadIdx.x; o < tile; o += 4 * pb::kKeyThreads) {
+      const uint64_t p0 = base + (uint64_t)o;
+      if (p0 >= n) break;
+      const bool whole = quad && p0 + 4 <= n && (p0 + 4 <= ca || p0 >= ca);
+      const uint64_t win = whole ? window64(p0 >= ca ? gb : ga, p0 >= ca ? p0 - ca : p0) : 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t f = gather_mer32(win, u, lut, nb);
-        const uint32_t r = revcomp_mer32(f, s.w);
-        const uint32_t m = f < r ? f : r;
-        kk[u] = ((((m >> sh) << 1) | (m & 1u)) << 1) | (in_b ? 1u : 0u);
-        atomicAdd(&h[kk[u] >> bsh], 1u);
-      }
-      *reinterpret_cast<uint4*>(keys + p0) = make_uint4(kk[0], kk[1], kk[2], kk[3]);
-      *reinterpret_cast<uint4*>(pos + p0) =
-          make_uint4((uint32_t)q0, (uint32_t)q0 + 1, (uint32_t)q0 + 2, (uint32_t)q0 + 3);
-    } else {
       for (int u = 0; u < 4; ++u) {
         const uint64_t p = p0 + u;
         if (p >= n) break;
         const bool in_b = p >= ca;
         const uint64_t q = in_b ? p - ca : p;
-        const uint32_t f = gather_mer32(window64(in_b ? gb : ga, q), 0, lut, nb);
-        const uint32_t r = revcomp_mer32(f, s.w);
-        const uint32_t m = f < r ? f : r;
-        const uint32_t key = ((((m >> sh) << 1) | (m & 1u)) << 1) | (in_b ? 1u : 0u);
-        keys[p] = key;
-        pos[p] = (uint32_t)q;
-        atomicAdd(&h[key >> bsh], 1u);
+        const uint32_t fw = whole ? gather_mer32(win, u, lut, nb) : gather_mer32(window64(in_b ? gb : ga, q), 0, lut, nb);
+        const uint32_t r = revcomp_mer32(fw, s.w);
+        const uint32_t m = fw < r ? fw : r;
+        f(p, mix_mer<uint32_t>(m >> sh, s.w), m & 1u, in_b, (uint32_t)q);
       }
     }
+  } else {
+    const int sh = 64 - 2 * s.w;
+    for (int64_t o = threadIdx.x; o < tile; o += pb::kKeyThreads) {
+      const uint64_t p = base + (uint64_t)o;
+      if (p >= n) break;
+      const bool in_b = p >= ca;
+      const uint64_t q = in_b ? p - ca : p;
+      const uint64_t m = canonical_mer_lut(in_b ? gb : ga, q, lut, nb, s.w);
+      f(p, mix_mer<uint64_t>(m >> sh, s.w), (uint32_t)m & 1u, in_b, (uint32_t)q);
+    }
   }
+}
+
+template <typename K>
+__device__ __forceinline__ void pb_lut(const SeedDesc& s, K (*lut)[256]) {
+  if constexpr (sizeof(K) == 4)
+    seed_lut_build32(s, lut);
+  else
+    seed_lut_build(s, lut);
+}
+
+template <typename K>
+__global__ void __launch_bounds__(pb::kKeyThreads) k_pb_keys(const uint32_t* __restrict__ ga, uint64_t ca,
+                                                             const uint32_t* __restrict__ gb, uint64_t cb, SeedDesc s,
+                                                             uint32_t* __restrict__ counts, int bbits, int64_t tile) {
+  extern __shared__ uint32_t h[];  // nbuckets counts
+  __shared__ K lut[8][256];
+  const int nbk = 1 << bbits, bsh = 2 * s.w - bbits;
+  pb_lut(s, lut);
+  for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) h[d] = 0;
+  __syncthreads();
+  pb_tile<K>(ga, ca, gb, cb, s, lut, tile,
+             [&](uint64_t, K m, uint32_t, bool, uint32_t) { atomicAdd(&h[(uint32_t)(m >> bsh)], 1u); });
   __syncthreads();
   uint32_t* row = counts + (int64_t)blockIdx.x * nbk;
-  for (int d = tid; d < nbk; d += pb::kKeyThreads) row[d] = h[d];
+  for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) row[d] = h[d];
 }
 
 // ------------------------------------------------------- bucket offsets
@@ -251,35 +273,34 @@ void pair_scan_small(const uint32_t* in, int n, uint32_t* out, uint32_t* total, 
 
 // ------------------------------------------------------------- scatter
 
-__global__ void __launch_bounds__(pb::kKeyThreads) k_pb_scatter(const uint32_t* __restrict__ keys,
-                                                                const uint32_t* __restrict__ pos, uint64_t n,
+template <typename K>
+__global__ void __launch_bounds__(pb::kKeyThreads) k_pb_scatter(const uint32_t* __restrict__ ga, uint64_t ca,
+                                                                const uint32_t* __restrict__ gb, uint64_t cb, SeedDesc s,
                                                                 const uint32_t* __restrict__ offsets, int bbits,
-                                                                int bsh, int64_t tile, uint2* __restrict__ out) {
+                                                                int64_t tile, uint2* __restrict__ out) {
   extern __shared__ uint32_t cur[];  // next free slot per bucket
-  const int nbk = 1 << bbits;
+  __shared__ K lut[8][256];
+  const int nbk = 1 << bbits, bsh = 2 * s.w - bbits;
+  const uint32_t rest = (uint32_t)(((uint64_t)1 << bsh) - 1);
   const uint32_t* row = offsets + (int64_t)blockIdx.x * nbk;
+  pb_lut(s, lut);
   for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) cur[d] = row[d];
   __syncthreads();
-  const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)tile;
-  const uint64_t end = min(n, base + (uint64_t)tile);
-  for (uint64_t i = base + threadIdx.x; i < end; i += pb::kKeyThreads) {
-    const uint32_t k = keys[i];
-    const uint32_t slot = atomicAdd(&cur[k >> bsh], 1u);
-    out[slot] = make_uint2(k, pos[i]);
-  }
+  pb_tile<K>(ga, ca, gb, cb, s, lut, tile, [&](uint64_t, K m, uint32_t strand, bool in_b, uint32_t q) {
+    const uint32_t slot = atomicAdd(&cur[(uint32_t)(m >> bsh)], 1u);
+    out[slot] = make_uint2(((uint32_t)m & rest) << 2 | strand << 1 | (in_b ? 1u : 0u), q);
+  });
 }
 
 // ---------------------------------------------------- in-bucket sort
 
 struct LocalSmem {
-  uint32_t whist[pb::kLocWarps][pb::kSmemDigit];  // per-warp digit counts, then each warp's first slot
+  uint32_t whist[pb::kLocWarps][pb::kMaxDigit];   // per-warp digit counts, then each warp's first slot
   uint32_t run[pb::kMaxDigit];                    // chunked sort: slots used so far by each digit
   uint32_t dstart[pb::kMaxDigit];                 // chunked sort: each digit's first slot in the bucket
-  uint32_t wpairs[pb::kLocWarps];
-  uint32_t total;
 };
 
-// In-bucket key: the mer bits below the bucket bits, then the genome bit.
+// In-bucket key: the rest of the mixed mer, then the genome bit.
 __device__ __forceinline__ uint32_t pb_lkey(uint32_t key, int lbits) {
   return (((key >> 2) << 1) | (key & 1u)) & ((1u << lbits) - 1u);
 }
@@ -313,53 +334,6 @@ __device__ __forceinline__ void pb_rank(const uint2* src, int n, int rounds, int
       __syncwarp();
     }
   }
-}
-
-// One stable LSD pass of a bucket held in shared memory (n <= kCap): rank,
-// one scan over (digit, warp) counts, scatter.  Digits of up to 9 bits.
-__device__ void pb_pass_smem(const uint2* src, uint2* dst, int n, int shift, uint32_t mask, int lbits,
-                             LocalSmem& S) {
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int ndig = (int)mask + 1;
-  const int rounds = (n + pb::kLocThreads - 1) / pb::kLocThreads;
-  for (int d = lane; d < ndig; d += 32) S.whist[wid][d] = 0;
-  __syncwarp();
-  uint2 item[pb::kLocItems];
-  uint32_t rank[pb::kLocItems];
-  pb_rank(src, n, rounds, shift, mask, lbits, S, item, rank);
-  __syncthreads();
-  // thread t: digits 2t and 2t + 1 (ndig is a power of two up to 512)
-  const int d0 = 2 * tid;
-  uint32_t c0 = 0, c1 = 0;
-  if (d0 < ndig) {
-#pragma unroll
-    for (int w = 0; w < pb::kLocWarps; ++w) {
-      c0 += S.whist[w][d0];
-      c1 += S.whist[w][d0 + 1];
-    }
-  }
-  uint32_t r = block_excl_scan256(c0 + c1, nullptr);
-  if (d0 < ndig) {
-#pragma unroll
-    for (int w = 0; w < pb::kLocWarps; ++w) {
-      const uint32_t x = S.whist[w][d0];
-      S.whist[w][d0] = r;
-      r += x;
-    }
-#pragma unroll
-    for (int w = 0; w < pb::kLocWarps; ++w) {
-      const uint32_t x = S.whist[w][d0 + 1];
-      S.whist[w][d0 + 1] = r;
-      r += x;
-    }
-  }
-  __syncthreads();
-  const int wbase = wid * rounds * 32;
-#pragma unroll
-  for (int k = 0; k < pb::kLocItems; ++k)
-    if (k < rounds && wbase + k * 32 + lane < n)
-      dst[S.whist[wid][(pb_lkey(item[k].x, lbits) >> shift) & mask] + rank[k]] = item[k];
-  __syncthreads();
 }
 
 // One stable LSD pass over a bucket too large for shared memory: src and
@@ -415,101 +389,54 @@ __device__ void pb_pass_chunked(const uint2* src, uint2* dst, int n, int shift, 
 
 // Runs of the sorted bucket v[0, n): element i opens a pair when it and
 // i + 1 hold the same mer from different genomes and neither i - 1 nor
-// i + 2 holds that mer.  Pairs are written in order to stage[0, count),
-// which must not overlap v; returns the count.
-__device__ uint32_t pb_pairs(const uint2* v, int n, uint2* stage, LocalSmem& S) {
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int per = min(16, max(1, (n + pb::kLocThreads - 1) / pb::kLocThreads));
-  uint32_t total = 0;
-  for (int c0 = 0; c0 < n; c0 += pb::kLocThreads * per) {
-    const int i0 = c0 + tid * per;  // thread t: elements i0 .. i0 + per - 1
-    uint32_t flags = 0;
-    for (int k = 0; k < per; ++k) {
-      const int i = i0 + k;
-      if (i + 1 >= n) break;
-      const uint32_t k0 = v[i].x, k1 = v[i + 1].x, m = k0 >> 2;  // key >> 2: the mer
-      if ((k1 >> 2) != m || ((k0 ^ k1) & 1u) == 0) continue;
-      if (i > 0 && (v[i - 1].x >> 2) == m) continue;
-      if (i + 2 < n && (v[i + 2].x >> 2) == m) continue;
-      flags |= 1u << k;
-    }
-    const uint32_t cnt = __popc(flags);
-    const uint32_t inc = warp_incl_scan(cnt);
-    if (lane == 31) S.wpairs[wid] = inc;
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t r = 0;
-      for (int w = 0; w < pb::kLocWarps; ++w) {
-        const uint32_t x = S.wpairs[w];
-        S.wpairs[w] = r;
-        r += x;
-      }
-      S.total = r;
-    }
-    __syncthreads();
-    uint32_t j = total + S.wpairs[wid] + inc - cnt;
-    const uint32_t chunk_pairs = S.total;
-    while (flags) {
-      const int k = __ffs(flags) - 1;
-      flags &= flags - 1;
-      const uint2 x = v[i0 + k], y = v[i0 + k + 1];
-      const bool a_first = (x.x & 1u) == 0;
-      const uint2 ea = a_first ? x : y, eb = a_first ? y : x;
-      // SetDirection (LM/MemHash.cpp:189-207): B is reversed relative to A
-      // when the two occurrences have different strand bits
-      const uint32_t rev = ((ea.x >> 1) ^ (eb.x >> 1)) & 1u;
-      stage[j++] = make_uint2(ea.y, eb.y | (rev << 31));
-    }
-    total += chunk_pairs;
-    __syncthreads();
+// i + 2 holds that mer.
+__device__ void pb_pairs(const uint2* v, int n, uint32_t* __restrict__ tab) {
+  for (int i = threadIdx.x; i + 1 < n; i += pb::kLocThreads) {
+    const uint32_t k0 = v[i].x, k1 = v[i + 1].x, m = k0 >> 2;  // key >> 2: the mer
+    if ((k1 >> 2) != m || ((k0 ^ k1) & 1u) == 0) continue;
+    if (i > 0 && (v[i - 1].x >> 2) == m) continue;
+    if (i + 2 < n && (v[i + 2].x >> 2) == m) continue;
+    const uint32_t p0 = v[i].y, p1 = v[i + 1].y;
+    // SetDirection (LM/MemHash.cpp:189-207): B is reversed relative to A
+    // when the two occurrences have different strand bits
+    tab[k0 & 1u ? p1 : p0] = (k0 & 1u ? p0 : p1) | (((k0 ^ k1) >> 1) & 1u) << 31;
   }
-  return total;
 }
 
 // Block b finds the unique pairs of bucket b.  A bucket of at most cap
-// (<= kCap) keys is loaded into shared memory as (in-bucket key | strand <<
-// 31, position) and split by its top in-bucket bits (up to 9) into at most
-// 512 groups of a few keys each (shared-memory atomics place a group's keys
-// in any order).  Then one thread per key: a key whose mer occurs exactly
-// twice in its group, once per genome, and which is the A occurrence, is a
-// pair (marked, and counted for its group); after one scan over the groups
-// each pair's slot is its group's first slot plus the number of the group's
-// pairs with a smaller mer.  If a group holds more than kGroupMax keys the
-// bucket is instead sorted by stable radix passes of up to 9 bits.  Larger
-// buckets are sorted in chunks between their region of `buf` and the same
-// region of `alt` in an odd number of passes of up to 6 bits, which leaves
-// them in `alt`.  The staged pairs go to the bucket's region of `buf`, which
-// the keys no longer occupy.
+// (<= kCap) keys is split in shared memory by its top in-bucket bits (up to
+// 9) into at most 512 groups of a few keys each (atomics place a group's keys
+// in any order).  Then one thread per key of A: a key whose mer occurs
+// exactly twice in its group, once per genome, is a pair.  Other buckets, and
+// one with a group of more than kGroupMax keys, are sorted in chunks between
+// their region of `buf` and the same region of `alt` in an odd number of
+// passes of up to 6 bits, which leaves them in `alt`.
 __global__ void __launch_bounds__(pb::kLocThreads) k_pb_local(uint2* __restrict__ buf, uint2* __restrict__ alt,
                                                               const uint32_t* __restrict__ bstart,
                                                               const uint32_t* __restrict__ bsize, int lbits, int npass,
-                                                              int dbits, int spass, int sbits, int cap,
-                                                              uint32_t* __restrict__ pcount) {
-  extern __shared__ __align__(16) uint2 sbuf[];  // 2 * kCap elements
+                                                              int dbits, int cap, uint32_t* __restrict__ tab) {
+  extern __shared__ __align__(16) uint2 sbuf[];  // kCap elements
   __shared__ LocalSmem S;
-  __shared__ uint32_t gcnt[pb::kGroups], gbeg[pb::kGroups], gcur[pb::kGroups], gpair[pb::kGroups];
-  constexpr uint32_t kMark = 1u << 30, kKey = kMark - 1u;
+  __shared__ uint32_t gcnt[pb::kGroups], gbeg[pb::kGroups], gcur[pb::kGroups];
   const int tid = threadIdx.x;
   const int b = blockIdx.x;
   const int n = (int)bsize[b];
   uint2* g = buf + bstart[b];
   uint2* h = alt + bstart[b];
-  uint32_t np;
-  if (n <= cap) {
+  bool sort = n > cap;
+  if (!sort) {
     // group bits: mer bits only (never the genome bit), at most 9
     const int hbits = lbits - 1 < 9 ? lbits - 1 : 9, lo = lbits - hbits, ng = 1 << hbits;
-    uint2* s0 = sbuf;
-    uint2* s1 = sbuf + pb::kCap;
-    for (int d = tid; d < pb::kGroups; d += pb::kLocThreads) {
-      gcnt[d] = 0;
-      gpair[d] = 0;
-    }
+    for (int d = tid; d < pb::kGroups; d += pb::kLocThreads) gcnt[d] = 0;
     __syncthreads();
-    for (int i = tid; i < n; i += pb::kLocThreads) {
-      const uint2 it = g[i];
-      const uint32_t lk = pb_lkey(it.x, lbits);
-      s0[i] = make_uint2(lk | (((it.x >> 1) & 1u) << 31), it.y);
-      atomicAdd(&gcnt[lk >> lo], 1u);
+    uint2 item[pb::kLocItems];
+#pragma unroll
+    for (int k = 0; k < pb::kLocItems; ++k) {
+      const int i = k * pb::kLocThreads + tid;
+      if (i < n) {
+        item[k] = g[i];
+        atomicAdd(&gcnt[pb_lkey(item[k].x, lbits) >> lo], 1u);
+      }
     }
     __syncthreads();
     // thread t: groups 2t and 2t + 1
@@ -518,67 +445,32 @@ __global__ void __launch_bounds__(pb::kLocThreads) k_pb_local(uint2* __restrict_
     const uint32_t st = block_excl_scan256(c0 + c1, nullptr);
     if (d0 < ng) gbeg[d0] = gcur[d0] = st;
     if (d0 + 1 < ng) gbeg[d0 + 1] = gcur[d0 + 1] = st + c0;
-    __syncthreads();
-    for (int i = tid; i < n; i += pb::kLocThreads) {
-      const uint2 e = s0[i];
-      s1[atomicAdd(&gcur[(e.x & kKey) >> lo], 1u)] = e;
-    }
-    const bool big = __syncthreads_or(c0 > (uint32_t)pb::kGroupMax || c1 > (uint32_t)pb::kGroupMax);
-    if (!big) {
-      // the A occurrence of each pair: its pair record into s0 (free now)
+    sort = __syncthreads_or(c0 > (uint32_t)pb::kGroupMax || c1 > (uint32_t)pb::kGroupMax);
+    if (!sort) {
+#pragma unroll
+      for (int k = 0; k < pb::kLocItems; ++k)
+        if (k * pb::kLocThreads + tid < n) sbuf[atomicAdd(&gcur[pb_lkey(item[k].x, lbits) >> lo], 1u)] = item[k];
+      __syncthreads();
       for (int i = tid; i < n; i += pb::kLocThreads) {
-        const uint32_t x = s1[i].x, lk = x & kKey, m = lk >> 1;
-        const int d = (int)(lk >> lo), e0 = (int)gbeg[d], e1 = e0 + (int)gcnt[d];
+        const uint32_t x = sbuf[i].x;
+        if (x & 1u) continue;  // the A occurrence of each pair
+        const int d = (int)(pb_lkey(x, lbits) >> lo), e0 = (int)gbeg[d], e1 = e0 + (int)gcnt[d];
         int cnt = 0, other = 0;
         for (int j = e0; j < e1; ++j)
-          if (((s1[j].x & kKey) >> 1) == m) {
+          if (((sbuf[j].x ^ x) >> 2) == 0) {
             ++cnt;
             if (j != i) other = j;
           }
-        if (cnt == 2 && (lk & 1u) == 0) {
-          const uint2 y = s1[other];
-          if (y.x & 1u) {
-            // SetDirection (LM/MemHash.cpp:189-207): B is reversed relative
-            // to A when the two occurrences have different strand bits
-            const uint32_t rev = (x ^ y.x) >> 31;
-            s0[i] = make_uint2(s1[i].y, y.y | (rev << 31));
-            atomicOr(&s1[i].x, kMark);
-            atomicAdd(&gpair[d], 1u);
-          }
+        if (cnt == 2 && (sbuf[other].x & 1u)) {
+          // SetDirection (LM/MemHash.cpp:189-207): B is reversed relative
+          // to A when the two occurrences have different strand bits
+          const uint2 y = sbuf[other];
+          tab[sbuf[i].y] = y.y | (((x ^ y.x) >> 1) & 1u) << 31;
         }
       }
-      __syncthreads();
-      const uint32_t q0 = d0 < ng ? gpair[d0] : 0u, q1 = d0 + 1 < ng ? gpair[d0 + 1] : 0u;
-      const uint32_t pst = block_excl_scan256(q0 + q1, &S.total);
-      if (d0 < ng) gcur[d0] = pst;
-      if (d0 + 1 < ng) gcur[d0 + 1] = pst + q0;
-      __syncthreads();
-      for (int i = tid; i < n; i += pb::kLocThreads) {
-        const uint32_t x = s1[i].x;
-        if (!(x & kMark)) continue;
-        const uint32_t m = (x & kKey) >> 1;
-        const int d = (int)((x & kKey) >> lo), e0 = (int)gbeg[d], e1 = e0 + (int)gcnt[d];
-        uint32_t r = 0;
-        for (int j = e0; j < e1; ++j) {
-          const uint32_t y = s1[j].x;
-          r += (y & kMark) && ((y & kKey) >> 1) < m;
-        }
-        g[gcur[d] + r] = s0[i];
-      }
-      np = S.total;
-    } else {
-      for (int i = tid; i < n; i += pb::kLocThreads) s0[i] = g[i];
-      __syncthreads();
-      const uint32_t mask = (1u << sbits) - 1u;
-      for (int p = 0; p < spass; ++p) {
-        pb_pass_smem(s0, s1, n, p * sbits, mask, lbits, S);
-        uint2* t = s0;
-        s0 = s1;
-        s1 = t;
-      }
-      np = pb_pairs(s0, n, g, S);
     }
-  } else {
+  }
+  if (sort) {
     const uint32_t mask = (1u << dbits) - 1u;
     const uint2* src = g;
     uint2* dst = h;
@@ -588,64 +480,56 @@ __global__ void __launch_bounds__(pb::kLocThreads) k_pb_local(uint2* __restrict_
       src = dst;
       dst = t;
     }
-    np = pb_pairs(src, n, g, S);  // npass is odd: the sorted bucket is in alt
+    pb_pairs(src, n, tab);  // npass is odd: the sorted bucket is in alt
   }
-  if (tid == 0) pcount[b] = np;
 }
 
 // ------------------------------------------------------------------ host
 
-int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
-                 PairStage* out) {
+template <typename K>
+static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
+                           uint32_t* tab) {
   const uint64_t n = ca + cb;
   const PairBucketGeom g = pair_bucket_geom(n, s.w);
   const int nbk = g.nbuckets;
   Workspace& ws = c->ws;
-  const uint64_t n4 = (n + 3) & ~3ull;  // positions start on a 16-byte boundary (vector stores)
-  uint32_t* kp = (uint32_t*)ws.get(c, 30, (size_t)n4 * 8 + 64);
+  uint2* altp = (uint2*)ws.get(c, 30, (size_t)n * 8 + 64);
   uint2* bufp = (uint2*)ws.get(c, 31, (size_t)n * 8 + 64);
   // count rows, then the tiles' first slots (ntiles x nbk each)
   uint32_t* counts = (uint32_t*)ws.get(c, 32, (size_t)g.ntiles * nbk * 8 + 64);
-  uint32_t* tabs = (uint32_t*)ws.get(c, 33, ((size_t)g.nchunks * nbk + 4 * (size_t)nbk) * 4 + 256);
-  if (!kp || !bufp || !counts || !tabs) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-  uint32_t* keys = kp;
-  uint32_t* pos = kp + n4;
+  uint32_t* tabs = (uint32_t*)ws.get(c, 33, ((size_t)g.nchunks * nbk + 2 * (size_t)nbk) * 4 + 256);
+  if (!altp || !bufp || !counts || !tabs) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   uint32_t* offs = counts + (size_t)g.ntiles * nbk;
   uint32_t* csum = tabs;
   uint32_t* bstart = csum + (size_t)g.nchunks * nbk;
   uint32_t* bsize = bstart + nbk;
-  uint32_t* pcount = bsize + nbk;
-  uint32_t* pbase = pcount + nbk;
-  static bool attr = false;  // once per process: more than 48 KB of dynamic shared memory
+  static bool attr = false;  // once per process and key type: more than 48 KB of dynamic shared memory
   if (!attr) {
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(2 * pb::kCap * sizeof(uint2))));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_keys<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
     attr = true;
   }
   const size_t hsm = (size_t)nbk * 4;
-  k_pb_keys<<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, keys, pos, counts, g.bbits,
-                                                                     g.tile);
+  k_pb_keys<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, counts, g.bbits, g.tile);
   const dim3 grid2((unsigned)((nbk + 255) / 256), (unsigned)g.nchunks);
   k_pb_csum<<<grid2, 256, 0, c->stream>>>(counts, g.ntiles, nbk, csum);
   k_pb_scan<<<1, 1024, 0, c->stream>>>(csum, g.nchunks, nbk, bstart, bsize);
   k_pb_offsets<<<grid2, 256, 0, c->stream>>>(counts, g.ntiles, nbk, csum, bstart, offs);
   stage_mark(c, "seed_scatter");
-  k_pb_scatter<<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(keys, pos, n, offs, g.bbits,
-                                                                        2 * s.w + 2 - g.bbits, g.tile, bufp);
+  k_pb_scatter<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, offs, g.bbits, g.tile, bufp);
   stage_mark(c, "seed_local");
   const int cap = std::min(c->pair_bucket_cap, pb::kCap);
-  k_pb_local<<<(unsigned)nbk, pb::kLocThreads, 2 * pb::kCap * sizeof(uint2), c->stream>>>(
-      bufp, (uint2*)kp, bstart, bsize, g.lbits, g.npass, g.dbits, g.spass, g.sbits, cap, pcount);
+  k_pb_local<<<(unsigned)nbk, pb::kLocThreads, pb::kCap * sizeof(uint2), c->stream>>>(
+      bufp, altp, bstart, bsize, g.lbits, g.npass, g.dbits, cap, tab);
   c->launches += 6;
   MVG_CUDA_TRY(cudaGetLastError());
-  out->stage = bufp;
-  out->bstart = bstart;
-  out->pcount = pcount;
-  out->pbase = pbase;
-  out->nbuckets = nbk;
   return 0;
+}
+
+int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
+                 uint32_t* tab) {
+  return s.w <= 15 ? pair_buckets_as<uint32_t>(c, ga, ca, gb, cb, s, tab)
+                   : pair_buckets_as<uint64_t>(c, ga, ca, gb, cb, s, tab);
 }
 
 }  // namespace mvg
