@@ -247,6 +247,8 @@ int mvg_destroy(mvg_handle h) {
   if (h->h_scalars) cudaFreeHost(h->h_scalars);
   if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->h_off) cudaFreeHost(h->h_off);
+  for (void* p : h->h_rows)
+    if (p) cudaFreeHost(p);
   for (cudaEvent_t ev : {h->fork, h->join, h->fork2, h->join2, h->fork4, h->join4, h->fork5,
                          h->join5})
     if (ev) cudaEventDestroy(ev);

@@ -14,26 +14,28 @@
 //
 //   k_gs_pack        each gap's sequences 2-bit packed into their own word
 //                    range (zero padded like translate32's buffer)
-//   k_gs_keys        canonical rank-0 seed mer of every gap position with the
-//                    gap's own seed: key = gap << 32 | mer bits | strand | genome
-//   radix sort       one stable LSD sort of all gaps' keys
-//   k_pair_count /   runs of one key per genome inside a gap (the unique-seed
-//   k_gs_pair_emit   enumeration), hash entry and bucket key gap << 16 | bucket
-//   radix sort       by bucket key: segments = (gap, bucket), seed order kept
-//   k_gs_replay      one warp per segment replays the reference's containment
-//                    tests, extensions and inserts (the genome matcher's warp
-//                    replay, with the gap's sequences and seed)
-//   k_gs_emit        GetMatchList order per gap: bucket, then MheCompare order
+//   k_gs_keys,       the seed join of pair_buckets.cu over all gaps' positions
+//   k_gs_scatter     at once, with keys (gap, canonical rank-0 seed mer of the
+//                    gap's own seed): the seeds unique in each gap, by A slot
+//   match_components the genome matcher's match list (match_components.cuh)
+//                    over all gaps, its buckets (gap, bucket): GetMatchList
+//                    order per gap
 //   host             EliminateOverlaps_v2 with std::sort (the order of equal
 //                    left ends is the library sort's, as in the reference),
 //                    LengthFilter, shift to genome coordinates
+//
+// A gap's positions take slots from a multiple of 32 on, with at least 31
+// empty ones after them, so that chains of seeds never cross into the next
+// gap and a warp's 32 slots are one gap's.  (A joint 64-bit radix sort of all
+// keys and a warp's replay per (gap, bucket) took 6.6 ms of device time for
+// 5,003 gaps of 200-20,000 bp, 43 Mbp; this takes GSMS ms.)
 #include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <thread>
 #include <vector>
 
-#include "match_common.cuh"
+#include "match_components.cuh"
 
 namespace mvg {
 
@@ -49,19 +51,19 @@ __constant__ SeedDesc c_gs_seed[32];
 struct GapDev {
   uint64_t src[2];   // first base of the gap in genome A / B
   uint64_t word[2];  // first packed word of the gap's A / B sequence
-  uint64_t key[2];   // first key slot of the gap's A / B positions
+  uint32_t slot[2];  // first slot of the gap's A / B positions
+  uint32_t cnt[2];   // seed positions
   uint32_t len[2];   // gap lengths
   int32_t w;         // seed weight
   int32_t pad;
 };
 
-// Index of the last gap whose field `off` is <= x (offsets ascending).
-__device__ __forceinline__ int gap_of(const GapDev* __restrict__ g, int n, int side, int which, uint64_t x) {
+// Index of the last gap whose packed words start at or before x.
+__device__ __forceinline__ int gap_of(const GapDev* __restrict__ g, int n, int side, uint64_t x) {
   int lo = 0, len = n;
   while (len > 0) {
     const int half = len >> 1;
-    const uint64_t v = which == 0 ? g[lo + half].word[side] : g[lo + half].key[side];
-    if (v <= x) {
+    if (g[lo + half].word[side] <= x) {
       lo += half + 1;
       len -= half + 1;
     } else {
@@ -79,7 +81,7 @@ __global__ void k_gs_pack(const uint8_t* __restrict__ ga, const uint8_t* __restr
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
     const int side = t < words_a ? 0 : 1;
     const uint64_t w = side ? t - words_a : t;
-    const int g = gap_of(gaps, ngaps, side, 0, w);
+    const int g = gap_of(gaps, ngaps, side, w);
     const GapDev& d = gaps[g];
     const uint8_t* s = (side ? gb : ga) + d.src[side];
     const uint64_t b0 = (w - d.word[side]) * 16;
@@ -98,180 +100,105 @@ __global__ void k_gs_pack(const uint8_t* __restrict__ ga, const uint8_t* __restr
   }
 }
 
-// One thread per seed position of all gaps (A positions, then B positions):
-// key = gap << kshift | (seed bits, strand) << 1 | genome, value = position
-// in the gap sequence, kshift = 2 * (largest seed weight) + 2 so that the
-// sort covers no unused bits.  The (2w+1)-bit SML key orders as the
-// reference's mers.
-__global__ void k_gs_keys(const uint32_t* __restrict__ pa, const uint32_t* __restrict__ pb,
-                          const GapDev* __restrict__ gaps, int ngaps, uint64_t keys_a, uint64_t keys_b, int kshift,
-                          uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  const uint64_t total = keys_a + keys_b, stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const int side = t < keys_a ? 0 : 1;
-    const uint64_t k = side ? t - keys_a : t;
-    const int g = gap_of(gaps, ngaps, side, 1, k);
-    const GapDev& d = gaps[g];
-    const SeedDesc& s = c_gs_seed[d.w];
-    const uint64_t p = k - d.key[side];
-    const uint64_t m = canonical_mer((side ? pb : pa) + d.word[side], p, s);
-    const uint64_t sml = ((m >> (64 - 2 * s.w)) << 1) | (m & 1ull);
-    keys[t] = ((uint64_t)g << kshift) | (sml << 1) | (uint64_t)side;
-    vals[t] = (uint32_t)p;
-  }
-}
-
-// Hash entries of the unique-seed pairs (k_pair_emit's HashMatch /
-// SetDirection / CalculateOffset, LM/MemHash.cpp:167-207,
-// LM/MatchHashEntry.cpp:141-162) with each gap's seed length; the bucket key
-// puts the gap above the bucket so one sort groups (gap, bucket) segments.
-__global__ void __launch_bounds__(256) k_gs_pair_emit(const uint64_t* __restrict__ keys,
-                                                      const uint32_t* __restrict__ pos, int64_t n,
-                                                      const uint32_t* __restrict__ tstart, int kshift,
-                                                      const GapDev* __restrict__ gaps, Mhe* __restrict__ mhe,
-                                                      uint64_t* __restrict__ bkey, uint32_t* __restrict__ order) {
-  const int64_t i0 = (int64_t)blockIdx.x * kPairTile + (int64_t)threadIdx.x * kPairItems;
-  __shared__ uint32_t tile_pairs;
-  uint32_t flags = 0;
+// The gap of every 32 slots (a CTA per gap).
+__global__ void k_gs_slots(const GapDev* __restrict__ gaps, uint32_t* __restrict__ ga, uint32_t* __restrict__ gb) {
+  const GapDev& d = gaps[blockIdx.x];
 #pragma unroll
-  for (int k = 0; k < kPairItems; ++k)
-    if (i0 + k < n && pair_flag(keys, n, i0 + k)) flags |= 1u << k;
-  uint32_t li = block_excl_scan256(__popc(flags), &tile_pairs) + tstart[blockIdx.x];
-  while (flags) {
-    const int k = __ffs(flags) - 1;
-    flags &= flags - 1;
-    const int64_t i = i0 + k;
-    const uint64_t k0 = keys[i], k1 = keys[i + 1];
-    const bool a_first = (k0 & 1ull) == 0;
-    const uint64_t ka = a_first ? k0 : k1, kb = a_first ? k1 : k0;
-    const uint32_t g = (uint32_t)(k0 >> kshift);
-    Mhe m;
-    m.s0 = (int64_t)(a_first ? pos[i] : pos[i + 1]) + 1;
-    m.s1 = (int64_t)(a_first ? pos[i + 1] : pos[i]) + 1;
-    m.len = c_gs_seed[gaps[g].w].L;
-    const bool ref_forward = !((ka >> 1) & 1ull);
-    if (ref_forward == (bool)((kb >> 1) & 1ull)) m.s1 = -m.s1;
-    m.off = m.s1 - m.s0;
-    if (m.s1 < 0) m.off -= m.len;
-    const int64_t ts = kTableSize;
-    mhe[li] = m;
-    bkey[li] = ((uint64_t)g << 16) | (uint64_t)(((m.off % ts) + ts) % ts);
-    order[li] = li;
-    ++li;
+  for (int side = 0; side < 2; ++side) {
+    const uint32_t w0 = d.slot[side] >> 5, n = d.cnt[side] ? (d.cnt[side] + 62) >> 5 : 0;
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) (side ? gb : ga)[w0 + k] = blockIdx.x;
   }
 }
 
-// Segment starts of the bucket-sorted entries: flag 1 where the bucket key
-// changes.
-__global__ void k_gs_seg_flags(const uint64_t* __restrict__ bkey, int64_t n, uint32_t* __restrict__ flag) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    flag[i] = (i == 0 || bkey[i] != bkey[i - 1]) ? 1u : 0u;
-}
+// All gaps as one matching problem over their slots.
+struct GapSet {
+  const uint32_t *pa, *pb;
+  const GapDev* gaps;
+  const uint32_t *ga, *gb;  // the gap of every 32 A / B slots
+  uint32_t slots[2];
+  int mbits;     // mer bits: the widest seed's
+  int32_t* out;  // rows (start A, start B, length) in gap coordinates
+  int mer_bits() const { return mbits; }
+  __device__ __forceinline__ int seed_len(uint32_t x) const { return c_gs_seed[gaps[ga[x >> 5]].w].L; }
+  __device__ __forceinline__ uint32_t key(uint32_t v, uint32_t x) const {
+    const uint32_t g = ga[x >> 5];
+    const GapDev& d = gaps[g];
+    return g << 16 | diag_bucket(seed_diag(v - d.slot[1], x - d.slot[0]), c_gs_seed[d.w].L);
+  }
+  __device__ __forceinline__ MatchView view(uint32_t x, uint32_t& a, uint32_t& b) const {
+    const GapDev& d = gaps[ga[x >> 5]];
+    a = d.slot[0];
+    b = d.slot[1];
+    return MatchView{{pa + d.word[0], pb + d.word[1]}, {d.len[0], d.len[1]}, c_gs_seed[d.w]};
+  }
+  __device__ __forceinline__ void row(uint64_t diag, uint32_t lo, uint32_t hi, uint64_t at) const {
+    const GapDev& d = gaps[ga[lo >> 5]];
+    const Mhe m = diag_entry(diag, lo, hi, c_gs_seed[d.w].L);
+    out[3 * at + 0] = (int32_t)(m.s0 - d.slot[0]);
+    out[3 * at + 1] = (int32_t)(m.s1 > 0 ? m.s1 - d.slot[1] : m.s1 + d.slot[1]);
+    out[3 * at + 2] = (int32_t)m.len;
+  }
+};
 
-__global__ void k_gs_seg_fill(const uint64_t* __restrict__ bkey, int64_t n, const uint32_t* __restrict__ flag,
-                              const uint32_t* __restrict__ sidx, uint32_t* __restrict__ seg_start,
-                              uint32_t* __restrict__ seg_gap) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (flag[i]) {
-      seg_start[sidx[i]] = (uint32_t)i;
-      seg_gap[sidx[i]] = (uint32_t)(bkey[i] >> 16);
-    }
-}
-
-// One warp per (gap, bucket) segment, taken in turn from a counter: the
-// reference's AddHashEntry sequence (LM/MemHash.cpp:209-251) over the
-// segment's seeds in key order.  32 seeds are tested at a time against the
-// bucket's sorted entries; the first one not contained is extended
-// (ExtendMatch, LM/MatchFinder.h:218-374, inside the gap's sequences) and
-// inserted at its lower_bound, and testing resumes after it.
-__global__ void __launch_bounds__(256, 3) k_gs_replay(const uint32_t* __restrict__ pa, const uint32_t* __restrict__ pb,
-                                                   const GapDev* __restrict__ gaps, const Mhe* __restrict__ mhe,
-                                                   const uint32_t* __restrict__ sorted,
-                                                   const uint32_t* __restrict__ seg_start,
-                                                   const uint32_t* __restrict__ seg_gap, uint32_t nseg,
-                                                   uint32_t nentries, Mhe* __restrict__ ent,
-                                                   uint32_t* __restrict__ nent, unsigned* __restrict__ counter) {
-  __shared__ ExtRing s_ring[8];
-  __shared__ MatchCtx s_ctx[8];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  MatchCtx& c = s_ctx[wid];
-  for (;;) {
-    uint32_t sg = 0;
-    if (lane == 0) sg = atomicAdd(counter, 1u);
-    sg = __shfl_sync(0xffffffffu, sg, 0);
-    if (sg >= nseg) return;
-    const uint32_t st = seg_start[sg];
-    const uint32_t cnt = (sg + 1 < nseg ? seg_start[sg + 1] : nentries) - st;
-    const GapDev& d = gaps[seg_gap[sg]];
-    if (lane == 0) {
-      c.g[0] = pa + d.word[0];
-      c.g[1] = pb + d.word[1];
-      c.n[0] = d.len[0];
-      c.n[1] = d.len[1];
-      c.s = c_gs_seed[d.w];
-    }
-    __syncwarp();
-    const int L = c.s.L;
-    Mhe* E = ent + st;
-    const uint32_t* sp = sorted + st;
-    int64_t n = 0;
-    for (uint32_t base = 0; base < cnt; base += 32) {
-      const uint32_t i = base + lane;
-      Mhe m = {0, 0, 0, 0};
-      if (i < cnt) m = mhe[sp[i]];
-      unsigned pending = __ballot_sync(0xffffffffu, i < cnt);
-      while (pending) {
-        bool coll_here = true;
-        if (pending & (1u << lane)) {
-          const int64_t at = lower_bound_mhe(E, n, m, L);
-          coll_here = at != n && !mhe_less(E[at], m, L) && !mhe_less(m, E[at], L);
-        }
-        const unsigned fresh = __ballot_sync(0xffffffffu, (pending & (1u << lane)) && !coll_here);
-        if (!fresh) break;
-        const int f = __ffs(fresh) - 1;
-        pending &= ~((2u << f) - 1u);
-        Mhe x;
-        x.s0 = __shfl_sync(0xffffffffu, m.s0, f);
-        x.s1 = __shfl_sync(0xffffffffu, m.s1, f);
-        x.len = __shfl_sync(0xffffffffu, m.len, f);
-        x.off = __shfl_sync(0xffffffffu, m.off, f);
-        warp_extend(c, x, s_ring[wid]);
-        const int64_t at = lower_bound_mhe(E, n, x, L);
-        for (int64_t hi = n - 1; hi >= at; hi -= 32) {
-          const int64_t k = hi - lane;
-          Mhe t;
-          if (k >= at) t = E[k];
-          __syncwarp();
-          if (k >= at) E[k + 1] = t;
-          __syncwarp();
-        }
-        if (lane == 0) E[at] = x;
-        __syncwarp();
-        ++n;
-      }
-    }
-    if (lane == 0) nent[sg] = (uint32_t)n;
-    __syncwarp();
+// Calls f(mixed key, strand, in B, slot) for every seed position of this
+// block's tile of slots (A's, then B's); a warp's 32 slots are one gap's.
+template <class F>
+__device__ __forceinline__ void gs_tile(const GapSet& P, int bits, int64_t tile, F f) {
+  const uint64_t n = (uint64_t)P.slots[0] + P.slots[1], base = (uint64_t)blockIdx.x * (uint64_t)tile;
+  for (int64_t o = threadIdx.x; o < tile; o += blockDim.x) {
+    const uint64_t p = base + (uint64_t)o;
+    if (p >= n) break;
+    const int side = p >= P.slots[0];
+    const uint32_t q = (uint32_t)(side ? p - P.slots[0] : p);
+    const uint32_t g = (side ? P.gb : P.ga)[q >> 5];
+    const GapDev& d = P.gaps[g];
+    const uint32_t x = q - d.slot[side];
+    if (x >= d.cnt[side]) continue;
+    const SeedDesc& s = c_gs_seed[d.w];
+    const uint64_t m = canonical_mer((side ? P.pb : P.pa) + d.word[side], x, s);
+    f(mix_mer<uint64_t>((uint64_t)g << P.mbits | m >> (64 - 2 * s.w), bits), (uint32_t)m & 1u, side, q);
   }
 }
 
-// Entries of each segment in bucket order (segments are already in (gap,
-// bucket) order), rows (start A, start B, length) in gap coordinates.
-__global__ void k_gs_emit(const Mhe* __restrict__ ent, const uint32_t* __restrict__ seg_start,
-                          const uint32_t* __restrict__ nent, const uint32_t* __restrict__ ooff, uint32_t nseg,
-                          int64_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t s = gw; s < nseg; s += nw) {
-    const Mhe* E = ent + seg_start[s];
-    for (uint32_t k = lane; k < nent[s]; k += 32) {
-      const uint64_t o = (uint64_t)ooff[s] + k;
-      out[3 * o + 0] = E[k].s0;
-      out[3 * o + 1] = E[k].s1;
-      out[3 * o + 2] = E[k].len;
+__global__ void __launch_bounds__(1024) k_gs_keys(GapSet P, int bits, int bbits, int64_t tile,
+                                                  uint32_t* __restrict__ counts) {
+  extern __shared__ uint32_t h[];  // nbuckets counts
+  const int nbk = 1 << bbits, bsh = bits - bbits;
+  for (int d = threadIdx.x; d < nbk; d += blockDim.x) h[d] = 0;
+  __syncthreads();
+  gs_tile(P, bits, tile, [&](uint64_t k, uint32_t, int, uint32_t) { atomicAdd(&h[(uint32_t)(k >> bsh)], 1u); });
+  __syncthreads();
+  for (int d = threadIdx.x; d < nbk; d += blockDim.x) counts[(int64_t)blockIdx.x * nbk + d] = h[d];
+}
+
+__global__ void __launch_bounds__(1024) k_gs_scatter(GapSet P, int bits, int bbits, int64_t tile,
+                                                     const uint32_t* __restrict__ offsets, uint2* __restrict__ out) {
+  extern __shared__ uint32_t cur[];  // next free slot per bucket
+  const int nbk = 1 << bbits, bsh = bits - bbits;
+  const uint32_t rest = (uint32_t)(((uint64_t)1 << bsh) - 1);
+  for (int d = threadIdx.x; d < nbk; d += blockDim.x) cur[d] = offsets[(int64_t)blockIdx.x * nbk + d];
+  __syncthreads();
+  gs_tile(P, bits, tile, [&](uint64_t k, uint32_t strand, int side, uint32_t q) {
+    out[atomicAdd(&cur[(uint32_t)(k >> bsh)], 1u)] = make_uint2(((uint32_t)k & rest) << 2 | strand << 1 | (uint32_t)side, q);
+  });
+}
+
+// First row of every gap, and their number.
+__global__ void k_gs_gap_rows(const uint32_t* __restrict__ key, uint32_t ncomp, const uint32_t* __restrict__ at,
+                              uint32_t rows, uint32_t ngaps, uint32_t* __restrict__ out) {
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g > ngaps) return;
+  uint32_t lo = 0, len = g < ngaps ? ncomp : 0;
+  while (len > 0) {
+    const uint32_t half = len >> 1;
+    if (key[lo + half] < g << 16) {
+      lo += half + 1;
+      len -= half + 1;
+    } else {
+      len = half;
     }
   }
+  out[g] = g == ngaps || lo == ncomp ? rows : at ? at[lo] : lo;
 }
 
 // ------------------------------------------------------------------ host
@@ -296,20 +223,20 @@ static int gs_upload_tables(int device) {
 }
 
 namespace {
-struct Anchor {
-  int64_t s[2];
-  int64_t len;
+struct Anchor {  // in gap coordinates
+  int32_t s[2];
+  int32_t len;
 };
-int64_t left_end(const Anchor& m, int q) { return m.s[q] < 0 ? -m.s[q] : m.s[q]; }
+int32_t left_end(const Anchor& m, int q) { return m.s[q] < 0 ? -m.s[q] : m.s[q]; }
 // CropStart / CropEnd (LM/UngappedLocalAlignment.h:137-152 over
 // LM/HybridAbstractMatch.h:271-290): a forward start follows the first
 // column, a reverse start the last.
-void crop_start(Anchor& m, int64_t k) {
+void crop_start(Anchor& m, int32_t k) {
   m.len -= k;
   for (int q = 0; q < 2; ++q)
     if (m.s[q] > 0) m.s[q] += k;
 }
-void crop_end(Anchor& m, int64_t k) {
+void crop_end(Anchor& m, int32_t k) {
   m.len -= k;
   for (int q = 0; q < 2; ++q)
     if (m.s[q] < 0) m.s[q] -= k;
@@ -319,68 +246,81 @@ void crop_end(Anchor& m, int64_t k) {
 // matches, then LengthFilter(12): per sequence, sort by left end and walk
 // the overlaps, cropping (CropRight / CropLeft in that sequence's
 // orientation) or deleting the shorter match; the cropped-off pieces are
-// single-sequence matches, which processNewMatch drops.
-int64_t filter_gap(Anchor* a, int64_t n, std::vector<Anchor*>& ml) {
+// single-sequence matches, which processNewMatch drops.  The sort moves
+// (left end, index) pairs: std::sort's result on equal left ends follows from
+// the sequence of comparisons alone.  Returns the number kept, at a[0 ..).
+struct FilterScratch {
+  struct Item {
+    int32_t left;
+    int32_t at;  // -1: deleted
+  };
+  std::vector<Item> ml;
+  std::vector<Anchor> kept;
+};
+int64_t filter_gap(Anchor* a, int64_t n, FilterScratch& F) {
+  auto& ml = F.ml;
   ml.resize(n);
-  for (int64_t k = 0; k < n; ++k) ml[k] = a + k;
+  for (int64_t k = 0; k < n; ++k) ml[k].at = (int32_t)k;
   if (n >= 2) {
     for (int q = 0; q < 2; ++q) {
-      std::sort(ml.begin(), ml.end(), [q](const Anchor* x, const Anchor* y) { return left_end(*x, q) < left_end(*y, q); });
+      for (auto& x : ml) x.left = left_end(a[x.at], q);
+      std::sort(ml.begin(), ml.end(),
+                [](const FilterScratch::Item& x, const FilterScratch::Item& y) { return x.left < y.left; });
       bool any_deleted = false;
       const int64_t m = (int64_t)ml.size();
       for (int64_t i = 0; i < m; ++i) {
-        if (!ml[i]) continue;
+        if (ml[i].at < 0) continue;
+        Anchor& A = a[ml[i].at];
         for (int64_t j = i + 1; j < m; ++j) {
-          if (!ml[j]) continue;
-          const int64_t len_i = ml[i]->len;
-          const int64_t over = len_i - (left_end(*ml[j], q) - left_end(*ml[i], q));
+          if (ml[j].at < 0) continue;
+          Anchor& B = a[ml[j].at];
+          const int32_t len_i = A.len;
+          const int32_t over = len_i - (left_end(B, q) - left_end(A, q));
           if (over <= 0) break;
-          if (ml[j]->len > len_i) {  // i is the shorter: crop its right end or delete it
+          if (B.len > len_i) {  // i is the shorter: crop its right end or delete it
             if (over >= len_i) {
-              ml[i] = nullptr;
+              ml[i].at = -1;
               any_deleted = true;
               break;  // the reference steps back to i, finds it deleted and moves on
             }
-            if (ml[i]->s[q] > 0) crop_end(*ml[i], over);
-            else crop_start(*ml[i], over);
+            if (A.s[q] > 0) crop_end(A, over);
+            else crop_start(A, over);
           } else {  // j is: crop its left end or delete it
-            if (over >= ml[j]->len) {
-              ml[j] = nullptr;
+            if (over >= B.len) {
+              ml[j].at = -1;
               any_deleted = true;
-            } else if (ml[j]->s[q] > 0) {
-              crop_start(*ml[j], over);
+            } else if (B.s[q] > 0) {
+              crop_start(B, over);
             } else {
-              crop_end(*ml[j], over);
+              crop_end(B, over);
             }
           }
         }
       }
-      if (any_deleted) ml.erase(std::remove(ml.begin(), ml.end(), nullptr), ml.end());
+      if (any_deleted)
+        ml.erase(std::remove_if(ml.begin(), ml.end(), [](const FilterScratch::Item& x) { return x.at < 0; }), ml.end());
     }
   }
-  int64_t k = 0;
-  std::vector<Anchor> kept;
-  kept.reserve(ml.size());
-  for (const Anchor* p : ml)
-    if (p->len >= kGsMinAnchor) kept.push_back(*p);
-  for (const Anchor& x : kept) a[k++] = x;
-  return k;
+  auto& kept = F.kept;
+  kept.clear();
+  for (const auto& x : ml)
+    if (a[x.at].len >= kGsMinAnchor) kept.push_back(a[x.at]);
+  std::copy(kept.begin(), kept.end(), a);
+  return (int64_t)kept.size();
 }
-}  // namespace
 
-namespace {
 // One chunk of a call's gaps: the searched gaps' device descriptors and
-// caller indices, the device pass's rows and segment tables, and the host
-// pass's filtered anchors.
+// caller indices, the device pass's rows (in pinned memory, per gap from
+// gap_row on, GetMatchList order) and the host pass's counts.
 struct GsChunk {
   std::vector<GapDev> gd;
   std::vector<uint32_t> gid;  // caller's gap index of each searched gap
-  uint64_t words[2] = {0, 0}, keys[2] = {0, 0};
-  std::vector<int64_t> rows;  // (start A, start B, length) per entry, GetMatchList order per gap
-  std::vector<uint32_t> seg_gap, seg_n;
-  std::vector<Anchor> anc;     // searched gap gi's survivors at [gap_r[gi], gap_r[gi] + nkept[gi])
-  std::vector<size_t> gap_r;
-  std::vector<int64_t> nkept;
+  uint64_t words[2] = {0, 0};
+  uint32_t slots[2] = {0, 0};
+  uint64_t keys[2] = {0, 0};
+  Anchor* rows = nullptr;
+  const uint32_t* gap_row = nullptr;  // null: no rows
+  std::vector<uint32_t> nkept;
 };
 
 // Runs fn(i) for i in [0, n) on up to nthreads host threads that claim runs
@@ -410,16 +350,29 @@ int host_threads_for(size_t items) {
 }
 }  // namespace
 
-// Host plan of gaps [g0, g1) (already validated): seed weights, word and key
-// ranges of the gaps that are searched.
-static int gs_plan(const int64_t* gaps, uint64_t g0, uint64_t g1, GsChunk& ch) {
-  for (uint64_t g = g0; g < g1; ++g) {
+// Slots of a chunk of gaps, and its most gaps: the seed join's buckets hold
+// 2,048 keys each up to 2^25 keys, and its keys 44 bits, 30 of them the
+// widest mer's.  Up to that, chunks of GSCHUNK slots: the host pass of one
+// chunk runs beside the device pass of the next.
+constexpr uint64_t kGsSlots = 1ull << 24;
+constexpr size_t kGsGaps = 1u << (kPairMaxBits - 30);
+
+// Host plan (gaps already validated): seed weights, word and slot ranges of
+// the gaps that are searched, in chunks.
+static int gs_plan(const int64_t* gaps, uint64_t ngaps, uint64_t total_slots, std::vector<GsChunk>& chunks) {
+  const uint64_t parts = std::max<uint64_t>(1, (total_slots + kGsSlots - 1) / kGsSlots);
+  const uint64_t share = total_slots / parts + 1;
+  chunks.emplace_back();
+  for (uint64_t g = 0; g < ngaps; ++g) {
     const int64_t* q = gaps + 4 * g;
     const unsigned w = mvg_default_seed_weight((uint64_t)(q[1] + q[3]) / 2);
     if (w < (unsigned)kGsMinWeight) continue;  // the reference returns without searching
     if (w > 15)
       return report_error(MVG_ERR_ARG, "gap of mean length above 5.9 Mbp (seed weight above 15): search it with "
                                        "mvg_pairwise_matches and the rank-0 seed");
+    if (chunks.back().gd.size() >= kGsGaps || (uint64_t)chunks.back().slots[0] + chunks.back().slots[1] >= share)
+      chunks.emplace_back();
+    GsChunk& ch = chunks.back();
     const int L = mvg_seed_length(mvg_get_seed((int)w, 0));
     GapDev d{};
     d.w = (int32_t)w;
@@ -428,9 +381,11 @@ static int gs_plan(const int64_t* gaps, uint64_t g0, uint64_t g1, GsChunk& ch) {
       d.src[s] = (uint64_t)q[2 * s];
       d.len[s] = (uint32_t)len;
       d.word[s] = ch.words[s];
-      d.key[s] = ch.keys[s];
+      d.slot[s] = ch.slots[s];
+      d.cnt[s] = len >= (uint64_t)L ? (uint32_t)(len - L + 1) : 0;
       ch.words[s] += packed_words(len);  // translate32's layout: two zero words after each gap
-      ch.keys[s] += len >= (uint64_t)L ? len - L + 1 : 0;
+      ch.keys[s] += d.cnt[s];
+      if (d.cnt[s]) ch.slots[s] += (d.cnt[s] + 62) & ~31u;
     }
     ch.gd.push_back(d);
     ch.gid.push_back((uint32_t)g);
@@ -438,163 +393,121 @@ static int gs_plan(const int64_t* gaps, uint64_t g0, uint64_t g1, GsChunk& ch) {
   return 0;
 }
 
-// Device pass of one chunk, from packing to the emitted rows, which are
-// copied to the host with the segment tables.  Synchronous.
-static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch) {
+// Device pass of one chunk, from packing to the rows, which are copied to the
+// pinned buffer `buf` with the gaps' first rows.  Synchronous.
+static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch, int buf) {
   const int ng = (int)ch.gd.size();
   if (ng == 0) return 0;
-  const std::vector<GapDev>& gd = ch.gd;
-  const uint64_t* words = ch.words;
-  const uint64_t* keys = ch.keys;
-  std::vector<int64_t>& rows = ch.rows;
-  std::vector<uint32_t>& seg_gap = ch.seg_gap;
-  std::vector<uint32_t>& seg_n = ch.seg_n;
-  const uint64_t nkeys = keys[0] + keys[1];
-  int rc = 0;
-  if (nkeys >= (1ull << 31)) return report_error(MVG_ERR_ARG, "gaps hold more than 2^31 seed positions");
   Workspace& ws = c->ws;
-  GapDev* d_gaps = (GapDev*)ws.get(c, kGsSlot + 0, gd.size() * sizeof(GapDev));
+  const uint64_t* words = ch.words;
+  const uint32_t wa = ch.slots[0] >> 5, wb = ch.slots[1] >> 5;
+  GapDev* d_gaps = (GapDev*)ws.get(c, kGsSlot + 0, ng * sizeof(GapDev));
   uint32_t* pa = (uint32_t*)ws.get(c, kGsSlot + 1, words[0] * 4 + 64);
   uint32_t* pb = (uint32_t*)ws.get(c, kGsSlot + 2, words[1] * 4 + 64);
-  uint64_t* k0 = (uint64_t*)ws.get(c, kGsSlot + 3, nkeys * 8);
-  uint64_t* k1 = (uint64_t*)ws.get(c, kGsSlot + 4, nkeys * 8);
-  uint32_t* v0 = (uint32_t*)ws.get(c, kGsSlot + 5, nkeys * 4);
-  uint32_t* v1 = (uint32_t*)ws.get(c, kGsSlot + 6, nkeys * 4);
-  int gbits = 1;
-  while ((1ll << gbits) < ng) ++gbits;
-  // (seed bits, strand, genome) below the gap index; a seed's bits are its
-  // pattern's selected positions, which for some table entries exceed the
-  // nominal weight (weight 11's rank-0 seed selects 12)
-  int wmax = 0;
-  for (const GapDev& d : gd) wmax = std::max(wmax, __builtin_popcountll(mvg_get_seed((int)d.w, 0)));
-  const int kshift = 2 * wmax + 2;
-  const int64_t ptiles = ((int64_t)nkeys + kPairTile - 1) / kPairTile;
-  uint32_t* sscr = (uint32_t*)ws.get(c, kGsSlot + 7, sort_scratch_words((int64_t)nkeys, std::max(kshift, 16) + gbits) * 4);  // both sorts below
-  uint32_t* tsum = (uint32_t*)ws.get(c, kGsSlot + 8, (ptiles + 4) * 4 + 64);
-  if (!d_gaps || !pa || !pb || !k0 || !k1 || !v0 || !v1 || !sscr || !tsum)
-    return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-  uint32_t* d_npairs = tsum + ptiles + 2;
+  uint32_t* gmap = (uint32_t*)ws.get(c, kGsSlot + 3, ((size_t)wa + wb) * 4 + 64);
+  uint32_t* tab = (uint32_t*)ws.get(c, 38, (size_t)ch.slots[0] * 4 + 64);
+  uint32_t* d_gap_row = (uint32_t*)ws.get(c, kGsSlot + 4, ((size_t)ng + 1) * 4);
+  if (!d_gaps || !pa || !pb || !gmap || !tab || !d_gap_row) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
   stage_mark(c, "gs_pack");
-  MVG_CUDA_TRY(cudaMemcpyAsync(d_gaps, gd.data(), gd.size() * sizeof(GapDev), cudaMemcpyHostToDevice, c->stream));
+  MVG_CUDA_TRY(cudaMemcpyAsync(d_gaps, ch.gd.data(), ng * sizeof(GapDev), cudaMemcpyHostToDevice, c->stream));
   k_gs_pack<<<grid_for(words[0] + words[1], 256), 256, 0, c->stream>>>(d_a, d_b, d_gaps, ng, words[0], words[1],
                                                                         pa, pb, c->d_err);
   c->launches++;
-  if (keys[0] == 0 || keys[1] == 0) {  // no seed in one genome's gaps: no match anywhere
+  if (ch.keys[0] == 0 || ch.keys[1] == 0) {  // no seed in one genome's gaps: no match anywhere
     MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return check_device_error(c);
   }
+  MVG_CUDA_TRY(cudaMemsetAsync(tab, 0xff, (size_t)ch.slots[0] * 4, c->stream));
   stage_mark(c, "gs_keys");
-  k_gs_keys<<<grid_for(nkeys, 256), 256, 0, c->stream>>>(pa, pb, d_gaps, ng, keys[0], keys[1], kshift, k0,
-                                                         v0);
-  c->launches++;
-  stage_mark(c, "gs_seed_sort");
-  int which = sort_pairs<uint64_t>(k0, v0, k1, v1, (int64_t)nkeys, kshift + gbits, sscr, c->stream, &c->launches,
-                                   c->d_err);
-  const uint64_t* sk = which ? k1 : k0;
-  const uint32_t* sv = which ? v1 : v0;
-  stage_mark(c, "gs_pairs");
-  k_pair_count<uint64_t><<<(unsigned)ptiles, 256, 0, c->stream>>>(sk, (int64_t)nkeys, tsum);
-  k_scan_bsums<<<1, 256, 0, c->stream>>>(tsum, ptiles, d_npairs);
-  c->launches += 2;
-  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, d_npairs, 4, cudaMemcpyDeviceToHost, c->stream));
-  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  if ((rc = check_device_error(c))) return rc;
-  const int64_t npairs = (int64_t)(uint32_t)c->h_scalars[0];
-  if (npairs > 0) {
-    Mhe* mhe = (Mhe*)ws.get(c, kGsSlot + 9, npairs * sizeof(Mhe));
-    Mhe* ent = (Mhe*)ws.get(c, kGsSlot + 10, npairs * sizeof(Mhe));
-    uint64_t* bk0 = (uint64_t*)ws.get(c, kGsSlot + 11, npairs * 8);
-    uint64_t* bk1 = (uint64_t*)ws.get(c, kGsSlot + 12, npairs * 8);
-    uint32_t* o0 = (uint32_t*)ws.get(c, kGsSlot + 13, npairs * 4);
-    uint32_t* o1 = (uint32_t*)ws.get(c, kGsSlot + 14, npairs * 4);
-    // per entry: segment flag, segment index; per segment: start, gap, entries, output offset
-    uint32_t* segtab = (uint32_t*)ws.get(c, kGsSlot + 15, (size_t)npairs * 4 * 6 + scan_scratch_words(npairs) * 8 + 256);
-    if (!mhe || !ent || !bk0 || !bk1 || !o0 || !o1 || !segtab)
-      return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-    uint32_t* flag = segtab;
-    uint32_t* sidx = flag + npairs;
-    uint32_t* seg_start = sidx + npairs;
-    uint32_t* d_seg_gap = seg_start + npairs;
-    uint32_t* nent = d_seg_gap + npairs;
-    uint32_t* ooff = nent + npairs;
-    uint32_t* scr = ooff + npairs;
-    uint32_t* totals = scr + scan_scratch_words(npairs) * 2;  // [0] segments, [1] entries, [2] counter
-    k_gs_pair_emit<<<(unsigned)ptiles, 256, 0, c->stream>>>(sk, sv, (int64_t)nkeys, tsum, kshift, d_gaps, mhe, bk0,
-                                                            o0);
-    c->launches++;
-    stage_mark(c, "gs_bucket_sort");
-    which = sort_pairs<uint64_t>(bk0, o0, bk1, o1, npairs, 16 + gbits, sscr, c->stream, &c->launches, c->d_err);
-    const uint64_t* sbk = which ? bk1 : bk0;
-    const uint32_t* sorted = which ? o1 : o0;
-    k_gs_seg_flags<<<grid_for(npairs, 256), 256, 0, c->stream>>>(sbk, npairs, flag);
-    exclusive_scan(flag, sidx, npairs, scr, totals, c->stream, &c->launches);
-    k_gs_seg_fill<<<grid_for(npairs, 256), 256, 0, c->stream>>>(sbk, npairs, flag, sidx, seg_start, d_seg_gap);
-    c->launches += 2;
-    MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, totals, 4, cudaMemcpyDeviceToHost, c->stream));
-    MVG_CUDA_TRY(cudaMemsetAsync(totals + 2, 0, 4, c->stream));
-    MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    const uint32_t nseg = (uint32_t)c->h_scalars[0];
-    int sms = 0;
-    MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    const uint32_t rblocks = std::min<uint32_t>((nseg + 7) / 8, (uint32_t)sms * 8);
-    stage_mark(c, "gs_replay");
-    k_gs_replay<<<rblocks, 256, 0, c->stream>>>(pa, pb, d_gaps, mhe, sorted, seg_start, d_seg_gap, nseg,
-                                                (uint32_t)npairs, ent, nent, totals + 2);
-    stage_mark(c, "gs_emit");
-    exclusive_scan(nent, ooff, nseg, scr, totals + 1, c->stream, &c->launches);
-    MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, totals + 1, 4, cudaMemcpyDeviceToHost, c->stream));
-    MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    const uint64_t nrows = (uint32_t)c->h_scalars[0];
-    int64_t* d_rows = (int64_t*)ws.get(c, kGsSlot + 3, nrows * 24 + 24);  // the key buffer is free again
-    if (!d_rows) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-    k_gs_emit<<<grid_for((uint64_t)nseg * 32, 256), 256, 0, c->stream>>>(ent, seg_start, nent, ooff, nseg, d_rows);
-    c->launches += 2;
-    rows.resize(nrows * 3);
-    seg_gap.resize(nseg);
-    seg_n.resize(nseg);
-    if (nrows) MVG_CUDA_TRY(cudaMemcpyAsync(rows.data(), d_rows, nrows * 24, cudaMemcpyDeviceToHost, c->stream));
-    MVG_CUDA_TRY(cudaMemcpyAsync(seg_gap.data(), d_seg_gap, (size_t)nseg * 4, cudaMemcpyDeviceToHost, c->stream));
-    MVG_CUDA_TRY(cudaMemcpyAsync(seg_n.data(), nent, (size_t)nseg * 4, cudaMemcpyDeviceToHost, c->stream));
-    stage_mark(c, "gs_copy");
-    MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if ((rc = check_device_error(c))) return rc;
+  int gbits = 1;
+  while ((1ll << gbits) < ng) ++gbits;
+  // a seed's bits are its pattern's selected positions, which for some table
+  // entries exceed the nominal weight (weight 11's rank-0 seed selects 12)
+  int wmax = 0;
+  for (const GapDev& d : ch.gd) wmax = std::max(wmax, __builtin_popcountll(mvg_get_seed((int)d.w, 0)));
+  GapSet P{pa, pb, d_gaps, gmap, gmap + wa, {ch.slots[0], ch.slots[1]}, 2 * wmax, nullptr};
+  const int bits = 2 * wmax + gbits;
+  if (bits > kPairMaxBits) return report_error(MVG_ERR_DEVICE, "gap search keys wider than the join's");
+  PairBucketBufs b;
+  int rc = pair_bucket_bufs(c, (uint64_t)ch.slots[0] + ch.slots[1], bits, &b);
+  if (rc) return rc;
+  static bool attr = false;  // once per process: more than 48 KB of dynamic shared memory
+  if (!attr) {
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
+    attr = true;
   }
+  const size_t hsm = (size_t)b.g.nbuckets * 4;
+  k_gs_slots<<<ng, 128, 0, c->stream>>>(d_gaps, gmap, gmap + wa);
+  k_gs_keys<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.counts);
+  pair_bucket_offsets(c, b);
+  stage_mark(c, "gs_scatter");
+  k_gs_scatter<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.offs, b.buf);
+  c->launches += 3;
+  stage_mark(c, "gs_join");
+  pair_bucket_join(c, b, tab);
+  MVG_CUDA_TRY(cudaGetLastError());
+  ComponentResult r;
+  auto room_for = [&](uint64_t rows) {
+    P.out = (int32_t*)ws.get(c, kGsSlot + 5, rows * 12 + 16);
+    return P.out ? 0 : report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  };
+  if ((rc = match_components(c, P, tab, (int64_t)ch.slots[0], 16 + gbits, room_for, &r))) return rc;
+  if (r.rows == 0) return 0;
+  stage_mark(c, "gs_copy");
+  k_gs_gap_rows<<<div_up(ng + 1, 256), 256, 0, c->stream>>>(r.C.key, r.ncomp, r.at, (uint32_t)r.rows, (uint32_t)ng,
+                                                            d_gap_row);
+  c->launches++;
+  const size_t head = (((size_t)ng + 1) * 4 + 255) & ~(size_t)255, need = head + r.rows * sizeof(Anchor);
+  if (c->h_rows_cap[buf] < need) {
+    if (c->h_rows[buf]) cudaFreeHost(c->h_rows[buf]);
+    c->h_rows[buf] = nullptr;
+    c->h_rows_cap[buf] = 0;
+    MVG_CUDA_TRY(cudaMallocHost(&c->h_rows[buf], need + need / 4));
+    c->h_rows_cap[buf] = need + need / 4;
+  }
+  ch.gap_row = (const uint32_t*)c->h_rows[buf];
+  ch.rows = (Anchor*)((uint8_t*)c->h_rows[buf] + head);
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_rows[buf], d_gap_row, ((size_t)ng + 1) * 4, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaMemcpyAsync(ch.rows, P.out, r.rows * sizeof(Anchor), cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return 0;
 }
 
 // Host pass of one chunk: per gap, overlap elimination and length filter,
-// then genome coordinates.  Gaps are independent and their anchor counts
-// differ by orders of magnitude, so host threads claim runs of gaps, each
-// converting, filtering and shifting its gaps' rows in place.
-static void gs_filter(GsChunk& ch) {
+// then the rows in genome coordinates from row `base` of the caller's output
+// on.  Gaps are independent and their anchor counts differ by orders of
+// magnitude, so host threads claim runs of gaps.  Returns the row after the
+// chunk's last.
+static uint64_t gs_filter(GsChunk& ch, int64_t* out, uint64_t cap, uint64_t base) {
   const int ng = (int)ch.gd.size();
-  ch.anc.resize(ch.rows.size() / 3);
-  ch.gap_r.assign(ng + 1, 0);  // rows of searched gap gi: [gap_r[gi], gap_r[gi+1])
-  for (size_t s = 0, r = 0, gi = 0; gi < (size_t)ng; ++gi) {
-    while (s < ch.seg_gap.size() && ch.seg_gap[s] == (uint32_t)gi) r += ch.seg_n[s++];
-    ch.gap_r[gi + 1] = r;
-  }
   ch.nkept.assign(ng, 0);
-  run_claimed(ng, host_threads_for(ch.anc.size()), [&](int gi) {
-    thread_local std::vector<Anchor*> scratch;
-    const size_t r0 = ch.gap_r[gi], r1 = ch.gap_r[gi + 1];
-    for (size_t k = r0; k < r1; ++k)
-      ch.anc[k] = Anchor{{ch.rows[3 * k], ch.rows[3 * k + 1]}, ch.rows[3 * k + 2]};
-    const int64_t k = filter_gap(ch.anc.data() + r0, (int64_t)(r1 - r0), scratch);
-    const GapDev& d = ch.gd[gi];
-    for (int64_t u = 0; u < k; ++u)
-      for (int q = 0; q < 2; ++q) {
-        int64_t& x = ch.anc[r0 + u].s[q];
-        x = x > 0 ? x + (int64_t)d.src[q] : x - (int64_t)d.src[q];
-      }
-    ch.nkept[gi] = k;
+  if (!ch.gap_row) return base;
+  const int nthreads = host_threads_for(ch.gap_row[ng]);
+  run_claimed(ng, nthreads, [&](int gi) {
+    thread_local FilterScratch scratch;
+    ch.nkept[gi] = (uint32_t)filter_gap(ch.rows + ch.gap_row[gi], ch.gap_row[gi + 1] - ch.gap_row[gi], scratch);
   });
+  std::vector<uint64_t> at(ng);
+  for (int gi = 0; gi < ng; ++gi) {
+    at[gi] = base;
+    base += ch.nkept[gi];
+  }
+  run_claimed(ng, nthreads, [&](int gi) {
+    const GapDev& d = ch.gd[gi];
+    for (uint32_t u = 0; u < ch.nkept[gi] && at[gi] + u < cap; ++u) {
+      const Anchor& x = ch.rows[ch.gap_row[gi] + u];
+      int64_t* o = out + 3 * (at[gi] + u);
+      for (int q = 0; q < 2; ++q) o[q] = x.s[q] > 0 ? x.s[q] + (int64_t)d.src[q] : x.s[q] - (int64_t)d.src[q];
+      o[2] = x.len;
+    }
+  });
+  return base;
 }
 
-// Gaps are searched in up to four chunks of about equal sequence: the host
-// pass of one chunk runs on host threads while the device pass of the next
-// runs on the GPU.
+// Gaps are searched in chunks: the host pass of one chunk runs on host
+// threads while the device pass of the next runs on the GPU.
 int gap_anchor_search_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t* d_b, uint64_t nb,
                           const int64_t* gaps, uint64_t ngaps, int64_t* out, uint64_t cap, uint64_t* gap_off,
                           uint64_t* count) {
@@ -603,72 +516,45 @@ int gap_anchor_search_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t
   if (ngaps >= (1ull << 31)) return report_error(MVG_ERR_ARG, "too many gaps");
   int rc = gs_upload_tables(c->device);
   if (rc) return rc;
-  uint64_t total_bases = 0;
+  uint64_t total_slots = 0;
   for (uint64_t g = 0; g < ngaps; ++g) {
     const int64_t* q = gaps + 4 * g;
     if (q[0] < 0 || q[1] < 0 || q[2] < 0 || q[3] < 0 || (uint64_t)(q[0] + q[1]) > na ||
         (uint64_t)(q[2] + q[3]) > nb)
       return report_error(MVG_ERR_RANGE, "gap outside its genome");
     if (q[1] >= (1ll << 31) || q[3] >= (1ll << 31)) return report_error(MVG_ERR_ARG, "gap longer than 2^31-1");
-    total_bases += (uint64_t)(q[1] + q[3]);
+    total_slots += (uint64_t)(q[1] + q[3]) + 62;
   }
-  const int nchunks = (int)std::max<uint64_t>(1, std::min<uint64_t>(4, total_bases / (32ull << 20)));
-  std::vector<uint64_t> bound(nchunks + 1, ngaps);
-  bound[0] = 0;
-  for (uint64_t g = 0, acc = 0, k = 1; g < ngaps && k < (uint64_t)nchunks; ++g) {
-    acc += (uint64_t)(gaps[4 * g + 1] + gaps[4 * g + 3]);
-    if (acc * nchunks >= total_bases * k) bound[k++] = g + 1;
-  }
-  std::vector<GsChunk> chunks(nchunks);
-  std::thread filt;  // the host pass of the previous chunk
+  std::vector<GsChunk> chunks;
+  if ((rc = gs_plan(gaps, ngaps, total_slots, chunks))) return rc;
+  uint64_t total = 0;  // rows of the chunks filtered so far
+  std::thread filt;    // the host pass of the previous chunk
   struct Joiner {
     std::thread& t;
     ~Joiner() {
       if (t.joinable()) t.join();
     }
   } joiner{filt};
-  for (int k = 0; k < nchunks; ++k) {
-    if ((rc = gs_plan(gaps, bound[k], bound[k + 1], chunks[k]))) return rc;
-    if ((rc = gs_device(c, d_a, d_b, chunks[k]))) return rc;
+  for (size_t k = 0; k < chunks.size(); ++k) {
+    if ((rc = gs_device(c, d_a, d_b, chunks[k], (int)(k & 1)))) return rc;
     HostSpan wait(c, "gs_filter_wait");
     if (filt.joinable()) filt.join();
-    filt = std::thread(gs_filter, std::ref(chunks[k]));
-  }
-  {
-    HostSpan wait(c, "gs_filter_wait");
-    filt.join();
+    GsChunk& ch = chunks[k];
+    if (k + 1 < chunks.size())
+      filt = std::thread([&ch, &total, out, cap] { total = gs_filter(ch, out, cap, total); });
+    else
+      total = gs_filter(ch, out, cap, total);
   }
   stage_end(c);
-  std::vector<uint64_t> per_gap(ngaps, 0);
-  uint64_t total = 0;
-  std::vector<std::pair<int, int>> where;  // (chunk, searched gap) in caller order
-  std::vector<uint64_t> obase;             // output row of each searched gap's first survivor
-  for (int k = 0; k < nchunks; ++k)
-    for (size_t gi = 0; gi < chunks[k].gd.size(); ++gi) {
-      const int64_t n = chunks[k].nkept[gi];
-      per_gap[chunks[k].gid[gi]] = (uint64_t)n;
-      where.push_back({k, (int)gi});
-      obase.push_back(total);
-      total += (uint64_t)n;
-    }
   if (gap_off) {
+    std::vector<uint64_t> per_gap(ngaps, 0);
+    for (const GsChunk& ch : chunks)
+      for (size_t gi = 0; gi < ch.gd.size(); ++gi) per_gap[ch.gid[gi]] = ch.nkept[gi];
     gap_off[0] = 0;
     for (uint64_t g = 0; g < ngaps; ++g) gap_off[g + 1] = gap_off[g] + per_gap[g];
   }
   *count = total;
   if (total > cap) return report_error(MVG_ERR_CAPACITY, "anchor output buffer too small");
-  // searched-gap order is the caller's gap order
-  run_claimed((int)where.size(), host_threads_for(total), [&](int i) {
-    const GsChunk& ch = chunks[where[i].first];
-    const int gi = where[i].second;
-    for (int64_t u = 0; u < ch.nkept[gi]; ++u) {
-      const Anchor& x = ch.anc[ch.gap_r[gi] + u];
-      int64_t* o = out + 3 * (obase[i] + (uint64_t)u);
-      o[0] = x.s[0];
-      o[1] = x.s[1];
-      o[2] = x.len;
-    }
-  });
   return 0;
 }
 

@@ -1,9 +1,7 @@
 // Device-side pieces of the seed matcher shared by the genome-pair matcher
 // (match.cu) and the batched gap anchor search (gapsearch.cu): the hash
-// entry, the unique-seed run test and its tile counts, MheCompare /
-// Contains, the reference's lower_bound probe sequence and the warp
-// ExtendMatch.  Included once per translation unit; nothing here has a
-// host-side symbol except the k_pair_count template.
+// entry, the unique-seed run test, MheCompare / Contains and ExtendMatch's
+// walk.
 #pragma once
 #include "mvg_internal.h"
 #include "prim.cuh"
@@ -22,6 +20,13 @@ struct MatchCtx {
   SeedDesc s;
 };
 
+// The same with the seed elsewhere (one of many).
+struct MatchView {
+  const uint32_t* g[2];
+  int64_t n[2];
+  const SeedDesc& s;
+};
+
 // ------------------------------------------------------------------ join
 
 // Both genomes' seeds sorted in one array by (seed bits, strand, genome).  A
@@ -38,29 +43,7 @@ __device__ __forceinline__ bool pair_flag(const K* __restrict__ keys, int64_t n,
   return (k1 >> 2) == cur && ((k0 ^ k1) & 1ull) && (i + 2 == n || ((uint64_t)keys[i + 2] >> 2) != cur);
 }
 
-constexpr int kPairItems = 8;  // consecutive keys per thread
-constexpr int kPairTile = 256 * kPairItems;
-
-// Pass 1: the number of pairs opened in each tile of kPairTile keys.
-template <typename K>
-__global__ void __launch_bounds__(256) k_pair_count(const K* __restrict__ keys, int64_t n, uint32_t* __restrict__ bsum) {
-  const int64_t i0 = (int64_t)blockIdx.x * kPairTile + (int64_t)threadIdx.x * kPairItems;
-  uint32_t c = 0;
-#pragma unroll 4
-  for (int k = 0; k < kPairItems; ++k)
-    if (i0 + k < n) c += pair_flag(keys, n, i0 + k);
-  for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
-  __shared__ uint32_t ws[8];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < 8; ++w) t += ws[w];
-    bsum[blockIdx.x] = t;
-  }
-}
-
-// ------------------------------------------------------- bucket replay
+// ------------------------------------------------------ hash entries
 
 // LM/MatchHashEntry.cpp:164-200 (Contains), two genomes, both present.
 __device__ __forceinline__ bool mhe_contains(const Mhe& c, const Mhe& m) {
@@ -92,24 +75,7 @@ __device__ __forceinline__ bool mhe_less(const Mhe& a, const Mhe& b, int L) {
   return mhe_strict_lt(a, b, L);
 }
 
-// std::lower_bound's bisection: the comparator is not a strict weak order,
-// so the probe sequence decides which entry is tested and is kept exactly.
-__device__ __forceinline__ int64_t lower_bound_mhe(const Mhe* __restrict__ v, int64_t n, const Mhe& x, int L) {
-  int64_t first = 0, len = n;
-  while (len > 0) {
-    int64_t half = len >> 1, mid = first + half;
-    if (mhe_less(v[mid], x, L)) {
-      first = mid + 1;
-      len = len - half - 1;
-    } else {
-      len = half;
-    }
-  }
-  return first;
-}
-
-// ExtendMatch (LM/MatchFinder.h:218-374) for two genomes, executed by a full
-// warp.  The reference cycles through four phases (jump left and right by
+// ExtendMatch (LM/MatchFinder.h:218-374) for two genomes.  The reference cycles through four phases (jump left and right by
 // the seed length until the first mismatching window, then try the L
 // single-base offsets left and right and move to the furthest matching one)
 // and restarts while a single-base phase moves.
@@ -122,26 +88,10 @@ __device__ __forceinline__ int64_t lower_bound_mhe(const Mhe* __restrict__ v, in
 // starts move by exactly those amounts and negative starts stay.  The room
 // a phase has (the genome-end clamp) is likewise C - ML or C' - MR.  So the
 // two sides never interact: each side's total is where its own walk stops.
-// The match bits are filled 1024 displacements at a time into a per-warp
-// ring, and each fill's 32 words are searched for the stop (stop_in_word),
-// one word per lane.  For a same-strand pair a window pair matches iff the
+// The match bits come 32 displacements at a time (ext_word), and each pair of
+// words is searched for the stop (stop_in_word).  For a same-strand pair a window pair matches iff the
 // pattern-selected bases are equal (equal canonical mers with equal strand
 // bits); other pairs use the canonical-mer test itself.
-constexpr int kExtRing = 128;    // words per side: the last 4096 displacements
-constexpr int kExtChunk = 1024;  // displacements per fill (32 per lane)
-
-struct ExtRing {
-  uint32_t w[2][kExtRing];
-};
-
-// 2-bit mask of the pattern's bases in a 64-bit window (base 0 in bits 63:62).
-__device__ __forceinline__ uint64_t pattern_mask64(const SeedDesc& s) {
-  uint64_t m = 0;
-  for (int r = 0; r < s.nruns; ++r)
-    for (int b = 0; b < s.run_len[r]; ++b) m |= 3ull << (62 - 2 * (s.run_start[r] + b));
-  return m;
-}
-
 // Window start (0-based) in genome q of the pair at displacement u from the
 // entry state's edge (st, len), or -1 outside the genome.
 __device__ __forceinline__ int64_t ext_start(int64_t st, int64_t len, int64_t u, int L, int64_t n) {
@@ -199,9 +149,10 @@ __device__ __forceinline__ uint32_t even_bits(uint64_t x) {
 // mask shifted by each selected base of the pattern tells for 32 windows at
 // once whether a selected base differs (about 150 instructions; 32 masked
 // 64-bit comparisons took 400).
-__device__ __forceinline__ uint32_t ext_word(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t U,
-                                             uint64_t pmask) {
+template <class C>  // MatchCtx or MatchView
+__device__ __forceinline__ uint32_t ext_word(const C& c, int64_t st0, int64_t st1, int64_t len, int64_t U) {
   const int L = c.s.L;
+  const uint64_t pmask = c.s.base_mask;
   const bool same = (st0 > 0) == (st1 > 0);
   uint32_t word = 0;
   if (same || c.s.sym) {
@@ -270,17 +221,6 @@ __device__ __forceinline__ uint32_t ext_word(const MatchCtx& c, int64_t st0, int
   return word;
 }
 
-// One warp's fill: match bits of displacements u0 .. u0 + 32 * nlanes - 1
-// into ring words (u0 / 32 + lane) mod RING, lanes below nlanes (no
-// synchronisation).
-template <int RING>
-__device__ __forceinline__ void ext_fill_ring(const MatchCtx& c, int64_t st0, int64_t st1, int64_t len, int64_t u0,
-                                              uint64_t pmask, uint32_t* ring, int nlanes = 32) {
-  const int lane = threadIdx.x & 31;
-  if (lane >= nlanes) return;
-  ring[((u0 >> 5) + lane) & (RING - 1)] = ext_word(c, st0, st1, len, u0 + lane * 32, pmask);
-}
-
 // Where a side's walk stops.  On one side of the entry the walk starts at
 // displacement 0 and, with bit(u) = "the window pair at displacement u
 // matches" (0 beyond the genome ends), jumps by L while the window L further
@@ -301,51 +241,6 @@ __device__ __forceinline__ uint32_t stop_in_word(uint32_t w, uint32_t w_next, bo
     have += sh;
   }
   return (w | (first ? 1u : 0u)) & (uint32_t)(y >> 1);
-}
-
-static __device__ void warp_extend(const MatchCtx& c, Mhe& m, ExtRing& R) {
-  const int lane = threadIdx.x & 31;
-  const int L = c.s.L;
-  const uint64_t pmask = pattern_mask64(c.s);
-  const int64_t e0 = m.s0, e1 = m.s1, elen = m.len;  // entry state S0
-  int64_t moved[2] = {0, 0};                          // ML, MR
-#pragma unroll 1
-  for (int sd = 0; sd < 2; ++sd) {
-    const int64_t sg = sd == 0 ? 1 : -1;
-    const int64_t s0 = sg * e0, s1 = sg * e1;
-    // room of this side: min over both genomes of the distance to the end
-    const int64_t r0 = s0 > 0 ? s0 - 1 : (s0 < 0 ? c.n[0] - elen + s0 + 1 : -1);
-    const int64_t r1 = s1 > 0 ? s1 - 1 : (s1 < 0 ? c.n[1] - elen + s1 + 1 : -1);
-    const int64_t room = r0 < r1 ? r0 : r1;
-    uint32_t* ring = R.w[sd];
-    int64_t filled = 0, checked = 0;  // displacements filled, words checked
-    for (int k = 0;; ++k) {
-      // most matches stop within a few windows: the first fill is 256 displacements
-      const int nlanes = k == 0 ? 8 : 32;
-      ext_fill_ring<kExtRing>(c, s0, s1, elen, filled, pmask, ring, nlanes);
-      __syncwarp();
-      filled += 32 * nlanes;
-      const int64_t last = filled / 32 - 1;  // words below it have their successor filled
-      const int64_t i = checked + lane;
-      uint32_t hit = 0;
-      if (i < last) hit = stop_in_word(ring[i & (kExtRing - 1)], ring[(i + 1) & (kExtRing - 1)], i == 0, L);
-      const unsigned any = __ballot_sync(0xffffffffu, hit != 0);
-      if (any) {
-        const int f = __ffs(any) - 1;  // the lowest word with a stop holds the first one
-        const uint32_t h = __shfl_sync(0xffffffffu, hit, f);
-        moved[sd] = 32 * (checked + f) + (__ffs(h) - 1);
-        break;
-      }
-      checked = last;
-      if (filled > room + 2 * kExtChunk + 64) {  // never reached: the bits beyond the room are clear
-        moved[sd] = room > 0 ? room : 0;
-        break;
-      }
-    }
-  }
-  m.len = elen + moved[0] + moved[1];
-  m.s0 = e0 > 0 ? e0 - moved[0] : e0 + moved[1];
-  m.s1 = e1 > 0 ? e1 - moved[0] : e1 + moved[1];
 }
 
 }  // namespace mvg

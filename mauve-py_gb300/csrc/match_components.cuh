@@ -34,6 +34,8 @@
 // seeds), two walks per segment on eight lanes each, and a compaction.  The
 // walks bound it: about 1,000 instructions for a group of eight lanes.
 #pragma once
+#include <algorithm>
+
 #include "match_common.cuh"
 
 namespace mvg {
@@ -72,10 +74,37 @@ __device__ __forceinline__ Mhe diag_entry(uint64_t d, uint32_t lo, uint32_t hi, 
   return m;
 }
 
-// ------------------------------------------------------------ pair table
+// What the kernels below ask of a matching problem P, by A position x (and
+// the table's value v there):
+//   seed_len(x)   the seed's length
+//   key(v, x)     sort key: the hash bucket (below the gap's number)
+//   view(x, a, b) packed sequences, lengths and seed, and the positions at
+//                 which they start among A's and B's
+//   row(...)      writes the entry of windows [lo, hi] on diagonal d as row at
+//   mer_bits()    width of the widest mer (host)
+// One genome pair: positions are the genomes'.
+struct OnePair {
+  MatchCtx c;
+  int64_t* out;
+  uint64_t cap;
+  int mer_bits() const { return 2 * c.s.w; }
+  __device__ __forceinline__ int seed_len(uint32_t) const { return c.s.L; }
+  __device__ __forceinline__ uint32_t key(uint32_t v, uint32_t x) const { return diag_bucket(seed_diag(v, x), c.s.L); }
+  __device__ __forceinline__ MatchView view(uint32_t, uint32_t& a, uint32_t& b) const {
+    a = b = 0;
+    return MatchView{{c.g[0], c.g[1]}, {c.n[0], c.n[1]}, c.s};
+  }
+  __device__ __forceinline__ void row(uint64_t d, uint32_t lo, uint32_t hi, uint64_t at) const {
+    if (at >= cap) return;
+    const Mhe m = diag_entry(d, lo, hi, c.s.L);
+    out[3 * at + 0] = m.s0;
+    out[3 * at + 1] = m.s1;
+    out[3 * at + 2] = m.len;
+  }
+};
 
-// From the joint sort (the bucketed join of pair_buckets.cu writes the table
-// itself): runs of exactly one key per genome.
+// The pair table from a joint sort of both genomes' keys (the bucketed join of
+// pair_buckets.cu writes it itself): runs of exactly one key per genome.
 template <typename K>
 __global__ void k_tab_runs(const K* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n,
                            uint32_t* __restrict__ tab) {
@@ -92,7 +121,8 @@ __global__ void k_tab_runs(const K* __restrict__ keys, const uint32_t* __restric
 // Segment heads (no pair of the diagonal in the L positions before) and
 // tails as bit masks over A's positions; per tile their counts (heads of all
 // tiles, then tails), and the number of pairs.
-__global__ void __launch_bounds__(256) k_seg_bits(const uint32_t* __restrict__ tab, int64_t n, int L,
+template <class P>
+__global__ void __launch_bounds__(256) k_seg_bits(P prob, const uint32_t* __restrict__ tab, int64_t n,
                                                   uint32_t* __restrict__ headw, uint32_t* __restrict__ tailw,
                                                   uint32_t* __restrict__ tcount, int64_t ntiles,
                                                   uint32_t* __restrict__ npairs) {
@@ -112,6 +142,7 @@ __global__ void __launch_bounds__(256) k_seg_bits(const uint32_t* __restrict__ t
     const uint32_t v = s[i];
     bool head = v != kNoSeed, tail = head;
     if (head) {
+      const int L = prob.seed_len((uint32_t)(base + i - 32));
       // along the diagonal B moves with A or against it; a value that wraps
       // is no pair's, but can be the empty table's (B position -1)
       const uint32_t back = v >> 31 ? 1u : 0xffffffffu;
@@ -146,10 +177,12 @@ __global__ void __launch_bounds__(256) k_seg_bits(const uint32_t* __restrict__ t
 
 // The ends in order of their A positions, heads then tails: key = bucket
 // (tails behind all heads), value = position.  toff: the scanned counts.
-__global__ void __launch_bounds__(128) k_seg_emit(const uint32_t* __restrict__ tab, int L,
+template <class P>
+__global__ void __launch_bounds__(128) k_seg_emit(P prob, const uint32_t* __restrict__ tab,
                                                   const uint32_t* __restrict__ headw, const uint32_t* __restrict__ tailw,
                                                   const uint32_t* __restrict__ toff, int64_t ntiles,
-                                                  uint32_t* __restrict__ key, uint32_t* __restrict__ val) {
+                                                  int tail_bit, uint32_t* __restrict__ key,
+                                                  uint32_t* __restrict__ val) {
   constexpr int kWords = kSegTile / 32;
   static_assert(kWords == 64, "two warps of head words, two of tail words");
   __shared__ uint32_t wsum[4];
@@ -164,7 +197,7 @@ __global__ void __launch_bounds__(128) k_seg_emit(const uint32_t* __restrict__ t
   while (bits) {
     const uint32_t x = (uint32_t)(w * 32) + (uint32_t)(__ffs(bits) - 1);
     bits &= bits - 1;
-    key[at] = diag_bucket(seed_diag(tab[x], x), L) + (tails ? kTableSize : 0);
+    key[at] = prob.key(tab[x], x) | (tails ? 1u << tail_bit : 0u);
     val[at++] = x;
   }
 }
@@ -172,7 +205,7 @@ __global__ void __launch_bounds__(128) k_seg_emit(const uint32_t* __restrict__ t
 // Sorted by bucket, a bucket's heads and tails have the same indices.  The
 // tail of head k is the first one at or behind it on its diagonal: index k
 // unless segments of the bucket interleave.
-__global__ void k_seg_pair(const uint32_t* __restrict__ tab, const uint32_t* __restrict__ head,
+static __global__ void k_seg_pair(const uint32_t* __restrict__ tab, const uint32_t* __restrict__ head,
                            const uint32_t* __restrict__ tkey, const uint32_t* __restrict__ tail, int64_t n,
                            uint32_t* __restrict__ last) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -192,13 +225,14 @@ __global__ void k_seg_pair(const uint32_t* __restrict__ tab, const uint32_t* __r
 // towards a neighbouring segment of the same bucket and diagonal stops when
 // it gets there.  Out: moved[task], and for the first n joined[k] (segment k
 // is connected to segment k + 1).
-__global__ void __launch_bounds__(256) k_seg_walk(MatchCtx c, const uint32_t* __restrict__ tab,
+template <class P>
+__global__ void __launch_bounds__(256) k_seg_walk(P prob, const uint32_t* __restrict__ tab,
                                                   const uint32_t* __restrict__ key, const uint32_t* __restrict__ head,
                                                   const uint32_t* __restrict__ last, int64_t n,
                                                   uint32_t* __restrict__ moved, uint8_t* __restrict__ joined) {
   const int64_t task = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   if (task >= 2 * n) return;
-  const int lane = threadIdx.x & 31, j = lane & 7, L = c.s.L;
+  const int lane = threadIdx.x & 31, j = lane & 7;
   const unsigned group = 0xffu << (lane & 24);
   const bool up = task < n;
   const int64_t k = up ? task : task - n;
@@ -210,13 +244,15 @@ __global__ void __launch_bounds__(256) k_seg_walk(MatchCtx c, const uint32_t* __
     limit = (int64_t)head[k + 1] - x;
   if (!up && k > 0 && key[k - 1] == key[k] && seed_diag(tab[last[k - 1]], last[k - 1]) == d)
     limit = (int64_t)x - last[k - 1];
-  const int64_t e1 = (int64_t)(v & 0x7fffffffu) + 1;
-  const int64_t s0 = up ? -((int64_t)x + 1) : (int64_t)x + 1;
+  uint32_t a0, b0;
+  const MatchView c = prob.view(x, a0, b0);
+  const int L = c.s.L;
+  const int64_t e0 = (int64_t)(x - a0) + 1, e1 = (int64_t)((v & 0x7fffffffu) - b0) + 1;
+  const int64_t s0 = up ? -e0 : e0;
   const int64_t s1 = (v >> 31 != 0) != up ? -e1 : e1;
-  const uint64_t pmask = pattern_mask64(c.s);
   uint32_t carry = 0;
   for (int64_t it = 0;; ++it) {
-    const uint32_t w = ext_word(c, s0, s1, L, (it * 8 + j) * 32, pmask);
+    const uint32_t w = ext_word(c, s0, s1, L, (it * 8 + j) * 32);
     uint32_t prev = __shfl_up_sync(group, w, 1, 8);
     if (j == 0) prev = carry;
     const int64_t idx = it * 8 + j - 1;  // the word whose successor is w
@@ -248,13 +284,13 @@ struct Components {
   uint32_t* lo;      // first window (A start)
   uint32_t* hi;      // last window
   uint32_t* seed;    // last seed
-  uint32_t* bucket;
+  uint32_t* key;     // its bucket's sort key
   uint64_t* diag;
   uint32_t* copies;  // entries the bucket holds of it
   uint64_t* time;    // flagged buckets: the component's smallest mer
 };
 
-__global__ void __launch_bounds__(256) k_comp_count(const uint8_t* __restrict__ joined, int64_t n,
+static __global__ void __launch_bounds__(256) k_comp_count(const uint8_t* __restrict__ joined, int64_t n,
                                                     uint32_t* __restrict__ tcount) {
   const int64_t i0 = (int64_t)blockIdx.x * kSegTile + (int64_t)threadIdx.x * 8;
   uint32_t cnt = 0, total;
@@ -276,7 +312,7 @@ __global__ void __launch_bounds__(256) k_comp_count(const uint8_t* __restrict__ 
 
 // Components from segments: the first one's head and downward walk, the last
 // one's tail and upward walk.
-__global__ void __launch_bounds__(256) k_comp_emit(const uint32_t* __restrict__ tab, const uint32_t* __restrict__ key,
+static __global__ void __launch_bounds__(256) k_comp_emit(const uint32_t* __restrict__ tab, const uint32_t* __restrict__ key,
                                                    const uint32_t* __restrict__ head, const uint32_t* __restrict__ last,
                                                    const uint32_t* __restrict__ moved, const uint8_t* __restrict__ joined,
                                                    int64_t n, const uint32_t* __restrict__ toff, Components C) {
@@ -294,7 +330,7 @@ __global__ void __launch_bounds__(256) k_comp_emit(const uint32_t* __restrict__ 
       const uint32_t x = head[k];
       C.lo[id] = x - moved[n + k];
       C.diag[id] = seed_diag(tab[x], x);
-      C.bucket[id] = key[k];
+      C.key[id] = key[k];
       C.copies[id] = 1;
       ++id;
     }
@@ -305,26 +341,28 @@ __global__ void __launch_bounds__(256) k_comp_emit(const uint32_t* __restrict__ 
   }
 }
 
-__device__ __forceinline__ void comp_row(const Components& C, uint32_t e, int L, int64_t* __restrict__ out, uint64_t at,
-                                         uint64_t cap) {
-  if (at >= cap) return;
-  const Mhe m = diag_entry(C.diag[e], C.lo[e], C.hi[e], L);
-  out[3 * at + 0] = m.s0;
-  out[3 * at + 1] = m.s1;
-  out[3 * at + 2] = m.len;
-}
-
 // The match list when no bucket is flagged (GetMatchList order: buckets, then
 // their entries, LM/MemHash.h:182-203), and the list of flagged buckets.
-__global__ void k_comp_out(Components C, const uint32_t* __restrict__ ncomp, int L, int64_t* __restrict__ out,
-                           uint64_t cap, uint32_t* __restrict__ bflag, uint32_t* __restrict__ flagged,
-                           uint32_t* __restrict__ nflagged) {
+template <class P>
+__global__ void k_comp_out(P prob, Components C, const uint32_t* __restrict__ ncomp, uint32_t* __restrict__ bflag,
+                           uint32_t* __restrict__ flagged, uint32_t* __restrict__ nflagged) {
   const uint32_t n = *ncomp;
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    comp_row(C, e, L, out, e, cap);
-    if (e + 1 < n && C.bucket[e] == C.bucket[e + 1] && C.lo[e + 1] <= C.seed[e] &&
-        atomicExch(&bflag[C.bucket[e]], 1u) == 0u)
-      flagged[atomicAdd(nflagged, 1u)] = C.bucket[e];
+    prob.row(C.diag[e], C.lo[e], C.hi[e], e);
+    if (e + 1 < n && C.key[e] == C.key[e + 1] && C.lo[e + 1] <= C.seed[e]) {
+      // the bucket's flag is the word of its first component
+      uint32_t lo = 0, len = e;
+      while (len > 0) {
+        const uint32_t half = len >> 1;
+        if (C.key[lo + half] < C.key[e]) {
+          lo += half + 1;
+          len -= half + 1;
+        } else {
+          len = half;
+        }
+      }
+      if (atomicExch(&bflag[lo], 1u) == 0u) flagged[atomicAdd(nflagged, 1u)] = C.key[e];
+    }
   }
 }
 
@@ -337,7 +375,7 @@ __device__ __forceinline__ void comp_range(const Components& C, uint32_t n, uint
     uint32_t lo = 0, len = n;
     while (len > 0) {
       const uint32_t half = len >> 1;
-      if (C.bucket[lo + half] < b + q) {
+      if (C.key[lo + half] < b + q) {
         lo += half + 1;
         len -= half + 1;
       } else {
@@ -353,11 +391,13 @@ __device__ __forceinline__ void comp_range(const Components& C, uint32_t n, uint
 // One CTA per flagged bucket: its components in entry order (they nearly are:
 // exchanges of neighbours until nothing moves), a component found from
 // several of its segments kept once.
-__global__ void __launch_bounds__(256) k_flag_sort(Components C, uint32_t n, int L, const uint32_t* __restrict__ flagged) {
+template <class P>
+__global__ void __launch_bounds__(256) k_flag_sort(P prob, Components C, uint32_t n, const uint32_t* __restrict__ flagged) {
   __shared__ uint32_t range[2];
   if (threadIdx.x == 0) comp_range(C, n, flagged[blockIdx.x], range[0], range[1]);
   __syncthreads();
   const uint32_t first = range[0], end = range[1];
+  const int L = prob.seed_len(C.lo[first]);
   for (bool again = true; again;) {
     bool moved = false;
     for (uint32_t parity = 0; parity < 2; ++parity) {
@@ -395,37 +435,46 @@ __global__ void __launch_bounds__(256) k_flag_sort(Components C, uint32_t n, int
 }
 
 // Mer of A's window at x as the reference orders seeds.
-__device__ __forceinline__ uint64_t seed_time(const MatchCtx& c, uint32_t x) {
-  return (canonical_mer(c.g[0], x, c.s) & c.s.seed_mask) >> (64 - 2 * c.s.w);
+template <class P>
+__device__ __forceinline__ uint64_t seed_time(const P& prob, uint32_t x) {
+  uint32_t a0, b0;
+  const MatchView c = prob.view(x, a0, b0);
+  return (canonical_mer(c.g[0], x - a0, c.s) & c.s.seed_mask) >> (64 - 2 * c.s.w);
 }
 
 // Work on the seeds of flagged buckets' components in pieces of kFlagPiece
-// positions: (component, first position).
+// positions: component, first position, the bucket's number in the list.
 constexpr uint32_t kFlagPiece = 1024;
 struct FlagWork {
   uint32_t* count;  // [0] pieces of whole components, [1] pieces of their seeds behind the next component's start
-  uint2* whole;     // null: count only
-  uint2* behind;
+  uint4* whole;     // null: count only
+  uint4* behind;
 };
 
-__global__ void k_flag_plan(Components C, uint32_t n, const uint32_t* __restrict__ bflag, FlagWork W) {
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    if (!bflag[C.bucket[e]] || !C.copies[e]) continue;
+// One CTA per flagged bucket.
+static __global__ void __launch_bounds__(256) k_flag_plan(Components C, uint32_t n, const uint32_t* __restrict__ flagged,
+                                                   FlagWork W) {
+  __shared__ uint32_t range[2];
+  if (threadIdx.x == 0) comp_range(C, n, flagged[blockIdx.x], range[0], range[1]);
+  __syncthreads();
+  for (uint32_t e = range[0] + threadIdx.x; e < range[1]; e += 256) {
+    if (!C.copies[e]) continue;
     uint32_t f = e + 1;
-    while (f < n && C.bucket[f] == C.bucket[e] && !C.copies[f]) ++f;
-    const bool over = f < n && C.bucket[f] == C.bucket[e] && C.lo[f] <= C.seed[e];
+    while (f < range[1] && !C.copies[f]) ++f;
+    const bool over = f < range[1] && C.lo[f] <= C.seed[e];
     for (int list = 0; list < (over ? 2 : 1); ++list) {
       const uint32_t x0 = list ? max(C.lo[f], C.lo[e]) : C.lo[e];
       const uint32_t pieces = (C.seed[e] - x0) / kFlagPiece + 1;
       const uint32_t at = atomicAdd(&W.count[list], pieces);
-      uint2* out = list ? W.behind : W.whole;
-      for (uint32_t q = 0; out && q < pieces; ++q) out[at + q] = make_uint2(e, x0 + q * kFlagPiece);
+      uint4* out = list ? W.behind : W.whole;
+      for (uint32_t q = 0; out && q < pieces; ++q) out[at + q] = make_uint4(e, x0 + q * kFlagPiece, blockIdx.x, 0u);
     }
   }
 }
 
 // Every component's smallest mer (a warp per piece).
-__global__ void k_flag_time(MatchCtx c, const uint32_t* __restrict__ tab, Components C, const uint2* __restrict__ work,
+template <class P>
+__global__ void k_flag_time(P prob, const uint32_t* __restrict__ tab, Components C, const uint4* __restrict__ work,
                             uint32_t pieces) {
   const int lane = threadIdx.x & 31;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -434,20 +483,21 @@ __global__ void k_flag_time(MatchCtx c, const uint32_t* __restrict__ tab, Compon
   const uint64_t d = C.diag[e];
   unsigned long long t = ~0ull;
   for (uint32_t x = x0 + lane; x <= x1; x += 32)
-    if (tab[x] == diag_seed(d, x)) t = min(t, (unsigned long long)seed_time(c, x));
+    if (tab[x] == diag_seed(d, x)) t = min(t, (unsigned long long)seed_time(prob, x));
   for (int s = 16; s > 0; s >>= 1) t = min(t, __shfl_xor_sync(0xffffffffu, t, s));
   if (lane == 0 && t != ~0ull) atomicMin((unsigned long long*)&C.time[e], t);
 }
 
-// The seeds behind the start of a component after their own: mer, position
-// and component, in any order (a warp per piece).
+// The seeds behind the start of a component after their own: mer, position,
+// component and bucket, in any order (a warp per piece).
 struct FlagSeeds {
   uint64_t* time;
-  uint32_t *x, *e;
+  uint32_t *x, *e, *number;
   uint32_t* id;     // 0, 1, ...
   uint32_t* count;
 };
-__global__ void k_flag_collect(MatchCtx c, const uint32_t* __restrict__ tab, Components C, const uint2* __restrict__ work,
+template <class P>
+__global__ void k_flag_collect(P prob, const uint32_t* __restrict__ tab, Components C, const uint4* __restrict__ work,
                                uint32_t pieces, FlagSeeds S) {
   const int lane = threadIdx.x & 31;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -459,7 +509,7 @@ __global__ void k_flag_collect(MatchCtx c, const uint32_t* __restrict__ tab, Com
     bool in = x <= x1 && tab[x] == diag_seed(d, x);
     uint64_t t = 0;
     if (in) {
-      t = seed_time(c, x);
+      t = seed_time(prob, x);
       in = t != t0;  // the component's first seed finds no entry
     }
     const unsigned all = __ballot_sync(0xffffffffu, in);
@@ -471,22 +521,16 @@ __global__ void k_flag_collect(MatchCtx c, const uint32_t* __restrict__ tab, Com
       S.time[at] = t;
       S.x[at] = x;
       S.e[at] = e;
+      S.number[at] = work[w].z;
       S.id[at] = at;
     }
   }
 }
 
-// The seeds' flagged-bucket numbers, in the order of ids (sorted by mer).
-__global__ void k_flag_bucket(Components C, const uint32_t* __restrict__ e, const uint32_t* __restrict__ id, uint32_t n,
-                              const uint32_t* __restrict__ bnumber, uint32_t* __restrict__ number) {
+// The seeds' bucket numbers in the order of ids (sorted by mer).
+static __global__ void k_flag_number(FlagSeeds S, const uint32_t* __restrict__ id, uint32_t n, uint32_t* __restrict__ number) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) number[i] = bnumber[C.bucket[e[id[i]]]];
-}
-
-// The flagged buckets' numbers in the list.
-__global__ void k_flag_numbers(const uint32_t* __restrict__ flagged, uint32_t n, uint32_t* __restrict__ bnumber) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) bnumber[flagged[i]] = i;
+  if (i < n) number[i] = S.number[id[i]];
 }
 
 // One CTA per flagged bucket tests its seeds in mer order, 1024 at a time
@@ -496,7 +540,8 @@ __global__ void k_flag_numbers(const uint32_t* __restrict__ flagged, uint32_t n,
 // of e, which contain it, b that start between e's start and the seed's and
 // are less, and the rest, which are not.  So lower_bound's bisection needs
 // only p, c, b and the number of all.
-__global__ void __launch_bounds__(1024) k_flag_test(Components C, uint32_t n, int L, const uint32_t* __restrict__ flagged,
+template <class P>
+__global__ void __launch_bounds__(1024) k_flag_test(P prob, Components C, uint32_t n, const uint32_t* __restrict__ flagged,
                                                     const uint32_t* __restrict__ number, const uint32_t* __restrict__ id,
                                                     uint32_t nseeds, FlagSeeds S) {
   __shared__ uint32_t range[4];
@@ -518,6 +563,7 @@ __global__ void __launch_bounds__(1024) k_flag_test(Components C, uint32_t n, in
   }
   __syncthreads();
   const uint32_t first = range[0], end = range[1], send = range[3];
+  const int L = prob.seed_len(C.lo[first]);
   for (uint32_t pos = range[2]; pos < send;) {
     bool missed = false;
     if (pos + tid < send) {
@@ -559,10 +605,182 @@ __global__ void __launch_bounds__(1024) k_flag_test(Components C, uint32_t n, in
 }
 
 // The match list with copies: at = exclusive sums of copies.
-__global__ void k_comp_out_copies(Components C, uint32_t n, const uint32_t* __restrict__ at, int L,
-                                  int64_t* __restrict__ out, uint64_t cap) {
+template <class P>
+__global__ void k_comp_out_copies(P prob, Components C, uint32_t n, const uint32_t* __restrict__ at) {
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
-    for (uint32_t q = 0; q < C.copies[e]; ++q) comp_row(C, e, L, out, (uint64_t)at[e] + q, cap);
+    for (uint32_t q = 0; q < C.copies[e]; ++q) prob.row(C.diag[e], C.lo[e], C.hi[e], (uint64_t)at[e] + q);
+}
+
+// ------------------------------------------------------------------ host
+
+// Exclusive scan of n counts and their sum: one launch where it fits.
+static void scan_counts(const uint32_t* in, int64_t n, uint32_t* out, uint32_t* scratch, uint32_t* total,
+                        cudaStream_t st, uint64_t* launches) {
+  if (n <= 16384) {
+    pair_scan_small(in, (int)n, out, total, st);
+    *launches += 1;
+  } else {
+    exclusive_scan(in, out, n, scratch, total, st, launches);
+  }
+}
+
+struct ComponentResult {
+  Components C;
+  uint32_t ncomp = 0;
+  uint64_t pairs = 0, rows = 0;
+  const uint32_t* at = nullptr;  // rows before each component (null: its index)
+};
+
+// The buckets k_comp_out flagged, exactly, and the rows again.
+template <class P, class F>
+int flagged_components(Ctx* c, P& prob, const uint32_t* tab, const uint32_t* flagged, uint32_t nflagged, F room_for,
+                       ComponentResult* out) {
+  const Components& C = out->C;
+  const uint32_t ncomp = out->ncomp;
+  Workspace& ws = c->ws;
+  // work and seed counts, sums, all components' first rows, scan scratch
+  uint32_t* w = (uint32_t*)ws.get(c, 37, ((size_t)ncomp + scan_scratch_words(ncomp) + 16) * 4);
+  if (!w) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  uint32_t *count = w, *cat = w + 16, *scratch = cat + ncomp;
+  MVG_CUDA_TRY(cudaMemsetAsync(count, 0, 64, c->stream));
+  k_flag_sort<<<nflagged, 256, 0, c->stream>>>(prob, C, ncomp, flagged);
+  FlagWork W{count, nullptr, nullptr};
+  k_flag_plan<<<nflagged, 256, 0, c->stream>>>(C, ncomp, flagged, W);
+  c->launches += 2;
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, count, 8, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  const uint32_t whole = ((const uint32_t*)c->h_scalars)[0], behind = ((const uint32_t*)c->h_scalars)[1];
+  // the pieces, and room for every position of the seeds' pieces
+  const size_t room = (size_t)behind * kFlagPiece;
+  W.whole = (uint4*)ws.get(c, 39, ((size_t)whole + behind) * 16 + 16);
+  uint64_t* t0 = (uint64_t*)ws.get(c, 40, room * 8 + 16);
+  uint64_t* t1 = (uint64_t*)ws.get(c, 41, room * 8 + 16);
+  uint32_t* u = (uint32_t*)ws.get(c, 42, room * 4 * 5 + 16);
+  uint32_t* sscr = (uint32_t*)ws.get(c, 43, sort_scratch_words((int64_t)room, 64) * 4);
+  if (!W.whole || !t0 || !t1 || !u || !sscr) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  W.behind = W.whole + whole;
+  W.count = count + 2;
+  FlagSeeds S{t0, u, u + room, u + 2 * room, u + 3 * room, count + 4};
+  k_flag_plan<<<nflagged, 256, 0, c->stream>>>(C, ncomp, flagged, W);
+  k_flag_time<<<div_up((int64_t)whole * 32, 256), 256, 0, c->stream>>>(prob, tab, C, W.whole, whole);
+  c->launches += 2;
+  if (behind) {
+    k_flag_collect<<<div_up((int64_t)behind * 32, 256), 256, 0, c->stream>>>(prob, tab, C, W.behind, behind, S);
+    c->launches++;
+  }
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, count + 4, 4, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  const uint32_t nseeds = ((const uint32_t*)c->h_scalars)[0];
+  if (nseeds) {
+    // by mer, then stably by bucket; the mers stay where they are for the tests
+    uint64_t* keys = (uint64_t*)ws.get(c, 48, (size_t)nseeds * 8);
+    if (!keys) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+    MVG_CUDA_TRY(cudaMemcpyAsync(keys, t0, (size_t)nseeds * 8, cudaMemcpyDeviceToDevice, c->stream));
+    uint32_t *id = S.id, *id_alt = u + 4 * room;
+    if (sort_pairs<uint64_t>(keys, id, t1, id_alt, nseeds, prob.mer_bits(), sscr, c->stream, &c->launches, c->d_err))
+      std::swap(id, id_alt);
+    uint32_t *number = (uint32_t*)keys, *number_alt = (uint32_t*)t1;
+    k_flag_number<<<div_up(nseeds, 256), 256, 0, c->stream>>>(S, id, nseeds, number);
+    int bits = 1;
+    while ((1u << bits) < nflagged) ++bits;
+    if (sort_pairs<uint32_t>(number, id, number_alt, id_alt, nseeds, bits, sscr, c->stream, &c->launches, c->d_err)) {
+      std::swap(number, number_alt);
+      std::swap(id, id_alt);
+    }
+    k_flag_test<<<nflagged, 1024, 0, c->stream>>>(prob, C, ncomp, flagged, number, id, nseeds, S);
+    c->launches += 2;
+  }
+  exclusive_scan(C.copies, cat, ncomp, scratch, count + 5, c->stream, &c->launches);
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, count + 5, 4, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  out->rows = ((const uint32_t*)c->h_scalars)[0];
+  out->at = cat;
+  if (int rc = room_for(out->rows)) return rc;
+  k_comp_out_copies<<<grid_for(ncomp, 256), 256, 0, c->stream>>>(prob, C, ncomp, cat);
+  c->launches++;
+  MVG_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
+// The match list of the pairs in tab (n A positions): rows through prob.row,
+// in order of buckets and of the entries in them.  key_bits: width of
+// prob.key; room_for(rows) is called before rows are written.  Waits for the
+// stream twice (three times more with flagged buckets); the rows' kernel may
+// still be running on return.
+template <class P, class F>
+int match_components(Ctx* c, P& prob, const uint32_t* tab, int64_t n, int key_bits, F room_for, ComponentResult* out) {
+  Workspace& ws = c->ws;
+  const int64_t ntiles = div_up(n, kSegTile);
+  uint32_t* masks = (uint32_t*)ws.get(c, 39, (size_t)ntiles * (kSegTile / 32) * 2 * 4);
+  // head and tail counts per tile, their offsets, scan scratch
+  uint32_t* tcount = (uint32_t*)ws.get(c, 44, ((size_t)ntiles * 4 + scan_scratch_words(2 * ntiles) + 16) * 4);
+  uint32_t* scal = (uint32_t*)ws.get(c, 34, 64);  // segment ends, pairs, components, flagged buckets
+  if (!masks || !tcount || !scal) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  uint32_t *headw = masks, *tailw = masks + ntiles * (kSegTile / 32);
+  uint32_t *toff = tcount + 2 * ntiles, *tscr = toff + 2 * ntiles;
+  MVG_CUDA_TRY(cudaMemsetAsync(scal, 0, 64, c->stream));
+  stage_mark(c, "segments");
+  k_seg_bits<<<(unsigned)ntiles, 256, 0, c->stream>>>(prob, tab, n, headw, tailw, tcount, ntiles, scal + 1);
+  c->launches++;
+  scan_counts(tcount, 2 * ntiles, toff, tscr, scal, c->stream, &c->launches);
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal, 8, cudaMemcpyDeviceToHost, c->stream));
+  if (int rc = check_device_error(c)) return rc;
+  const int64_t ends = ((const uint32_t*)c->h_scalars)[0], nseg = ends / 2;
+  out->pairs = ((const uint32_t*)c->h_scalars)[1];
+  if (out->pairs == 0) return 0;
+
+  uint32_t* k0 = (uint32_t*)ws.get(c, 40, ends * 4);
+  uint32_t* v0 = (uint32_t*)ws.get(c, 41, ends * 4);
+  uint32_t* k1 = (uint32_t*)ws.get(c, 42, ends * 4);
+  uint32_t* v1 = (uint32_t*)ws.get(c, 48, ends * 4);
+  uint32_t* sscr = (uint32_t*)ws.get(c, 43, sort_scratch_words(ends, key_bits + 1) * 4);
+  // per segment: last position, two walks, the join with the next one; its
+  // tiles' component counts and offsets; per component (at most one per
+  // segment) its fields, its bucket's flag and the list of flagged buckets
+  const int64_t ctiles = div_up(nseg, kSegTile);
+  uint64_t* blk = (uint64_t*)ws.get(
+      c, 45, (size_t)nseg * (8 * 2 + 4 * 7 + 4 * 3 + 1) + (2 * ctiles + scan_scratch_words(ctiles)) * 4 + 256);
+  if (!k0 || !v0 || !k1 || !v1 || !sscr || !blk) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  Components& C = out->C;
+  C.diag = blk;
+  C.time = blk + nseg;
+  uint32_t* w = (uint32_t*)(blk + 2 * nseg);
+  auto take = [&](int64_t k) {
+    uint32_t* p = w;
+    w += k;
+    return p;
+  };
+  C.lo = take(nseg);
+  C.hi = take(nseg);
+  C.seed = take(nseg);
+  C.key = take(nseg);
+  C.copies = take(nseg);
+  uint32_t *bflag = take(nseg), *flagged = take(nseg);
+  uint32_t *last = take(nseg), *moved = take(2 * nseg);
+  uint32_t *ccount = take(ctiles), *coff = take(ctiles), *cscr = take(scan_scratch_words(ctiles));
+  uint8_t* joined = (uint8_t*)w;
+  if (int rc = room_for((uint64_t)nseg)) return rc;
+  k_seg_emit<<<(unsigned)ntiles, 128, 0, c->stream>>>(prob, tab, headw, tailw, toff, ntiles, key_bits, k0, v0);
+  stage_mark(c, "segment_sort");
+  const bool alt = sort_pairs<uint32_t>(k0, v0, k1, v1, ends, key_bits + 1, sscr, c->stream, &c->launches, c->d_err) != 0;
+  const uint32_t *key = alt ? k1 : k0, *head = alt ? v1 : v0, *tail = head + nseg;
+  stage_mark(c, "walks");
+  k_seg_pair<<<div_up(nseg, 256), 256, 0, c->stream>>>(tab, head, key, tail, nseg, last);
+  k_seg_walk<<<div_up(2 * nseg * 8, 256), 256, 0, c->stream>>>(prob, tab, key, head, last, nseg, moved, joined);
+  stage_mark(c, "components");
+  MVG_CUDA_TRY(cudaMemsetAsync(bflag, 0, (size_t)nseg * 4, c->stream));
+  k_comp_count<<<(unsigned)ctiles, 256, 0, c->stream>>>(joined, nseg, ccount);
+  scan_counts(ccount, ctiles, coff, cscr, scal + 2, c->stream, &c->launches);
+  k_comp_emit<<<(unsigned)ctiles, 256, 0, c->stream>>>(tab, key, head, last, moved, joined, nseg, coff, C);
+  k_comp_out<<<grid_for(nseg, 256), 256, 0, c->stream>>>(prob, C, scal + 2, bflag, flagged, scal + 3);
+  c->launches += 6;
+  stage_mark(c, "flagged");
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal + 2, 8, cudaMemcpyDeviceToHost, c->stream));
+  if (int rc = check_device_error(c)) return rc;
+  out->ncomp = ((const uint32_t*)c->h_scalars)[0];
+  out->rows = out->ncomp;
+  const uint32_t nflagged = ((const uint32_t*)c->h_scalars)[1];
+  return nflagged ? flagged_components(c, prob, tab, flagged, nflagged, room_for, out) : 0;
 }
 
 }  // namespace mvg

@@ -33,6 +33,7 @@ __device__ __forceinline__ void set_error(uint32_t* err, uint32_t code) {
 struct SeedDesc {
   uint64_t pattern;
   uint64_t seed_mask;  // top 2w bits
+  uint64_t base_mask;  // the pattern's bases in a 64-bit window (base 0 in bits 63:62)
   int L, w;
   int nruns;
   // the pattern reads the same reversed (every rank-0 seed of weight >= 5
@@ -151,6 +152,14 @@ __device__ __forceinline__ uint32_t gather_mer32(uint64_t win, int u, const uint
   for (int c = 0; c < 8; ++c)
     if (c < nb) f |= lut[c][(uint32_t)(win >> (56 - 8 * c - 2 * u)) & 255u];
   return f;
+}
+
+// A bijection of keys of `bits` bits whose top bits depend on all of the key's.
+template <typename K>
+__device__ __forceinline__ K mix_mer(K m, int bits) {
+  m ^= m >> (bits / 2);
+  m *= (K)0x9E3779B97F4A7C15ull;
+  return m & ((((K)1 << (bits - 1)) << 1) - 1);
 }
 
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }

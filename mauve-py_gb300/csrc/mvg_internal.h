@@ -40,6 +40,8 @@ struct Ctx {
   uint32_t* d_err = nullptr;     // device error word
   uint32_t* h_err = nullptr;     // pinned mirror
   uint64_t* h_scalars = nullptr; // pinned scalars for small device->host reads
+  void* h_rows[2] = {};          // pinned: the gap search's rows of a chunk, filtered while the next is searched
+  size_t h_rows_cap[2] = {};
   uint8_t* h_stage = nullptr;    // pinned staging of one call's host->device copies (bump allocated)
   size_t h_stage_cap = 0, h_stage_used = 0;
   void* h_off = nullptr;         // pinned buffer for gap-DP offsets read back from the device
@@ -141,12 +143,21 @@ int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s
 // unique in both genomes (tab holds ~0 elsewhere).
 constexpr uint64_t kPairBucketMaxKeys = 1ull << 25;
 constexpr int kPairRestBits = 30;                      // mer bits below the bucket's
-constexpr int kPairBucketMaxWeight = (14 + kPairRestBits) / 2;  // with 2^14 buckets
+constexpr int kPairMaxBits = 14 + kPairRestBits;       // with 2^14 buckets
 struct PairBucketGeom {
   int bbits, nbuckets, npass, dbits, lbits;
   int64_t tile, ntiles, nchunks;
 };
-PairBucketGeom pair_bucket_geom(uint64_t n, int w);
+// The parts of it another key source uses (n keys of `bits` bits): buffers,
+// tile offsets from the count rows, the join of the filled buckets.
+struct PairBucketBufs {
+  PairBucketGeom g;
+  uint2 *alt, *buf;
+  uint32_t *counts, *offs, *csum, *bstart, *bsize;
+};
+int pair_bucket_bufs(Ctx* c, uint64_t n, int bits, PairBucketBufs* b);
+void pair_bucket_offsets(Ctx* c, const PairBucketBufs& b);
+void pair_bucket_join(Ctx* c, const PairBucketBufs& b, uint32_t* tab);
 int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
                  uint32_t* tab);
 // Exclusive scan of n <= 16384 counts in one launch; *total gets the sum.

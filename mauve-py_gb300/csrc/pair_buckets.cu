@@ -50,12 +50,12 @@ constexpr int kGroupMax = 256;  // larger groups: the bucket is sorted instead
 constexpr int kChunkTiles = 32;
 }  // namespace pb
 
-PairBucketGeom pair_bucket_geom(uint64_t n, int w) {
+PairBucketGeom pair_bucket_geom(uint64_t n, int bits) {
   PairBucketGeom g;
   int bb = 4;
   while (bb < 14 && ((uint64_t)2048 << bb) < n) ++bb;  // about 2048 keys per bucket at most
-  if (bb < 2 * w - kPairRestBits) bb = 2 * w - kPairRestBits;
-  if (bb > 2 * w) bb = 2 * w;
+  if (bb < bits - kPairRestBits) bb = bits - kPairRestBits;
+  if (bb > bits) bb = bits;
   g.bbits = bb;
   g.nbuckets = 1 << bb;
   g.tile = std::max<int64_t>(16384, 4ll * g.nbuckets);
@@ -63,7 +63,7 @@ PairBucketGeom pair_bucket_geom(uint64_t n, int w) {
   g.nchunks = (g.ntiles + pb::kChunkTiles - 1) / pb::kChunkTiles;
   // in-bucket key: the rest of the mixed mer, then the genome bit; an odd
   // number of passes leaves a sort's result in the scratch copy
-  const int lbits = 2 * w - bb + 1;
+  const int lbits = bits - bb + 1;
   int np = (lbits + 5) / 6;
   if ((np & 1) == 0) ++np;
   g.npass = np;
@@ -73,14 +73,6 @@ PairBucketGeom pair_bucket_geom(uint64_t n, int w) {
 }
 
 // ------------------------------------------------------------------ keys
-
-// A bijection of 2w-bit mers whose top bits depend on all of the mer's.
-template <typename K>
-__device__ __forceinline__ K mix_mer(K m, int w) {
-  m ^= m >> w;
-  m *= (K)0x9E3779B97F4A7C15ull;
-  return m & ((((K)1 << (2 * w - 1)) << 1) - 1);
-}
 
 // Calls f(global index, mixed mer, strand, in B, position) for every position
 // of this block's tile.  K = uint32_t: w <= 15, four positions from one
@@ -108,7 +100,7 @@ __device__ __forceinline__ void pb_tile(const uint32_t* __restrict__ ga, uint64_
         const uint32_t fw = whole ? gather_mer32(win, u, lut, nb) : gather_mer32(window64(in_b ? gb : ga, q), 0, lut, nb);
         const uint32_t r = revcomp_mer32(fw, s.w);
         const uint32_t m = fw < r ? fw : r;
-        f(p, mix_mer<uint32_t>(m >> sh, s.w), m & 1u, in_b, (uint32_t)q);
+        f(p, mix_mer<uint32_t>(m >> sh, 2 * s.w), m & 1u, in_b, (uint32_t)q);
       }
     }
   } else {
@@ -119,7 +111,7 @@ __device__ __forceinline__ void pb_tile(const uint32_t* __restrict__ ga, uint64_
       const bool in_b = p >= ca;
       const uint64_t q = in_b ? p - ca : p;
       const uint64_t m = canonical_mer_lut(in_b ? gb : ga, q, lut, nb, s.w);
-      f(p, mix_mer<uint64_t>(m >> sh, s.w), (uint32_t)m & 1u, in_b, (uint32_t)q);
+      f(p, mix_mer<uint64_t>(m >> sh, 2 * s.w), (uint32_t)m & 1u, in_b, (uint32_t)q);
     }
   }
 }
@@ -486,42 +478,62 @@ __global__ void __launch_bounds__(pb::kLocThreads) k_pb_local(uint2* __restrict_
 
 // ------------------------------------------------------------------ host
 
+int pair_bucket_bufs(Ctx* c, uint64_t n, int bits, PairBucketBufs* b) {
+  b->g = pair_bucket_geom(n, bits);
+  const PairBucketGeom& g = b->g;
+  const int nbk = g.nbuckets;
+  Workspace& ws = c->ws;
+  b->alt = (uint2*)ws.get(c, 30, (size_t)n * 8 + 64);
+  b->buf = (uint2*)ws.get(c, 31, (size_t)n * 8 + 64);
+  // count rows, then the tiles' first slots (ntiles x nbk each)
+  b->counts = (uint32_t*)ws.get(c, 32, (size_t)g.ntiles * nbk * 8 + 64);
+  uint32_t* tabs = (uint32_t*)ws.get(c, 33, ((size_t)g.nchunks * nbk + 2 * (size_t)nbk) * 4 + 256);
+  if (!b->alt || !b->buf || !b->counts || !tabs) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  b->offs = b->counts + (size_t)g.ntiles * nbk;
+  b->csum = tabs;
+  b->bstart = tabs + (size_t)g.nchunks * nbk;
+  b->bsize = b->bstart + nbk;
+  return 0;
+}
+
+void pair_bucket_offsets(Ctx* c, const PairBucketBufs& b) {
+  const PairBucketGeom& g = b.g;
+  const dim3 grid2((unsigned)((g.nbuckets + 255) / 256), (unsigned)g.nchunks);
+  k_pb_csum<<<grid2, 256, 0, c->stream>>>(b.counts, g.ntiles, g.nbuckets, b.csum);
+  k_pb_scan<<<1, 1024, 0, c->stream>>>(b.csum, g.nchunks, g.nbuckets, b.bstart, b.bsize);
+  k_pb_offsets<<<grid2, 256, 0, c->stream>>>(b.counts, g.ntiles, g.nbuckets, b.csum, b.bstart, b.offs);
+  c->launches += 3;
+}
+
+void pair_bucket_join(Ctx* c, const PairBucketBufs& b, uint32_t* tab) {
+  const PairBucketGeom& g = b.g;
+  const int cap = std::min(c->pair_bucket_cap, pb::kCap);
+  k_pb_local<<<(unsigned)g.nbuckets, pb::kLocThreads, pb::kCap * sizeof(uint2), c->stream>>>(
+      b.buf, b.alt, b.bstart, b.bsize, g.lbits, g.npass, g.dbits, cap, tab);
+  c->launches++;
+}
+
 template <typename K>
 static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
                            uint32_t* tab) {
-  const uint64_t n = ca + cb;
-  const PairBucketGeom g = pair_bucket_geom(n, s.w);
-  const int nbk = g.nbuckets;
-  Workspace& ws = c->ws;
-  uint2* altp = (uint2*)ws.get(c, 30, (size_t)n * 8 + 64);
-  uint2* bufp = (uint2*)ws.get(c, 31, (size_t)n * 8 + 64);
-  // count rows, then the tiles' first slots (ntiles x nbk each)
-  uint32_t* counts = (uint32_t*)ws.get(c, 32, (size_t)g.ntiles * nbk * 8 + 64);
-  uint32_t* tabs = (uint32_t*)ws.get(c, 33, ((size_t)g.nchunks * nbk + 2 * (size_t)nbk) * 4 + 256);
-  if (!altp || !bufp || !counts || !tabs) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
-  uint32_t* offs = counts + (size_t)g.ntiles * nbk;
-  uint32_t* csum = tabs;
-  uint32_t* bstart = csum + (size_t)g.nchunks * nbk;
-  uint32_t* bsize = bstart + nbk;
+  PairBucketBufs b;
+  if (int rc = pair_bucket_bufs(c, ca + cb, 2 * s.w, &b)) return rc;
+  const PairBucketGeom& g = b.g;
   static bool attr = false;  // once per process and key type: more than 48 KB of dynamic shared memory
   if (!attr) {
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_keys<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
     attr = true;
   }
-  const size_t hsm = (size_t)nbk * 4;
-  k_pb_keys<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, counts, g.bbits, g.tile);
-  const dim3 grid2((unsigned)((nbk + 255) / 256), (unsigned)g.nchunks);
-  k_pb_csum<<<grid2, 256, 0, c->stream>>>(counts, g.ntiles, nbk, csum);
-  k_pb_scan<<<1, 1024, 0, c->stream>>>(csum, g.nchunks, nbk, bstart, bsize);
-  k_pb_offsets<<<grid2, 256, 0, c->stream>>>(counts, g.ntiles, nbk, csum, bstart, offs);
+  const size_t hsm = (size_t)g.nbuckets * 4;
+  k_pb_keys<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, b.counts, g.bbits, g.tile);
+  pair_bucket_offsets(c, b);
   stage_mark(c, "seed_scatter");
-  k_pb_scatter<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, offs, g.bbits, g.tile, bufp);
+  k_pb_scatter<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, b.offs, g.bbits, g.tile,
+                                                                           b.buf);
+  c->launches += 2;
   stage_mark(c, "seed_local");
-  const int cap = std::min(c->pair_bucket_cap, pb::kCap);
-  k_pb_local<<<(unsigned)nbk, pb::kLocThreads, pb::kCap * sizeof(uint2), c->stream>>>(
-      bufp, altp, bstart, bsize, g.lbits, g.npass, g.dbits, cap, tab);
-  c->launches += 6;
+  pair_bucket_join(c, b, tab);
   MVG_CUDA_TRY(cudaGetLastError());
   return 0;
 }
