@@ -20,15 +20,22 @@
 //   match_components the genome matcher's match list (match_components.cuh)
 //                    over all gaps, its buckets (gap, bucket): GetMatchList
 //                    order per gap
-//   host             EliminateOverlaps_v2 with std::sort (the order of equal
-//                    left ends is the library sort's, as in the reference),
-//                    LengthFilter, shift to genome coordinates
+//   k_gs_filter      EliminateOverlaps_v2 and LengthFilter per gap, where no
+//                    two matches have equal left ends (any sort gives the
+//                    reference's order then)
+//   host             the same with std::sort for the other gaps (the order of
+//                    equal left ends is the library sort's, as in the
+//                    reference) and for gaps of more matches than shared
+//                    memory takes
 //
 // A gap's positions take slots from a multiple of 32 on, with at least 31
 // empty ones after them, so that chains of seeds never cross into the next
 // gap and a warp's 32 slots are one gap's.  (A joint 64-bit radix sort of all
 // keys and a warp's replay per (gap, bucket) took 6.6 ms of device time for
-// 5,003 gaps of 200-20,000 bp, 43 Mbp; this takes GSMS ms.)
+// 5,003 gaps of 200-20,000 bp, 43 Mbp; the device passes
+// here take 4.0 ms.)
+#include <string.h>
+
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -201,6 +208,208 @@ __global__ void k_gs_gap_rows(const uint32_t* __restrict__ key, uint32_t ncomp, 
   out[g] = g == ngaps || lo == ncomp ? rows : at ? at[lo] : lo;
 }
 
+struct Anchor {  // in gap coordinates
+  int32_t s[2];
+  int32_t len;
+};
+__host__ __device__ __forceinline__ int32_t left_end(const Anchor& m, int q) { return m.s[q] < 0 ? -m.s[q] : m.s[q]; }
+// CropStart / CropEnd (LM/UngappedLocalAlignment.h:137-152 over
+// LM/HybridAbstractMatch.h:271-290): a forward start follows the first
+// column, a reverse start the last.
+__host__ __device__ __forceinline__ void crop_start(Anchor& m, int32_t k) {
+  m.len -= k;
+  for (int q = 0; q < 2; ++q)
+    if (m.s[q] > 0) m.s[q] += k;
+}
+__host__ __device__ __forceinline__ void crop_end(Anchor& m, int32_t k) {
+  m.len -= k;
+  for (int q = 0; q < 2; ++q)
+    if (m.s[q] < 0) m.s[q] -= k;
+}
+
+// EliminateOverlaps_v2's walk over one sequence's overlaps
+// (LM/ProgressiveAligner.h:302-392, eliminate_both = false): item k's match
+// is a[at[k * STEP]], in order of left ends; a match that overlaps a longer one is
+// cropped (CropRight / CropLeft in the sequence's orientation) or, when
+// nothing is left of it, deleted (at = -1); the cropped-off pieces are
+// single-sequence matches, which processNewMatch drops.
+template <int STEP>
+__host__ __device__ __forceinline__ void walk_overlaps(Anchor* a, int32_t* at, int64_t m, int q) {
+  for (int64_t i = 0; i < m; ++i) {
+    if (at[i * STEP] < 0) continue;
+    Anchor& A = a[at[i * STEP]];
+    for (int64_t j = i + 1; j < m; ++j) {
+      if (at[j * STEP] < 0) continue;
+      Anchor& B = a[at[j * STEP]];
+      const int32_t len_i = A.len;
+      const int32_t over = len_i - (left_end(B, q) - left_end(A, q));
+      if (over <= 0) break;
+      if (B.len > len_i) {  // i is the shorter: crop its right end or delete it
+        if (over >= len_i) {
+          at[i * STEP] = -1;
+          break;  // the reference steps back to i, finds it deleted and moves on
+        }
+        if (A.s[q] > 0) crop_end(A, over);
+        else crop_start(A, over);
+      } else {  // j is: crop its left end or delete it
+        if (over >= B.len)
+          at[j * STEP] = -1;
+        else if (B.s[q] > 0)
+          crop_start(B, over);
+        else
+          crop_end(B, over);
+      }
+    }
+  }
+}
+
+// Overlap elimination and length filter of one gap per CTA: its matches sorted
+// in shared memory by their left ends in A and walked, the rest by their left
+// ends in B and walked, and the kept ones written over the gap's rows.  A
+// match whose left end no earlier match reaches starts a run that shares
+// nothing with the matches before it (walking only shortens them), so threads
+// walk runs.  What the host has to do is left in todo[g]: 0 nothing; 1 all of
+// it, the rows as they were (more than kGsFilterRows matches, or two equal
+// left ends in A); m > 1 the B half of the gap's first m rows, which the A half
+// left in order (two equal left ends in B).  Latency of the sorts and the
+// longest run's walk bound it.  (On 16 host threads, all of it: 1.9 ms per
+// 180,000 matches; a walk by one thread per gap: 0.46 ms.)
+constexpr int kGsFilterRows = 1536;
+constexpr int kGsFilterThreads = 128;
+__global__ void __launch_bounds__(kGsFilterThreads)
+    k_gs_filter(Anchor* __restrict__ rows, const uint32_t* __restrict__ gap_row, uint32_t* __restrict__ kept,
+                uint32_t* __restrict__ todo) {
+  constexpr int T = kGsFilterThreads;
+  __shared__ uint64_t key[kGsFilterRows];  // the sort's keys; then the runs' heads and the warps' counts
+  __shared__ Anchor a[kGsFilterRows];
+  __shared__ int32_t order[kGsFilterRows];
+  __shared__ int32_t reach[T / 32];
+  uint8_t* const head = reinterpret_cast<uint8_t*>(key);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = blockIdx.x;
+  const uint32_t r0 = gap_row[g];
+  const int n = (int)(gap_row[g + 1] - r0);
+  if (n == 0 || n > kGsFilterRows) {
+    if (tid == 0) {
+      kept[g] = 0;
+      todo[g] = n > 0;
+    }
+    return;
+  }
+  for (int i = tid; i < n; i += T) {
+    a[i] = rows[r0 + i];
+    order[i] = i;
+  }
+  int m = n;  // matches left, in order
+  for (int q = 0; q < 2; ++q) {
+    int size = 2;  // the sort's; keys from m on count as larger than all others
+    while (size < m) size <<= 1;
+    __syncthreads();
+    for (int i = tid; i < m; i += T) key[i] = (uint64_t)(uint32_t)left_end(a[order[i]], q) << 32 | (uint32_t)order[i];
+    __syncthreads();
+    for (int len = 2; len <= size; len <<= 1)
+      for (int step = len >> 1; step > 0; step >>= 1) {
+        const bool first = step == len >> 1;  // mirrored pairs: every pair ascends
+        for (int i = tid; i < size / 2; i += T) {
+          const int blk = i & ~(step - 1), in = i & (step - 1);
+          const int lo = 2 * blk + in, hi = first ? 2 * blk + len - 1 - in : lo + step;
+          if (hi >= m) continue;
+          const uint64_t x = key[lo], y = key[hi];
+          if (x > y) {
+            key[lo] = y;
+            key[hi] = x;
+          }
+        }
+        __syncthreads();
+      }
+    bool tie = false;
+    for (int i = tid + 1; i < m; i += T) tie |= key[i] >> 32 == key[i - 1] >> 32;
+    if (__syncthreads_or(tie)) {
+      if (q == 1)
+        for (int i = tid; i < m; i += T) rows[r0 + i] = a[order[i]];
+      if (tid == 0) {
+        kept[g] = 0;
+        todo[g] = q == 0 ? 1u : (uint32_t)m;
+      }
+      return;
+    }
+    // the farthest end before each thread's matches, which are consecutive
+    const int per = (m + T - 1) / T, lo = min(tid * per, m), hi = min(lo + per, m);
+    int32_t far = 0;
+    for (int i = lo; i < hi; ++i) {
+      const int x = (int)(uint32_t)key[i];
+      order[i] = x;
+      far = max(far, (int32_t)(key[i] >> 32) + a[x].len);
+    }
+    int32_t scan = far;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int32_t v = __shfl_up_sync(0xffffffffu, scan, d);
+      if (lane >= d) scan = max(scan, v);
+    }
+    if (lane == 31) reach[warp] = scan;
+    scan = __shfl_up_sync(0xffffffffu, scan, 1);
+    if (lane == 0) scan = 0;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) scan = max(scan, reach[w]);
+    for (int i = lo; i < hi; ++i) {
+      const Anchor& x = a[order[i]];
+      const int32_t l = left_end(x, q);
+      head[i] = l >= scan;
+      scan = max(scan, l + x.len);
+    }
+    __syncthreads();
+    for (int i = tid; i < m; i += T)
+      if (head[i]) {
+        int e = i + 1;
+        while (e < m && !head[e]) ++e;
+        if (e > i + 1) walk_overlaps<1>(a, order + i, e - i, q);
+      }
+    __syncthreads();
+    if (tid < 32) {  // the matches left, in order
+      int w = 0;
+      for (int base = 0; base < m; base += 32) {
+        const int x = base + lane < m ? order[base + lane] : -1;
+        const unsigned b = __ballot_sync(0xffffffffu, x >= 0);
+        __syncwarp();
+        if (x >= 0) order[w + __popc(b & ((1u << lane) - 1u))] = x;
+        w += __popc(b);
+      }
+      if (lane == 0) reach[0] = w;
+    }
+    __syncthreads();
+    m = reach[0];
+  }
+  if (tid < 32) {
+    int w = 0;
+    for (int base = 0; base < m; base += 32) {
+      const int i = base + lane;
+      const bool in = i < m && a[order[i < m ? i : 0]].len >= kGsMinAnchor;
+      const unsigned b = __ballot_sync(0xffffffffu, in);
+      if (in) rows[r0 + w + __popc(b & ((1u << lane) - 1u))] = a[order[i]];
+      w += __popc(b);
+    }
+    if (lane == 0) {
+      kept[g] = (uint32_t)w;
+      todo[g] = 0;
+    }
+  }
+}
+
+// The kept rows of every gap in genome coordinates, at its first output row.
+__global__ void k_gs_out(const Anchor* __restrict__ rows, const uint32_t* __restrict__ gap_row,
+                         const uint32_t* __restrict__ kept, const uint32_t* __restrict__ at,
+                         const GapDev* __restrict__ gaps, int64_t* __restrict__ out) {
+  const int g = blockIdx.x;
+  const GapDev& d = gaps[g];
+  for (uint32_t u = threadIdx.x; u < kept[g]; u += blockDim.x) {
+    const Anchor x = rows[gap_row[g] + u];
+    int64_t* o = out + 3 * ((uint64_t)at[g] + u);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) o[q] = x.s[q] > 0 ? x.s[q] + (int64_t)d.src[q] : x.s[q] - (int64_t)d.src[q];
+    o[2] = x.len;
+  }
+}
+
 // ------------------------------------------------------------------ host
 
 static std::mutex g_gs_mu;
@@ -223,32 +432,10 @@ static int gs_upload_tables(int device) {
 }
 
 namespace {
-struct Anchor {  // in gap coordinates
-  int32_t s[2];
-  int32_t len;
-};
-int32_t left_end(const Anchor& m, int q) { return m.s[q] < 0 ? -m.s[q] : m.s[q]; }
-// CropStart / CropEnd (LM/UngappedLocalAlignment.h:137-152 over
-// LM/HybridAbstractMatch.h:271-290): a forward start follows the first
-// column, a reverse start the last.
-void crop_start(Anchor& m, int32_t k) {
-  m.len -= k;
-  for (int q = 0; q < 2; ++q)
-    if (m.s[q] > 0) m.s[q] += k;
-}
-void crop_end(Anchor& m, int32_t k) {
-  m.len -= k;
-  for (int q = 0; q < 2; ++q)
-    if (m.s[q] < 0) m.s[q] -= k;
-}
-
-// EliminateOverlaps_v2 (eliminate_both = false) on one gap's two-sequence
-// matches, then LengthFilter(12): per sequence, sort by left end and walk
-// the overlaps, cropping (CropRight / CropLeft in that sequence's
-// orientation) or deleting the shorter match; the cropped-off pieces are
-// single-sequence matches, which processNewMatch drops.  The sort moves
-// (left end, index) pairs: std::sort's result on equal left ends follows from
-// the sequence of comparisons alone.  Returns the number kept, at a[0 ..).
+// One gap's overlap elimination and length filter with the sort the reference
+// uses: std::sort's result on equal left ends follows from the sequence of
+// comparisons alone, so (left end, index) pairs are sorted.  from: the first
+// sequence (1: A's half is done).  Returns the number kept, at a[0 ..).
 struct FilterScratch {
   struct Item {
     int32_t left;
@@ -257,48 +444,17 @@ struct FilterScratch {
   std::vector<Item> ml;
   std::vector<Anchor> kept;
 };
-int64_t filter_gap(Anchor* a, int64_t n, FilterScratch& F) {
+int64_t filter_gap(Anchor* a, int64_t n, int from, FilterScratch& F) {
   auto& ml = F.ml;
   ml.resize(n);
   for (int64_t k = 0; k < n; ++k) ml[k].at = (int32_t)k;
   if (n >= 2) {
-    for (int q = 0; q < 2; ++q) {
+    for (int q = from; q < 2; ++q) {
       for (auto& x : ml) x.left = left_end(a[x.at], q);
       std::sort(ml.begin(), ml.end(),
                 [](const FilterScratch::Item& x, const FilterScratch::Item& y) { return x.left < y.left; });
-      bool any_deleted = false;
-      const int64_t m = (int64_t)ml.size();
-      for (int64_t i = 0; i < m; ++i) {
-        if (ml[i].at < 0) continue;
-        Anchor& A = a[ml[i].at];
-        for (int64_t j = i + 1; j < m; ++j) {
-          if (ml[j].at < 0) continue;
-          Anchor& B = a[ml[j].at];
-          const int32_t len_i = A.len;
-          const int32_t over = len_i - (left_end(B, q) - left_end(A, q));
-          if (over <= 0) break;
-          if (B.len > len_i) {  // i is the shorter: crop its right end or delete it
-            if (over >= len_i) {
-              ml[i].at = -1;
-              any_deleted = true;
-              break;  // the reference steps back to i, finds it deleted and moves on
-            }
-            if (A.s[q] > 0) crop_end(A, over);
-            else crop_start(A, over);
-          } else {  // j is: crop its left end or delete it
-            if (over >= B.len) {
-              ml[j].at = -1;
-              any_deleted = true;
-            } else if (B.s[q] > 0) {
-              crop_start(B, over);
-            } else {
-              crop_end(B, over);
-            }
-          }
-        }
-      }
-      if (any_deleted)
-        ml.erase(std::remove_if(ml.begin(), ml.end(), [](const FilterScratch::Item& x) { return x.at < 0; }), ml.end());
+      walk_overlaps<2>(a, &ml[0].at, (int64_t)ml.size(), q);
+      ml.erase(std::remove_if(ml.begin(), ml.end(), [](const FilterScratch::Item& x) { return x.at < 0; }), ml.end());
     }
   }
   auto& kept = F.kept;
@@ -310,17 +466,21 @@ int64_t filter_gap(Anchor* a, int64_t n, FilterScratch& F) {
 }
 
 // One chunk of a call's gaps: the searched gaps' device descriptors and
-// caller indices, the device pass's rows (in pinned memory, per gap from
-// gap_row on, GetMatchList order) and the host pass's counts.
+// caller indices, and the device pass's results in pinned memory: the kept
+// rows in genome coordinates and the matches of the gaps left to the host (in
+// GetMatchList order).
 struct GsChunk {
   std::vector<GapDev> gd;
   std::vector<uint32_t> gid;  // caller's gap index of each searched gap
   uint64_t words[2] = {0, 0};
   uint32_t slots[2] = {0, 0};
   uint64_t keys[2] = {0, 0};
+  const int64_t* out = nullptr;  // rows of the gaps filtered on the device, gap by gap
+  std::vector<uint32_t> nkept;   // rows per gap
+  std::vector<uint32_t> todo;    // gaps left to the host, ascending
+  std::vector<uint32_t> todo_at, todo_n;  // their matches: rows[todo_at ..]
+  std::vector<uint8_t> todo_q;            // the sequence to begin with
   Anchor* rows = nullptr;
-  const uint32_t* gap_row = nullptr;  // null: no rows
-  std::vector<uint32_t> nkept;
 };
 
 // Runs fn(i) for i in [0, n) on up to nthreads host threads that claim runs
@@ -346,14 +506,16 @@ void run_claimed(int n, int nthreads, F&& fn) {
 
 int host_threads_for(size_t items) {
   const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  return (int)std::min<uint64_t>(hw, std::max<uint64_t>(1, items / 20000));
+  return (int)std::min<uint64_t>(hw, std::max<uint64_t>(1, items / 10000));
 }
 }  // namespace
 
 // Slots of a chunk of gaps, and its most gaps: the seed join's buckets hold
 // 2,048 keys each up to 2^25 keys, and its keys 44 bits, 30 of them the
-// widest mer's.  Up to that, chunks of GSCHUNK slots: the host pass of one
-// chunk runs beside the device pass of the next.
+// widest mer's.  Below that a chunk is as
+// large as this because the host pass of one chunk runs beside the device
+// pass of the next (43 Mbp in gaps: 5.9 ms with 2^23 slots, 5.2 with 2^24, 5.8
+// with 2^25, 5.6 in one chunk).
 constexpr uint64_t kGsSlots = 1ull << 24;
 constexpr size_t kGsGaps = 1u << (kPairMaxBits - 30);
 
@@ -393,11 +555,13 @@ static int gs_plan(const int64_t* gaps, uint64_t ngaps, uint64_t total_slots, st
   return 0;
 }
 
-// Device pass of one chunk, from packing to the rows, which are copied to the
-// pinned buffer `buf` with the gaps' first rows.  Synchronous.
+// Device pass of one chunk, from packing to the kept rows, which are copied to
+// the pinned buffer `buf` with the matches of the gaps left to the host.
+// Synchronous.
 static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch, int buf) {
   const int ng = (int)ch.gd.size();
   if (ng == 0) return 0;
+  ch.nkept.assign(ng, 0);
   Workspace& ws = c->ws;
   const uint64_t* words = ch.words;
   const uint32_t wa = ch.slots[0] >> 5, wb = ch.slots[1] >> 5;
@@ -406,8 +570,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   uint32_t* pb = (uint32_t*)ws.get(c, kGsSlot + 2, words[1] * 4 + 64);
   uint32_t* gmap = (uint32_t*)ws.get(c, kGsSlot + 3, ((size_t)wa + wb) * 4 + 64);
   uint32_t* tab = (uint32_t*)ws.get(c, 38, (size_t)ch.slots[0] * 4 + 64);
-  uint32_t* d_gap_row = (uint32_t*)ws.get(c, kGsSlot + 4, ((size_t)ng + 1) * 4);
-  if (!d_gaps || !pa || !pb || !gmap || !tab || !d_gap_row) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  if (!d_gaps || !pa || !pb || !gmap || !tab) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
   stage_mark(c, "gs_pack");
   MVG_CUDA_TRY(cudaMemcpyAsync(d_gaps, ch.gd.data(), ng * sizeof(GapDev), cudaMemcpyHostToDevice, c->stream));
@@ -455,54 +618,104 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   };
   if ((rc = match_components(c, P, tab, (int64_t)ch.slots[0], 16 + gbits, room_for, &r))) return rc;
   if (r.rows == 0) return 0;
-  stage_mark(c, "gs_copy");
+  stage_mark(c, "gs_filter");
+  // per gap: first match, rows kept, left to the host, first output row; their sum (k_gs_filter's todo)
+  uint32_t* d_tab = (uint32_t*)ws.get(c, kGsSlot + 4, ((size_t)ng * 4 + 2) * 4);
+  int64_t* d_out = (int64_t*)ws.get(c, kGsSlot + 6, r.rows * 24);
+  if (!d_tab || !d_out) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+  uint32_t *gap_row = d_tab, *kept = d_tab + ng + 1, *todo = kept + ng, *at = todo + ng, *sum = at + ng;
+  Anchor* d_rows = (Anchor*)P.out;
   k_gs_gap_rows<<<div_up(ng + 1, 256), 256, 0, c->stream>>>(r.C.key, r.ncomp, r.at, (uint32_t)r.rows, (uint32_t)ng,
-                                                            d_gap_row);
-  c->launches++;
-  const size_t head = (((size_t)ng + 1) * 4 + 255) & ~(size_t)255, need = head + r.rows * sizeof(Anchor);
-  if (c->h_rows_cap[buf] < need) {
-    if (c->h_rows[buf]) cudaFreeHost(c->h_rows[buf]);
-    c->h_rows[buf] = nullptr;
-    c->h_rows_cap[buf] = 0;
-    MVG_CUDA_TRY(cudaMallocHost(&c->h_rows[buf], need + need / 4));
-    c->h_rows_cap[buf] = need + need / 4;
+                                                            gap_row);
+  k_gs_filter<<<ng, kGsFilterThreads, 0, c->stream>>>(d_rows, gap_row, kept, todo);
+  pair_scan_small(kept, ng, at, sum, c->stream);
+  k_gs_out<<<ng, 64, 0, c->stream>>>(d_rows, gap_row, kept, at, d_gaps, d_out);
+  c->launches += 4;
+  stage_mark(c, "gs_copy");
+  auto pinned = [&](size_t need) -> uint8_t* {
+    if (c->h_rows_cap[buf] < need) {
+      if (c->h_rows[buf]) cudaFreeHost(c->h_rows[buf]);
+      c->h_rows[buf] = nullptr;
+      c->h_rows_cap[buf] = 0;
+      if (cudaMallocHost(&c->h_rows[buf], need + need / 4) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_rows[buf] = nullptr;
+        return nullptr;
+      }
+      c->h_rows_cap[buf] = need + need / 4;
+    }
+    return (uint8_t*)c->h_rows[buf];
+  };
+  const size_t tab_bytes = ((size_t)ng * 4 + 2) * 4;
+  uint32_t* h = (uint32_t*)pinned(std::max(tab_bytes, (size_t)r.rows * 24 + 256));
+  if (!h) return report_error(MVG_ERR_NOMEM, "pinned allocation failed");
+  MVG_CUDA_TRY(cudaMemcpyAsync(h, d_tab, tab_bytes, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  std::vector<uint32_t> first(h, h + ng + 1);
+  ch.nkept.assign(h + ng + 1, h + 2 * ng + 1);
+  const uint64_t nout = h[4 * ng + 1];
+  uint64_t nrows = 0;
+  for (int g = 0; g < ng; ++g)
+    if (const uint32_t t = h[2 * ng + 1 + g]) {
+      ch.todo.push_back((uint32_t)g);
+      ch.todo_q.push_back(t > 1);
+      ch.todo_n.push_back(t > 1 ? t : first[g + 1] - first[g]);
+      ch.todo_at.push_back((uint32_t)nrows);
+      nrows += ch.todo_n.back();
+    }
+  const bool all = ch.todo.size() > 32;  // one copy of every row instead of a copy per gap
+  if (all) {
+    nrows = r.rows;
+    for (size_t k = 0; k < ch.todo.size(); ++k) ch.todo_at[k] = first[ch.todo[k]];
   }
-  ch.gap_row = (const uint32_t*)c->h_rows[buf];
-  ch.rows = (Anchor*)((uint8_t*)c->h_rows[buf] + head);
-  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_rows[buf], d_gap_row, ((size_t)ng + 1) * 4, cudaMemcpyDeviceToHost, c->stream));
-  MVG_CUDA_TRY(cudaMemcpyAsync(ch.rows, P.out, r.rows * sizeof(Anchor), cudaMemcpyDeviceToHost, c->stream));
+  const size_t rows_at = (nout * 24 + 255) & ~(size_t)255;
+  uint8_t* base = pinned(rows_at + nrows * sizeof(Anchor));
+  if (!base) return report_error(MVG_ERR_NOMEM, "pinned allocation failed");
+  ch.out = (const int64_t*)base;
+  ch.rows = (Anchor*)(base + rows_at);
+  if (nout) MVG_CUDA_TRY(cudaMemcpyAsync(base, d_out, nout * 24, cudaMemcpyDeviceToHost, c->stream));
+  if (all) MVG_CUDA_TRY(cudaMemcpyAsync(ch.rows, d_rows, nrows * sizeof(Anchor), cudaMemcpyDeviceToHost, c->stream));
+  for (size_t k = 0; k < ch.todo.size() && !all; ++k)
+    MVG_CUDA_TRY(cudaMemcpyAsync(ch.rows + ch.todo_at[k], d_rows + first[ch.todo[k]], ch.todo_n[k] * sizeof(Anchor),
+                                 cudaMemcpyDeviceToHost, c->stream));
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return 0;
 }
 
-// Host pass of one chunk: per gap, overlap elimination and length filter,
-// then the rows in genome coordinates from row `base` of the caller's output
-// on.  Gaps are independent and their anchor counts differ by orders of
-// magnitude, so host threads claim runs of gaps.  Returns the row after the
-// chunk's last.
-static uint64_t gs_filter(GsChunk& ch, int64_t* out, uint64_t cap, uint64_t base) {
-  const int ng = (int)ch.gd.size();
-  ch.nkept.assign(ng, 0);
-  if (!ch.gap_row) return base;
-  const int nthreads = host_threads_for(ch.gap_row[ng]);
-  run_claimed(ng, nthreads, [&](int gi) {
+// Host pass of one chunk: the gaps the device left (their sizes differ by
+// orders of magnitude, so host threads claim them), and all rows to the
+// caller's output from row `base` on.  Returns the row after the chunk's last.
+static uint64_t gs_finish(GsChunk& ch, int64_t* out, uint64_t cap, uint64_t base) {
+  const size_t nt = ch.todo.size();
+  uint64_t nrows = 0;
+  for (uint32_t n : ch.todo_n) nrows += n;
+  run_claimed((int)nt, host_threads_for(nrows), [&](int k) {
     thread_local FilterScratch scratch;
-    ch.nkept[gi] = (uint32_t)filter_gap(ch.rows + ch.gap_row[gi], ch.gap_row[gi + 1] - ch.gap_row[gi], scratch);
+    ch.nkept[ch.todo[k]] = (uint32_t)filter_gap(ch.rows + ch.todo_at[k], ch.todo_n[k], ch.todo_q[k], scratch);
   });
-  std::vector<uint64_t> at(ng);
-  for (int gi = 0; gi < ng; ++gi) {
-    at[gi] = base;
-    base += ch.nkept[gi];
-  }
-  run_claimed(ng, nthreads, [&](int gi) {
-    const GapDev& d = ch.gd[gi];
-    for (uint32_t u = 0; u < ch.nkept[gi] && at[gi] + u < cap; ++u) {
-      const Anchor& x = ch.rows[ch.gap_row[gi] + u];
-      int64_t* o = out + 3 * (at[gi] + u);
+  const int64_t* src = ch.out;
+  size_t g = 0;
+  auto copy = [&](size_t to) {  // the device's rows of gaps [g, to), none of them in todo
+    uint64_t n = 0;
+    for (; g < to; ++g) n += ch.nkept[g];
+    const uint64_t fit = base < cap ? std::min(n, cap - base) : 0;
+    if (fit) memcpy(out + 3 * base, src, fit * 24);
+    src += 3 * n;
+    base += n;
+  };
+  for (size_t k = 0; k < nt; ++k) {
+    copy(ch.todo[k]);
+    const GapDev& d = ch.gd[g];
+    for (uint32_t u = 0; u < ch.nkept[g]; ++u, ++base) {
+      if (base >= cap) continue;
+      const Anchor& x = ch.rows[ch.todo_at[k] + u];
+      int64_t* o = out + 3 * base;
       for (int q = 0; q < 2; ++q) o[q] = x.s[q] > 0 ? x.s[q] + (int64_t)d.src[q] : x.s[q] - (int64_t)d.src[q];
       o[2] = x.len;
     }
-  });
+    ++g;
+  }
+  copy(ch.nkept.size());
   return base;
 }
 
@@ -541,9 +754,9 @@ int gap_anchor_search_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t
     if (filt.joinable()) filt.join();
     GsChunk& ch = chunks[k];
     if (k + 1 < chunks.size())
-      filt = std::thread([&ch, &total, out, cap] { total = gs_filter(ch, out, cap, total); });
+      filt = std::thread([&ch, &total, out, cap] { total = gs_finish(ch, out, cap, total); });
     else
-      total = gs_filter(ch, out, cap, total);
+      total = gs_finish(ch, out, cap, total);
   }
   stage_end(c);
   if (gap_off) {
