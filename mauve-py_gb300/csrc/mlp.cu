@@ -9,16 +9,17 @@
 //
 // Forward hidden layers: tcgen05 tensor-core GEMMs fed by TMA with bias,
 // GELU and (last layer) the 256 -> 2 output layer in the epilogue
-// (mlp_tc.cuh).  Backward GEMMs, and the forward when the tcgen05 path is
-// switched off or an operand does not meet its TMA rules: C[M x N] (fp32) =
-// op(A)[M x K] * op(B)[K x N] with bf16 operands; a 64x64 block tile, four
-// warps of 32x32 (2 x 4 mma.sync tiles), K step 32 staged in shared memory
-// with both operands stored k-contiguous so every fragment is one 32-bit
-// shared load.
+// (mlp_tc.cuh).  Forward when the tcgen05 path is switched off or an operand
+// does not meet its TMA rules: C[M x N] (fp32) = A[M x K] * B[N x K]^T with
+// bf16 operands; a 64x64 block tile, four warps of 32x32 (2 x 4 mma.sync
+// tiles), K step 32 staged in shared memory with both operands stored
+// k-contiguous so every fragment is one 32-bit shared load.  Backward:
+// mlp_grad.cuh.
 #include <cuda_bf16.h>
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "mvg_internal.h"
@@ -51,11 +52,8 @@ struct MlpState {
   float* z[3] = {};       // pre-activations
   __nv_bfloat16* h[3] = {};  // activations
   float* out = nullptr;   // [n x kOut]
-  float* dh = nullptr;    // [n x kHid] fp32 upstream gradient
-  float* dz32 = nullptr;  // [n x kHid] fp32 dZ (bias gradients)
-  __nv_bfloat16* dz = nullptr;  // [n x kHid] bf16 dZ (GEMM operand)
-  __nv_bfloat16* dout = nullptr;  // [n x kOut]
-  float* dout32 = nullptr;
+  __nv_bfloat16* dz[3] = {};  // [n x kHid] bf16 dZ (GEMM operands)
+  float* part = nullptr;  // partial sums of the backward pass (kPartFloats)
   float* loss = nullptr;
   bool ready = false;
 };
@@ -70,8 +68,6 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// op(A)[m][k] = TA ? A[k * lda + m] : A[m * lda + k];  op(B)[k][n] = TB ? B[n * ldb + k] : B[k * ldb + n]
-template <bool TA, bool TB>
 __global__ void __launch_bounds__(128) k_gemm_bf16(const __nv_bfloat16* __restrict__ A, int lda,
                                                    const __nv_bfloat16* __restrict__ B, int ldb,
                                                    float* __restrict__ C, int ldc, int M, int N, int K) {
@@ -92,21 +88,14 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const __nv_bfloat16* __restri
   const __nv_bfloat16 zero = __float2bfloat16(0.f);
   for (int k0 = 0; k0 < K; k0 += BK) {
     for (int e = tid; e < BM * BK; e += 128) {
-      const int mm = e / BK, kk = e % BK;  // k fastest: coalesced when A is row-major
+      const int mm = e / BK, kk = e % BK;  // k fastest: coalesced
       const int gm = m0 + mm, gk = k0 + kk;
-      As[mm][kk] = (gm < M && gk < K) ? (TA ? A[(int64_t)gk * lda + gm] : A[(int64_t)gm * lda + gk]) : zero;
+      As[mm][kk] = (gm < M && gk < K) ? A[(int64_t)gm * lda + gk] : zero;
     }
     for (int e = tid; e < BN * BK; e += 128) {
-      int nn, kk;
-      if (TB) {
-        nn = e / BK;
-        kk = e % BK;
-      } else {
-        kk = e / BN;
-        nn = e % BN;
-      }
+      const int nn = e / BK, kk = e % BK;
       const int gn = n0 + nn, gk = k0 + kk;
-      Bs[nn][kk] = (gn < N && gk < K) ? (TB ? B[(int64_t)gn * ldb + gk] : B[(int64_t)gk * ldb + gn]) : zero;
+      Bs[nn][kk] = (gn < N && gk < K) ? B[(int64_t)gn * ldb + gk] : zero;
     }
     __syncthreads();
 #pragma unroll
@@ -146,11 +135,10 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const __nv_bfloat16* __restri
     }
 }
 
-template <bool TA, bool TB>
 static void gemm(cudaStream_t st, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C, int ldc,
                  int M, int N, int K, uint64_t* launches) {
   dim3 grid((N + 63) / 64, (M + 63) / 64);
-  k_gemm_bf16<TA, TB><<<grid, 128, 0, st>>>(A, lda, B, ldb, C, ldc, M, N, K);
+  k_gemm_bf16<<<grid, 128, 0, st>>>(A, lda, B, ldb, C, ldc, M, N, K);
   ++*launches;
 }
 
@@ -163,6 +151,7 @@ __device__ __forceinline__ float gelu_grad(float x) {
 
 }  // namespace mvg
 
+#include "mlp_grad.cuh"
 #include "mlp_tc.cuh"
 
 namespace mvg {
@@ -179,46 +168,6 @@ __global__ void k_bias_gelu(float* __restrict__ z, const float* __restrict__ b, 
 __global__ void k_bias_add(float* __restrict__ z, const float* __restrict__ b, int64_t n, int d) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * d; e += (int64_t)gridDim.x * blockDim.x)
     z[e] += b[e % d];
-}
-
-// loss = mean over rows of sum_k (o - t)^2; dO = 2 (o - t) / n
-__global__ void k_mse(const float* __restrict__ o, const float* __restrict__ tgt, int64_t n, float* __restrict__ d32,
-                      __nv_bfloat16* __restrict__ d16, float* __restrict__ loss) {
-  float s = 0.f;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * kOut; e += (int64_t)gridDim.x * blockDim.x) {
-    const float diff = o[e] - tgt[e];
-    s += diff * diff;
-    const float gd = 2.f * diff / (float)n;
-    d32[e] = gd;
-    d16[e] = __float2bfloat16(gd);
-  }
-  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (float)n);
-}
-
-__global__ void k_gelu_back(const float* __restrict__ dh, const float* __restrict__ z, float* __restrict__ dz32,
-                            __nv_bfloat16* __restrict__ dz, int64_t total) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const float v = dh[e] * gelu_grad(z[e]);
-    dz32[e] = v;
-    dz[e] = __float2bfloat16(v);
-  }
-}
-
-// column sums of x [n x d] into out[d] (one block per column group)
-__global__ void k_colsum(const float* __restrict__ x, int64_t n, int d, float* __restrict__ out) {
-  const int col = blockIdx.x;
-  float s = 0.f;
-  for (int64_t r = threadIdx.x; r < n; r += blockDim.x) s += x[r * d + col];
-  for (int q = 16; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
-  __shared__ float ws[8];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-    out[col] = t;
-  }
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, int64_t n) {
@@ -369,22 +318,14 @@ static int mlp_alloc(Ctx* c, MlpState& s, int64_t n) {
       cudaFree(s.h[q]);
     }
     cudaFree(s.out);
-    cudaFree(s.dh);
-    cudaFree(s.dz32);
-    cudaFree(s.dz);
-    cudaFree(s.dout);
-    cudaFree(s.dout32);
+    for (int q = 0; q < 3; ++q) cudaFree(s.dz[q]);
     bool ok = true;
     for (int q = 0; q < 3; ++q) {
       ok = ok && cudaMalloc(&s.z[q], n * kHid * 4) == cudaSuccess;
       ok = ok && cudaMalloc(&s.h[q], rows8(n) * kHid * 2) == cudaSuccess;
+      ok = ok && cudaMalloc(&s.dz[q], n * kHid * 2) == cudaSuccess;
     }
     ok = ok && cudaMalloc(&s.out, n * kOut * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&s.dh, n * kHid * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&s.dz32, n * kHid * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&s.dz, n * kHid * 2) == cudaSuccess;
-    ok = ok && cudaMalloc(&s.dout, n * kOut * 2) == cudaSuccess;
-    ok = ok && cudaMalloc(&s.dout32, n * kOut * 4) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
       s.cap = 0;
@@ -406,12 +347,9 @@ static void mlp_free(MlpState& s) {
     cudaFree(s.z[q]);
     cudaFree(s.h[q]);
   }
+  for (int q = 0; q < 3; ++q) cudaFree(s.dz[q]);
   cudaFree(s.out);
-  cudaFree(s.dh);
-  cudaFree(s.dz32);
-  cudaFree(s.dz);
-  cudaFree(s.dout);
-  cudaFree(s.dout32);
+  cudaFree(s.part);
   s = MlpState();
 }
 
@@ -504,39 +442,88 @@ static void mlp_forward(Ctx* c, MlpState& s, const __nv_bfloat16* X, int64_t n, 
       return;
     }
   }
-  gemm<false, true>(st, X, kIn, s.wb + kOffW1, kIn, s.z[0], kHid, nn, kHid, kIn, &c->launches);
+  gemm(st, X, kIn, s.wb + kOffW1, kIn, s.z[0], kHid, nn, kHid, kIn, &c->launches);
   k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[0], s.w + kOffB1, s.h[0], n, kHid);
-  gemm<false, true>(st, s.h[0], kHid, s.wb + kOffW2, kHid, s.z[1], kHid, nn, kHid, kHid, &c->launches);
+  gemm(st, s.h[0], kHid, s.wb + kOffW2, kHid, s.z[1], kHid, nn, kHid, kHid, &c->launches);
   k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[1], s.w + kOffB2, s.h[1], n, kHid);
-  gemm<false, true>(st, s.h[1], kHid, s.wb + kOffW3, kHid, s.z[2], kHid, nn, kHid, kHid, &c->launches);
+  gemm(st, s.h[1], kHid, s.wb + kOffW3, kHid, s.z[2], kHid, nn, kHid, kHid, &c->launches);
   k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[2], s.w + kOffB3, s.h[2], n, kHid);
-  gemm<false, true>(st, s.h[2], kHid, s.wb + kOffW4, kHid, s.out, kOut, nn, kOut, kHid, &c->launches);
+  gemm(st, s.h[2], kHid, s.wb + kOffW4, kHid, s.out, kOut, nn, kOut, kHid, &c->launches);
   k_bias_add<<<eltwise_grid(n * kOut), 256, 0, st>>>(s.out, s.w + kOffB4, n, kOut);
   c->launches += 4;
 }
 
+// Partial sums of the backward pass: dW, db1 and db2, and the output layer's.
+constexpr int64_t kPartW = (int64_t)kGradSplits * kHid * (kIn + 2 * kHid);
+constexpr int64_t kPartB = (int64_t)kGradParts * kHid;
+constexpr int64_t kPartFloats = kPartW + 2 * kPartB + (int64_t)kGradTopParts * kTopPart;
+
+// Per device: k_grad_z's shared-memory opt-in.
+static int grad_kernel_ready(int device) {
+  static bool ready[64] = {};
+  if (device >= 0 && device < 64 && ready[device]) return 0;
+  MVG_CUDA_TRY(cudaFuncSetAttribute(k_grad_z, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradZSmem));
+  if (device >= 0 && device < 64) ready[device] = true;
+  return 0;
+}
+
 // Gradients of the mean-squared loss into s.g (overwritten), loss into s.loss.
-static void mlp_backward(Ctx* c, MlpState& s, const __nv_bfloat16* X, const float* tgt, int64_t n) {
+static int mlp_backward(Ctx* c, MlpState& s, const __nv_bfloat16* X, const float* tgt, int64_t n) {
   cudaStream_t st = c->stream;
-  const int nn = (int)n;
-  cudaMemsetAsync(s.loss, 0, 4, st);
-  k_mse<<<eltwise_grid(n * kOut), 256, 0, st>>>(s.out, tgt, n, s.dout32, s.dout, s.loss);
-  // layer 4: dW4 = dO^T H3, db4 = sum dO, dH3 = dO W4
-  gemm<true, false>(st, s.dout, kOut, s.h[2], kHid, s.g + kOffW4, kHid, kOut, kHid, nn, &c->launches);
-  k_colsum<<<kOut, 256, 0, st>>>(s.dout32, n, kOut, s.g + kOffB4);
-  gemm<false, false>(st, s.dout, kOut, s.wb + kOffW4, kHid, s.dh, kHid, nn, kHid, kOut, &c->launches);
-  c->launches += 2;
-  const int64_t offW[3] = {kOffW1, kOffW2, kOffW3};
-  const int64_t offB[3] = {kOffB1, kOffB2, kOffB3};
-  for (int q = 2; q >= 0; --q) {
-    k_gelu_back<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.dh, s.z[q], s.dz32, s.dz, n * kHid);
-    k_colsum<<<kHid, 256, 0, st>>>(s.dz32, n, kHid, s.g + offB[q]);
-    const __nv_bfloat16* in = q == 0 ? X : s.h[q - 1];
-    const int din = q == 0 ? kIn : kHid;
-    gemm<true, false>(st, s.dz, kHid, in, din, s.g + offW[q], din, kHid, din, nn, &c->launches);
-    if (q > 0) gemm<false, false>(st, s.dz, kHid, s.wb + offW[q], kHid, s.dh, kHid, nn, kHid, kHid, &c->launches);
-    c->launches += 2;
+  int rc = grad_kernel_ready(c->device);
+  if (rc) return rc;
+  if (!s.part && cudaMalloc(&s.part, kPartFloats * 4) != cudaSuccess) {
+    cudaGetLastError();
+    s.part = nullptr;
+    return report_error(MVG_ERR_NOMEM, "MLP gradient allocation failed");
   }
+  float* part_w[3] = {s.part, s.part + (int64_t)kGradSplits * kHid * kIn,
+                      s.part + (int64_t)kGradSplits * kHid * (kIn + kHid)};
+  float* part_b[2] = {s.part + kPartW, s.part + kPartW + kPartB};
+  float* part_top = s.part + kPartW + 2 * kPartB;
+  const int64_t offW[4] = {kOffW1, kOffW2, kOffW3, kOffW4};
+  const int64_t offB[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
+
+  const int64_t top_rows = ((n + kGradTopParts - 1) / kGradTopParts + 15) / 16 * 16;
+  const int top = (int)((n + top_rows - 1) / top_rows);
+  k_grad_top<<<top, kHid, 0, st>>>(s.out, tgt, s.wb + kOffW4, s.z[2], s.h[2], n, top_rows, s.dz[2], part_top);
+  const int zrows = (int)std::min<int64_t>(kGradParts, (n + kGradTile - 1) / kGradTile);
+  for (int q = 1; q >= 0; --q)
+    k_grad_z<<<dim3(kHid / kGradTile, zrows), kGradThreads, kGradZSmem, st>>>(s.dz[q + 1], s.wb + offW[q + 1], s.z[q],
+                                                                             n, s.dz[q], part_b[q]);
+  const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(kGradSplits, n / kGradSplitRows));
+  const int64_t rows = ((n + splits - 1) / splits + kGradK - 1) / kGradK * kGradK;
+  GradWs W;
+  int tiles = 0;
+  for (int q = 0; q < 3; ++q) {
+    const int din = q == 0 ? kIn : kHid;
+    const __nv_bfloat16* in = q == 0 ? X : s.h[q - 1];
+    W.l[q] = {s.dz[q], in, part_w[q], din, ((uintptr_t)in & 15) == 0, tiles};
+    tiles += kHid / kGradTile * ((din + kGradTile - 1) / kGradTile);
+  }
+  k_grad_w<<<dim3(tiles, splits), kGradThreads, 0, st>>>(W, n, rows);
+
+  GradSegs G;
+  int k = 0, blocks = 0;
+  auto seg = [&](const float* part, float* out, int64_t len, int64_t pitch, int parts, float scale = 1.f) {
+    G.s[k] = {part, out, len, pitch, parts, scale};
+    G.block[k++] = blocks;
+    blocks += (int)((len + 127) / 128);
+  };
+  for (int q = 0; q < 3; ++q) {
+    const int64_t len = (int64_t)kHid * (q == 0 ? kIn : kHid);
+    seg(part_w[q], s.g + offW[q], len, len, splits);
+    if (q < 2) seg(part_b[q], s.g + offB[q], kHid, kHid, zrows);
+  }
+  seg(part_top, s.g + offB[2], kHid, kTopPart, top);
+  seg(part_top + kHid, s.g + offW[3], kOut * kHid, kTopPart, top);
+  seg(part_top + 3 * kHid, s.g + offB[3], kOut, kTopPart, top);
+  seg(part_top + 3 * kHid + kOut, s.loss, 1, kTopPart, top, 1.f / (float)n);
+  G.block[k] = blocks;
+  k_grad_sum<<<blocks, 1024, 0, st>>>(G);
+  c->launches += 5;
+  MVG_CUDA_TRY(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace mvg
@@ -638,7 +625,7 @@ int mvg_mlp_grad_dev(mvg_handle h, const void* d_x_bf16, const float* d_target, 
   if (rc) return rc;
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
   mlp_forward(c, s, (const __nv_bfloat16*)d_x_bf16, n, n, true);
-  mlp_backward(c, s, (const __nv_bfloat16*)d_x_bf16, d_target, n);
+  if ((rc = mlp_backward(c, s, (const __nv_bfloat16*)d_x_bf16, d_target, n))) return rc;
   if (h_grads) MVG_CUDA_TRY(cudaMemcpyAsync(h_grads, s.g, kNumParams * 4, cudaMemcpyDeviceToHost, c->stream));
   float loss = 0;
   MVG_CUDA_TRY(cudaMemcpyAsync(&loss, s.loss, 4, cudaMemcpyDeviceToHost, c->stream));
@@ -659,7 +646,7 @@ int mvg_mlp_train_step_dev(mvg_handle h, const void* d_x_bf16, const float* d_ta
   if (rc) return rc;
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
   mlp_forward(c, s, (const __nv_bfloat16*)d_x_bf16, n, n, true);
-  mlp_backward(c, s, (const __nv_bfloat16*)d_x_bf16, d_target, n);
+  if ((rc = mlp_backward(c, s, (const __nv_bfloat16*)d_x_bf16, d_target, n))) return rc;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
   MVG_CUDA_TRY(cudaMemsetAsync(s.loss + 1, 0, 4, c->stream));
