@@ -421,7 +421,7 @@ static void mlp_forward(Ctx* c, MlpState& s, const __nv_bfloat16* X, int64_t n, 
       const int K = q == 0 ? kIn : kHid;
       const int64_t a_rows = q == 0 ? x_rows : rows8(n);
       ok = a_rows % 8 == 0 && tc_map(&ma[q], q == 0 ? X : s.h[q - 1], a_rows, K, K, kTcM) &&
-           tc_map(&mw[q], s.wb + offW[q], kTcN, K, K, kTcN);
+           tc_map(&mw[q], s.wb + offW[q], kHid, K, K, kTcN);
     }
     if (ok) {
       for (int q = 0; q < 3; ++q) {
@@ -434,8 +434,18 @@ static void mlp_forward(Ctx* c, MlpState& s, const __nv_bfloat16* X, int64_t n, 
           ep.b_out = s.w + kOffB4;
           ep.out = s.out;
         }
-        k_mlp_layer_tc<<<(int)((n + kTcM - 1) / kTcM), kTcThreads, kTcSmem, st>>>(ma[q], mw[q], nn,
-                                                                                   q == 0 ? kIn : kHid, ep, c->d_err);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)((n + kTcM - 1) / kTcM * kTcParts));
+        cfg.blockDim = dim3(kTcThreads);
+        cfg.dynamicSmemBytes = kTcSmem;
+        cfg.stream = st;
+        cudaLaunchAttribute cluster;
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = kTcParts;
+        cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+        cfg.attrs = &cluster;
+        cfg.numAttrs = q == 2;
+        cudaLaunchKernelEx(&cfg, k_mlp_layer_tc, ma[q], mw[q], nn, q == 0 ? kIn : kHid, ep, c->d_err);
       }
       c->launches += 3;
       ++c->mlp_tc_passes;

@@ -7,15 +7,22 @@
 // epilogue (out = H W4^T + b4, with H rounded to bf16 as the next GEMM's
 // operand would be).
 //
-// A CTA of 128 threads owns 128 rows and all 256 columns: the accumulator
-// is 128 TMEM lanes x 256 fp32 columns (tcgen05.alloc).  K moves in chunks
-// of 64 through a two-stage shared-memory ring filled by TMA: thread 0
-// issues the two tile loads of a stage (A 128 x 64, W 256 x 64, 48 KB) on
-// the stage's "full" mbarrier; thread 32 waits for it, issues four
-// tcgen05.mma.kind::f16 (M 128, N 256, K 16) and commits them to the
-// stage's "empty" mbarrier, which frees the stage for the next load.  Two
-// CTAs fit on an SM (96 KB of stages each, 512 TMEM columns in all), so one
-// CTA's epilogue runs under the other's main loop.
+// A CTA of 128 threads owns 128 rows and 64 of the 256 columns: the
+// accumulator is 128 TMEM lanes x 64 fp32 columns (tcgen05.alloc).  K moves
+// in chunks of 64 through a ring of shared-memory stages filled by TMA:
+// thread 0 issues the two tile loads of a stage (A 128 x 64, W 64 x 64, 24
+// KB) on the stage's "full" mbarrier; thread 32 waits for it, issues four
+// tcgen05.mma.kind::f16 (M 128, N 64, K 16) and commits them to the stage's
+// "empty" mbarrier, which frees the stage for the next load.  Two CTAs fit on
+// an SM, so one CTA's epilogue runs under the other's main loop.
+//
+// Blocks and the epilogue's erff bound it, not the products: at 4,096 rows
+// CTAs of all 256 columns left 120 of 152 SMs idle, and a thread per row wrote
+// 256 columns row by row (39 us a layer).  64 columns per CTA and stores by
+// way of shared memory, 128 bytes of a row at a time, take the three layers
+// and their call from 136 to 75 us (100,000 rows: 443 to 425).  In the
+// last layer the four CTAs of a row tile are a cluster and hand the output's
+// running sums on in column order, so that they add up as in one thread.
 //
 // Shared-memory operand layout: 8 x 8 core matrices (8 rows of 16 bytes)
 // without swizzle, K-major.  The tensor maps view a K-contiguous bf16
@@ -36,9 +43,10 @@
 
 namespace mvg {
 
-constexpr int kTcM = 128, kTcN = 256, kTcK = 64, kTcStages = 2, kTcThreads = 128;
+constexpr int kTcM = 128, kTcN = 64, kTcK = 64, kTcStages = 3, kTcThreads = 128;
+constexpr int kTcParts = kHid / kTcN;  // CTAs per row tile
 constexpr uint32_t kTcBytesA = kTcM * kTcK * 2;  // 16 KB
-constexpr uint32_t kTcBytesB = kTcN * kTcK * 2;  // 32 KB
+constexpr uint32_t kTcBytesB = kTcN * kTcK * 2;  // 8 KB
 constexpr uint32_t kTcStageBytes = kTcBytesA + kTcBytesB;
 constexpr uint32_t kTcSmem = kTcStages * kTcStageBytes + 1024;  // + alignment slack
 constexpr unsigned long long kTcWaitNs = 1ull << 30;
@@ -97,6 +105,10 @@ __device__ __forceinline__ void tc_load(uint32_t dst, const CUtensorMap* map, in
       : "memory");
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
 __global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const __grid_constant__ CUtensorMap map_a,
                                                              const __grid_constant__ CUtensorMap map_w, int M, int K,
                                                              TcEpilogue ep, uint32_t* err) {
@@ -104,9 +116,11 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const __grid_consta
   __shared__ __align__(8) uint64_t s_full[kTcStages], s_empty[kTcStages], s_done;
   __shared__ uint32_t s_tmem;
   __shared__ int s_fail, s_issued, s_consumed;
+  __shared__ float2 s_out[kTcThreads];  // the output layer's sums over the columns before this CTA's
   const uint32_t base = ((uint32_t)__cvta_generic_to_shared(tc_smem) + 1023u) & ~1023u;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * kTcM;
+  const int part = (int)blockIdx.x % kTcParts;
+  const int n0 = part * kTcN, m0 = (int)blockIdx.x / kTcParts * kTcM;
   const int nk = (K + kTcK - 1) / kTcK;
   const uint32_t full0 = (uint32_t)__cvta_generic_to_shared(&s_full[0]);
   const uint32_t empty0 = (uint32_t)__cvta_generic_to_shared(&s_empty[0]);
@@ -149,7 +163,7 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const __grid_consta
                    "r"(kTcStageBytes)
                    : "memory");
       tc_load(sa, &map_a, i * (kTcK / 8), m0 / 8, full0 + 8 * s);
-      tc_load(sb, &map_w, i * (kTcK / 8), 0, full0 + 8 * s);
+      tc_load(sb, &map_w, i * (kTcK / 8), n0 / 8, full0 + 8 * s);
     }
     s_issued = i;
   } else if (tid == 32) {  // MMA issuer
@@ -193,12 +207,16 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const __grid_consta
     for (int i = s_consumed; i < s_issued; ++i) tc_wait(full0 + 8 * (i % kTcStages), (uint32_t)(i / kTcStages) & 1u);
   }
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  // warp w reads TMEM lanes 32 w .. 32 w + 31: lane t holds row m0 + 32 w + t
+  const int row0 = m0 + wid * 32, row = row0 + lane;
+  uint32_t hb[kTcN / 2];  // this row's activations
   if (ok) {
-    // warp w reads TMEM lanes 32 w .. 32 w + 31: lane t holds row m0 + 32 w + t
-    const int row = m0 + wid * 32 + lane;
-    const bool live = row < M;
-    float o0 = 0.f, o1 = 0.f;
-#pragma unroll 1
+    // the stages are free: 32 rows of 32 columns per warp, rows 36 words apart
+    // (a row's four-word pieces fall into distinct banks across eight rows)
+    constexpr int kPitch = 36;
+    float* const tile = reinterpret_cast<float*>(tc_smem + (base - (uint32_t)__cvta_generic_to_shared(tc_smem))) +
+                        wid * 32 * kPitch;
+#pragma unroll
     for (int c0 = 0; c0 < kTcN; c0 += 32) {
       uint32_t v[32];
       const uint32_t taddr = tmem + ((uint32_t)(wid * 32) << 16) + (uint32_t)c0;
@@ -212,36 +230,75 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const __grid_consta
           : "r"(taddr)
           : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-      if (!live) continue;
       float x[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]) + __ldg(ep.bias + c0 + j);
+      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]) + __ldg(ep.bias + n0 + c0 + j);
       if (ep.z) {
-        float4* dz = reinterpret_cast<float4*>(ep.z + (int64_t)row * kTcN + c0);
+        __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 8; ++q) dz[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<float4*>(tile + lane * kPitch + 4 * q) =
+              make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {  // four rows at a time, eight lanes each
+          const int r = 4 * q + (lane >> 3);
+          if (row0 + r < M)
+            *reinterpret_cast<float4*>(ep.z + (int64_t)(row0 + r) * kHid + n0 + c0 + 4 * (lane & 7)) =
+                *reinterpret_cast<const float4*>(tile + r * kPitch + 4 * (lane & 7));
+        }
       }
-      uint32_t hb[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const __nv_bfloat162 pr = __floats2bfloat162_rn(gelu(x[2 * j]), gelu(x[2 * j + 1]));
-        hb[j] = *reinterpret_cast<const uint32_t*>(&pr);
-        if (ep.w_out) {
-          const float2 hf = __bfloat1622float2(pr);
-          const int cc = c0 + 2 * j;
-          o0 += hf.x * __bfloat162float(ep.w_out[cc]) + hf.y * __bfloat162float(ep.w_out[cc + 1]);
-          o1 += hf.x * __bfloat162float(ep.w_out[kTcN + cc]) + hf.y * __bfloat162float(ep.w_out[kTcN + cc + 1]);
-        }
-      }
-      if (ep.h) {
-        uint4* dh = reinterpret_cast<uint4*>(ep.h + (int64_t)row * kTcN + c0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dh[q] = make_uint4(hb[4 * q], hb[4 * q + 1], hb[4 * q + 2], hb[4 * q + 3]);
+        hb[c0 / 2 + j] = *reinterpret_cast<const uint32_t*>(&pr);
       }
     }
-    if (ep.w_out && live) {
-      ep.out[(int64_t)row * 2] = o0 + ep.b_out[0];
-      ep.out[(int64_t)row * 2 + 1] = o1 + ep.b_out[1];
+    if (ep.h) {
+      uint32_t* const words = reinterpret_cast<uint32_t*>(tile);
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<uint4*>(words + lane * kPitch + 4 * q) =
+            make_uint4(hb[4 * q], hb[4 * q + 1], hb[4 * q + 2], hb[4 * q + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int r = 4 * q + (lane >> 3);
+        if (row0 + r < M)
+          *reinterpret_cast<uint4*>(ep.h + (int64_t)(row0 + r) * kHid + n0 + 8 * (lane & 7)) =
+              *reinterpret_cast<const uint4*>(words + r * kPitch + 4 * (lane & 7));
+      }
+    }
+  }
+  if (ep.w_out) {  // the CTAs of the cluster in turn
+    float o0 = 0.f, o1 = 0.f;
+    cluster_sync();
+    for (int turn = 0; turn < kTcParts; ++turn) {
+      if (turn == part && ok) {
+        if (turn > 0) {
+          o0 = s_out[tid].x;
+          o1 = s_out[tid].y;
+        }
+#pragma unroll
+        for (int j = 0; j < kTcN / 2; ++j) {
+          const float2 hf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hb[j]));
+          const int cc = n0 + 2 * j;
+          o0 += hf.x * __bfloat162float(ep.w_out[cc]) + hf.y * __bfloat162float(ep.w_out[cc + 1]);
+          o1 += hf.x * __bfloat162float(ep.w_out[kHid + cc]) + hf.y * __bfloat162float(ep.w_out[kHid + cc + 1]);
+        }
+        if (turn < kTcParts - 1) {
+          uint32_t there;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                       : "=r"(there)
+                       : "r"((uint32_t)__cvta_generic_to_shared(&s_out[tid])), "r"(turn + 1));
+          asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(there), "f"(o0), "f"(o1) : "memory");
+        } else if (row < M) {
+          ep.out[(int64_t)row * 2] = o0 + ep.b_out[0];
+          ep.out[(int64_t)row * 2 + 1] = o1 + ep.b_out[1];
+        }
+      }
+      if (turn < kTcParts - 1) cluster_sync();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
