@@ -34,7 +34,7 @@
 // there, and a stage that meets an error leaves it in the error word, which
 // the later stages test.  (Flags, scans and candidates as separate passes
 // over the LUT, 35 launches and nine waits, took 396 us for 4.6 million
-// bases in 64 blocks; this takes 215.)
+// bases in 64 blocks; this takes 189.)
 #include "mvg_internal.h"
 #include "prim.cuh"
 
@@ -285,21 +285,22 @@ __global__ void __launch_bounds__(256) k_fix_zero(int32_t* lut, int64_t n, const
 
 enum FillMode : int { kFill = 0, kSmooth = 1 };
 
-__device__ __forceinline__ bool gap_start(const int32_t* lut, int64_t i, int mode) {
-  const int32_t lo = lut[i - 1], m = lut[i];
+__device__ __forceinline__ bool gap_start(int32_t lo, int32_t m, int mode) {  // of lut[i - 1], lut[i]
   if (lo == -1) return false;
   return mode == kSmooth ? m != (int32_t)((uint32_t)lo + 1u) : m == -1;
 }
 
-// A tile's gap starts in order: thread t of step j looks at entry 256 j + t,
-// and s_at[8 j + warp] gets the tile's gap starts before that warp's.
-__device__ __forceinline__ uint32_t tile_starts(const int32_t* lut, int64_t n, int mode, int64_t t0,
-                                                unsigned (&ball)[kTile / 256], uint32_t* s_at) {
+// A tile's gap starts: thread t of step j looks at entry 256 j + t (m[j]; the
+// entry before it lo[j]), and s_at[8 j + warp] gets the tile's gap starts
+// before that warp's.  Returns their number.
+__device__ __forceinline__ uint32_t tile_starts(const int32_t (&lo)[kTile / 256], const int32_t (&m)[kTile / 256],
+                                                int64_t n, int mode, int64_t t0, unsigned (&ball)[kTile / 256],
+                                                uint32_t* s_at) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < kTile / 256; ++j) {
     const int64_t i = t0 + 256 * j + threadIdx.x;
-    ball[j] = __ballot_sync(0xffffffffu, i > 0 && i < n && gap_start(lut, i, mode));
+    ball[j] = __ballot_sync(0xffffffffu, i > 0 && i < n && gap_start(lo[j], m[j], mode));
     if (lane == 0) s_at[8 * j + wid] = __popc(ball[j]);
   }
   __syncthreads();
@@ -320,69 +321,94 @@ __global__ void __launch_bounds__(256) k_fill_count(int32_t* lut, int64_t n, int
     fix_zero(lut, n, z, err);
     __syncthreads();
   }
+  const int64_t t0 = (int64_t)blockIdx.x * kTile;
+  int32_t lo[kTile / 256], m[kTile / 256];
+#pragma unroll
+  for (int j = 0; j < kTile / 256; ++j) {
+    const int64_t i = t0 + 256 * j + threadIdx.x;
+    m[j] = i < n ? lut[i] : 0;
+    lo[j] = __shfl_up_sync(0xffffffffu, m[j], 1);
+    if ((threadIdx.x & 31) == 0 && i > 0 && i < n) lo[j] = lut[i - 1];
+  }
   unsigned ball[kTile / 256];
-  const uint32_t count = tile_starts(lut, n, mode, (int64_t)blockIdx.x * kTile, ball, s_at);
+  const uint32_t count = tile_starts(lo, m, n, mode, t0, ball, s_at);
   if (threadIdx.x == 0) tile[blockIdx.x] = count;
 }
 
 // Gap starts g (lower = g-1, L = lut[lower]) in order, and the first u in
 // g+1 .. min(n-1, g+width) with lut[u] - L == u - lower (int32 arithmetic),
-// reach = u, or g when there is none.  A thread tries the next eight entries
-// itself (a substitution's partner is the next one); what is left the warp
-// searches together, 32 entries per step.
+// reach = u, or g when there is none.  The tile is in shared memory, its gap
+// starts are listed there, and a thread per gap start tries the next eight
+// entries (a substitution's partner is the next one); what is left the warp
+// searches together, 32 entries per step.  (From global memory, a thread per
+// entry: 36 us for 4.6 million entries that are not in L2; this takes 16.)
 __global__ void __launch_bounds__(256) k_fill_search(const int32_t* __restrict__ lut, int64_t n, int width, int mode,
                                                      const uint32_t* __restrict__ tile, int32_t* __restrict__ cand,
                                                      int32_t* __restrict__ reach, int32_t* __restrict__ lval,
                                                      const uint32_t* err) {
+  constexpr int kProbe = 8;
   __shared__ uint32_t s_at[kTile / 32];
+  __shared__ int32_t s_lut[kTile + 1 + kProbe];  // entries t0 - 1 ..
+  __shared__ uint16_t s_start[kTile];
   if (err && *(const volatile uint32_t*)err) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t t0 = (int64_t)blockIdx.x * kTile;
-  unsigned ball[kTile / 256];
-  if (tile_starts(lut, n, mode, t0, ball, s_at) == 0) return;
-  const uint32_t first = tile[blockIdx.x];
-#pragma unroll 1
-  for (int j = 0; j < kTile / 256; ++j) {
-    unsigned b = ball[0];  // ball[j]; the array stays in registers
+  int32_t lo[kTile / 256], m[kTile / 256];
 #pragma unroll
-    for (int q = 1; q < kTile / 256; ++q) b = j == q ? ball[q] : b;
-    if (b == 0) continue;
-    const int64_t gs = t0 + 256 * j + threadIdx.x, lower = gs - 1;
-    const uint32_t at = first + s_at[8 * j + wid] + __popc(b & ((1u << lane) - 1u));
-    const int64_t last = gs + width < n - 1 ? gs + width : n - 1;
-    bool open = b >> lane & 1;
-    int32_t L = 0;
+  for (int j = 0; j < kTile / 256; ++j) {
+    const int64_t i = t0 + 256 * j + threadIdx.x;
+    m[j] = i < n ? lut[i] : 0;
+  }
+  if (threadIdx.x <= kProbe) {
+    const int64_t i = threadIdx.x == 0 ? t0 - 1 : t0 + kTile + threadIdx.x - 1;
+    s_lut[threadIdx.x == 0 ? 0 : kTile + threadIdx.x] = i >= 0 && i < n ? lut[i] : 0;
+  }
+#pragma unroll
+  for (int j = 0; j < kTile / 256; ++j) s_lut[1 + 256 * j + threadIdx.x] = m[j];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kTile / 256; ++j) lo[j] = s_lut[256 * j + threadIdx.x];
+  unsigned ball[kTile / 256];
+  const int count = (int)tile_starts(lo, m, n, mode, t0, ball, s_at);
+#pragma unroll
+  for (int j = 0; j < kTile / 256; ++j)
+    if (ball[j] >> lane & 1)
+      s_start[s_at[8 * j + wid] + __popc(ball[j] & ((1u << lane) - 1u))] = (uint16_t)(256 * j + threadIdx.x);
+  __syncthreads();
+  const uint32_t first = tile[blockIdx.x];
+  for (int k0 = wid * 32; k0 < count; k0 += 256) {
+    const int k = k0 + lane;
+    bool open = k < count;
+    const int q = open ? s_start[k] : 0;
+    const int64_t gs = t0 + q;
+    const int32_t L = s_lut[q];
     if (open) {
-      L = lut[lower];
-      cand[at] = (int32_t)gs;
-      lval[at] = L;
+      cand[first + k] = (int32_t)gs;
+      lval[first + k] = L;
+      // entries gs + 1 .. last that this thread tries
+      const int64_t last = gs + width < n - 1 ? gs + width : n - 1;
+      const int tries = last - gs < kProbe ? (int)(last - gs) : kProbe;
       int32_t u = (int32_t)gs;
-#pragma unroll 1
-      for (int64_t up = gs + 1; up <= gs + 8; ++up) {
-        if (up > last) {
+      for (int d = 1; d <= tries; ++d)
+        if ((int32_t)((uint32_t)s_lut[q + 1 + d] - (uint32_t)L) == d + 1) {
+          u = (int32_t)gs + d;
           open = false;
           break;
         }
-        if ((int32_t)((uint32_t)lut[up] - (uint32_t)L) == (int32_t)(up - lower)) {
-          u = (int32_t)up;
-          open = false;
-          break;
-        }
-      }
-      reach[at] = u;
+      open = open && last - gs > kProbe;
+      reach[first + k] = u;
     }
     for (unsigned left = __ballot_sync(0xffffffffu, open); left; left &= left - 1) {
       const int src = __ffs(left) - 1;
-      const int64_t g0 = gs - lane + src, l0 = g0 - 1;
+      const int64_t g0 = t0 + __shfl_sync(0xffffffffu, q, src), l0 = g0 - 1;
       const int64_t end = g0 + width < n - 1 ? g0 + width : n - 1;
       const int32_t L0 = __shfl_sync(0xffffffffu, L, src);
-      const uint32_t a0 = __shfl_sync(0xffffffffu, at, src);
-      for (int64_t base = g0 + 9; base <= end; base += 32) {
+      for (int64_t base = g0 + 1 + kProbe; base <= end; base += 32) {
         const int64_t up = base + lane;
         const unsigned hit = __ballot_sync(
             0xffffffffu, up <= end && (int32_t)((uint32_t)lut[up] - (uint32_t)L0) == (int32_t)(up - l0));
         if (hit) {
-          if (lane == 0) reach[a0] = (int32_t)(base + __ffs(hit) - 1);
+          if (lane == 0) reach[first + k0 + src] = (int32_t)(base + __ffs(hit) - 1);
           break;
         }
       }
