@@ -33,52 +33,57 @@ constexpr float kGapOpen = -400.0f;
 constexpr float kGapExtend = 0.0f;
 constexpr float kTermGap = kGapOpen / 2;  // TERMGAPS_Half
 constexpr unsigned kSmoothWindow = 21;
-constexpr double kSmoothCeil = 999.0;
-constexpr double kMinBestColScore = 90.0;
-constexpr double kMinSmoothScore = 90.0;
+constexpr float kSmoothCeil = 999.0f;
+constexpr float kMinBestColScore = 90.0f;
+constexpr float kMinSmoothScore = 90.0f;
 constexpr unsigned kAnchorSpacing = 96;
 constexpr unsigned kInsane = 0xffffffffu;
 
-bool is_gap(uint8_t c) { return c == '-' || c == '.'; }
-
-// DNA letter of a column character; 4 (the wildcard) for anything else.
-unsigned letter(uint8_t c) {
-  switch (c) {
-    case 'A': case 'a': return 0;
-    case 'C': case 'c': return 1;
-    case 'G': case 'g': return 2;
-    case 'T': case 't': case 'U': case 'u': return 3;
-    default: return 4;
+// Per character: its DNA letter, 4 (the wildcard) for anything else, with bit
+// 3 set for a gap character; per letter pair: the centred score, 0 where
+// either is no base.
+struct Tables {
+  uint8_t letter[256];
+  float pair[8][8];
+  Tables() {
+    for (int c = 0; c < 256; ++c) letter[c] = 4;
+    for (int k = 0; k < 4; ++k) letter["ACGT"[k] + 0u] = letter["acgt"[k] + 0u] = (uint8_t)k;
+    letter[(int)'U'] = letter[(int)'u'] = 3;
+    letter[(int)'-'] = letter[(int)'.'] = 4 | 8;
+    for (int i = 0; i < 8; ++i)
+      for (int j = 0; j < 8; ++j) pair[i][j] = i < 4 && j < 4 ? kNucSp[i][j] + kCenter : 0.0f;
   }
-}
+};
+const Tables kTables;
 
-// The per-column score of LetterObjScoreXP for the pair (one sequence each).
-void column_scores(const uint8_t* a, const uint8_t* b, unsigned n, std::vector<float>& score) {
-  std::vector<float> mm(n, 0.0f), gg(n, 0.0f);
+// The per-column score of LetterObjScoreXP for the pair (one sequence each):
+// the letters' scores, then each gap run's penalty spread over its columns
+// (every column is in one run at most, so this is the same one addition).
+void column_scores(const uint8_t* a, const uint8_t* b, unsigned n, float* score) {
+  const Tables& T = kTables;
+  auto both_gaps = [&](unsigned c) { return (T.letter[a[c]] & T.letter[b[c]] & 8) != 0; };
   unsigned start = 0, end = n - 1;
   for (unsigned c = 0; c < n; ++c)
-    if (!is_gap(a[c]) || !is_gap(b[c])) {
+    if (!both_gaps(c)) {
       start = c;
       break;
     }
   for (int c = (int)n - 1; c >= 0; --c)
-    if (!is_gap(a[c]) || !is_gap(b[c])) {
+    if (!both_gaps((unsigned)c)) {
       end = (unsigned)c;
       break;
     }
-  for (unsigned c = start; c <= end; ++c) {
-    const unsigned l1 = letter(a[c]), l2 = letter(b[c]);
-    if (l1 >= 4 || l2 >= 4) continue;
-    mm[c] = (float)kNucSp[l1][l2] + kCenter;
-  }
+  for (unsigned c = 0; c < start; ++c) score[c] = 0.0f;
+  for (unsigned c = end + 1; c < n; ++c) score[c] = 0.0f;
   bool gapping[2] = {false, false};
   unsigned gap_left = 0;
   float cur = 0.0f;
   for (unsigned c = start; c <= end; ++c) {
-    const bool g[2] = {is_gap(a[c]), is_gap(b[c])};
-    if (g[0] && g[1]) continue;
-    if (g[0] || g[1]) {
-      const int q = g[0] ? 0 : 1;
+    const unsigned l1 = T.letter[a[c]], l2 = T.letter[b[c]];
+    score[c] = T.pair[l1 & 7][l2 & 7];
+    if ((l1 | l2) & 8) {
+      if (l1 & l2 & 8) continue;
+      const int q = l1 & 8 ? 0 : 1;
       if (!gapping[q]) {
         gap_left = c;
         cur += c == start ? kTermGap : kGapOpen;
@@ -90,7 +95,7 @@ void column_scores(const uint8_t* a, const uint8_t* b, unsigned n, std::vector<f
     }
     if (gapping[0] || gapping[1]) {  // spread the run's penalty over its columns
       const float per_site = cur / (float)(c - gap_left);
-      for (unsigned k = gap_left; k < c; ++k) gg[k] = per_site;
+      for (unsigned k = gap_left; k < c; ++k) score[k] += per_site;
       gap_left = kInsane;
       cur = 0.0f;
     }
@@ -100,43 +105,38 @@ void column_scores(const uint8_t* a, const uint8_t* b, unsigned n, std::vector<f
     cur -= kGapOpen;
     cur += kTermGap;
     const float per_site = cur / (float)(n - gap_left);
-    for (unsigned k = gap_left; k < n; ++k) gg[k] = per_site;
+    for (unsigned k = gap_left; k < n; ++k) score[k] += per_site;
   }
-  score.assign(n, 0.0f);
-  const float w = 1.0f;  // sequence weight product of two one-sequence profiles
-  for (unsigned c = 0; c < n; ++c) score[c] += w * (mm[c] + gg[c]);
 }
 
-float ceil_score(float x) { return (float)(x > kSmoothCeil ? kSmoothCeil : x); }
+float ceil_score(float x) { return x > kSmoothCeil ? kSmoothCeil : x; }
 
 }  // namespace
 }  // namespace mvg
 
 using namespace mvg;
 
-void mvg::anchor_columns(const uint8_t* row_a, const uint8_t* row_b, unsigned n, std::vector<unsigned>& out) {
+void mvg::anchor_columns(const uint8_t* row_a, const uint8_t* row_b, unsigned n, std::vector<unsigned>& out,
+                         AnchorScratch& scratch) {
   out.clear();
   if (n == 0) return;
-  std::vector<float> score, smooth(n, 0.0f);
+  std::vector<unsigned>& best = scratch.best;
+  if (scratch.score.size() < n) scratch.score.resize(n);
+  float* const score = scratch.score.data();
   column_scores(row_a, row_b, n, score);
-  // WindowSmooth
+  // WindowSmooth, and FindBestColsComboPP on the columns it covers (the
+  // others' smoothed score is 0)
+  best.clear();
   if (n > kSmoothWindow) {
     const unsigned w2 = kSmoothWindow / 2;
     float total = 0.0f;
     for (unsigned i = 0; i < kSmoothWindow; ++i) total += ceil_score(score[i]);
     for (unsigned i = w2;; ++i) {
-      smooth[i] = total / (float)kSmoothWindow;
+      if (score[i] >= kMinBestColScore && total / (float)kSmoothWindow >= kMinSmoothScore) best.push_back(i);
       if (i == n - w2 - 1) break;
       total -= ceil_score(score[i - w2]);
       total += ceil_score(score[i + w2 + 1]);
     }
-  }
-  // FindBestColsComboPP
-  std::vector<unsigned> best;
-  for (unsigned c = 0; c < n; ++c) {
-    if (score[c] < kMinBestColScore) continue;
-    if (smooth[c] < kMinSmoothScore) continue;
-    best.push_back(c);
   }
   // MergeBestCols: two candidates within a window keep the better scoring;
   // more keep the one nearest the first, among all but the window's last
@@ -174,7 +174,8 @@ extern "C" int mvg_anchor_columns(const uint8_t* row_a, const uint8_t* row_b, ui
   if (!ncols_out || (ncols && (!row_a || !row_b)) || (cap && !cols)) return report_error(MVG_ERR_ARG, "null argument");
   if (ncols >= (1ull << 31)) return report_error(MVG_ERR_ARG, "window longer than 2^31 columns");
   std::vector<unsigned> found;
-  anchor_columns(row_a, row_b, (unsigned)ncols, found);
+  AnchorScratch scratch;
+  anchor_columns(row_a, row_b, (unsigned)ncols, found, scratch);
   const uint64_t m = found.size();
   for (uint64_t k = 0; k < m && k < cap; ++k) cols[k] = found[k];
   *ncols_out = m;

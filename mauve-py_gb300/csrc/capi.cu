@@ -72,6 +72,21 @@ int check_device_error(Ctx* c) {
   }
 }
 
+uint8_t* pinned_buf(Ctx* c, int which, size_t need) {
+  if (c->h_rows_cap[which] < need) {
+    if (c->h_rows[which]) cudaFreeHost(c->h_rows[which]);
+    c->h_rows[which] = nullptr;
+    c->h_rows_cap[which] = 0;
+    if (cudaMallocHost(&c->h_rows[which], need + need / 4) != cudaSuccess) {
+      cudaGetLastError();
+      c->h_rows[which] = nullptr;
+      return nullptr;
+    }
+    c->h_rows_cap[which] = need + need / 4;
+  }
+  return (uint8_t*)c->h_rows[which];
+}
+
 int upload_base_table();
 int upload_score_table();
 

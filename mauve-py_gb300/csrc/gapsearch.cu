@@ -632,22 +632,8 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   k_gs_out<<<ng, 64, 0, c->stream>>>(d_rows, gap_row, kept, at, d_gaps, d_out);
   c->launches += 4;
   stage_mark(c, "gs_copy");
-  auto pinned = [&](size_t need) -> uint8_t* {
-    if (c->h_rows_cap[buf] < need) {
-      if (c->h_rows[buf]) cudaFreeHost(c->h_rows[buf]);
-      c->h_rows[buf] = nullptr;
-      c->h_rows_cap[buf] = 0;
-      if (cudaMallocHost(&c->h_rows[buf], need + need / 4) != cudaSuccess) {
-        cudaGetLastError();
-        c->h_rows[buf] = nullptr;
-        return nullptr;
-      }
-      c->h_rows_cap[buf] = need + need / 4;
-    }
-    return (uint8_t*)c->h_rows[buf];
-  };
   const size_t tab_bytes = ((size_t)ng * 4 + 2) * 4;
-  uint32_t* h = (uint32_t*)pinned(std::max(tab_bytes, (size_t)r.rows * 24 + 256));
+  uint32_t* h = (uint32_t*)pinned_buf(c, buf, std::max(tab_bytes, (size_t)r.rows * 24 + 256));
   if (!h) return report_error(MVG_ERR_NOMEM, "pinned allocation failed");
   MVG_CUDA_TRY(cudaMemcpyAsync(h, d_tab, tab_bytes, cudaMemcpyDeviceToHost, c->stream));
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -669,7 +655,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
     for (size_t k = 0; k < ch.todo.size(); ++k) ch.todo_at[k] = first[ch.todo[k]];
   }
   const size_t rows_at = (nout * 24 + 255) & ~(size_t)255;
-  uint8_t* base = pinned(rows_at + nrows * sizeof(Anchor));
+  uint8_t* base = pinned_buf(c, buf, rows_at + nrows * sizeof(Anchor));
   if (!base) return report_error(MVG_ERR_NOMEM, "pinned allocation failed");
   ch.out = (const int64_t*)base;
   ch.rows = (Anchor*)(base + rows_at);
@@ -690,7 +676,7 @@ static uint64_t gs_finish(GsChunk& ch, int64_t* out, uint64_t cap, uint64_t base
   uint64_t nrows = 0;
   for (uint32_t n : ch.todo_n) nrows += n;
   run_claimed((int)nt, host_threads_for(nrows), [&](int k) {
-    thread_local FilterScratch scratch;
+    FilterScratch scratch;
     ch.nkept[ch.todo[k]] = (uint32_t)filter_gap(ch.rows + ch.todo_at[k], ch.todo_n[k], ch.todo_q[k], scratch);
   });
   const int64_t* src = ch.out;

@@ -15,9 +15,13 @@ struct LcbWindow {
   int density;
 };
 
-// refineAlignment's windows of one LCB (LM/ProgressiveAligner.cpp:1119-1165).
-std::vector<LcbWindow> lcb_windows(const uint8_t* row_a, const uint8_t* row_b, uint64_t ncols,
-                                   double max_window_size);
+// Bases (columns that are not '-') of each row before every column.
+using LcbCounts = std::vector<uint64_t>[2];
+
+// refineAlignment's windows of one LCB (LM/ProgressiveAligner.cpp:1119-1165);
+// pre gets the rows' counts.
+std::vector<LcbWindow> lcb_windows(const uint8_t* row_a, const uint8_t* row_b, uint64_t ncols, double max_window_size,
+                                   LcbCounts& pre);
 
 // RefineW's column-window width for a density class in the final refinement
 // pass (0 = the window is left as it is).
@@ -25,6 +29,11 @@ uint64_t refine_width(int density);
 
 // MUSCLE's anchor columns of a window (FindAnchorColsPP for two sequences),
 // ascending.
-void anchor_columns(const uint8_t* row_a, const uint8_t* row_b, unsigned n, std::vector<unsigned>& cols);
+struct AnchorScratch {
+  std::vector<float> score;
+  std::vector<unsigned> best;
+};
+void anchor_columns(const uint8_t* row_a, const uint8_t* row_b, unsigned n, std::vector<unsigned>& cols,
+                    AnchorScratch& scratch);
 
 }  // namespace mvg

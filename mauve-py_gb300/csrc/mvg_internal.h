@@ -134,6 +134,9 @@ inline uint64_t packed_words(uint64_t n) { return (n * 2) / 32 + (((n * 2) % 32)
 
 int upload_base_table();
 int grid_for(uint64_t n, int threads);
+// One of the context's two kept pinned buffers (h_rows), grown to `need` bytes
+// (its contents are lost when it grows); null when the allocation fails.
+uint8_t* pinned_buf(Ctx* c, int which, size_t need);
 int pack_sequence(Ctx* c, const uint8_t* d_seq, uint64_t n, uint32_t* d_packed);
 int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
              uint64_t* d_mer_out, SmlKeys* keep, int slot_base);

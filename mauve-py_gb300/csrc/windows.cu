@@ -53,13 +53,18 @@ constexpr uint64_t kRefineWidth[3] = {0, 500, 200};
 
 // refineAlignment's windows of one LCB (removeLargeGapsPP, then halving by
 // IsDenseEnough), each with its density class.
-std::vector<Window> lcb_windows(const uint8_t* row_a, const uint8_t* row_b, uint64_t ncols, double max_window_size) {
+std::vector<Window> lcb_windows(const uint8_t* row_a, const uint8_t* row_b, uint64_t ncols, double max_window_size,
+                                LcbCounts& pre) {
   const uint8_t* rows[2] = {row_a, row_b};
   // prefix base counts, for the bases of any column range
-  std::vector<uint64_t> pre[2];
   for (int q = 0; q < 2; ++q) {
-    pre[q].assign(ncols + 1, 0);
-    for (uint64_t c = 0; c < ncols; ++c) pre[q][c + 1] = pre[q][c] + (rows[q][c] != '-');
+    pre[q].resize(ncols + 1);
+    uint64_t n = 0;
+    for (uint64_t c = 0; c < ncols; ++c) {
+      pre[q][c] = n;
+      n += rows[q][c] != '-';
+    }
+    pre[q][ncols] = n;
   }
   // removeLargeGapsPP: cut out every stretch of more than max_gap_length
   // columns in which the genomes are never aligned to each other, keeping
@@ -142,7 +147,8 @@ extern "C" int mvg_refine_windows(const uint8_t* row_a, const uint8_t* row_b, ui
   if (!nwindows || (ncols && (!row_a || !row_b)) || (cap && !windows) || !(max_window_size > kMinWindowSize))
     return report_error(MVG_ERR_ARG, "bad argument");
   *nwindows = 0;
-  const std::vector<Window> wins = lcb_windows(row_a, row_b, ncols, max_window_size);
+  LcbCounts pre;
+  const std::vector<Window> wins = lcb_windows(row_a, row_b, ncols, max_window_size, pre);
   uint64_t n = 0;
   for (const Window& w : wins) {
     if (n < cap) {
@@ -163,7 +169,8 @@ extern "C" int mvg_refine_fast_ranges(const uint8_t* row_a, const uint8_t* row_b
     return report_error(MVG_ERR_ARG, "bad argument");
   *nranges = 0;
   uint64_t n = 0;
-  for (const Window& w : lcb_windows(row_a, row_b, ncols, max_window_size)) {
+  LcbCounts pre;
+  for (const Window& w : lcb_windows(row_a, row_b, ncols, max_window_size, pre)) {
     const uint64_t width = kRefineWidth[w.density];
     if (w.gap || width == 0) continue;
     for (uint64_t lo = w.lo; lo < w.hi; lo += width) {  // RefineW's column windows (MU/refinew.cpp:113-118)
