@@ -311,7 +311,7 @@ int mvg_sml_build_dev(mvg_handle h, const uint8_t* d_seq, uint64_t n, uint64_t s
   int rc = pack_sequence(h, d_seq, n, g);
   if (rc) return rc;
   if (cnt) {
-    rc = sml_sort(h, g, cnt, s, d_pos_out, d_mer_out, nullptr, 0);
+    rc = sml_sort(h, g, cnt, s, d_pos_out, d_mer_out);
     if (rc) return rc;
   }
   return check_device_error(h);

@@ -139,7 +139,7 @@ int grid_for(uint64_t n, int threads);
 uint8_t* pinned_buf(Ctx* c, int which, size_t need);
 int pack_sequence(Ctx* c, const uint8_t* d_seq, uint64_t n, uint32_t* d_packed);
 int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
-             uint64_t* d_mer_out, SmlKeys* keep, int slot_base);
+             uint64_t* d_mer_out);
 // Both genomes' keys ((seed bits, strand, genome) with A = 0) sorted in one array.
 // The bucketed seed join (pair_buckets.cu) for at most kPairBucketMaxKeys
 // keys: tab[position in A] = position in B | reverse << 31 for every seed

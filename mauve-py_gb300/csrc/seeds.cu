@@ -10,7 +10,7 @@
 //                   strand bit, (2w+1) bits in all, which orders exactly like
 //                   the reference's 64-bit bmer.mer.
 //   radix sort      stable LSD over those 2w+1 bits (prim.cuh).
-//   k_seed_keys_pair  the pairwise matcher's keys: both genomes in one array,
+//   k_seed_keys_tiles the pairwise matcher's keys: both genomes in one array,
 //                   a genome bit below the SML key, sorted once.
 #include <string.h>
 
@@ -124,9 +124,9 @@ __global__ void k_seed_keys(const uint32_t* __restrict__ g, uint64_t count, Seed
   }
 }
 
-// Both genomes' keys in one array for the pairwise matcher: the SML key
-// (seed bits, strand bit) followed by a genome bit (A = 0, B = 1); values are
-// positions.  Sorted stably, every seed's occurrences in the two genomes are
+// With PAIR, both genomes' keys in one array for the pairwise matcher: the SML
+// key (seed bits, strand bit) followed by a genome bit (A = 0, B = 1); values
+// are positions.  Without, one genome's SML keys (cb = 0, pos unused).  Sorted stably, every seed's occurrences in the two genomes are
 // adjacent, each genome's in position order.  Blocks build the seed's gather
 // table once and then take sort tiles of os::kTile positions in turn.  With
 // 32-bit keys (weight <= 15) a thread makes the keys of 4 consecutive
@@ -134,13 +134,15 @@ __global__ void k_seed_keys(const uint32_t* __restrict__ g, uint64_t count, Seed
 // counts0 is null, each tile's first-pass digit counts are written as its
 // count row (counts0) and added into its chunk's sums (csum0), the layout
 // rts_sort_pairs reads when told the keys come counted.
-template <typename K>
-__global__ void __launch_bounds__(256) k_seed_keys_pair(const uint32_t* __restrict__ ga, uint64_t ca,
+template <typename K, bool PAIR>
+__global__ void __launch_bounds__(256) k_seed_keys_tiles(const uint32_t* __restrict__ ga, uint64_t ca,
                                                         const uint32_t* __restrict__ gb, uint64_t cb, SeedDesc s,
                                                         K* __restrict__ keys, uint32_t* __restrict__ pos,
                                                         uint32_t* __restrict__ counts0, uint32_t* __restrict__ csum0,
                                                         int64_t ntiles, int64_t ctiles) {
   constexpr bool k32 = sizeof(K) == 4;
+  // the key of strand-carrying seed bits m
+  auto key_of = [](auto m, bool in_b) { return (K)(PAIR ? m << 1 | (in_b ? 1 : 0) : m); };
   __shared__ uint32_t h[8][256];
   __shared__ __align__(8) uint32_t lutw[k32 ? 8 * 256 : 2 * 8 * 256];
   const int tid = threadIdx.x, wid = tid >> 5;
@@ -177,11 +179,11 @@ __global__ void __launch_bounds__(256) k_seed_keys_pair(const uint32_t* __restri
             const uint32_t f = gather_mer32(win, u, lut32, nb);
             const uint32_t r = revcomp_mer32(f, s.w);
             const uint32_t m = f < r ? f : r;
-            kk[u] = ((((m >> sh) << 1) | (m & 1u)) << 1) | (in_b ? 1u : 0u);
+            kk[u] = key_of((m >> sh) << 1 | (m & 1u), in_b);
           }
           *reinterpret_cast<uint4*>(keys + p0) = make_uint4(kk[0], kk[1], kk[2], kk[3]);
-          *reinterpret_cast<uint4*>(pos + p0) =
-              make_uint4((uint32_t)q0, (uint32_t)q0 + 1, (uint32_t)q0 + 2, (uint32_t)q0 + 3);
+          if constexpr (PAIR)
+            *reinterpret_cast<uint4*>(pos + p0) = make_uint4((uint32_t)q0, (uint32_t)q0 + 1, (uint32_t)q0 + 2, (uint32_t)q0 + 3);
           if (count) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) atomicAdd(&h[wid][kk[u] & 255u], 1u);
@@ -195,9 +197,9 @@ __global__ void __launch_bounds__(256) k_seed_keys_pair(const uint32_t* __restri
             const uint32_t f = gather_mer32(window64(in_b ? gb : ga, q), 0, lut32, nb);
             const uint32_t r = revcomp_mer32(f, s.w);
             const uint32_t m = f < r ? f : r;
-            const uint32_t key = ((((m >> sh) << 1) | (m & 1u)) << 1) | (in_b ? 1u : 0u);
+            const uint32_t key = key_of((m >> sh) << 1 | (m & 1u), in_b);
             keys[p] = (K)key;
-            pos[p] = (uint32_t)q;
+            if constexpr (PAIR) pos[p] = (uint32_t)q;
             if (count) atomicAdd(&h[wid][key & 255u], 1u);
           }
         }
@@ -211,9 +213,9 @@ __global__ void __launch_bounds__(256) k_seed_keys_pair(const uint32_t* __restri
         const bool in_b = p >= ca;
         const uint64_t q = in_b ? p - ca : p;
         const uint64_t m = canonical_mer_lut(in_b ? gb : ga, q, lut64, nb, s.w);
-        const K key = (K)(((((m >> shift) << 1) | (m & 1ull)) << 1) | (in_b ? 1ull : 0ull));
+        const K key = key_of((m >> shift) << 1 | (m & 1ull), in_b);
         keys[p] = key;
-        pos[p] = (uint32_t)q;
+        if constexpr (PAIR) pos[p] = (uint32_t)q;
         if (count) atomicAdd(&h[wid][(uint32_t)key & 255u], 1u);
       }
     }
@@ -258,30 +260,41 @@ int pack_sequence(Ctx* c, const uint8_t* d_seq, uint64_t n, uint32_t* d_packed) 
 
 template <typename K>
 static int sml_sort_impl(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
-                         uint64_t* d_mer_out, SmlKeys* keep, int sb) {
+                         uint64_t* d_mer_out) {
   const int nbits = 2 * s.w + 1;
   Workspace& ws = c->ws;
-  K* k0 = (K*)ws.get(c, sb + 0, count * sizeof(K));
-  K* k1 = (K*)ws.get(c, sb + 1, count * sizeof(K));
-  uint32_t* v0 = (uint32_t*)ws.get(c, sb + 2, count * sizeof(uint32_t));
-  uint32_t* v1 = (uint32_t*)ws.get(c, sb + 3, count * sizeof(uint32_t));
-  uint32_t* scr = (uint32_t*)ws.get(c, sb + 4, sort_scratch_words(count, nbits) * sizeof(uint32_t));
+  uint32_t* scr = (uint32_t*)ws.get(c, 4, sort_scratch_words(count, nbits) * sizeof(uint32_t));
+  K* k0 = (K*)ws.get(c, 0, count * sizeof(K));
+  if (count < (1ull << 31)) {  // the reduce-then-scan sort's range
+    constexpr bool pairs = sizeof(K) == 4;
+    K* const keys[2] = {k0, pairs ? nullptr : (K*)ws.get(c, 1, count * sizeof(K))};
+    void* const buf[2] = {ws.get(c, 2, count * (pairs ? 8 : 4)), ws.get(c, 3, count * (pairs ? 8 : 4))};
+    if (!k0 || (!pairs && !keys[1]) || !buf[0] || !buf[1] || !scr)
+      return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
+    const RtsGeom g = rts_geom((int64_t)count, nbits);
+    uint32_t* csum = rts_csum(scr, g);
+    MVG_CUDA_TRY(cudaMemsetAsync(csum, 0, (size_t)g.npass * g.nchunks * 256 * 4, c->stream));
+    k_seed_keys_tiles<K, false><<<(unsigned)std::min<int64_t>(g.ntiles, 152 * 4), 256, 0, c->stream>>>(
+        d_packed, count, nullptr, 0, s, k0, nullptr, rts_counts(scr), csum, g.ntiles, g.ctiles);
+    c->launches++;
+    rts_sort_mers<K>(keys, buf, (int64_t)count, nbits, MersOut<K>{d_mer_out, d_pos_out, s.w}, scr, c->stream,
+                     &c->launches);
+    MVG_CUDA_TRY(cudaGetLastError());
+    return 0;
+  }
+  K* k1 = (K*)ws.get(c, 1, count * sizeof(K));
+  uint32_t* v0 = (uint32_t*)ws.get(c, 2, count * sizeof(uint32_t));
+  uint32_t* v1 = (uint32_t*)ws.get(c, 3, count * sizeof(uint32_t));
   if (!k0 || !k1 || !v0 || !v1 || !scr) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   k_seed_keys<K><<<grid_for(count, 256), 256, 0, c->stream>>>(d_packed, count, s, k0, v0);
   c->launches++;
-  int which = sort_pairs<K>(k0, v0, k1, v1, (int64_t)count, nbits, scr, c->stream, &c->launches, c->d_err);
-  K* ks = which ? k1 : k0;
-  uint32_t* vs = which ? v1 : v0;
-  if (d_pos_out) MVG_CUDA_TRY(cudaMemcpyAsync(d_pos_out, vs, count * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->stream));
+  const int which = sort_pairs<K>(k0, v0, k1, v1, (int64_t)count, nbits, scr, c->stream, &c->launches, c->d_err);
+  if (d_pos_out)
+    MVG_CUDA_TRY(cudaMemcpyAsync(d_pos_out, which ? v1 : v0, count * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                                 c->stream));
   if (d_mer_out) {
-    k_key_to_mer<K><<<grid_for(count, 256), 256, 0, c->stream>>>(ks, count, s.w, d_mer_out);
+    k_key_to_mer<K><<<grid_for(count, 256), 256, 0, c->stream>>>(which ? k1 : k0, count, s.w, d_mer_out);
     c->launches++;
-  }
-  if (keep) {
-    keep->keys = ks;
-    keep->pos = vs;
-    keep->wide = sizeof(K) == 8;
-    keep->count = count;
   }
   MVG_CUDA_TRY(cudaGetLastError());
   return 0;
@@ -343,12 +356,12 @@ static int pair_sort_impl(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_
   if ((int64_t)count < (1ll << 31)) {  // the sort_pairs range of the reduce-then-scan sort
     uint32_t* csum = rts_csum(scr, g);
     MVG_CUDA_TRY(cudaMemsetAsync(csum, 0, (size_t)g.npass * g.nchunks * 256 * 4, c->stream));
-    k_seed_keys_pair<K><<<grid, 256, 0, c->stream>>>(ga, ca, gb, cb, s, k0, v0, rts_counts(scr), csum, g.ntiles,
-                                                      g.ctiles);
+    k_seed_keys_tiles<K, true><<<grid, 256, 0, c->stream>>>(ga, ca, gb, cb, s, k0, v0, rts_counts(scr), csum, g.ntiles,
+                                                            g.ctiles);
     c->launches++;
     which = rts_sort_pairs<K>(k0, v0, k1, v1, (int64_t)count, nbits, scr, c->stream, &c->launches, true);
   } else {
-    k_seed_keys_pair<K><<<grid, 256, 0, c->stream>>>(ga, ca, gb, cb, s, k0, v0, nullptr, nullptr, g.ntiles, 1);
+    k_seed_keys_tiles<K, true><<<grid, 256, 0, c->stream>>>(ga, ca, gb, cb, s, k0, v0, nullptr, nullptr, g.ntiles, 1);
     c->launches++;
     which = sort_pairs<K>(k0, v0, k1, v1, (int64_t)count, nbits, scr, c->stream, &c->launches, c->d_err);
   }
@@ -367,9 +380,9 @@ int pair_sort(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint6
 }
 
 int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
-             uint64_t* d_mer_out, SmlKeys* keep, int slot_base) {
-  if (2 * s.w + 1 <= 32) return sml_sort_impl<uint32_t>(c, d_packed, count, s, d_pos_out, d_mer_out, keep, slot_base);
-  return sml_sort_impl<uint64_t>(c, d_packed, count, s, d_pos_out, d_mer_out, keep, slot_base);
+             uint64_t* d_mer_out) {
+  if (2 * s.w + 1 <= 32) return sml_sort_impl<uint32_t>(c, d_packed, count, s, d_pos_out, d_mer_out);
+  return sml_sort_impl<uint64_t>(c, d_packed, count, s, d_pos_out, d_mer_out);
 }
 
 }  // namespace mvg
