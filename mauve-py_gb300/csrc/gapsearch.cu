@@ -147,12 +147,15 @@ struct GapSet {
   }
 };
 
-// Calls f(mixed key, strand, in B, slot) for every seed position of this
-// block's tile of slots (A's, then B's); a warp's 32 slots are one gap's.
+// Calls f(mixed keys, strands, in B, first slot, valid) for groups of four
+// slots of this block's tile (A's, then B's), of which those with a bit in
+// `valid` hold a seed position; a warp's slots, and so a group's, are aligned
+// pieces of gaps.  A seed of the table is at most 23 bases long up to weight
+// 15, so a group's seeds lie in one 32-base window.
 template <class F>
 __device__ __forceinline__ void gs_tile(const GapSet& P, int bits, int64_t tile, F f) {
   const uint64_t n = (uint64_t)P.slots[0] + P.slots[1], base = (uint64_t)blockIdx.x * (uint64_t)tile;
-  for (int64_t o = threadIdx.x; o < tile; o += blockDim.x) {
+  for (int64_t o = 4 * threadIdx.x; o < tile; o += 4 * blockDim.x) {
     const uint64_t p = base + (uint64_t)o;
     if (p >= n) break;
     const int side = p >= P.slots[0];
@@ -162,8 +165,17 @@ __device__ __forceinline__ void gs_tile(const GapSet& P, int bits, int64_t tile,
     const uint32_t x = q - d.slot[side];
     if (x >= d.cnt[side]) continue;
     const SeedDesc& s = c_gs_seed[d.w];
-    const uint64_t m = canonical_mer((side ? P.pb : P.pa) + d.word[side], x, s);
-    f(mix_mer<uint64_t>((uint64_t)g << P.mbits | m >> (64 - 2 * s.w), bits), (uint32_t)m & 1u, side, q);
+    const uint64_t win = window64((side ? P.pb : P.pa) + d.word[side], x);
+    uint64_t key[4];
+    uint32_t strand[4], valid = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint64_t fw = gather_seed(win << 2 * u, s), r = revcomp_mer(fw, s.w), m = fw < r ? fw : r;
+      key[u] = mix_mer<uint64_t>((uint64_t)g << P.mbits | m >> (64 - 2 * s.w), bits);
+      strand[u] = (uint32_t)m & 1u;
+      valid |= (x + u < d.cnt[side] ? 1u : 0u) << u;
+    }
+    f(key, strand, side, q, valid);
   }
 }
 
@@ -173,7 +185,11 @@ __global__ void __launch_bounds__(1024) k_gs_keys(GapSet P, int bits, int bbits,
   const int nbk = 1 << bbits, bsh = bits - bbits;
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) h[d] = 0;
   __syncthreads();
-  gs_tile(P, bits, tile, [&](uint64_t k, uint32_t, int, uint32_t) { atomicAdd(&h[(uint32_t)(k >> bsh)], 1u); });
+  gs_tile(P, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&)[4], int, uint32_t, uint32_t valid) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (valid >> u & 1) atomicAdd(&h[(uint32_t)(k[u] >> bsh)], 1u);
+  });
   __syncthreads();
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) counts[(int64_t)blockIdx.x * nbk + d] = h[d];
 }
@@ -185,8 +201,14 @@ __global__ void __launch_bounds__(1024) k_gs_scatter(GapSet P, int bits, int bbi
   const uint32_t rest = (uint32_t)(((uint64_t)1 << bsh) - 1);
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) cur[d] = offsets[(int64_t)blockIdx.x * nbk + d];
   __syncthreads();
-  gs_tile(P, bits, tile, [&](uint64_t k, uint32_t strand, int side, uint32_t q) {
-    out[atomicAdd(&cur[(uint32_t)(k >> bsh)], 1u)] = make_uint2(((uint32_t)k & rest) << 2 | strand << 1 | (uint32_t)side, q);
+  gs_tile(P, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&strand)[4], int side, uint32_t q, uint32_t valid) {
+    uint32_t slot[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (valid >> u & 1) slot[u] = atomicAdd(&cur[(uint32_t)(k[u] >> bsh)], 1u);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (valid >> u & 1) out[slot[u]] = make_uint2(((uint32_t)k[u] & rest) << 2 | strand[u] << 1 | (uint32_t)side, q + u);
   });
 }
 
@@ -598,7 +620,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   static bool attr = false;  // once per process: more than 48 KB of dynamic shared memory
   if (!attr) {
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneCta));
     attr = true;
   }
   const size_t hsm = (size_t)b.g.nbuckets * 4;
@@ -606,7 +628,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   k_gs_keys<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.counts);
   pair_bucket_offsets(c, b);
   stage_mark(c, "gs_scatter");
-  k_gs_scatter<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.offs, b.buf);
+  k_gs_scatter<<<(unsigned)b.g.ntiles, 1024, kOneCta, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.offs, b.buf);
   c->launches += 3;
   stage_mark(c, "gs_join");
   pair_bucket_join(c, b, tab);

@@ -145,9 +145,11 @@ __device__ __forceinline__ uint32_t revcomp_mer32(uint32_t mer, int w) {
   return (r << (32 - 2 * w)) | 1u;
 }
 
-// The forward mer of the position u bases into a 64-bit window (u + L <= 32).
-__device__ __forceinline__ uint32_t gather_mer32(uint64_t win, int u, const uint32_t (*lut)[256], int nb) {
-  uint32_t f = 0;
+// The forward mer of the position u bases into a 64-bit window, left-aligned
+// in K (u + L <= 32, and no byte shift below zero: 8 nb + 2 u <= 64).
+template <typename K>
+__device__ __forceinline__ K gather_mer(uint64_t win, int u, const K (*lut)[256], int nb) {
+  K f = 0;
 #pragma unroll
   for (int c = 0; c < 8; ++c)
     if (c < nb) f |= lut[c][(uint32_t)(win >> (56 - 8 * c - 2 * u)) & 255u];

@@ -147,6 +147,7 @@ int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s
 constexpr uint64_t kPairBucketMaxKeys = 1ull << 25;
 constexpr int kPairRestBits = 30;                      // mer bits below the bucket's
 constexpr int kPairMaxBits = 14 + kPairRestBits;       // with 2^14 buckets
+constexpr int kOneCta = 120 * 1024;  // dynamic shared memory of the join's scatter: one CTA per SM
 struct PairBucketGeom {
   int bbits, nbuckets, npass, dbits, lbits;
   int64_t tile, ntiles, nchunks;

@@ -48,9 +48,19 @@ constexpr int kMaxDigit = 64;   // chunked in-bucket passes: digits of at most 6
 constexpr int kGroups = 512;    // groups of a bucket: its top 9 in-bucket bits
 constexpr int kGroupMax = 256;  // larger groups: the bucket is sorted instead
 constexpr int kChunkTiles = 32;
+constexpr uint64_t kInL2 = 96ull << 20;  // of 129 MB
 }  // namespace pb
 
-PairBucketGeom pair_bucket_geom(uint64_t n, int bits) {
+// Keys of a tile.  A tile writes its keys of a bucket as a run at the bucket's
+// next slots, at random times, so the open sectors are those of all the tiles
+// in flight: one CTA per SM (kOneCta), and once the keys outgrow L2, tiles of
+// two keys per bucket, 38 MB of 24 million keys in flight.  Smaller tiles cost
+// more count rows, larger ones leave L2 with partial sectors (24 million keys,
+// 16,384 buckets: keys and scatter 0.52 ms with one key per bucket and tile,
+// 0.49 with two, 0.53 with four, 0.73 with eight, 0.75 with four and two CTAs
+// per SM).  Below that, eight (9.2 million: 0.15 ms, 0.18 with two).
+// Tiles fill whole waves of the CTAs.
+PairBucketGeom pair_bucket_geom(uint64_t n, int bits, int sms) {
   PairBucketGeom g;
   int bb = 4;
   while (bb < 14 && ((uint64_t)2048 << bb) < n) ++bb;  // about 2048 keys per bucket at most
@@ -58,7 +68,10 @@ PairBucketGeom pair_bucket_geom(uint64_t n, int bits) {
   if (bb > bits) bb = bits;
   g.bbits = bb;
   g.nbuckets = 1 << bb;
-  g.tile = std::max<int64_t>(16384, 4ll * g.nbuckets);
+  const uint64_t per = n * 8 <= pb::kInL2 ? 8 : 2;
+  const uint64_t wave = (uint64_t)sms * std::max<uint64_t>(16384, per * g.nbuckets);
+  const uint64_t waves = std::max<uint64_t>(1, (n + wave / 2) / wave);
+  g.tile = (int64_t)((n / (waves * sms) + 1 + 4095) & ~4095ull);
   g.ntiles = (int64_t)((n + g.tile - 1) / g.tile);
   g.nchunks = (g.ntiles + pb::kChunkTiles - 1) / pb::kChunkTiles;
   // in-bucket key: the rest of the mixed mer, then the genome bit; an odd
@@ -74,44 +87,47 @@ PairBucketGeom pair_bucket_geom(uint64_t n, int bits) {
 
 // ------------------------------------------------------------------ keys
 
-// Calls f(global index, mixed mer, strand, in B, position) for every position
-// of this block's tile.  K = uint32_t: w <= 15, four positions from one
-// 32-base window where they fit.
+// The reverse complement of a mer left-aligned in K, its strand bit set.
+__device__ __forceinline__ uint32_t revcomp_in(uint32_t m, int w) { return revcomp_mer32(m, w); }
+__device__ __forceinline__ uint64_t revcomp_in(uint64_t m, int w) { return revcomp_mer(m, w); }
+
+// Calls f(mixed mers, strands, in B, first position, how many) for groups of
+// up to four consecutive positions of this block's tile, made from one
+// 32-base window where they fit.  K = uint32_t: w <= 15.  (A position per
+// thread and call left one window load in flight per thread: the keys of 24
+// million seeds of weight 17 took 0.21 ms, in groups 0.15.)
 template <typename K, class F>
 __device__ __forceinline__ void pb_tile(const uint32_t* __restrict__ ga, uint64_t ca, const uint32_t* __restrict__ gb,
                                         uint64_t cb, const SeedDesc& s, const K (*lut)[256], int64_t tile, F f) {
   const int nb = seed_bytes(s);
   const uint64_t n = ca + cb;
   const uint64_t base = (uint64_t)blockIdx.x * (uint64_t)tile;
-  if constexpr (sizeof(K) == 4) {
-    const bool quad = nb <= 7;
-    const int sh = 32 - 2 * s.w;
-    for (int64_t o = 4 * threadIdx.x; o < tile; o += 4 * pb::kKeyThreads) {
-      const uint64_t p0 = base + (uint64_t)o;
-      if (p0 >= n) break;
-      const bool whole = quad && p0 + 4 <= n && (p0 + 4 <= ca || p0 >= ca);
-      const uint64_t win = whole ? window64(p0 >= ca ? gb : ga, p0 >= ca ? p0 - ca : p0) : 0;
+  const bool quad = nb <= 7;
+  const int sh = 8 * (int)sizeof(K) - 2 * s.w;
+  for (int64_t o = 4 * threadIdx.x; o < tile; o += 4 * pb::kKeyThreads) {
+    const uint64_t p0 = base + (uint64_t)o;
+    if (p0 >= n) break;
+    K m[4];
+    uint32_t strand[4];
+    auto take = [&](int k, K fw) {
+      const K r = revcomp_in(fw, s.w), c = fw < r ? fw : r;
+      m[k] = mix_mer<K>(c >> sh, 2 * s.w);
+      strand[k] = (uint32_t)c & 1u;
+    };
+    if (quad && p0 + 4 <= n && (p0 + 4 <= ca || p0 >= ca)) {
+      const bool in_b = p0 >= ca;
+      const uint64_t q0 = in_b ? p0 - ca : p0;
+      const uint64_t win = window64(in_b ? gb : ga, q0);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint64_t p = p0 + u;
-        if (p >= n) break;
+      for (int u = 0; u < 4; ++u) take(u, gather_mer<K>(win, u, lut, nb));
+      f(m, strand, in_b, (uint32_t)q0, 4);
+    } else {
+      for (uint64_t p = p0; p < p0 + 4 && p < n; ++p) {
         const bool in_b = p >= ca;
         const uint64_t q = in_b ? p - ca : p;
-        const uint32_t fw = whole ? gather_mer32(win, u, lut, nb) : gather_mer32(window64(in_b ? gb : ga, q), 0, lut, nb);
-        const uint32_t r = revcomp_mer32(fw, s.w);
-        const uint32_t m = fw < r ? fw : r;
-        f(p, mix_mer<uint32_t>(m >> sh, 2 * s.w), m & 1u, in_b, (uint32_t)q);
+        take(0, gather_mer<K>(window64(in_b ? gb : ga, q), 0, lut, nb));
+        f(m, strand, in_b, (uint32_t)q, 1);
       }
-    }
-  } else {
-    const int sh = 64 - 2 * s.w;
-    for (int64_t o = threadIdx.x; o < tile; o += pb::kKeyThreads) {
-      const uint64_t p = base + (uint64_t)o;
-      if (p >= n) break;
-      const bool in_b = p >= ca;
-      const uint64_t q = in_b ? p - ca : p;
-      const uint64_t m = canonical_mer_lut(in_b ? gb : ga, q, lut, nb, s.w);
-      f(p, mix_mer<uint64_t>(m >> sh, 2 * s.w), (uint32_t)m & 1u, in_b, (uint32_t)q);
     }
   }
 }
@@ -135,7 +151,11 @@ __global__ void __launch_bounds__(pb::kKeyThreads) k_pb_keys(const uint32_t* __r
   for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) h[d] = 0;
   __syncthreads();
   pb_tile<K>(ga, ca, gb, cb, s, lut, tile,
-             [&](uint64_t, K m, uint32_t, bool, uint32_t) { atomicAdd(&h[(uint32_t)(m >> bsh)], 1u); });
+             [&](const K(&m)[4], const uint32_t(&)[4], bool, uint32_t, int count) {
+#pragma unroll
+               for (int u = 0; u < 4; ++u)
+                 if (u < count) atomicAdd(&h[(uint32_t)(m[u] >> bsh)], 1u);
+             });
   __syncthreads();
   uint32_t* row = counts + (int64_t)blockIdx.x * nbk;
   for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) row[d] = h[d];
@@ -278,10 +298,17 @@ __global__ void __launch_bounds__(pb::kKeyThreads) k_pb_scatter(const uint32_t* 
   pb_lut(s, lut);
   for (int d = threadIdx.x; d < nbk; d += pb::kKeyThreads) cur[d] = row[d];
   __syncthreads();
-  pb_tile<K>(ga, ca, gb, cb, s, lut, tile, [&](uint64_t, K m, uint32_t strand, bool in_b, uint32_t q) {
-    const uint32_t slot = atomicAdd(&cur[(uint32_t)(m >> bsh)], 1u);
-    out[slot] = make_uint2(((uint32_t)m & rest) << 2 | strand << 1 | (in_b ? 1u : 0u), q);
-  });
+  pb_tile<K>(ga, ca, gb, cb, s, lut, tile,
+             [&](const K(&m)[4], const uint32_t(&strand)[4], bool in_b, uint32_t q, int count) {
+               uint32_t slot[4];
+#pragma unroll
+               for (int u = 0; u < 4; ++u)
+                 if (u < count) slot[u] = atomicAdd(&cur[(uint32_t)(m[u] >> bsh)], 1u);
+#pragma unroll
+               for (int u = 0; u < 4; ++u)
+                 if (u < count)
+                   out[slot[u]] = make_uint2(((uint32_t)m[u] & rest) << 2 | strand[u] << 1 | (in_b ? 1u : 0u), q + u);
+             });
 }
 
 // ---------------------------------------------------- in-bucket sort
@@ -479,7 +506,9 @@ __global__ void __launch_bounds__(pb::kLocThreads) k_pb_local(uint2* __restrict_
 // ------------------------------------------------------------------ host
 
 int pair_bucket_bufs(Ctx* c, uint64_t n, int bits, PairBucketBufs* b) {
-  b->g = pair_bucket_geom(n, bits);
+  int sms = 0;
+  MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  b->g = pair_bucket_geom(n, bits, sms);
   const PairBucketGeom& g = b->g;
   const int nbk = g.nbuckets;
   Workspace& ws = c->ws;
@@ -522,14 +551,14 @@ static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32
   static bool attr = false;  // once per process and key type: more than 48 KB of dynamic shared memory
   if (!attr) {
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_keys<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneCta));
     attr = true;
   }
   const size_t hsm = (size_t)g.nbuckets * 4;
   k_pb_keys<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, b.counts, g.bbits, g.tile);
   pair_bucket_offsets(c, b);
   stage_mark(c, "seed_scatter");
-  k_pb_scatter<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, b.offs, g.bbits, g.tile,
+  k_pb_scatter<K><<<(unsigned)g.ntiles, pb::kKeyThreads, kOneCta, c->stream>>>(ga, ca, gb, cb, s, b.offs, g.bbits, g.tile,
                                                                            b.buf);
   c->launches += 2;
   stage_mark(c, "seed_local");

@@ -448,8 +448,9 @@ int rts_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int
 // positions.  Between passes 32-bit keys travel with their values in 8-byte
 // pairs: a tile's run of a digit is 8 keys on average, which as pairs fills
 // two whole sectors with one store each instead of parts of four with two.
-// (3.98 million 31-bit keys, a scatter pass: 34 us in two arrays, PAIRUS as
-// pairs.  Tiles twice as large were slower, 0.32 against 0.29 ms for the SML.)
+// (3.98 million 31-bit keys, a scatter pass: 34 us in two arrays with
+// ranks by __match_any_sync, 24 as pairs with ranks by eight ballots; tiles
+// half as large again or twice as large are no faster.)
 // keys[0] holds the keys; buf[0], buf[1]: n pairs each, or for 64-bit keys n
 // values, with keys[1].
 template <typename K>

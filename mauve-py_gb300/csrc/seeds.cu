@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) k_seed_keys_tiles(const uint32_t* __restr
           uint32_t kk[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const uint32_t f = gather_mer32(win, u, lut32, nb);
+            const uint32_t f = gather_mer<uint32_t>(win, u, lut32, nb);
             const uint32_t r = revcomp_mer32(f, s.w);
             const uint32_t m = f < r ? f : r;
             kk[u] = key_of((m >> sh) << 1 | (m & 1u), in_b);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) k_seed_keys_tiles(const uint32_t* __restr
             if (p >= n) break;
             const bool in_b = p >= ca;
             const uint64_t q = in_b ? p - ca : p;
-            const uint32_t f = gather_mer32(window64(in_b ? gb : ga, q), 0, lut32, nb);
+            const uint32_t f = gather_mer<uint32_t>(window64(in_b ? gb : ga, q), 0, lut32, nb);
             const uint32_t r = revcomp_mer32(f, s.w);
             const uint32_t m = f < r ? f : r;
             const uint32_t key = key_of((m >> sh) << 1 | (m & 1u), in_b);
