@@ -220,61 +220,107 @@ static __global__ void k_seg_pair(const uint32_t* __restrict__ tab, const uint32
 
 // ----------------------------------------------------------------- walks
 
-// One side of ExtendMatch from a segment end on eight lanes: tasks [0, n)
-// from the tails to higher A positions, [n, 2n) from the heads down.  A walk
-// towards a neighbouring segment of the same bucket and diagonal stops when
-// it gets there.  Out: moved[task], and for the first n joined[k] (segment k
-// is connected to segment k + 1).
+// One side of ExtendMatch from a segment end: tasks [0, n) from the tails to
+// higher A positions, [n, 2n) from the heads down.  A walk towards a
+// neighbouring segment of the same bucket and diagonal stops when it gets
+// there.
+template <class P>
+struct SegTask {
+  const bool up;
+  const int64_t k;
+  const uint32_t x;  // the seed it starts from
+  uint32_t a0, b0;   // where its sequences begin
+  const MatchView c;
+  int64_t limit;     // distance to the neighbour
+  int64_t s0, s1;
+
+  __device__ __forceinline__ SegTask(const P& prob, const uint32_t* tab, const uint32_t* key, const uint32_t* head,
+                                     const uint32_t* last, int64_t n, int64_t task)
+      : up(task < n), k(up ? task : task - n), x(up ? last[k] : head[k]), c(prob.view(x, a0, b0)) {
+    const uint32_t v = tab[x];
+    const uint64_t d = seed_diag(v, x);
+    limit = INT64_MAX;
+    if (up && k + 1 < n && key[k + 1] == key[k] && seed_diag(tab[head[k + 1]], head[k + 1]) == d)
+      limit = (int64_t)head[k + 1] - x;
+    if (!up && k > 0 && key[k - 1] == key[k] && seed_diag(tab[last[k - 1]], last[k - 1]) == d)
+      limit = (int64_t)x - last[k - 1];
+    const int64_t e0 = (int64_t)(x - a0) + 1, e1 = (int64_t)((v & 0x7fffffffu) - b0) + 1;
+    s0 = up ? -e0 : e0;
+    s1 = (v >> 31 != 0) != up ? -e1 : e1;
+  }
+
+  // Words of 32 displacements from word `start` on, LANES (this lane is the
+  // j-th of `group`) at a time, `rounds` times: the displacement of the stop,
+  // the limit or beyond when it gets there, -1 when neither is reached.
+  // Word start - 1 and those before have been looked at.
+  template <int LANES>
+  __device__ __forceinline__ int64_t walk(int64_t start, int64_t rounds, unsigned group, int j) const {
+    const int L = c.s.L;
+    uint32_t carry = 0;
+    for (int64_t it = 0; it < rounds; ++it) {
+      const int64_t at = start + it * LANES;
+      const uint32_t w = ext_word(c, s0, s1, L, (at + j) * 32);
+      uint32_t prev = __shfl_up_sync(group, w, 1, LANES);
+      if (j == 0) prev = carry;
+      const int64_t idx = at + j - 1;  // the word whose successor is w
+      const uint32_t hit = idx >= start ? stop_in_word(prev, w, idx == 0, L) : 0u;
+      const unsigned any = __ballot_sync(group, hit != 0);
+      if (any) {
+        const int f = __ffs(any) - 1;  // a lane of this group
+        return __shfl_sync(group, 32 * idx + (__ffs(hit) - 1), f % LANES, LANES);
+      }
+      if (32 * (at + LANES - 1) >= limit) return limit;
+      carry = __shfl_sync(group, w, LANES - 1, LANES);
+    }
+    return -1;
+  }
+
+  // moved: what the walk covered; joined[k]: segment k is connected to k + 1.
+  __device__ __forceinline__ void done(int64_t q, int64_t task, uint32_t* moved, uint8_t* joined) const {
+    moved[task] = (uint32_t)(q < limit ? q : 0);
+    if (up) joined[k] = q >= limit;
+  }
+};
+
+// Two lanes per task look at the first words, as far as most walks go; the
+// warp's other tasks go on in fours, eight lanes each, and what is left then
+// one by one with the whole warp.  The instructions of making and searching
+// words bound short walks, latency the few long ones: eight lanes per task
+// throughout took 1.06 ms for the walks of 5,003 gaps and 0.045 ms for the 4.6
+// Mbp recoded pair's, this 0.42 and 0.037 (two lanes throughout: 0.44 and
+// 0.125).
 template <class P>
 __global__ void __launch_bounds__(256) k_seg_walk(P prob, const uint32_t* __restrict__ tab,
                                                   const uint32_t* __restrict__ key, const uint32_t* __restrict__ head,
                                                   const uint32_t* __restrict__ last, int64_t n,
                                                   uint32_t* __restrict__ moved, uint8_t* __restrict__ joined) {
-  const int64_t task = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  if (task >= 2 * n) return;
-  const int lane = threadIdx.x & 31, j = lane & 7;
-  const unsigned group = 0xffu << (lane & 24);
-  const bool up = task < n;
-  const int64_t k = up ? task : task - n;
-  const uint32_t x = up ? last[k] : head[k];
-  const uint32_t v = tab[x];
-  const uint64_t d = seed_diag(v, x);
-  int64_t limit = INT64_MAX;  // distance to the neighbour
-  if (up && k + 1 < n && key[k + 1] == key[k] && seed_diag(tab[head[k + 1]], head[k + 1]) == d)
-    limit = (int64_t)head[k + 1] - x;
-  if (!up && k > 0 && key[k - 1] == key[k] && seed_diag(tab[last[k - 1]], last[k - 1]) == d)
-    limit = (int64_t)x - last[k - 1];
-  uint32_t a0, b0;
-  const MatchView c = prob.view(x, a0, b0);
-  const int L = c.s.L;
-  const int64_t e0 = (int64_t)(x - a0) + 1, e1 = (int64_t)((v & 0x7fffffffu) - b0) + 1;
-  const int64_t s0 = up ? -e0 : e0;
-  const int64_t s1 = (v >> 31 != 0) != up ? -e1 : e1;
-  uint32_t carry = 0;
-  for (int64_t it = 0;; ++it) {
-    const uint32_t w = ext_word(c, s0, s1, L, (it * 8 + j) * 32);
-    uint32_t prev = __shfl_up_sync(group, w, 1, 8);
-    if (j == 0) prev = carry;
-    const int64_t idx = it * 8 + j - 1;  // the word whose successor is w
-    const uint32_t hit = idx >= 0 ? stop_in_word(prev, w, idx == 0, L) : 0u;
-    const unsigned any = __ballot_sync(group, hit != 0);
-    if (any) {
-      const int f = __ffs(any) - 1;
-      if (lane == f) {
-        const int64_t q = 32 * idx + (__ffs(hit) - 1);
-        moved[task] = (uint32_t)(q < limit ? q : 0);
-        if (up) joined[k] = q >= limit;
-      }
-      return;
-    }
-    if (32 * (it * 8 + 7) >= limit) {
-      if (j == 0) {
-        moved[task] = 0;
-        if (up) joined[k] = 1;
-      }
-      return;
-    }
-    carry = __shfl_sync(group, w, 7, 8);
+  constexpr int kEight = 1;  // rounds of eight lanes
+  constexpr int kFrom8 = 2 - 1, kFrom32 = kFrom8 + 8 * kEight - 1;  // a walk's last word has no successor yet
+  const int lane = threadIdx.x & 31;
+  const int64_t first = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / 2;  // the warp's first task
+  const int64_t task = first + lane / 2;
+  bool open = false;
+  if (task < 2 * n) {
+    const SegTask<P> t(prob, tab, key, head, last, n, task);
+    const int64_t q = t.template walk<2>(0, 1, 3u << (lane & 30), lane & 1);
+    open = q < 0;
+    if (!open && (lane & 1) == 0) t.done(q, task, moved, joined);
+  }
+  const unsigned left = __ballot_sync(0xffffffffu, open) & 0x55555555u;
+  const int more = __popc(left);
+  unsigned rest = 0;
+  for (int r = lane >> 3; r < more; r += 4) {
+    const int at = (int)__fns(left, 0, r + 1);
+    const SegTask<P> t(prob, tab, key, head, last, n, first + at / 2);
+    const int64_t q = t.template walk<8>(kFrom8, kEight, 0xffu << (lane & 24), lane & 7);
+    if (q < 0) rest |= 1u << at;
+    else if ((lane & 7) == 0) t.done(q, first + at / 2, moved, joined);
+  }
+  for (rest = __reduce_or_sync(0xffffffffu, rest); rest; rest &= rest - 1) {
+    const int64_t mine = first + (__ffs(rest) - 1) / 2;
+    const SegTask<P> t(prob, tab, key, head, last, n, mine);
+    const int64_t q = t.template walk<32>(kFrom32, INT64_MAX, 0xffffffffu, lane);
+    if (lane == 0) t.done(q, mine, moved, joined);
   }
 }
 
@@ -766,7 +812,7 @@ int match_components(Ctx* c, P& prob, const uint32_t* tab, int64_t n, int key_bi
   const uint32_t *key = alt ? k1 : k0, *head = alt ? v1 : v0, *tail = head + nseg;
   stage_mark(c, "walks");
   k_seg_pair<<<div_up(nseg, 256), 256, 0, c->stream>>>(tab, head, key, tail, nseg, last);
-  k_seg_walk<<<div_up(2 * nseg * 8, 256), 256, 0, c->stream>>>(prob, tab, key, head, last, nseg, moved, joined);
+  k_seg_walk<<<div_up(2 * nseg * 2, 256), 256, 0, c->stream>>>(prob, tab, key, head, last, nseg, moved, joined);
   stage_mark(c, "components");
   MVG_CUDA_TRY(cudaMemsetAsync(bflag, 0, (size_t)nseg * 4, c->stream));
   k_comp_count<<<(unsigned)ctiles, 256, 0, c->stream>>>(joined, nseg, ccount);

@@ -67,3 +67,25 @@ def test_segment_edges(ctx, weight):
             b[q] = ord("ACGT"["ACGT".index(chr(b[q])) - 1])
     for x, y in ((a, b), (a, synth.revcomp(b)), (b[L // 2:], a[:-3]), (a[:2048], b), (a[:2049], synth.revcomp(b))):
         np.testing.assert_array_equal(ctx.pairwise_matches(x, y, seed), O.pairwise_matches(x, y, seed))
+
+
+@pytest.mark.parametrize("gap", [20, 40, 63, 64, 65, 96, 200, 255, 256, 288, 289, 320, 1000, 1290, 1330, 4000])
+@pytest.mark.parametrize("flip", [False, True])
+def test_walks_across_repeats(ctx, gap, flip):
+    """Segments of one diagonal with a repeat of `gap` bases between them,
+    whose seeds match but are not unique: walks of every length, some of which
+    end on a substitution in the repeat."""
+    rng = np.random.default_rng(gap)
+    a, b = [], []
+    for k in range(12):
+        u, v, r = (synth.random_bases(rng, n) for n in (150, 170, gap))
+        rb = r.copy()
+        if k % 3:
+            rb[int(rng.integers(0, gap))::max(1, gap // (k % 3))] = ord("A")
+        a += [u, r, v, r, synth.random_bases(rng, 60)]
+        b += [u, rb, v, synth.random_bases(rng, 80), rb]
+    a, b = np.concatenate(a), np.concatenate(b)
+    if flip:
+        b = synth.revcomp(b)
+    seed = mvg.get_seed(15, 0)
+    np.testing.assert_array_equal(ctx.pairwise_matches(a, b, seed), O.pairwise_matches(a, b, seed))
