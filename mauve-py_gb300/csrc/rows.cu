@@ -5,47 +5,97 @@
 // the gap character is '-' (MUSCLE's MSA gap).  The characters are copied
 // as given (ASCII bases or 0..3 codes alike).
 //
-// One warp per problem: 32 edges per step, each lane's source positions from
-// a ballot prefix of the edges before it.
+// A warp takes 128 edges per step, each lane's source positions from a ballot
+// prefix of the edges before it.  One warp per problem, or, where there are
+// too few problems to fill the device that way, a CTA of 32, whose warps count
+// their shares of the path first.
 #include "mvg_internal.h"
 
 namespace mvg {
 
-__global__ void k_path_rows(const uint8_t* __restrict__ sa, const uint64_t* __restrict__ oa,
-                            const uint8_t* __restrict__ sb, const uint64_t* __restrict__ ob, int64_t nprob,
-                            const char* __restrict__ paths, const uint64_t* __restrict__ path_off,
-                            const int64_t* __restrict__ path_len, uint8_t* __restrict__ rows_a,
-                            uint8_t* __restrict__ rows_b, uint32_t* err) {
+// Edges [t0, t1) of one path on one warp, whose first takes character i of A
+// and j of B; both move on.  Returns whether an edge was none, or past a
+// sequence's end.
+__device__ __forceinline__ bool rows_of(const uint8_t* __restrict__ A, int64_t la, const uint8_t* __restrict__ B,
+                                        int64_t lb, const char* __restrict__ P, int64_t t0, int64_t t1,
+                                        uint8_t* __restrict__ RA, uint8_t* __restrict__ RB, int64_t& i, int64_t& j) {
+  constexpr int kSteps = 4;  // loads in flight
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < nprob; p += nw) {
+  bool bad = false;
+  for (; t0 < t1; t0 += 32 * kSteps) {
+    char e[kSteps];
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s) {
+      const int64_t t = t0 + 32 * s + lane;
+      e[s] = t < t1 ? P[t] : 'X';
+    }
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s) {
+      const int64_t t = t0 + 32 * s + lane;
+      const bool ia = e[s] == 'M' || e[s] == 'D', ib = e[s] == 'M' || e[s] == 'I';
+      const unsigned ma = __ballot_sync(0xffffffffu, ia), mb = __ballot_sync(0xffffffffu, ib);
+      const int64_t pa = i + __popc(ma & below), pb = j + __popc(mb & below);
+      if (t < t1) {
+        bad |= !ia && !ib;
+        bad |= (ia && pa >= la) || (ib && pb >= lb);
+        RA[t] = ia && pa < la ? A[pa] : (uint8_t)'-';
+        RB[t] = ib && pb < lb ? B[pb] : (uint8_t)'-';
+      }
+      i += __popc(ma);
+      j += __popc(mb);
+    }
+  }
+  return bad;
+}
+
+// WARPS warps per problem: 1 (eight problems per CTA) or 32 (a CTA each).
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS == 1 ? 256 : 1024)
+    k_path_rows(const uint8_t* __restrict__ sa, const uint64_t* __restrict__ oa, const uint8_t* __restrict__ sb,
+                const uint64_t* __restrict__ ob, int64_t nprob, const char* __restrict__ paths,
+                const uint64_t* __restrict__ path_off, const int64_t* __restrict__ path_len,
+                uint8_t* __restrict__ rows_a, uint8_t* __restrict__ rows_b, uint32_t* err) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t first = WARPS == 1 ? (int64_t)blockIdx.x * 8 + wid : blockIdx.x;
+  const int64_t step = WARPS == 1 ? (int64_t)gridDim.x * 8 : gridDim.x;
+  for (int64_t p = first; p < nprob; p += step) {
     const uint8_t* A = sa + oa[p];
     const uint8_t* B = sb + ob[p];
     const int64_t la = (int64_t)(oa[p + 1] - oa[p]), lb = (int64_t)(ob[p + 1] - ob[p]);
     const int64_t n = path_len[p];
     const char* P = paths + path_off[p];
-    uint8_t* RA = rows_a + path_off[p];
-    uint8_t* RB = rows_b + path_off[p];
-    int64_t i = 0, j = 0;  // characters of A and B consumed before this step
-    bool bad = false;
-    for (int64_t t0 = 0; t0 < n; t0 += 32) {
-      const int64_t t = t0 + lane;
-      const char e = t < n ? P[t] : 'X';
-      const bool ia = t < n && (e == 'M' || e == 'D');
-      const bool ib = t < n && (e == 'M' || e == 'I');
-      bad |= t < n && !ia && !ib;
-      const unsigned ma = __ballot_sync(0xffffffffu, ia), mb = __ballot_sync(0xffffffffu, ib);
-      const int64_t pa = i + __popc(ma & below), pb = j + __popc(mb & below);
-      if (t < n) {
-        bad |= (ia && pa >= la) || (ib && pb >= lb);
-        RA[t] = ia ? (pa < la ? A[pa] : (uint8_t)'-') : (uint8_t)'-';
-        RB[t] = ib ? (pb < lb ? B[pb] : (uint8_t)'-') : (uint8_t)'-';
+    int64_t i = 0, j = 0, t0 = 0, t1 = n;  // characters of A and B consumed before t0
+    if constexpr (WARPS > 1) {
+      __shared__ int64_t s_a[WARPS], s_b[WARPS];
+      const int64_t share = ((n + WARPS - 1) / WARPS + 31) & ~(int64_t)31;
+      t0 = min(n, wid * share);
+      t1 = min(n, t0 + share);
+      int64_t ca = 0, cb = 0;
+#pragma unroll 4
+      for (int64_t t = t0 + lane; t < t1; t += 32) {
+        const char e = P[t];
+        ca += e == 'M' || e == 'D';
+        cb += e == 'M' || e == 'I';
       }
-      i += __popc(ma);
-      j += __popc(mb);
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) {
+        ca += __shfl_xor_sync(0xffffffffu, ca, d);
+        cb += __shfl_xor_sync(0xffffffffu, cb, d);
+      }
+      __syncthreads();  // the last problem's counts are read
+      if (lane == 0) {
+        s_a[wid] = ca;
+        s_b[wid] = cb;
+      }
+      __syncthreads();
+      for (int w = 0; w < wid; ++w) {
+        i += s_a[w];
+        j += s_b[w];
+      }
     }
-    bad |= i != la || j != lb;  // the path must consume both sequences
+    bool bad = rows_of(A, la, B, lb, P, t0, t1, rows_a + path_off[p], rows_b + path_off[p], i, j);
+    if (wid % WARPS == WARPS - 1) bad |= i != la || j != lb;  // the path must consume both sequences
     if (__any_sync(0xffffffffu, bad) && lane == 0) set_error(err, kDevRange);
   }
 }
@@ -68,9 +118,18 @@ extern "C" int mvg_path_rows_dev(mvg_handle h, const uint8_t* d_seq_a, const uin
   Ctx* c = rows_ctx(h);
   MVG_CUDA_TRY(cudaSetDevice(c->device));
   MVG_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
-  const int grid = grid_for((uint64_t)nprob * 32, 256);
-  k_path_rows<<<grid, 256, 0, c->stream>>>(d_seq_a, d_off_a, d_seq_b, d_off_b, nprob, d_paths, d_path_off,
-                                           d_path_len, d_rows_a, d_rows_b, c->d_err);
+  // Below four problems per SM a warp per problem leaves most of the device
+  // idle: the call took 162 us for one path of 10,000 edges with a warp, 26
+  // with a CTA, and for 600 of 4,000 edges 65 and 38.  From there on CTAs of
+  // short paths cost more than they give (2,000 of 4,000 edges: 67 and 68 us,
+  // of 300: 26 and 42).
+  constexpr int64_t kCtaProblems = 608;
+  if (nprob <= kCtaProblems)
+    k_path_rows<32><<<(unsigned)nprob, 1024, 0, c->stream>>>(d_seq_a, d_off_a, d_seq_b, d_off_b, nprob, d_paths,
+                                                             d_path_off, d_path_len, d_rows_a, d_rows_b, c->d_err);
+  else
+    k_path_rows<1><<<grid_for((uint64_t)nprob * 32, 256), 256, 0, c->stream>>>(
+        d_seq_a, d_off_a, d_seq_b, d_off_b, nprob, d_paths, d_path_off, d_path_len, d_rows_a, d_rows_b, c->d_err);
   c->launches++;
   MVG_CUDA_TRY(cudaGetLastError());
   const int rc = check_device_error(c);
