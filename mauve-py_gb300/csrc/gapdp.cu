@@ -902,9 +902,8 @@ static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vec
 
 // Every base code must be 0..3 (the kernels mask to 2 bits; this reports it).
 static int check_codes(Ctx* c, const uint8_t* d_sa, uint64_t na, const uint8_t* d_sb, uint64_t nb) {
-  k_check_codes<<<grid_for(na / 16 + 1, 256), 256, 0, c->stream>>>(d_sa, na, c->d_err);
-  k_check_codes<<<grid_for(nb / 16 + 1, 256), 256, 0, c->stream>>>(d_sb, nb, c->d_err);
-  c->launches += 2;
+  k_check_codes<<<dim3(grid_for(std::max(na, nb) / 16 + 1, 256), 2), 256, 0, c->stream>>>(d_sa, na, d_sb, nb, c->d_err);
+  c->launches++;
   MVG_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -964,8 +963,7 @@ int gapdp_batch_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const uin
   rc = run_full(c, in, ids, la, lb);
   if (rc) return rc;
   stage_end(c);
-  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return check_device_error(c);
+  return check_device_error(c);  // waits for the stream
 }
 
 int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const uint8_t* d_sb, const uint64_t* d_ob,
@@ -1127,10 +1125,9 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
   rc = run_full(c, in, fallback, la, lb);
   if (rc) return rc;
   stage_end(c);
-  MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (h_used_band) memcpy(h_used_band, acc.data(), (size_t)nprob);
   if (banded_cells) *banded_cells = bc;
-  return check_device_error(c);
+  return check_device_error(c);  // waits for the stream
 }
 
 // --------------------------------------------------------- INT32 probe

@@ -504,7 +504,11 @@ __global__ void __launch_bounds__(kDpThreads, 2) k_gapdp_t(DpJob J) {
 }
 
 // Flags any byte above 3 in a concatenated code buffer.
-__global__ void k_check_codes(const uint8_t* __restrict__ s, uint64_t n, uint32_t* err) {
+// Both arrays in one launch: blockIdx.y 0 and 1.
+__global__ void k_check_codes(const uint8_t* __restrict__ sa, uint64_t na, const uint8_t* __restrict__ sb, uint64_t nb,
+                              uint32_t* err) {
+  const uint8_t* const s = blockIdx.y ? sb : sa;
+  const uint64_t n = blockIdx.y ? nb : na;
   uint32_t bad = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t n16 = (((uintptr_t)s & 15) == 0) ? n / 16 : 0;
