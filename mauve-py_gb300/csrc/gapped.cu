@@ -19,7 +19,7 @@
 // buffer, runs every problem of every LCB in one batched gap-DP call, rebuilds
 // the rows of every problem on the GPU (k_path_rows) and splices them into
 // the LCBs' rows, the last pass's into the caller's buffers.  What bounds it
-// is this host work: 120 LCBs, 1.44 million columns, take 3.8 ms of which
+// is this host work: 120 LCBs, 1.44 million columns, take 3.8 ms, of which
 // the gap-DP calls are 1.3 (the plans' literal rows, the characters and their
 // codes as vectors of their own, grown byte by byte, merged and spliced by way
 // of further vectors: 10.3).

@@ -1,5 +1,6 @@
 // The pairwise matcher's match list from its seeds, without replaying the
-// reference's hash table seed by seed (included by match.cu).
+// reference's hash table seed by seed (included by match.cu and
+// gapsearch.cu).
 //
 // The reference (AddHashEntry, LM/MemHash.cpp:209-251) takes the unique seeds
 // in mer order; a seed that lower_bound finds contained in an entry of its
@@ -31,8 +32,7 @@
 //
 // So: a table of B positions by A position, segment ends by looking L
 // positions to either side, one sort of the ends by bucket (not of the
-// seeds), two walks per segment on eight lanes each, and a compaction.  The
-// walks bound it: about 1,000 instructions for a group of eight lanes.
+// seeds), two walks per segment, and a compaction.
 #pragma once
 #include <algorithm>
 

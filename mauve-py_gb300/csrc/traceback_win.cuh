@@ -2,10 +2,9 @@
 //
 // BitTraceBack (MU/bittraceback.cpp:138-210) is a serial walk from (LA, LB)
 // to (0, 0); walked one thread per problem, every step is a dependent global
-// load, and the longest path of a batch sets the traceback's time.  Both
-// traceback layouts (strips, gapdp_kernel.cuh; ring, gapdp_ring.cuh) store
-// 128-byte rows of 32 lane words, and the walk visits rows in non-increasing
-// order.  So one warp walks one long path: all lanes run the same walk, the
+// load, and the longest path of a batch sets the traceback's time.  The banded
+// strips (gapdp_kernel.cuh) store 128-byte rows of 32 lane words, and the walk
+// visits rows in non-increasing order.  So one warp walks one long path: all lanes run the same walk, the
 // rows come through shared memory in windows of kTbRows rows, the window
 // below the current one is prefetched with cp.async while the walk runs, and
 // lane 0 writes the path.  Short paths keep the thread-per-problem walker.

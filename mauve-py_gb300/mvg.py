@@ -490,11 +490,11 @@ class Context:
         _check(load_library().mvg_set_band_gate(self._h, int(min_match)))
 
     def set_dp_spin_limit(self, polls=1 << 26):
-        """Polls before a whole-CTA gap-DP wait gives up (watchdog); see mvg_set_dp_spin_limit."""
+        """Polls before a full-DP strip's wait for its predecessor gives up (watchdog); see mvg_set_dp_spin_limit."""
         _check(load_library().mvg_set_dp_spin_limit(self._h, int(polls)))
 
     def set_dp_coop_strips(self, strips):
-        """Full-DP problems of at least this many strips go to a whole CTA; see mvg_set_dp_coop_strips."""
+        """Full-DP problems of at least this many strips are pipelined strip by strip; see mvg_set_dp_coop_strips."""
         _check(load_library().mvg_set_dp_coop_strips(self._h, int(strips)))
 
     def set_mlp_tcgen05(self, on=True):
