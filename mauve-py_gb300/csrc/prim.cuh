@@ -479,8 +479,127 @@ void rts_sort_mers(K* const (&keys)[2], void* const (&buf)[2], int64_t n, int nb
   }
 }
 
-// The sort the workspace paths use: reduce-then-scan passes below 2^31
-// elements, the older three-kernel passes above.  scratch:
+// --------------------------------------------------- one CTA's radix sort
+//
+// Up to 8,192 pairs in one launch: a thread holds eight in registers, warp w
+// the 256 from 256 w on; a pass ranks them as k_rts_scatter does and exchanges
+// them through shared memory.  In place.  (Three launches per pass, each
+// waiting for the one before, took 45 us for the 20-bit keys of a few thousand
+// segments; this 12.)
+constexpr int kSmallSort = 8192;
+template <typename K>
+constexpr size_t small_sort_smem(int warps) {
+  return (size_t)warps * 256 * (sizeof(K) + 4) + (size_t)warps * 256 * 4;
+}
+
+template <typename K>
+__global__ void __launch_bounds__(1024) k_small_sort(K* __restrict__ keys, uint32_t* __restrict__ vals, int n,
+                                                     int npass, int dbits) {
+  extern __shared__ __align__(16) uint8_t ss_smem[];
+  __shared__ uint32_t wsum[8];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
+  K* const skey = reinterpret_cast<K*>(ss_smem);
+  uint32_t* const sval = reinterpret_cast<uint32_t*>(skey + warps * 256);
+  uint32_t* const wofs = sval + warps * 256;  // [warp][digit]: counts, then first slots
+  const int first = wid * 256 + lane, ndig = 1 << dbits;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  K key[8];
+  uint32_t val[8], rank[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int i = first + 32 * k;
+    key[k] = i < n ? keys[i] : (K)0;
+    val[k] = i < n ? vals[i] : 0u;
+  }
+  for (int p = 0; p < npass; ++p) {
+    const int shift = p * dbits;
+    for (int d = lane; d < ndig; d += 32) wofs[wid * ndig + d] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool live = first + 32 * k < n;
+      const uint32_t d = (uint32_t)(key[k] >> shift) & (ndig - 1);
+      uint32_t peers = __ballot_sync(0xffffffffu, live);
+      for (int b = 0; b < dbits; ++b) {
+        const uint32_t m = __ballot_sync(0xffffffffu, d >> b & 1u);
+        peers &= d >> b & 1u ? m : ~m;
+      }
+      const uint32_t before = wofs[wid * ndig + d];
+      rank[k] = before + __popc(peers & lt_mask);
+      __syncwarp();
+      if (live && (peers & lt_mask) == 0) wofs[wid * ndig + d] = before + __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    // threads 0 .. 255: digit tid's count in every warp, then its first slots
+    uint32_t total = 0, inc = 0;
+    if (tid < 256) {
+      if (tid < ndig)
+        for (int w = 0; w < warps; ++w) total += wofs[w * ndig + tid];
+      inc = warp_incl_scan(total);
+      if (lane == 31) wsum[wid] = inc;
+    }
+    __syncthreads();
+    if (tid < ndig) {
+      uint32_t run = inc - total;
+      for (int w = 0; w < wid; ++w) run += wsum[w];
+      for (int w = 0; w < warps; ++w) {
+        const uint32_t c = wofs[w * ndig + tid];
+        wofs[w * ndig + tid] = run;
+        run += c;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (first + 32 * k < n) {
+        const uint32_t at = wofs[wid * ndig + ((uint32_t)(key[k] >> shift) & (ndig - 1))] + rank[k];
+        skey[at] = key[k];
+        sval[at] = val[k];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int i = first + 32 * k;
+      if (i < n) {
+        key[k] = skey[i];
+        val[k] = sval[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int i = first + 32 * k;
+    if (i < n) {
+      keys[i] = key[k];
+      vals[i] = val[k];
+    }
+  }
+}
+
+// false when the device does not give it the shared memory.
+template <typename K>
+bool small_sort_pairs(K* keys, uint32_t* vals, int n, int nbits, cudaStream_t st, uint64_t* launches) {
+  static bool ready[64] = {};  // per device: the opt-in for more than 48 KB
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+  if (!ready[dev]) {
+    if (cudaFuncSetAttribute(k_small_sort<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)small_sort_smem<K>(32)) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    ready[dev] = true;
+  }
+  const int warps = n <= 2048 ? 8 : (n + 255) / 256;
+  const int npass = (nbits + 7) / 8, dbits = (nbits + npass - 1) / npass;
+  k_small_sort<K><<<1, 32 * warps, small_sort_smem<K>(warps), st>>>(keys, vals, n, npass, dbits);
+  if (launches) *launches += 1;
+  return true;
+}
+
+// The sort the workspace paths use: one CTA's for a few thousand elements,
+// reduce-then-scan passes below 2^31, the older three-kernel passes above.  scratch:
 // sort_scratch_words(n, nbits) words.
 inline int64_t sort_scratch_words(int64_t n, int nbits) {
   const int64_t a = radix_scratch_words(n), b = rts_scratch_words(n, nbits);
@@ -491,6 +610,8 @@ template <typename K>
 int sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n, int nbits, uint32_t* scratch,
                cudaStream_t st, uint64_t* launches, uint32_t* err) {
   (void)err;
+  if (n <= 0) return 0;
+  if (n <= kSmallSort && nbits > 0 && small_sort_pairs<K>(keys, vals, (int)n, nbits, st, launches)) return 0;
   if (n < (1ll << 31)) return rts_sort_pairs<K>(keys, vals, keys_alt, vals_alt, n, nbits, scratch, st, launches);
   return radix_sort_pairs<K>(keys, vals, keys_alt, vals_alt, n, nbits, scratch, st, launches);
 }

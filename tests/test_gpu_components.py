@@ -89,3 +89,16 @@ def test_walks_across_repeats(ctx, gap, flip):
         b = synth.revcomp(b)
     seed = mvg.get_seed(15, 0)
     np.testing.assert_array_equal(ctx.pairwise_matches(a, b, seed), O.pairwise_matches(a, b, seed))
+
+
+@pytest.mark.parametrize("n", [2_000, 60_000, 230_000, 262_000, 300_000])
+@pytest.mark.parametrize("weight", [15, 17])
+def test_segment_order_around_one_cta_s_sort(ctx, n, weight):
+    """From a few segment ends to twice as many as one CTA sorts."""
+    rng = np.random.default_rng(n + weight)
+    a = synth.random_bases(rng, n)
+    b = synth._substitute(rng, a, rng.random(n) < 0.06)
+    b[n // 3:n // 2] = synth.revcomp(b[n // 3:n // 2])
+    seed = mvg.get_seed(weight, 0)
+    got = ctx.pairwise_matches(a, b, seed)
+    np.testing.assert_array_equal(got, O.pairwise_matches(a, b, seed))
