@@ -217,10 +217,12 @@ __global__ void __launch_bounds__(1024) k_pb_scan(const uint32_t* __restrict__ c
   if (d0 >= nbk) return;
   uint32_t start = wsum[wid] + inc - mine;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    bstart[d0 + k] = start;
-    bsize[d0 + k] = tot[k];
-    start += tot[k];
+  for (int k = 0; k < kPer; k += 4) {  // 16 bytes at a time: nbk is a multiple of 4, both arrays aligned
+    if (d0 + k >= nbk) break;
+    const uint32_t s1 = start + tot[k], s2 = s1 + tot[k + 1], s3 = s2 + tot[k + 2];
+    *reinterpret_cast<uint4*>(bstart + d0 + k) = make_uint4(start, s1, s2, s3);
+    *reinterpret_cast<uint4*>(bsize + d0 + k) = make_uint4(tot[k], tot[k + 1], tot[k + 2], tot[k + 3]);
+    start = s3 + tot[k + 3];
   }
 }
 

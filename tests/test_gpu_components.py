@@ -102,3 +102,14 @@ def test_segment_order_around_one_cta_s_sort(ctx, n, weight):
     seed = mvg.get_seed(weight, 0)
     got = ctx.pairwise_matches(a, b, seed)
     np.testing.assert_array_equal(got, O.pairwise_matches(a, b, seed))
+
+
+@pytest.mark.parametrize("seed", [0b1, 0b11, 0b101, 0b1101, 0b10111])
+def test_fewest_buckets(ctx, seed):
+    """Seeds of so few bases that the join has four to sixteen buckets."""
+    rng = np.random.default_rng(seed)
+    for n in (3, 9, 40, 200):
+        a, b = synth.random_bases(rng, n), synth.random_bases(rng, n + 2)
+        np.testing.assert_array_equal(ctx.pairwise_matches(a, b, seed), O.pairwise_matches(a, b, seed))
+    same = np.frombuffer(b"ACGTTGCAAC", np.uint8)
+    np.testing.assert_array_equal(ctx.pairwise_matches(same, same, seed), O.pairwise_matches(same, same, seed))
