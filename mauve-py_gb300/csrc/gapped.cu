@@ -32,7 +32,6 @@
 #include <functional>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -180,12 +179,10 @@ class Team {
  public:
   explicit Team(size_t n) {
     const size_t hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    for (size_t t = 1; t < std::min(hw, n); ++t) {
-      try {
-        pool_.emplace_back([this, t] { worker(t); });
-      } catch (const std::system_error&) {
-        break;  // fewer threads
-      }
+    try {
+      pool_.reserve(hw);
+      for (size_t t = 1; t < std::min(hw, n); ++t) pool_.emplace_back([this, t] { worker(t); });
+    } catch (...) {  // fewer threads, and none to leave behind
     }
   }
   ~Team() {
