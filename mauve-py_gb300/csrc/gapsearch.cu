@@ -295,9 +295,10 @@ __host__ __device__ __forceinline__ void walk_overlaps(Anchor* a, int32_t* at, i
 // left ends in A); m > 1 the B half of the gap's first m rows, which the A half
 // left in order (two equal left ends in B).  Latency of the sorts and the
 // longest run's walk bound it.  (On 16 host threads, all of it: 1.9 ms per
-// 180,000 matches; a walk by one thread per gap: 0.46 ms.)
+// 180,000 matches; a walk by one thread per gap: 0.46 ms; with 128 threads
+// 0.124 ms, with 256 0.102.)
 constexpr int kGsFilterRows = 1536;
-constexpr int kGsFilterThreads = 128;
+constexpr int kGsFilterThreads = 256;
 __global__ void __launch_bounds__(kGsFilterThreads)
     k_gs_filter(Anchor* __restrict__ rows, const uint32_t* __restrict__ gap_row, uint32_t* __restrict__ kept,
                 uint32_t* __restrict__ todo) {
