@@ -113,3 +113,15 @@ def test_fewest_buckets(ctx, seed):
         np.testing.assert_array_equal(ctx.pairwise_matches(a, b, seed), O.pairwise_matches(a, b, seed))
     same = np.frombuffer(b"ACGTTGCAAC", np.uint8)
     np.testing.assert_array_equal(ctx.pairwise_matches(same, same, seed), O.pairwise_matches(same, same, seed))
+
+
+@pytest.mark.parametrize("weight", [16, 21, 22, 23, 25, 31])
+def test_join_and_sort_on_both_sides_of_their_line(ctx, weight):
+    """Seeds of up to 22 bases go through the bucketed join, longer ones through
+    the sort of both genomes' keys."""
+    rng = np.random.default_rng(weight)
+    a = synth.random_bases(rng, 30_000)
+    b = synth._substitute(rng, a, rng.random(len(a)) < 0.01)
+    b = np.concatenate([b[:12_000], synth.revcomp(b[12_000:20_000]), b[500:1500], b[20_000:]])
+    seed = (1 << weight) - 1  # solid: any weight up to 31
+    np.testing.assert_array_equal(ctx.pairwise_matches(a, b, seed), O.pairwise_matches(a, b, seed))
