@@ -147,13 +147,25 @@ struct GapSet {
   }
 };
 
+// The gather tables (gather_mer) of the weights in `weights` (bit w; the
+// default weights are odd, 5 to 15), 6 window bytes each: seeds of up to 23
+// bases.  (Gathering run by run, some 190 instructions per position, took 0.48
+// ms for the keys of 43 Mbp and 0.58 for their scatter, with the tables 0.32 and
+// 0.53.)
+constexpr int kGsTables = 6, kGsTableBytes = 6;
+constexpr int kGsLutBytes = kGsTables * kGsTableBytes * 256 * 4;
+using GsLut = uint32_t (*)[kGsTableBytes][256];
+__device__ __forceinline__ void gs_lut(uint32_t weights, GsLut lut) {
+  for (int t = 0; t < kGsTables; ++t)
+    if (weights >> (kGsMinWeight + 2 * t) & 1) seed_lut_build32(c_gs_seed[kGsMinWeight + 2 * t], lut[t]);
+}
+
 // Calls f(mixed keys, strands, in B, first slot, valid) for groups of four
 // slots of this block's tile (A's, then B's), of which those with a bit in
 // `valid` hold a seed position; a warp's slots, and so a group's, are aligned
-// pieces of gaps.  A seed of the table is at most 23 bases long up to weight
-// 15, so a group's seeds lie in one 32-base window.
+// pieces of gaps.  A group's seeds lie in one 32-base window.
 template <class F>
-__device__ __forceinline__ void gs_tile(const GapSet& P, int bits, int64_t tile, F f) {
+__device__ __forceinline__ void gs_tile(const GapSet& P, GsLut lut, int bits, int64_t tile, F f) {
   const uint64_t n = (uint64_t)P.slots[0] + P.slots[1], base = (uint64_t)blockIdx.x * (uint64_t)tile;
   for (int64_t o = 4 * threadIdx.x; o < tile; o += 4 * blockDim.x) {
     const uint64_t p = base + (uint64_t)o;
@@ -165,27 +177,35 @@ __device__ __forceinline__ void gs_tile(const GapSet& P, int bits, int64_t tile,
     const uint32_t x = q - d.slot[side];
     if (x >= d.cnt[side]) continue;
     const SeedDesc& s = c_gs_seed[d.w];
+    const uint32_t(*const table)[256] = lut[(d.w - kGsMinWeight) >> 1];
+    const int nb = seed_bytes(s), w = s.w;
     const uint64_t win = window64((side ? P.pb : P.pa) + d.word[side], x);
     uint64_t key[4];
     uint32_t strand[4], valid = 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint64_t fw = gather_seed(win << 2 * u, s), r = revcomp_mer(fw, s.w), m = fw < r ? fw : r;
-      key[u] = mix_mer<uint64_t>((uint64_t)g << P.mbits | m >> (64 - 2 * s.w), bits);
-      strand[u] = (uint32_t)m & 1u;
+      uint32_t fw = 0;
+#pragma unroll
+      for (int c = 0; c < kGsTableBytes; ++c)
+        if (c < nb) fw |= table[c][(uint32_t)(win >> (56 - 8 * c - 2 * u)) & 255u];
+      const uint32_t r = revcomp_mer32(fw, w), m = fw < r ? fw : r;
+      key[u] = mix_mer<uint64_t>((uint64_t)g << P.mbits | m >> (32 - 2 * w), bits);
+      strand[u] = m & 1u;
       valid |= (x + u < d.cnt[side] ? 1u : 0u) << u;
     }
     f(key, strand, side, q, valid);
   }
 }
 
-__global__ void __launch_bounds__(1024) k_gs_keys(GapSet P, int bits, int bbits, int64_t tile,
+__global__ void __launch_bounds__(1024) k_gs_keys(GapSet P, uint32_t weights, int bits, int bbits, int64_t tile,
                                                   uint32_t* __restrict__ counts) {
-  extern __shared__ uint32_t h[];  // nbuckets counts
+  extern __shared__ uint32_t h[];  // nbuckets counts, the gather tables
   const int nbk = 1 << bbits, bsh = bits - bbits;
+  GsLut lut = reinterpret_cast<GsLut>(h + nbk);
+  gs_lut(weights, lut);
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) h[d] = 0;
   __syncthreads();
-  gs_tile(P, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&)[4], int, uint32_t, uint32_t valid) {
+  gs_tile(P, lut, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&)[4], int, uint32_t, uint32_t valid) {
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (valid >> u & 1) atomicAdd(&h[(uint32_t)(k[u] >> bsh)], 1u);
@@ -194,14 +214,16 @@ __global__ void __launch_bounds__(1024) k_gs_keys(GapSet P, int bits, int bbits,
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) counts[(int64_t)blockIdx.x * nbk + d] = h[d];
 }
 
-__global__ void __launch_bounds__(1024) k_gs_scatter(GapSet P, int bits, int bbits, int64_t tile,
+__global__ void __launch_bounds__(1024) k_gs_scatter(GapSet P, uint32_t weights, int bits, int bbits, int64_t tile,
                                                      const uint32_t* __restrict__ offsets, uint2* __restrict__ out) {
-  extern __shared__ uint32_t cur[];  // next free slot per bucket
+  extern __shared__ uint32_t cur[];  // next free slot per bucket, the gather tables
   const int nbk = 1 << bbits, bsh = bits - bbits;
+  GsLut lut = reinterpret_cast<GsLut>(cur + nbk);
+  gs_lut(weights, lut);
   const uint32_t rest = (uint32_t)(((uint64_t)1 << bsh) - 1);
   for (int d = threadIdx.x; d < nbk; d += blockDim.x) cur[d] = offsets[(int64_t)blockIdx.x * nbk + d];
   __syncthreads();
-  gs_tile(P, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&strand)[4], int side, uint32_t q, uint32_t valid) {
+  gs_tile(P, lut, bits, tile, [&](const uint64_t(&k)[4], const uint32_t(&strand)[4], int side, uint32_t q, uint32_t valid) {
     uint32_t slot[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -611,7 +633,10 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   // a seed's bits are its pattern's selected positions, which for some table
   // entries exceed the nominal weight (weight 11's rank-0 seed selects 12)
   int wmax = 0;
-  for (const GapDev& d : ch.gd) wmax = std::max(wmax, __builtin_popcountll(mvg_get_seed((int)d.w, 0)));
+  uint32_t weights = 0;
+  for (const GapDev& d : ch.gd) weights |= 1u << d.w;
+  for (int w = kGsMinWeight; w < 32; ++w)
+    if (weights >> w & 1) wmax = std::max(wmax, __builtin_popcountll(mvg_get_seed(w, 0)));
   GapSet P{pa, pb, d_gaps, gmap, gmap + wa, {ch.slots[0], ch.slots[1]}, 2 * wmax, nullptr};
   const int bits = 2 * wmax + gbits;
   if (bits > kPairMaxBits) return report_error(MVG_ERR_DEVICE, "gap search keys wider than the join's");
@@ -620,16 +645,17 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   if (rc) return rc;
   static bool attr = false;  // once per process: more than 48 KB of dynamic shared memory
   if (!attr) {
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
+    MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4 + kGsLutBytes));
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneCta));
     attr = true;
   }
-  const size_t hsm = (size_t)b.g.nbuckets * 4;
+  const size_t hsm = (size_t)b.g.nbuckets * 4 + kGsLutBytes;
+  static_assert(16384 * 4 + kGsLutBytes <= kOneCta, "the scatter's shared memory");
   k_gs_slots<<<ng, 128, 0, c->stream>>>(d_gaps, gmap, gmap + wa);
-  k_gs_keys<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.counts);
+  k_gs_keys<<<(unsigned)b.g.ntiles, 1024, hsm, c->stream>>>(P, weights, bits, b.g.bbits, b.g.tile, b.counts);
   pair_bucket_offsets(c, b);
   stage_mark(c, "gs_scatter");
-  k_gs_scatter<<<(unsigned)b.g.ntiles, 1024, kOneCta, c->stream>>>(P, bits, b.g.bbits, b.g.tile, b.offs, b.buf);
+  k_gs_scatter<<<(unsigned)b.g.ntiles, 1024, kOneCta, c->stream>>>(P, weights, bits, b.g.bbits, b.g.tile, b.offs, b.buf);
   c->launches += 3;
   stage_mark(c, "gs_join");
   pair_bucket_join(c, b, tab);
