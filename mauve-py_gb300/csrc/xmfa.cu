@@ -49,6 +49,21 @@ __device__ __forceinline__ uint8_t xmfa_byte(const XmfaPiece& pc, uint64_t o, co
   return pos == 80 || c == pc.len ? (uint8_t)'\n' : (pc.row == 0 ? rows_a : rows_b)[pc.src + c];
 }
 
+// Short texts: pieces along grid.y, each piece's output bytes spread over
+// grid.x, so that no thread looks for its piece.
+__global__ void __launch_bounds__(256) k_xmfa_bytes(const XmfaPiece* __restrict__ pieces, int64_t npieces,
+                                                    const uint8_t* __restrict__ blob,
+                                                    const uint8_t* __restrict__ rows_a,
+                                                    const uint8_t* __restrict__ rows_b, uint8_t* __restrict__ out) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (int64_t k = blockIdx.y; k < npieces; k += gridDim.y) {
+    const XmfaPiece pc = pieces[k];
+    const uint64_t n = pc.row < 0 ? pc.len : pc.len + (pc.len + 79) / 80;
+    for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += step)
+      out[pc.dst + o] = xmfa_byte(pc, o, blob, rows_a, rows_b);
+  }
+}
+
 // A thread per 16 bytes of the text, four at a time: four columns of one line
 // from the two aligned words that hold them (where both lie in the row), other
 // bytes one by one.  The copy to the host (52 us for 9.6 MB at 184 GB/s) and
@@ -210,8 +225,20 @@ extern "C" int mvg_xmfa_write_dev(mvg_handle h, const char* file_a, const char* 
   if (int rc = h2d_async(c, d_pieces, pieces.data(), pieces.size() * sizeof(XmfaPiece), c->stream)) return rc;
   if (int rc = h2d_async(c, d_blob, blob.data(), blob.size(), c->stream)) return rc;
   const int64_t np = (int64_t)pieces.size();
-  k_xmfa_assemble<<<(unsigned)((total + 4095) / 4096), 256, 0, c->stream>>>(d_pieces, np, d_blob, d_rows_a, d_rows_b,
-                                                                            col_off[nblocks], total, d_out);
+  // a byte per thread up to here: the other kernel's search for the piece costs
+  // a short text 3 to 7 us (80,227 bases in 7 blocks: the call 58 and 62 us,
+  // 20,000 in 200: 101 and 108), a long one gains (300,000 in 50: 78 and 76,
+  // 4.6 million in 64: 142 and 138)
+  constexpr uint64_t kShortText = 400000;
+  if (total <= kShortText) {
+    uint64_t widest = 0;  // output bytes of the largest piece
+    for (const XmfaPiece& pc : pieces) widest = std::max(widest, pc.row < 0 ? pc.len : pc.len + (pc.len + 79) / 80);
+    const dim3 grid((unsigned)std::max<uint64_t>((widest + 1023) / 1024, 1), (unsigned)std::min<int64_t>(np, 65535));
+    k_xmfa_bytes<<<grid, 256, 0, c->stream>>>(d_pieces, np, d_blob, d_rows_a, d_rows_b, d_out);
+  } else {
+    k_xmfa_assemble<<<(unsigned)((total + 4095) / 4096), 256, 0, c->stream>>>(d_pieces, np, d_blob, d_rows_a, d_rows_b,
+                                                                              col_off[nblocks], total, d_out);
+  }
   c->launches++;
   MVG_CUDA_TRY(cudaGetLastError());
   MVG_CUDA_TRY(cudaMemcpyAsync(out, d_out, total, cudaMemcpyDeviceToHost, c->stream));

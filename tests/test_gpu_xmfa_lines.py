@@ -1,4 +1,4 @@
-"""XMFA text where its pieces meet: rows of one to a few columns, of whole
+"""XMFA text where its pieces meet, short and long enough for either kernel: rows of one to a few columns, of whole
 lines and one more or less, empty blocks, absent sequences, and rows that
 start off a word boundary, against the text put together line by line."""
 import numpy as np
@@ -41,7 +41,8 @@ def text_of(names, starts, lengths, rows, off):
 
 @pytest.mark.parametrize("shift", [(0, 0), (1, 2), (3, 16)])
 @pytest.mark.parametrize("widths", [[1], [79], [80], [81], [1, 2, 3, 4, 5, 0, 1, 1], [160, 161, 159, 0, 80],
-                                    [4, 76, 77, 78, 400], [5000, 1, 12_345], [3] * 300])
+                                    [4, 76, 77, 78, 400], [5000, 1, 12_345], [3] * 300, [180_000, 7],
+                                    [196_000], [300_001, 1, 80, 79, 5]])
 def test_text_of_uneven_blocks(ctx, widths, shift):
     import torch
     rng = np.random.default_rng(sum(widths) + len(widths))
