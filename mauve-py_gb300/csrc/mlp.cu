@@ -11,10 +11,11 @@
 // GELU and (last layer) the 256 -> 2 output layer in the epilogue
 // (mlp_tc.cuh).  Forward when the tcgen05 path is switched off or an operand
 // does not meet its TMA rules: C[M x N] (fp32) = A[M x K] * B[N x K]^T with
-// bf16 operands; a 64x64 block tile, four warps of 32x32 (2 x 4 mma.sync
-// tiles), K step 32 staged in shared memory with both operands stored
-// k-contiguous so every fragment is one 32-bit shared load.  Backward:
-// mlp_grad.cuh.
+// bf16 operands (k_gemm_bf16 for the output layer; a 64x64 block tile, four
+// warps of 32x32 (2 x 4 mma.sync tiles), K step 32 staged in shared memory with
+// both operands stored k-contiguous so every fragment is one 32-bit shared load)
+// and, for the hidden layers with bias and GELU, k_mlp_layer_mma (mlp_grad.cuh,
+// which also holds the backward pass).
 #include <cuda_bf16.h>
 #include <math.h>
 #include <string.h>
@@ -155,15 +156,6 @@ __device__ __forceinline__ float gelu_grad(float x) {
 #include "mlp_tc.cuh"
 
 namespace mvg {
-
-__global__ void k_bias_gelu(float* __restrict__ z, const float* __restrict__ b, __nv_bfloat16* __restrict__ h,
-                            int64_t n, int d) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * d; e += (int64_t)gridDim.x * blockDim.x) {
-    const float v = z[e] + b[e % d];
-    z[e] = v;
-    h[e] = __float2bfloat16(gelu(v));
-  }
-}
 
 __global__ void k_bias_add(float* __restrict__ z, const float* __restrict__ b, int64_t n, int d) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * d; e += (int64_t)gridDim.x * blockDim.x)
@@ -452,12 +444,13 @@ static void mlp_forward(Ctx* c, MlpState& s, const __nv_bfloat16* X, int64_t n, 
       return;
     }
   }
-  gemm(st, X, kIn, s.wb + kOffW1, kIn, s.z[0], kHid, nn, kHid, kIn, &c->launches);
-  k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[0], s.w + kOffB1, s.h[0], n, kHid);
-  gemm(st, s.h[0], kHid, s.wb + kOffW2, kHid, s.z[1], kHid, nn, kHid, kHid, &c->launches);
-  k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[1], s.w + kOffB2, s.h[1], n, kHid);
-  gemm(st, s.h[1], kHid, s.wb + kOffW3, kHid, s.z[2], kHid, nn, kHid, kHid, &c->launches);
-  k_bias_gelu<<<eltwise_grid(n * kHid), 256, 0, st>>>(s.z[2], s.w + kOffB3, s.h[2], n, kHid);
+  const int64_t offW[3] = {kOffW1, kOffW2, kOffW3}, offB[3] = {kOffB1, kOffB2, kOffB3};
+  for (int q = 0; q < 3; ++q) {
+    const __nv_bfloat16* in = q == 0 ? X : s.h[q - 1];
+    k_mlp_layer_mma<<<(unsigned)((n + kGradTile - 1) / kGradTile * 4), kGradThreads, 0, st>>>(
+        in, ((uintptr_t)in & 15) == 0, s.wb + offW[q], s.w + offB[q], n, q == 0 ? kIn : kHid, train ? s.z[q] : nullptr,
+        s.h[q]);
+  }
   gemm(st, s.h[2], kHid, s.wb + kOffW4, kHid, s.out, kOut, nn, kOut, kHid, &c->launches);
   k_bias_add<<<eltwise_grid(n * kOut), 256, 0, st>>>(s.out, s.w + kOffB4, n, kOut);
   c->launches += 4;

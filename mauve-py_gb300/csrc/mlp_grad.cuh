@@ -1,5 +1,6 @@
-// Backward pass of the band-proposal MLP (included by mlp.cu after the GELU
-// helpers).  Four kinds of launch:
+// Backward pass of the band-proposal MLP, and its forward layers off the TMA
+// path (included by mlp.cu after the GELU helpers).  The backward pass is four
+// kinds of launch:
 //
 //   k_grad_top    loss, dO and the 256 -> 2 output layer's gradients, and
 //                 dZ3 = (dO W4) * gelu'(Z3)
@@ -54,6 +55,85 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr)
                : "memory");
+}
+
+// A hidden layer of the forward pass for operands off TMA's rules: z = A W^T +
+// b, h = GELU(z) for A [M x K], W [256 x K] (K a multiple of 8), a CTA per 64 x
+// 64 tile, three stages of 32 columns in flight.  The products are added in the
+// order of the plain GEMM it stands in for (k_gemm_bf16, 16 at a time), so its
+// results are the same bits; with that and a launch for bias and GELU the forward
+// call took 148 us over 1,003 rows and 1.10 ms over 100,001, now 70 and 382.  wide: A may be loaded 16 bytes at a
+// time.  z may be null.
+__global__ void __launch_bounds__(kGradThreads) k_mlp_layer_mma(const __nv_bfloat16* __restrict__ A, int wide,
+                                                                const __nv_bfloat16* __restrict__ W,
+                                                                const float* __restrict__ bias, int64_t M, int K,
+                                                                float* __restrict__ z, __nv_bfloat16* __restrict__ h) {
+  constexpr int kStages = 3, kPitch = kGradK + 8;
+  __shared__ __align__(16) __nv_bfloat16 s_a[kStages][kGradTile][kPitch], s_b[kStages][kGradTile][kPitch];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int n0 = ((int)blockIdx.x & 3) * kGradTile;
+  const int64_t m0 = (int64_t)(blockIdx.x >> 2) * kGradTile;
+  const int steps = (K + kGradK - 1) / kGradK, wm = (wid >> 1) * 32, wn = (wid & 1) * 32;
+  auto load = [&](int step) {
+    const int s = step % kStages;
+    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(&s_a[s][0][0]);
+    const uint32_t b0 = (uint32_t)__cvta_generic_to_shared(&s_b[s][0][0]);
+#pragma unroll
+    for (int e = tid; e < kGradTile * (kGradK / 8); e += kGradThreads) {
+      const int r = e >> 2, q = (e & 3) * 8, k = step * kGradK + q;
+      const bool in = k < K, live = in && m0 + r < M;
+      cp16(b0 + (r * kPitch + q) * 2, W + (in ? (int64_t)(n0 + r) * K + k : 0), in);
+      if (wide) {
+        cp16(a0 + (r * kPitch + q) * 2, A + (live ? (m0 + r) * K + k : 0), live);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s_a[s][r][q + u] = live ? A[(m0 + r) * K + k + u] : __float2bfloat16(0.f);
+      }
+    }
+  };
+  float acc[2][4][4] = {};
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    if (s < steps) load(s);
+    cp_commit();
+  }
+  for (int step = 0; step < steps; ++step) {
+    cp_wait<kStages - 2>();
+    __syncthreads();
+    if (step + kStages - 1 < steps) load(step + kStages - 1);
+    cp_commit();
+    const int s = step % kStages;
+    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(&s_a[s][0][0]);
+    const uint32_t b0 = (uint32_t)__cvta_generic_to_shared(&s_b[s][0][0]);
+#pragma unroll
+    for (int k = 0; k < kGradK; k += 16) {
+      uint32_t a[2][4], b[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldsm4(a[i], a0 + ((wm + i * 16 + (lane & 15)) * kPitch + k + (lane >> 4) * 8) * 2);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)  // matrices (n, k), (n, k + 8), (n + 8, k), (n + 8, k + 8)
+        ldsm4(b[j], b0 + ((wn + j * 16 + (lane & 7) + (lane >> 4) * 8) * kPitch + k + ((lane >> 3) & 1) * 8) * 2);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], a[i], &b[j >> 1][(j & 1) * 2]);
+    }
+  }
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int64_t r = m0 + wm + i * 16 + half * 8 + g;
+      if (r >= M) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = n0 + wn + j * 8 + 2 * t;
+        const float v0 = acc[i][j][2 * half] + bias[c], v1 = acc[i][j][2 * half + 1] + bias[c + 1];
+        if (z) *reinterpret_cast<float2*>(z + r * kHid + c) = make_float2(v0, v1);
+        *reinterpret_cast<__nv_bfloat162*>(h + r * kHid + c) = __floats2bfloat162_rn(gelu(v0), gelu(v1));
+      }
+    }
 }
 
 // part layout of k_grad_top, per CTA: db3 [256], dW4 [2 x 256], db4 [2], loss.
