@@ -266,18 +266,14 @@ static int tb_long_plan(Ctx* c, const std::vector<uint32_t>& slot_len, std::vect
   long_slots->clear();
   *long_path = INT_MAX;
   *grid = 0;
-  static bool attr = false;  // once per process: more than 48 KB of shared memory
-  static int cap = 0;
-  int sms = 0;
-  MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  if (!attr) {
+  if (!c->tb_grid) {
+    int sms = 0, bps = 0;
+    MVG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_traceback_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTbSmem));
-    int bps = 0;
     MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_traceback_win, kTbWarps * 32, kTbSmem));
-    cap = std::max(1, bps) * kTbWarps;
-    attr = true;
+    c->tb_grid = sms * std::max(1, bps);
   }
-  const size_t round = (size_t)cap * (size_t)sms;
+  const size_t round = (size_t)c->tb_grid * kTbWarps;
   std::vector<uint32_t> lens;
   for (uint32_t L : slot_len)
     if (L >= (uint32_t)kTbLongPath) lens.push_back(L);
@@ -296,7 +292,7 @@ static int tb_long_plan(Ctx* c, const std::vector<uint32_t>& slot_len, std::vect
   long_slots->resize(sel.size());
   for (size_t q = 0; q < sel.size(); ++q) (*long_slots)[q] = sel[q].second;
   const int n = (int)long_slots->size();
-  *grid = std::min(sms * (cap / kTbWarps), (n + kTbWarps - 1) / kTbWarps);
+  *grid = std::min(c->tb_grid, (n + kTbWarps - 1) / kTbWarps);
   *long_path = (int)thr;
   return 0;
 }

@@ -643,11 +643,10 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   PairBucketBufs b;
   int rc = pair_bucket_bufs(c, (uint64_t)ch.slots[0] + ch.slots[1], bits, &b);
   if (rc) return rc;
-  static bool attr = false;  // once per process: more than 48 KB of dynamic shared memory
-  if (!attr) {
+  if (!c->search_ready) {  // more than 48 KB of dynamic shared memory
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_keys, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4 + kGsLutBytes));
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_gs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneCta));
-    attr = true;
+    c->search_ready = true;
   }
   const size_t hsm = (size_t)b.g.nbuckets * 4 + kGsLutBytes;
   static_assert(16384 * 4 + kGsLutBytes <= kOneCta, "the scatter's shared memory");

@@ -62,6 +62,11 @@ struct Ctx {
   int dp_coop_strips = 16;               // full-DP problems of at least this many strips run on a warp per strip
   int strip_grid = 0, walk_grid = 0, sms = 0;  // full DP: resident CTAs of the strips and walk kernels, SMs (0: not asked yet)
   int ring_grid[2] = {};                 // resident CTAs of the tall and the low ring launch (0: not asked yet)
+  int tb_grid = 0;                       // resident CTAs of the banded strips' walk of long paths (0: not asked yet)
+  // Kernels of more than 48 KB of dynamic shared memory are allowed it per
+  // device, so once per handle: the seed join's (32- and 64-bit mers) and the
+  // gap search's.
+  bool join_ready[2] = {}, search_ready = false;
   cudaGraphExec_t dp_exec[2] = {};       // the executable graph of each DP lane, updated per call
   uint64_t graph_launches = 0;
   int mlp_tc = 1;              // MLP forward hidden layers on tcgen05 (else mma.sync)

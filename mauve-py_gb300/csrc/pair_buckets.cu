@@ -553,11 +553,11 @@ static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32
   PairBucketBufs b;
   if (int rc = pair_bucket_bufs(c, ca + cb, 2 * s.w, &b)) return rc;
   const PairBucketGeom& g = b.g;
-  static bool attr = false;  // once per process and key type: more than 48 KB of dynamic shared memory
-  if (!attr) {
+  bool& ready = c->join_ready[sizeof(K) == 8];
+  if (!ready) {  // more than 48 KB of dynamic shared memory
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_keys<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 64) * 4));
     MVG_CUDA_TRY(cudaFuncSetAttribute(k_pb_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneCta));
-    attr = true;
+    ready = true;
   }
   const size_t hsm = (size_t)g.nbuckets * 4;
   k_pb_keys<K><<<(unsigned)g.ntiles, pb::kKeyThreads, hsm, c->stream>>>(ga, ca, gb, cb, s, b.counts, g.bbits, g.tile);
