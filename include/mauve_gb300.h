@@ -563,7 +563,9 @@ int mvg_xmfa_write_dev(mvg_handle h, const char* file_a, const char* file_b, con
 
 /* Upper bound on the device bytes the gap-DP traceback arena may use.  Each
  * call uses min(bound, 60% of free device memory); problems run in waves of
- * mixed sizes that fit it.  Default: no bound beyond the 60% cap. */
+ * mixed sizes that fit it, and a problem of the full DP that alone would not
+ * fit keeps fewer of its states (also with mvg_set_dp_checkpoint off).  The
+ * buffer itself may be an eighth larger.  Default: no bound beyond the 60% cap. */
 int mvg_set_tb_arena(mvg_handle h, uint64_t bytes);
 
 /* Gap-DP kernel shape: rows per lane for the full DP (4 or 8) and for banded

@@ -488,10 +488,11 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   if (!c->strip_grid) {
     int bps = 0;
     MVG_CUDA_TRY(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
-    MVG_CUDA_TRY(cudaFuncSetAttribute(k_strip_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
-    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_strip_walk, kWalkWarps * 32, kWalkSmem));
+    for (auto walk : {k_strip_walk<false>, k_strip_walk<true>})
+      MVG_CUDA_TRY(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_strip_walk<true>, kWalkWarps * 32, kWalkSmem));
     c->walk_grid = c->sms * std::max(1, bps);
-    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_strips, kStWarps * 32, 0));
+    MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_gapdp_strips<true>, kStWarps * 32, 0));
     c->strip_grid = c->sms * std::max(1, bps);
   }
   // A pass of fewer strips than the chip has warp schedulers is bound by the
@@ -503,29 +504,40 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   const bool few = strips_all <= 4 * c->sms;
   const int max_rows = few ? 4 : c->dp_rows;
   const int min_piped = few ? 2 : c->dp_coop_strips;
-  std::vector<uint64_t> bytes(nwork), cells(nwork);
+  std::vector<uint64_t> bytes(nwork), cells(nwork), shapes(nwork);
   std::vector<char> piped(nwork), direct(nwork);
   std::vector<uint32_t> strips(nwork);
   uint64_t total = 0, most = 0, most_least = 0;
-  for (int64_t w = 0; w < nwork; ++w) {
+  auto shape = [&](int64_t w, uint64_t limit) {
     const uint32_t p = ids[w];
-    const StripShape h = strip_shape((int)la[p], (int)lb[p], max_rows, ckpt);
+    const StripShape h = strip_shape_within(strip_shape((int)la[p], (int)lb[p], max_rows, ckpt), limit);
     bytes[w] = strip_slot_bytes(h);
-    cells[w] = (uint64_t)la[p] * (uint64_t)lb[p];
     strips[w] = (uint32_t)h.n;
     piped[w] = h.n >= min_piped;
     direct[w] = h.direct;
-    total += bytes[w];
+    shapes[w] = strip_slot(0, h);
     most = std::max(most, bytes[w]);
+    return h;
+  };
+  for (int64_t w = 0; w < nwork; ++w) {
+    const StripShape h = shape(w, ~0ull);
+    cells[w] = (uint64_t)h.LA * (uint64_t)h.LB;
+    total += bytes[w];
     most_least = std::max(most_least, std::min(bytes[w], strip_least_bytes(h, c->dp_rows, ckpt)));
   }
-  uint64_t arena = arena_bound(c, kDpSlots.arena, total);
-  if (most_least > arena) return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
-  arena = std::max(arena, most);
+  const uint64_t arena = arena_bound(c, kDpSlots.arena, total);
+  const bool sparse = most > arena;  // slots cut to fit
+  if (sparse) {
+    most = 0;
+    for (int64_t w = 0; w < nwork; ++w) shape(w, arena);
+  }
+  if (std::max(most, most_least) > arena)
+    return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
   sub.reset(new HostSpan(c, "dp_sort"));
   const std::vector<uint32_t> idx = largest_first(cells);
   sub.reset(new HostSpan(c, "dp_waves"));
-  const DpWaves W = deal_waves(idx, piped, bytes, arena);
+  DpWaves W = deal_waves(idx, piped, bytes, arena);
+  for (int64_t q = 0; q < nwork; ++q) W.off[q] |= shapes[W.item[q]];
   const size_t nwaves = W.begin.size() - 1;
   // one upload: the slots' problems, then per wave the pipelined strips in
   // claim order (pairs) and the walk's slots (checkpointed, then direct)
@@ -582,7 +594,7 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     J.sb = in.sb;
     J.ob = in.ob;
     J.order = d_order + w0;
-    J.slot_off = d_off + w0;
+    J.slots = d_off + w0;
     J.units = reinterpret_cast<const uint2*>(d_order + units_at[wv]);
     J.nwork = (int)n;
     J.npipe = (int)W.nbig[wv];
@@ -597,12 +609,13 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     J.spin_limit = c->dp_spin_limit;
     stage_mark(c, "dp");
     if (J.npipe) {
-      k_strip_unwritten<<<dim3(std::min(J.npipe, 4096), 8), 256, 0, c->stream>>>(J);
+      (sparse ? k_strip_unwritten<true> : k_strip_unwritten<false>)<<<dim3(std::min(J.npipe, 4096), 8), 256, 0,
+                                                                      c->stream>>>(J);
       c->launches++;
     }
     const int64_t units = J.nunits + (n - J.npipe);
-    k_gapdp_strips<<<(int)std::min<int64_t>(c->strip_grid, (units + kStWarps - 1) / kStWarps), kStWarps * 32, 0,
-                     c->stream>>>(J);
+    const int ctas = (int)std::min<int64_t>(c->strip_grid, (units + kStWarps - 1) / kStWarps);
+    (sparse ? k_gapdp_strips<true> : k_gapdp_strips<false>)<<<ctas, kStWarps * 32, 0, c->stream>>>(J);
     stage_mark(c, "traceback");
     WalkJob K;
     K.sa = in.sa;
@@ -610,11 +623,11 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     K.sb = in.sb;
     K.ob = in.ob;
     K.order = J.order;
-    K.slot_off = J.slot_off;
+    K.slots = J.slots;
     K.todo = d_order + todo_at[wv];
     K.nwork = J.nwork;
     K.nck = nck[wv];
-    K.max_rows = J.max_rows;
+    K.max_rows = max_rows;
     K.ckpt = ckpt;
     K.arena = arena_p;
     K.end_edge = d_edge;
@@ -625,7 +638,8 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
     K.env = in.env;
     K.counter = J.counter + 2;
     const int64_t walkers = std::max<int64_t>(K.nck, (n - K.nck + kWalkWarps - 1) / kWalkWarps);
-    k_strip_walk<<<(int)std::min<int64_t>(c->walk_grid, walkers), kWalkWarps * 32, kWalkSmem, c->stream>>>(K);
+    const int walk_ctas = (int)std::min<int64_t>(c->walk_grid, walkers);
+    (sparse ? k_strip_walk<true> : k_strip_walk<false>)<<<walk_ctas, kWalkWarps * 32, kWalkSmem, c->stream>>>(K);
     c->launches += 2;
     if (int e = rec.check(cudaGetLastError(), "kernel launch")) return e;
   }

@@ -46,7 +46,8 @@
 //
 // What a strip leaves for the traceback (per problem slot, StripShape):
 //   rows    the bottom row of every strip but the last, (V, next D~) per column;
-//   states  checkpointed problems: every kStBlock steps, all lanes' state;
+//   states  checkpointed problems: every kStBlock steps (or a multiple), all
+//           lanes' state;
 //   bits    direct problems: the traceback nibbles of every step.
 // Nibbles belong to the cell that the move arrives at: bits 0-1 where V comes
 // from (3 = M, 0 = D, 1 = I, ties in that order), bit 2 set if the next row's
@@ -63,19 +64,31 @@ namespace mvg {
 constexpr int kStWarps = 4;
 constexpr int kStGroup = 1024;             // problems whose strips are claimed level by level
 constexpr unsigned long long kStUnwritten = 0x8080808080808080ull;  // V far below any score
-constexpr int kStBlock = 64;               // steps between stored states
+constexpr int kStBlockBits = 6;
+constexpr int kStBlock = 1 << kStBlockBits;  // steps of a block, and between stored states where there is room
 constexpr int kStDirectCols = 700;         // direct bits up to this LB ...
 constexpr int64_t kStDirectCells = 4 << 20;  // ... and this many cells
 constexpr int kStScaledMax = 400000;       // min(LA, LB) up to which scaled scores fit 32 bits
 constexpr int32_t kOpen2 = 2 * kGap;       // open plus close
 
 // How a problem is run: rows per lane, strips, and what is stored for the
-// traceback.  The bits of a problem of few columns cost less than computing
+// traceback: its bits, or the state every 1 << every steps (a block, or a
+// multiple).  The bits of a problem of few columns cost less than computing
 // most of its blocks again.
 struct StripShape {
-  int LA, LB, R, n, S, nb;
+  int LA, LB, R, n, S, every;
   bool direct;
 };
+
+MVG_HD uint64_t strip_rows_bytes(const StripShape& h) { return ((uint64_t)(h.n - 1) * h.LB * 8 + 255) & ~255ull; }
+// stored states of a strip
+MVG_HD int strip_states(const StripShape& h) { return (h.S - 1) >> h.every; }
+// one state: R (V, next I~) pairs and (V above-left, next D~) per lane
+MVG_HD uint64_t strip_state_bytes(const StripShape& h) { return (uint64_t)(h.R + 1) * 32 * 8; }
+MVG_HD uint64_t strip_slot_bytes(const StripShape& h) {
+  const uint64_t rest = h.direct ? (uint64_t)h.n * h.S * 16 * h.R : (uint64_t)h.n * strip_states(h) * strip_state_bytes(h);
+  return (strip_rows_bytes(h) + rest + 255) & ~255ull;
+}
 
 MVG_HD StripShape strip_shape(int LA, int LB, int max_rows, bool ckpt) {
   StripShape h;
@@ -84,22 +97,54 @@ MVG_HD StripShape strip_shape(int LA, int LB, int max_rows, bool ckpt) {
   h.R = max_rows < 8 || LA <= 128 ? 4 : 8;
   h.n = (LA + 32 * h.R - 1) / (32 * h.R);
   h.S = LB + 31;
-  h.nb = (h.S + kStBlock - 1) / kStBlock;
+  h.every = kStBlockBits;
   const int least = LA < LB ? LA : LB;
   h.direct = least <= kStScaledMax && (!ckpt || (LB <= kStDirectCols && (int64_t)LA * LB <= kStDirectCells));
   return h;
 }
-MVG_HD uint64_t strip_rows_bytes(const StripShape& h) { return ((uint64_t)(h.n - 1) * h.LB * 8 + 255) & ~255ull; }
-// one state: R (V, next I~) pairs and (V above-left, next D~) per lane
-MVG_HD uint64_t strip_state_bytes(const StripShape& h) { return (uint64_t)(h.R + 1) * 32 * 8; }
-MVG_HD uint64_t strip_slot_bytes(const StripShape& h) {
-  const uint64_t rest = h.direct ? (uint64_t)h.n * h.S * 16 * h.R : (uint64_t)h.n * (h.nb - 1) * strip_state_bytes(h);
-  return (strip_rows_bytes(h) + rest + 255) & ~255ull;
+
+// The shape of a problem whose slot would take more than `limit`: checkpointed
+// in the taller strips, with as many states as fit.
+inline StripShape strip_shape_within(StripShape h, uint64_t limit) {
+  if (strip_slot_bytes(h) <= limit) return h;
+  h.direct = false;
+  h.R = h.LA <= 128 ? 4 : 8;
+  h.n = (h.LA + 32 * h.R - 1) / (32 * h.R);
+  while (strip_slot_bytes(h) > limit && strip_states(h) > 0) ++h.every;
+  return h;
+}
+
+// A slot as the kernels get it: its byte offset in the arena (a multiple of
+// 256) with the shape below it.
+inline uint64_t strip_slot(uint64_t offset, const StripShape& h) {
+  return offset | (uint64_t)(h.every << 2 | (h.R == 8 ? 2 : 0) | (h.direct ? 1 : 0));
+}
+MVG_HD uint64_t strip_slot_offset(uint64_t slot) { return slot & ~255ull; }
+
+// The shape of problem p in slot w.  SPARSE: as the slot has it.  A pass whose
+// slots were not cut to fit a bound takes it from the lengths: with the states'
+// interval and the slot's shape in registers the batch's forward pass took 2%
+// longer.
+template <bool SPARSE, class Job>
+__device__ __forceinline__ StripShape strip_shape_of(const Job& J, uint32_t p, int w) {
+  const int LA = (int)(J.oa[p + 1] - J.oa[p]), LB = (int)(J.ob[p + 1] - J.ob[p]);
+  if (!SPARSE) return strip_shape(LA, LB, J.max_rows, J.ckpt);
+  const uint64_t slot = J.slots[w];
+  StripShape h;
+  h.LA = LA;
+  h.LB = LB;
+  h.R = slot & 2 ? 8 : 4;
+  h.n = (LA + 32 * h.R - 1) / (32 * h.R);
+  h.S = LB + 31;
+  h.every = (int)(slot >> 2 & 63);
+  h.direct = slot & 1;
+  return h;
 }
 
 // The least arena bound at which a problem is taken: its cell states at 16
 // bytes each, every 128 columns and 32 * max_rows rows (or its nibbles), as
-// the entry point has always had it.  A slot above the bound oversteps it.
+// the entry point has always had it.  The rows alone, which a slot cannot do
+// without, are half of that at most.
 MVG_HD uint64_t strip_least_bytes(const StripShape& h, int max_rows, bool ckpt) {
   const uint64_t n = ((uint64_t)h.LA + 32 * max_rows - 1) / (32 * max_rows), LB = h.LB;
   return ckpt ? ((n - 1) * LB + n * ((LB + 127) / 128 - 1) * 32 * max_rows) * 16 : n * (LB + 31) * 16 * max_rows;
@@ -111,7 +156,7 @@ struct StripJob {
   const uint8_t* sb;
   const uint64_t* ob;
   const uint32_t* order;       // slot -> problem: pipelined problems first, each part largest first
-  const uint64_t* slot_off;    // byte offset of each slot in the arena
+  const uint64_t* slots;       // strip_slot
   const uint2* units;          // pipelined strips in claim order: slot, strip
   int nwork, npipe, nunits;
   int max_rows;
@@ -126,11 +171,12 @@ struct StripJob {
 
 // Before a pass: the pipelined slots' rows unwritten.  Slots along grid.x,
 // shares of a slot's rows along grid.y.
+template <bool SPARSE>
 __global__ void k_strip_unwritten(StripJob J) {
   for (int w = blockIdx.x; w < J.npipe; w += gridDim.x) {
     const uint32_t p = J.order[w];
-    const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
-    ulonglong2* rows = reinterpret_cast<ulonglong2*>(J.arena + J.slot_off[w]);
+    const StripShape h = strip_shape_of<SPARSE>(J, p, w);
+    ulonglong2* rows = reinterpret_cast<ulonglong2*>(J.arena + strip_slot_offset(J.slots[w]));
     const int64_t n = (int64_t)(strip_rows_bytes(h) / 16);
     for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.y * blockDim.x)
       rows[i] = make_ulonglong2(kStUnwritten, kStUnwritten);
@@ -338,8 +384,9 @@ __device__ bool strip_run(const StripJob& J, StripSmem& sm, const StripShape& h,
   for (int s0 = 0; s0 < S; s0 += 32) {
     if (!stage(s0 + lane)) return false;
     fetch(s0 + 32 + lane);
-    if (!BITS && s0 > 0 && (s0 & (kStBlock - 1)) == 0) {
-      int2* st = reinterpret_cast<int2*>(rest) + ((int64_t)k * (h.nb - 1) + s0 / kStBlock - 1) * ((R + 1) * 32) + lane;
+    if (!BITS && s0 > 0 && (s0 & ((1 << h.every) - 1)) == 0) {
+      int2* st = reinterpret_cast<int2*>(rest) +
+                 ((int64_t)k * strip_states(h) + (s0 >> h.every) - 1) * ((R + 1) * 32) + lane;
 #pragma unroll
       for (int r = 0; r < R; ++r) st[r * 32] = make_int2(V[r], I[r]);
       st[R * 32] = make_int2(dg, D);
@@ -379,6 +426,7 @@ __device__ bool strip_run(const StripJob& J, StripSmem& sm, const StripShape& h,
 // 5 CTAs of 4 warps per SM and 16 steps unrolled (96 registers): on the
 // 4,000-pair batch 22.7 ms against 23.8 at 4 steps, 24.5 at 7 CTAs and 4 steps
 // (72 registers) and 32.5 at 9 CTAs; 2 or 8 warps per CTA measure the same.
+template <bool SPARSE>
 __global__ void __launch_bounds__(kStWarps * 32, 5) k_gapdp_strips(StripJob J) {
   __shared__ StripSmem smem[kStWarps];
   const int lane = threadIdx.x & 31;
@@ -392,8 +440,8 @@ __global__ void __launch_bounds__(kStWarps * 32, 5) k_gapdp_strips(StripJob J) {
     const int w = (int)unit.x;
     if (w >= J.nwork) break;
     const uint32_t p = J.order[w];
-    const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
-    uint8_t* slot = J.arena + J.slot_off[w];
+    const StripShape h = strip_shape_of<SPARSE>(J, p, w);
+    uint8_t* slot = J.arena + strip_slot_offset(J.slots[w]);
     int k = (int)unit.y;
     const int end = piped ? k + 1 : h.n;
     bool ok = true;
@@ -430,7 +478,7 @@ struct WalkJob {
   const uint8_t* sb;
   const uint64_t* ob;
   const uint32_t* order;
-  const uint64_t* slot_off;
+  const uint64_t* slots;
   const uint32_t* todo;  // slots: the first nck checkpointed, the others direct, each part largest first
   int nwork, nck, max_rows;
   bool ckpt;
@@ -452,8 +500,70 @@ struct WalkSmem {
 };
 constexpr size_t kWalkSmem = sizeof(WalkSmem);
 
-// Steps s0 .. s1 of strip k computed again; step s goes to nib[s & mask].
+// The state of strip k at step s0 from the one at step sa (st; null: the
+// strip's start), left in sm.prof as a stored state: for slots whose states are
+// some blocks apart.  Not inlined, and without the caller's structures: this is
+// the exception, walk_block's registers are the rule's.
 template <int R>
+__device__ __noinline__ void walk_to(StripSmem& sm, const uint8_t* A, int LA, const uint8_t* B, int LB,
+                                     const int2* row_in, const int2* st, int k, int sa, int s0) {
+  const int lane = threadIdx.x & 31;
+  int32_t V[R], I[R], dg = k == 0 && lane == 0 && LA > 1 ? kGap : kOpen2, D = 0, e[3];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int2 v = st ? st[r * 32] : make_int2(kOpen2, kNeg);
+    V[r] = v.x;
+    I[r] = v.y;
+  }
+  if (st) {
+    dg = st[R * 32].x;
+    D = st[R * 32].y;
+  }
+  __syncwarp();
+  strip_profile<R, false>(sm, A, k * 32 * R, LA);
+  const int x0 = sa - 1 - lane;
+  uint32_t sel = x0 >= 0 && x0 < LB ? (B[x0] & 3u) * 512u : 0u;
+  for (int c = sa; c < s0; c += 32) {
+    const int xc = c + lane;
+    int4 in = make_int4(kOpen2, kNeg, 0, 0);
+    if (xc < LB) {
+      if (k > 0) {
+        const int2 above = row_in[xc];
+        in.x = above.x;
+        in.y = above.y;
+      }
+      in.z = (int)((B[xc] & 3u) * 512u);
+    }
+    __syncwarp();
+    sm.ring[xc & 31] = in;
+    __syncwarp();
+#pragma unroll 1
+    for (int q = 0; q < 32; ++q) {
+      int32_t uV = __shfl_up_sync(0xffffffffu, V[R - 1], 1);
+      int32_t uD = __shfl_up_sync(0xffffffffu, D, 1);
+      sel = __shfl_up_sync(0xffffffffu, sel, 1);
+      strip_input(sm, c + q, lane, uV, uD, sel);
+      const int x = c + q - lane;
+      if (x >= 0 && x < LB) {
+        int32_t sc[R];
+        strip_scores<R>(sm, sel, sc);
+        uint32_t nib = 0;
+        D = uD;
+        strip_column<R, false, false>(V, I, sc, dg, D, nib, -1, e);
+        dg = uV;
+      }
+    }
+  }
+  __syncwarp();
+  int2* to = reinterpret_cast<int2*>(sm.prof) + lane;
+  static_assert((R + 1) * 32 * 8 <= sizeof(sm.prof), "a state fits the profile");
+#pragma unroll
+  for (int r = 0; r < R; ++r) to[r * 32] = make_int2(V[r], I[r]);
+  to[R * 32] = make_int2(dg, D);
+}
+
+// Steps s0 .. s1 of strip k computed again; step s goes to nib[s & mask].
+template <int R, bool SPARSE>
 __device__ void walk_block(const WalkJob& J, StripSmem& sm, void* nibs, int mask, const StripShape& h,
                            const uint8_t* slot, uint32_t p, int k, int s0, int s1) {
   const int lane = threadIdx.x & 31;
@@ -470,8 +580,13 @@ __device__ void walk_block(const WalkJob& J, StripSmem& sm, void* nibs, int mask
     dg = k == 0 && lane == 0 && h.LA > 1 ? kGap : kOpen2;
     D = 0;
   } else {
+    const int sa = SPARSE ? s0 & ~((1 << h.every) - 1) : s0;
     const int2* st = reinterpret_cast<const int2*>(slot + strip_rows_bytes(h)) +
-                     ((int64_t)k * (h.nb - 1) + s0 / kStBlock - 1) * ((R + 1) * 32) + lane;
+                     ((int64_t)k * strip_states(h) + (sa >> h.every) - 1) * ((R + 1) * 32) + lane;
+    if (SPARSE && sa != s0) {
+      walk_to<R>(sm, J.sa + J.oa[p], h.LA, B, LB, row_in, sa > 0 ? st : nullptr, k, sa, s0);
+      st = reinterpret_cast<const int2*>(sm.prof) + lane;
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int2 v = st[r * 32];
@@ -538,7 +653,7 @@ __device__ void walk_block(const WalkJob& J, StripSmem& sm, void* nibs, int mask
 
 // The walk.  COOP: the CTA's first warp walks while the others wait in
 // walk_help for the steps it wants.  Returns the path's length, 0 on failure.
-template <int R, bool COOP>
+template <int R, bool SPARSE, bool COOP>
 __device__ int64_t walk_path(const WalkJob& J, WalkSmem& sm, const StripShape& h, const uint8_t* slot, uint32_t p) {
   constexpr int SR = 32 * R;
   constexpr int kMask = COOP ? kWalkWarps * kStBlock - 1 : kStBlock - 1;
@@ -626,7 +741,7 @@ __device__ int64_t walk_path(const WalkJob& J, WalkSmem& sm, const StripShape& h
           sm.want_n = nblk;
         }
         __syncthreads();
-        walk_block<R>(J, sm.strip[0], sm.nib, kMask, h, slot, p, k, s0, s1);
+        walk_block<R, SPARSE>(J, sm.strip[0], sm.nib, kMask, h, slot, p, k, s0, s1);
         __syncthreads();
         s0 -= (nblk - 1) * kStBlock;
       } else {
@@ -660,7 +775,7 @@ __device__ int64_t walk_path(const WalkJob& J, WalkSmem& sm, const StripShape& h
 }
 
 // The CTA's other warps: warp w computes the block w before the walk's.
-template <int R>
+template <int R, bool SPARSE>
 __device__ void walk_help(const WalkJob& J, WalkSmem& sm, const StripShape& h, const uint8_t* slot, uint32_t p) {
   const int w = threadIdx.x >> 5;
   for (;;) {
@@ -668,7 +783,7 @@ __device__ void walk_help(const WalkJob& J, WalkSmem& sm, const StripShape& h, c
     const int k = sm.want_k, s0 = (sm.want_s & ~(kStBlock - 1)) - w * kStBlock;
     if (k < 0) return;
     if (w < sm.want_n)
-      walk_block<R>(J, sm.strip[w], sm.nib, kWalkWarps * kStBlock - 1, h, slot, p, k, s0, s0 + kStBlock - 1);
+      walk_block<R, SPARSE>(J, sm.strip[w], sm.nib, kWalkWarps * kStBlock - 1, h, slot, p, k, s0, s0 + kStBlock - 1);
     __syncthreads();
   }
 }
@@ -691,6 +806,7 @@ __device__ void walk_compact(char* path, int64_t limit, int64_t n, int t, int nt
   }
 }
 
+template <bool SPARSE>
 __global__ void __launch_bounds__(kWalkWarps * 32) k_strip_walk(WalkJob J) {
   extern __shared__ __align__(16) uint8_t walk_smem[];
   WalkSmem& sm = *reinterpret_cast<WalkSmem*>(walk_smem);
@@ -703,19 +819,20 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_strip_walk(WalkJob J) {
     if (sm.claim >= J.nck) break;
     const int w = (int)J.todo[sm.claim];
     const uint32_t p = J.order[w];
-    const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
-    const uint8_t* slot = J.arena + J.slot_off[w];
+    const StripShape h = strip_shape_of<SPARSE>(J, p, w);
+    const uint8_t* slot = J.arena + strip_slot_offset(J.slots[w]);
     if (wib == 0) {
-      const int64_t n = h.R == 8 ? walk_path<8, true>(J, sm, h, slot, p) : walk_path<4, true>(J, sm, h, slot, p);
+      const int64_t n =
+          h.R == 8 ? walk_path<8, SPARSE, true>(J, sm, h, slot, p) : walk_path<4, SPARSE, true>(J, sm, h, slot, p);
       if (lane == 0) {
         sm.want_k = -1;
         sm.path_n = n;
       }
       __syncthreads();
     } else if (h.R == 8) {
-      walk_help<8>(J, sm, h, slot, p);
+      walk_help<8, SPARSE>(J, sm, h, slot, p);
     } else {
-      walk_help<4>(J, sm, h, slot, p);
+      walk_help<4, SPARSE>(J, sm, h, slot, p);
     }
     walk_compact(J.paths + J.path_off[p], (int64_t)h.LA + h.LB, sm.path_n, (int)threadIdx.x, kWalkWarps * 32,
                  [] { __syncthreads(); });
@@ -727,9 +844,10 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_strip_walk(WalkJob J) {
     if (q >= J.nwork) break;
     const int w = (int)J.todo[q];
     const uint32_t p = J.order[w];
-    const StripShape h = strip_shape((int)(J.oa[p + 1] - J.oa[p]), (int)(J.ob[p + 1] - J.ob[p]), J.max_rows, J.ckpt);
-    const uint8_t* slot = J.arena + J.slot_off[w];
-    const int64_t n = h.R == 8 ? walk_path<8, false>(J, sm, h, slot, p) : walk_path<4, false>(J, sm, h, slot, p);
+    const StripShape h = strip_shape_of<SPARSE>(J, p, w);
+    const uint8_t* slot = J.arena + strip_slot_offset(J.slots[w]);
+    const int64_t n =
+        h.R == 8 ? walk_path<8, SPARSE, false>(J, sm, h, slot, p) : walk_path<4, SPARSE, false>(J, sm, h, slot, p);
     __syncwarp();
     walk_compact(J.paths + J.path_off[p], (int64_t)h.LA + h.LB, n, lane, 32, [] { __syncwarp(); });
   }

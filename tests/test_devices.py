@@ -1,5 +1,6 @@
-"""Handles on several devices of one process: every kernel is launched with
-the shared memory it was allowed on its own device (no GPU: fake_device)."""
+"""What the host side asks of the devices (no GPU: fake_device): on several
+devices of one process every kernel is launched with the shared memory it was
+allowed on its own; the traceback arena stays within its bound."""
 import ctypes
 
 import numpy as np
@@ -56,3 +57,43 @@ def test_second_device(lib, call, arg):
         assert call(lib, h, arg) == 0, lib.mvg_last_error()
         assert lib.fake_refused() == 0
         lib.mvg_destroy(h)
+
+
+def _least(la, lb, checkpoints=True):
+    """The least arena bound at which the gap DP takes a problem."""
+    strips = -(-la // 256)
+    if not checkpoints:
+        return strips * (lb + 31) * 128
+    return ((strips - 1) * lb + strips * (-(-lb // 128) - 1) * 256) * 16
+
+
+# Slots that the shape chosen for speed would make larger than the bound:
+# stored bits, half-height strips, one strip of many states, many strips of few
+# columns, bits by request.
+@pytest.mark.parametrize("la,lb,checkpoints", [(5900, 700, True), (5000, 1500, True), (200, 40000, True),
+                                               (200000, 120, True), (5900, 690, False)])
+def test_arena_bound(lib, la, lb, checkpoints):
+    h = ctypes.c_void_p()
+    assert lib.mvg_create(ctypes.byref(h), 0) == 0
+    least = _least(la, lb, checkpoints)
+    bound = max(least // 256 * 256 + 256, 1 << 20)
+    lib.mvg_set_dp_checkpoint(h, int(checkpoints))
+    a, b = np.zeros(la, np.uint8), np.zeros(lb, np.uint8)
+    oa, ob, po = (np.array([0, n], np.uint64) for n in (la, lb, la + lb))
+    score, path, plen = np.zeros(1, np.int32), np.zeros(la + lb, np.uint8), np.zeros(1, np.int64)
+
+    def call():
+        return lib.mvg_gapdp_batch(h, _p(a), _p(oa), _p(b), _p(ob), i64(1), _p(score), _p(path), _p(po), _p(plen))
+
+    for by_free_memory in (False, True):  # the bound asked for, then 60% of free memory
+        assert lib.mvg_set_tb_arena(h, u64(2**64 - 1 if by_free_memory else bound)) == 0
+        lib.fake_reset(int(bound / 0.6) + 2 if by_free_memory else 1 << 40)
+        assert call() == 0, lib.mvg_last_error()
+        assert lib.fake_largest() <= bound + bound // 8 + 512  # a buffer is made an eighth larger than asked for
+        lib.mvg_destroy(h)
+        assert lib.mvg_create(ctypes.byref(h), 0) == 0
+        lib.mvg_set_dp_checkpoint(h, int(checkpoints))
+    lib.fake_reset(1 << 40)
+    if lib.mvg_set_tb_arena(h, u64(least - 1)) == 0:
+        assert call() == 5  # MVG_ERR_CAPACITY
+    lib.mvg_destroy(h)
