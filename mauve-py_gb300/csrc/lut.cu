@@ -45,6 +45,12 @@ constexpr int kTile = 4096;  // columns, or LUT entries, per tile
 constexpr int kLutThreads = 256;
 constexpr int kGroups = kTile / 16;  // a thread's 16 consecutive columns
 
+// Whether the error word is set, the same for all of the CTA's threads: CTAs of
+// the same launch may set it at any time.
+__device__ __forceinline__ bool cta_failed(const uint32_t* err) {
+  return __syncthreads_or(err && threadIdx.x == 0 && *(const volatile uint32_t*)err);
+}
+
 // ------------------------------------------------------------ construction
 
 // Sixteen characters from p, `have` of them readable (0 for the rest).
@@ -169,7 +175,7 @@ __global__ void __launch_bounds__(kLutThreads) k_lut_walk(const uint8_t* __restr
                                                           const int64_t* __restrict__ r_start, int64_t n,
                                                           unsigned long long* __restrict__ keys, uint32_t* err) {
   __shared__ uint32_t s_ex[kGroups], s_bases[kGroups], s_same[kGroups];
-  if (*(volatile uint32_t*)err) return;  // offsets that decrease
+  if (cta_failed(err)) return;  // offsets that decrease
   const uint64_t first = col_off[0], t0 = first + (uint64_t)blockIdx.x * kTile;
   const uint64_t end = col_off[nblocks], t1 = t0 + kTile < end ? t0 + kTile : end;
   const Group x = load_group(g, r, t0 + threadIdx.x * 16, t1);
@@ -316,7 +322,7 @@ __device__ __forceinline__ uint32_t tile_starts(const int32_t (&lo)[kTile / 256]
 __global__ void __launch_bounds__(256) k_fill_count(int32_t* lut, int64_t n, int mode, const ZeroFix z,
                                                     uint32_t* __restrict__ tile, uint32_t* err) {
   __shared__ uint32_t s_at[kTile / 32];
-  if (err && *(volatile uint32_t*)err) return;
+  if (cta_failed(err)) return;
   if (z.on && blockIdx.x == 0) {
     fix_zero(lut, n, z, err);
     __syncthreads();
