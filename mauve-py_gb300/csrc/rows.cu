@@ -15,11 +15,11 @@ namespace mvg {
 
 // Edges [t0, t1) of one path on one warp, whose first takes character i of A
 // and j of B; both move on.  Returns whether an edge was none, or past a
-// sequence's end.
+// sequence's end.  kSteps: steps of 32 edges whose loads are in flight.
+template <int kSteps>
 __device__ __forceinline__ bool rows_of(const uint8_t* __restrict__ A, int64_t la, const uint8_t* __restrict__ B,
                                         int64_t lb, const char* __restrict__ P, int64_t t0, int64_t t1,
                                         uint8_t* __restrict__ RA, uint8_t* __restrict__ RB, int64_t& i, int64_t& j) {
-  constexpr int kSteps = 4;  // loads in flight
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   bool bad = false;
@@ -94,7 +94,14 @@ __global__ void __launch_bounds__(WARPS == 1 ? 256 : 1024)
         j += s_b[w];
       }
     }
-    bool bad = rows_of(A, la, B, lb, P, t0, t1, rows_a + path_off[p], rows_b + path_off[p], i, j);
+    bool bad = false;
+    if (WARPS == 1) {  // a rest of up to 32 edges, or a short path, in one step (100,000 of 30: 44 and 37 us)
+      const int64_t rest = n > 32 ? min(n, (n + 95) / 128 * 128) : 0;
+      bad = rows_of<4>(A, la, B, lb, P, 0, rest, rows_a + path_off[p], rows_b + path_off[p], i, j);
+      bad |= rows_of<1>(A, la, B, lb, P, rest, n, rows_a + path_off[p], rows_b + path_off[p], i, j);
+    } else {
+      bad = rows_of<4>(A, la, B, lb, P, t0, t1, rows_a + path_off[p], rows_b + path_off[p], i, j);
+    }
     if (wid % WARPS == WARPS - 1) bad |= i != la || j != lb;  // the path must consume both sequences
     if (__any_sync(0xffffffffu, bad) && lane == 0) set_error(err, kDevRange);
   }
