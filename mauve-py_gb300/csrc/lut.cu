@@ -346,13 +346,13 @@ __global__ void __launch_bounds__(256) k_fill_count(int32_t* lut, int64_t n, int
 // reach = u, or g when there is none.  The tile is in shared memory, its gap
 // starts are listed there, and a thread per gap start tries the next eight
 // entries (a substitution's partner is the next one); what is left the warp
-// searches together, 32 entries per step.  (From global memory, a thread per
+// searches together.  (From global memory, a thread per
 // entry: 36 us for 4.6 million entries that are not in L2; this takes 16.)
 __global__ void __launch_bounds__(256) k_fill_search(const int32_t* __restrict__ lut, int64_t n, int width, int mode,
                                                      const uint32_t* __restrict__ tile, int32_t* __restrict__ cand,
                                                      int32_t* __restrict__ reach, int32_t* __restrict__ lval,
                                                      const uint32_t* err) {
-  constexpr int kProbe = 8;
+  constexpr int kProbe = 8, kAhead = 8;
   __shared__ uint32_t s_at[kTile / 32];
   __shared__ int32_t s_lut[kTile + 1 + kProbe];  // entries t0 - 1 ..
   __shared__ uint16_t s_start[kTile];
@@ -409,15 +409,24 @@ __global__ void __launch_bounds__(256) k_fill_search(const int32_t* __restrict__
       const int64_t g0 = t0 + __shfl_sync(0xffffffffu, q, src), l0 = g0 - 1;
       const int64_t end = g0 + width < n - 1 ? g0 + width : n - 1;
       const int32_t L0 = __shfl_sync(0xffffffffu, L, src);
-      for (int64_t base = g0 + 1 + kProbe; base <= end; base += 32) {
-        const int64_t up = base + lane;
-        const unsigned hit = __ballot_sync(
-            0xffffffffu, up <= end && (int32_t)((uint32_t)lut[up] - (uint32_t)L0) == (int32_t)(up - l0));
-        if (hit) {
-          if (lane == 0) reach[first + k0 + src] = (int32_t)(base + __ffs(hit) - 1);
-          break;
-        }
+      // 32 entries, then 256 at a time
+      auto partner = [&](int64_t up) {
+        return up <= end && (int32_t)((uint32_t)lut[up] - (uint32_t)L0) == (int32_t)(up - l0);
+      };
+      int64_t base = g0 + 1 + kProbe;
+      unsigned hit = __ballot_sync(0xffffffffu, partner(base + lane));
+      for (base += 32; !hit && base <= end;) {
+        bool is[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) is[k] = partner(base + 32 * k + lane);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+          if (!hit) {
+            hit = __ballot_sync(0xffffffffu, is[k]);
+            base += 32;
+          }
       }
+      if (hit && lane == 0) reach[first + k0 + src] = (int32_t)(base - 32 + __ffs(hit) - 1);
     }
   }
 }
