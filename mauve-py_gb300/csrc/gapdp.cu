@@ -668,13 +668,25 @@ static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_
   // stay on one warp unless their strips are at least 4 strip heights wide
   // (bands of 1,100 columns on 5,000 rows, which no ring height takes: at 8
   // they were one warp's chain of 28,000 steps, 6.6 ms; at 4, 2.9 ms).
+  // Where the problems alone fill two thirds of the warps, one warp each costs
+  // less up to 8 strip heights (1,400 columns on 5,000 rows: 500 bands 21.3 ms
+  // with a warp and 8.5 with a CTA each, 2,000 bands 23.2 and 26.4).
+  int dev_sms = 0;
+  MVG_CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
+  void (*kern)(DpJob) = rows == 8 ? k_gapdp_t<8> : rows == 4 ? k_gapdp_t<4> : rows == 2 ? k_gapdp_t<2> : k_gapdp_t<1>;
+  int bps = 0;
+  MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kDpThreads, 0));
+  if (bps < 1) bps = 1;
+  const int grid = dev_sms * bps;
+  const int64_t nwarps = (int64_t)grid * (kDpThreads / 32);
+  const uint64_t wide = 3 * nwork >= 2 * nwarps ? 8 : 4;
   std::vector<char> is_big(nwork);
   for (int64_t w = 0; w < nwork; ++w) {
     const uint32_t p = ids[w];
     const Band b = make_band((int)la[p], (int)lb[p], h_delta[p], h_half[p], 32 * rows);
     cells[w] = band_cells(b);
     bytes[w] = (band_tb_words(b, rows) * 4 + 255) & ~255ull;
-    is_big[w] = b.nstrips >= kCoopMinStrips && cells[w] >= (uint64_t)la[p] * 4 * 32 * rows;
+    is_big[w] = b.nstrips >= kCoopMinStrips && cells[w] >= (uint64_t)la[p] * wide * 32 * rows;
     maxlb = std::max(maxlb, lb[p]);
     total += bytes[w];
     most = std::max(most, bytes[w]);
@@ -690,14 +702,6 @@ static int run_band_strips(Ctx* c, const DpInputs& in, const std::vector<uint32_
   for (int64_t q = 0; q < nwork; ++q) order[q] = ids[W.item[q]];
 
   sub.reset(new HostSpan(c, "dp_copy"));
-  int dev_sms = 0;
-  MVG_CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
-  void (*kern)(DpJob) = rows == 8 ? k_gapdp_t<8> : rows == 4 ? k_gapdp_t<4> : rows == 2 ? k_gapdp_t<2> : k_gapdp_t<1>;
-  int bps = 0;
-  MVG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kDpThreads, 0));
-  if (bps < 1) bps = 1;
-  const int grid = dev_sms * bps;
-  const int64_t nwarps = (int64_t)grid * (kDpThreads / 32);
   Workspace& ws = c->ws;
   const int64_t rb_stride = maxlb + 2;
   const DpSlots& sl = kDpSlotsBand;
