@@ -229,11 +229,18 @@ extern "C" int mvg_xmfa_write_dev(mvg_handle h, const char* file_a, const char* 
   // a short text 3 to 7 us (80,227 bases in 7 blocks: the call 58 and 62 us,
   // 20,000 in 200: 101 and 108), a long one gains (300,000 in 50: 78 and 76,
   // 4.6 million in 64: 142 and 138)
-  constexpr uint64_t kShortText = 400000;
+  // Its grid is the widest piece by all pieces, so not for a wide block among
+  // many small ones (100,000 bases and 500 of one: 245,000 CTAs, the call 304
+  // and 182 us; 5,000 and 1,000 of one: 25,000, 313 and 307; 3,000 blocks of
+  // 10: 15,000, 802 and 801).
+  constexpr uint64_t kShortText = 400000, kShortCtas = 16384;
+  dim3 grid(1, (unsigned)std::min<int64_t>(np, 65535));
   if (total <= kShortText) {
-    uint64_t widest = 0;  // output bytes of the largest piece
+    uint64_t widest = 1;  // output bytes of the largest piece
     for (const XmfaPiece& pc : pieces) widest = std::max(widest, pc.row < 0 ? pc.len : pc.len + (pc.len + 79) / 80);
-    const dim3 grid((unsigned)std::max<uint64_t>((widest + 1023) / 1024, 1), (unsigned)std::min<int64_t>(np, 65535));
+    grid.x = (unsigned)((widest + 1023) / 1024);
+  }
+  if (total <= kShortText && (uint64_t)grid.x * grid.y <= kShortCtas) {
     k_xmfa_bytes<<<grid, 256, 0, c->stream>>>(d_pieces, np, d_blob, d_rows_a, d_rows_b, d_out);
   } else {
     k_xmfa_assemble<<<(unsigned)((total + 4095) / 4096), 256, 0, c->stream>>>(d_pieces, np, d_blob, d_rows_a, d_rows_b,
