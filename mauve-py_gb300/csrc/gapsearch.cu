@@ -664,7 +664,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
     P.out = (int32_t*)ws.get(c, kGsSlot + 5, rows * 12 + 16);
     return P.out ? 0 : report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   };
-  if ((rc = match_components(c, P, tab, (int64_t)ch.slots[0], 16 + gbits, room_for, &r))) return rc;
+  if ((rc = match_components(c, P, tab, &b, (int64_t)ch.slots[0], 16 + gbits, room_for, &r))) return rc;
   if (r.rows == 0) return 0;
   stage_mark(c, "gs_filter");
   // per gap: first match, rows kept, left to the host, first output row; their sum (k_gs_filter's todo)

@@ -50,8 +50,9 @@ int pairwise_matches_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t*
   if (!tab) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   MVG_CUDA_TRY(cudaMemsetAsync(tab, 0xff, na * 4, c->stream));
   stage_mark(c, "sml_sort");
+  PairBucketBufs join;
   if (bucketed) {
-    if ((rc = pair_buckets(c, ga, ca, gb, cb, s, tab))) return rc;
+    if ((rc = pair_buckets(c, ga, ca, gb, cb, s, tab, &join))) return rc;
   } else {
     SmlKeys sk;
     if ((rc = pair_sort(c, ga, ca, gb, cb, s, &sk))) return rc;
@@ -72,7 +73,7 @@ int pairwise_matches_dev(Ctx* c, const uint8_t* d_a, uint64_t na, const uint8_t*
   prob.out = d_out;
   prob.cap = cap;
   ComponentResult r;
-  if ((rc = match_components(c, prob, tab, (int64_t)na, 16, [](uint64_t) { return 0; }, &r))) return rc;
+  if ((rc = match_components(c, prob, tab, bucketed ? &join : nullptr, (int64_t)na, 16, [](uint64_t) { return 0; }, &r))) return rc;
   stage_end(c);
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
   c->stats.pairs = r.pairs;

@@ -120,7 +120,8 @@ __global__ void k_tab_runs(const K* __restrict__ keys, const uint32_t* __restric
 
 // Segment heads (no pair of the diagonal in the L positions before) and
 // tails as bit masks over A's positions; per tile their counts (heads of all
-// tiles, then tails), and the number of pairs.  Most pairs have their
+// tiles, then tails), and the number of pairs; what the join left (left) beside
+// them.  Most pairs have their
 // diagonal's neighbour right beside them; the others' searches go through a
 // list, so that a warp's lanes all have one to do.  (Searched where they lie,
 // one lane in a warp kept it for L steps: bits, counts and lists of the ends of
@@ -129,7 +130,8 @@ template <class P>
 __global__ void __launch_bounds__(256) k_seg_bits(P prob, const uint32_t* __restrict__ tab, int64_t n,
                                                   uint32_t* __restrict__ headw, uint32_t* __restrict__ tailw,
                                                   uint32_t* __restrict__ tcount, int64_t ntiles,
-                                                  uint32_t* __restrict__ npairs) {
+                                                  uint32_t* __restrict__ npairs, const uint32_t* __restrict__ left,
+                                                  uint32_t* __restrict__ left_out) {
   __shared__ uint32_t s[kSegTile + 64];
   __shared__ uint16_t list[2 * kSegTile];  // entries of s to search from, 2 i + 1 for a tail
   __shared__ uint32_t bits[2][kSegTile / 32];
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(256) k_seg_bits(P prob, const uint32_t* __rest
     tcount[blockIdx.x] = sum[0];
     tcount[ntiles + blockIdx.x] = sum[1];
     if (sum[2]) atomicAdd(npairs, sum[2]);
+    if (left && blockIdx.x == 0) *left_out = *left;
   }
 }
 
@@ -767,27 +770,39 @@ int flagged_components(Ctx* c, P& prob, const uint32_t* tab, const uint32_t* fla
 
 // The match list of the pairs in tab (n A positions): rows through prob.row,
 // in order of buckets and of the entries in them.  key_bits: width of
-// prob.key; room_for(rows) is called before rows are written.  Waits for the
-// stream twice (three times more with flagged buckets); the rows' kernel may
-// still be running on return.
+// prob.key; room_for(rows) is called before rows are written.  join: the join
+// that made the table, whose buckets of repeated mers may be to do (or null).
+// Waits for the stream twice (once more for such buckets, three times more with
+// flagged ones); the rows' kernel may still be running on return.
 template <class P, class F>
-int match_components(Ctx* c, P& prob, const uint32_t* tab, int64_t n, int key_bits, F room_for, ComponentResult* out) {
+int match_components(Ctx* c, P& prob, uint32_t* tab, const PairBucketBufs* join, int64_t n, int key_bits, F room_for,
+                     ComponentResult* out) {
   Workspace& ws = c->ws;
   const int64_t ntiles = div_up(n, kSegTile);
   uint32_t* masks = (uint32_t*)ws.get(c, 39, (size_t)ntiles * (kSegTile / 32) * 2 * 4);
   // head and tail counts per tile, their offsets, scan scratch
   uint32_t* tcount = (uint32_t*)ws.get(c, 44, ((size_t)ntiles * 4 + scan_scratch_words(2 * ntiles) + 16) * 4);
-  uint32_t* scal = (uint32_t*)ws.get(c, 34, 64);  // segment ends, pairs, components, flagged buckets
+  uint32_t* scal = (uint32_t*)ws.get(c, 34, 64);  // segment ends, pairs, what the join left; components, flagged buckets
   if (!masks || !tcount || !scal) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   uint32_t *headw = masks, *tailw = masks + ntiles * (kSegTile / 32);
   uint32_t *toff = tcount + 2 * ntiles, *tscr = toff + 2 * ntiles;
-  MVG_CUDA_TRY(cudaMemsetAsync(scal, 0, 64, c->stream));
-  stage_mark(c, "segments");
-  k_seg_bits<<<(unsigned)ntiles, 256, 0, c->stream>>>(prob, tab, n, headw, tailw, tcount, ntiles, scal + 1);
-  c->launches++;
-  scan_counts(tcount, 2 * ntiles, toff, tscr, scal, c->stream, &c->launches);
-  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal, 8, cudaMemcpyDeviceToHost, c->stream));
-  if (int rc = check_device_error(c)) return rc;
+  const uint32_t* left = join ? join->pieces.count : nullptr;
+  for (;;) {
+    MVG_CUDA_TRY(cudaMemsetAsync(scal, 0, 64, c->stream));
+    stage_mark(c, "segments");
+    k_seg_bits<<<(unsigned)ntiles, 256, 0, c->stream>>>(prob, tab, n, headw, tailw, tcount, ntiles, scal + 1, left,
+                                                        scal + 2);
+    c->launches++;
+    scan_counts(tcount, 2 * ntiles, toff, tscr, scal, c->stream, &c->launches);
+    MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal, 12, cudaMemcpyDeviceToHost, c->stream));
+    if (int rc = check_device_error(c)) return rc;
+    if (((const uint32_t*)c->h_scalars)[2] == 0) break;
+    // few inputs have any: asked for here, where the host waits anyway (a
+    // launch that looks for them took 8 of 231 us of a 1 Mbp pair)
+    left = nullptr;
+    stage_mark(c, "repeats");
+    pair_bucket_repeats(c, *join, tab);
+  }
   const int64_t ends = ((const uint32_t*)c->h_scalars)[0], nseg = ends / 2;
   out->pairs = ((const uint32_t*)c->h_scalars)[1];
   if (out->pairs == 0) return 0;
@@ -833,12 +848,12 @@ int match_components(Ctx* c, P& prob, const uint32_t* tab, int64_t n, int key_bi
   stage_mark(c, "components");
   MVG_CUDA_TRY(cudaMemsetAsync(bflag, 0, (size_t)nseg * 4, c->stream));
   k_comp_count<<<(unsigned)ctiles, 256, 0, c->stream>>>(joined, nseg, ccount);
-  scan_counts(ccount, ctiles, coff, cscr, scal + 2, c->stream, &c->launches);
+  scan_counts(ccount, ctiles, coff, cscr, scal + 3, c->stream, &c->launches);
   k_comp_emit<<<(unsigned)ctiles, 256, 0, c->stream>>>(tab, key, head, last, moved, joined, nseg, coff, C);
-  k_comp_out<<<grid_for(nseg, 256), 256, 0, c->stream>>>(prob, C, scal + 2, bflag, flagged, scal + 3);
+  k_comp_out<<<grid_for(nseg, 256), 256, 0, c->stream>>>(prob, C, scal + 3, bflag, flagged, scal + 4);
   c->launches += 6;
   stage_mark(c, "flagged");
-  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal + 2, 8, cudaMemcpyDeviceToHost, c->stream));
+  MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal + 3, 8, cudaMemcpyDeviceToHost, c->stream));
   if (int rc = check_device_error(c)) return rc;
   out->ncomp = ((const uint32_t*)c->h_scalars)[0];
   out->rows = out->ncomp;

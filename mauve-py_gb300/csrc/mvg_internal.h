@@ -153,6 +153,13 @@ constexpr uint64_t kPairBucketMaxKeys = 1ull << 25;
 constexpr int kPairRestBits = 30;                      // mer bits below the bucket's
 constexpr int kPairMaxBits = 14 + kPairRestBits;       // with 2^14 buckets
 constexpr int kOneCta = 120 * 1024;  // dynamic shared memory of the join's scatter: one CTA per SM
+// Pieces of large buckets: (bucket, number, the bucket's first, their number),
+// and at a bucket's first what its pieces left and how many are done.
+struct PairPieces {
+  uint4* piece;
+  uint2* left;
+  uint32_t* count;
+};
 struct PairBucketGeom {
   int bbits, nbuckets, npass, dbits, lbits;
   int64_t tile, ntiles, nchunks;
@@ -163,12 +170,16 @@ struct PairBucketBufs {
   PairBucketGeom g;
   uint2 *alt, *buf;
   uint32_t *counts, *offs, *csum, *bstart, *bsize;
+  PairPieces pieces;
 };
 int pair_bucket_bufs(Ctx* c, uint64_t n, int bits, PairBucketBufs* b);
 void pair_bucket_offsets(Ctx* c, const PairBucketBufs& b);
+// The join leaves buckets of repeated mers (*b.pieces.count of them, on the
+// device) to pair_bucket_repeats, which adds their pairs to the table.
 void pair_bucket_join(Ctx* c, const PairBucketBufs& b, uint32_t* tab);
+void pair_bucket_repeats(Ctx* c, const PairBucketBufs& b, uint32_t* tab);
 int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
-                 uint32_t* tab);
+                 uint32_t* tab, PairBucketBufs* b);
 // Exclusive scan of n <= 16384 counts in one launch; *total gets the sum.
 void pair_scan_small(const uint32_t* in, int n, uint32_t* out, uint32_t* total, cudaStream_t st);
 int pair_sort(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,

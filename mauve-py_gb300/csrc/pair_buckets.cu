@@ -21,10 +21,14 @@
 //                 (shared-memory atomics)
 //   k_pb_local    one block per bucket: grouped by the next 9 bits in shared
 //                 memory, then a thread per key looks for its mer in its
-//                 group; larger buckets are sorted in chunks through global
-//                 memory and their runs taken.  A mer with one position in
-//                 each genome goes to the table: position in B, the strand
-//                 relation in bit 31, at the position in A.
+//                 group.  A mer with one position in each genome goes to the
+//                 table: position in B, the strand relation in bit 31, at the
+//                 position in A.
+//   k_pb_repeats  (where there are any; match_components asks) larger buckets,
+//                 which repeated mers (runs of N, tandem repeats) make, by way of a hash table of their mers; those
+//                 above 8,192 keys piece by piece, each piece leaving what may
+//                 be unique.  A bucket of more mers than the table holds is
+//                 sorted in chunks through global memory and its runs taken.
 //
 // With in-bucket keys of 32 bits this takes seeds of weight up to 22 (24 M
 // seeds of weight 17 in 1.06 ms, against 1.38 ms of a 64-bit radix sort
@@ -46,7 +50,10 @@ constexpr int kCap = 3072;      // bucket elements sorted in shared memory
 constexpr int kLocItems = kCap / kLocThreads;
 constexpr int kMaxDigit = 64;   // chunked in-bucket passes: digits of at most 6 bits
 constexpr int kGroups = 512;    // groups of a bucket: its top 9 in-bucket bits
-constexpr int kGroupMax = 256;  // larger groups: the bucket is sorted instead
+constexpr int kGroupMax = 256;  // larger groups: the bucket goes through the hash table
+constexpr int kPiece = 8192;    // larger buckets: keys of a piece
+constexpr int kRepeatCtas = 608;
+constexpr int kProbes = 512;    // table entries looked at for a mer before the bucket is sorted instead
 constexpr int kChunkTiles = 32;
 constexpr uint64_t kInL2 = 96ull << 20;  // of 129 MB
 }  // namespace pb
@@ -178,12 +185,14 @@ __global__ void __launch_bounds__(256) k_pb_csum(const uint32_t* __restrict__ co
 
 // One block of 1024 threads, 16 consecutive buckets per thread (nbk <=
 // 16384): every bucket's total over the chunks and its start (exclusive
-// scan over buckets).
+// scan over buckets), and the pieces of the large ones.
 __global__ void __launch_bounds__(1024) k_pb_scan(const uint32_t* __restrict__ csum, int64_t nchunks, int nbk,
-                                                  uint32_t* __restrict__ bstart, uint32_t* __restrict__ bsize) {
+                                                  uint32_t* __restrict__ bstart, uint32_t* __restrict__ bsize,
+                                                  PairPieces P) {
   constexpr int kPer = 16;
-  __shared__ uint32_t wsum[32];
+  __shared__ uint32_t wsum[32], npieces;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid == 0) npieces = 0;
   const int d0 = tid * kPer;
   uint32_t tot[kPer];
 #pragma unroll
@@ -214,7 +223,6 @@ __global__ void __launch_bounds__(1024) k_pb_scan(const uint32_t* __restrict__ c
     wsum[lane] = y - x;
   }
   __syncthreads();
-  if (d0 >= nbk) return;
   uint32_t start = wsum[wid] + inc - mine;
 #pragma unroll
   for (int k = 0; k < kPer; k += 4) {  // 16 bytes at a time: nbk is a multiple of 4, both arrays aligned
@@ -224,6 +232,15 @@ __global__ void __launch_bounds__(1024) k_pb_scan(const uint32_t* __restrict__ c
     *reinterpret_cast<uint4*>(bsize + d0 + k) = make_uint4(tot[k], tot[k + 1], tot[k + 2], tot[k + 3]);
     start = s3 + tot[k + 3];
   }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k)
+    if (d0 + k < nbk && tot[k] > (uint32_t)pb::kPiece) {
+      const uint32_t m = (tot[k] + pb::kPiece - 1) / pb::kPiece, at = atomicAdd(&npieces, m);
+      for (uint32_t q = 0; q < m; ++q) P.piece[at + q] = make_uint4((uint32_t)(d0 + k), q, at, m);
+      P.left[at] = make_uint2(0u, 0u);
+    }
+  __syncthreads();
+  if (tid == 0) *P.count = npieces;
 }
 
 // Block (x, c): chunk c's tiles' first slots per bucket (offs): the
@@ -311,6 +328,126 @@ __global__ void __launch_bounds__(pb::kKeyThreads) k_pb_scatter(const uint32_t* 
                  if (u < count)
                    out[slot[u]] = make_uint2(((uint32_t)m[u] & rest) << 2 | strand[u] << 1 | (in_b ? 1u : 0u), q + u);
              });
+}
+
+// ------------------------------------------- buckets of repeated mers
+
+// A mer of a bucket: x the mer, with its positions in A (0, 1, or 2 for more)
+// in bits 31:30; y its position in B and strand (bit 31), kNone before one was
+// seen, kMany after two.  Free entries have all bits set, as no x or y has:
+// there is no count 3, and no position of 31 bits.
+constexpr uint32_t kNone = 0xffffffffu, kMany = 0xfffffffeu;
+
+__device__ __forceinline__ uint32_t table_at(uint32_t mer, uint32_t entries) {
+  return __umulhi(mer * 0x9E3779B1u, entries);
+}
+
+// Counts a key; false: no room for its mer.  Entries only ever gain, and a mer
+// seen too often is left alone, so a run of one mer costs two shared reads a
+// key.
+__device__ __forceinline__ bool table_add(uint2* T, uint32_t entries, uint2 key) {
+  const uint32_t mer = key.x >> 2, one = key.x & 1u ? 0u : 1u << 30;
+  uint32_t i = table_at(mer, entries);
+  for (int probe = 0; probe < pb::kProbes; ++probe) {
+    uint32_t x = *(volatile uint32_t*)&T[i].x;
+    bool made = false;
+    if (x == kNone) {
+      x = atomicCAS(&T[i].x, kNone, mer | one);
+      made = x == kNone;
+    }
+    if (made || (x & 0x3fffffffu) == mer) {
+      if (one) {
+        while (!made && x >> 31 == 0) {  // counted none or one so far
+          const uint32_t was = atomicCAS(&T[i].x, x, x + one);
+          made = was == x;
+          x = was;
+        }
+      } else {
+        uint32_t y = *(volatile uint32_t*)&T[i].y;
+        if (y == kNone) y = atomicCAS(&T[i].y, kNone, key.y | (key.x >> 1 & 1u) << 31);
+        if (y != kNone && y != kMany) *(volatile uint32_t*)&T[i].y = kMany;
+      }
+      return true;
+    }
+    if (++i == entries) i = 0;
+  }
+  return false;
+}
+
+// The entry of a mer that was counted.
+__device__ __forceinline__ uint2 table_find(const uint2* T, uint32_t entries, uint32_t mer) {
+  uint32_t i = table_at(mer, entries);
+  while ((T[i].x & 0x3fffffffu) != mer) i = i + 1 == entries ? 0 : i + 1;
+  return T[i];
+}
+
+// v[0, n) counted in an emptied table, by the block; false: too many mers.
+__device__ bool table_fill(uint2* T, uint32_t entries, const uint2* v, int n) {
+  constexpr int kAhead = 4;
+  for (uint32_t i = threadIdx.x; i < entries; i += pb::kLocThreads) T[i] = make_uint2(kNone, kNone);
+  __syncthreads();
+  bool ok = true;
+  for (int i0 = threadIdx.x; i0 < n && ok; i0 += kAhead * pb::kLocThreads) {
+    uint2 key[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (i0 + k * pb::kLocThreads < n) key[k] = v[i0 + k * pb::kLocThreads];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (i0 + k * pb::kLocThreads < n) ok = table_add(T, entries, key[k]) && ok;
+  }
+  return !__syncthreads_or(!ok);
+}
+
+// The pairs of v[0, n) by way of the table; false: too many mers.
+__device__ __noinline__ bool table_pairs(uint2* T, uint32_t entries, const uint2* v, int n, uint32_t* __restrict__ tab) {
+  if (!table_fill(T, entries, v, n)) return false;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += pb::kLocThreads) {
+    const uint2 key = v[i];
+    if (key.x & 1u) continue;  // a pair's position in A
+    const uint2 e = table_find(T, entries, key.x >> 2);
+    if (e.x >> 30 == 1u && e.y != kNone && e.y != kMany)
+      tab[key.y] = (e.y & 0x7fffffffu) | ((key.x >> 1 & 1u) ^ e.y >> 31) << 31;
+  }
+  return true;
+}
+
+// What may be unique of the piece v[0, n), appended to the bucket's list: the
+// keys of mers with one position at most in either genome, and two keys in A
+// for every other mer, so that it stays out.  left: the list's length (bit 31:
+// it is not the whole bucket) and the pieces done.
+__device__ __noinline__ void table_thin(uint2* T, uint32_t entries, const uint2* v, int n, uint2* list, uint2* left) {
+  const int lane = threadIdx.x & 31;
+  if (!table_fill(T, entries, v, n)) {
+    if (threadIdx.x == 0) atomicOr(&left->x, 1u << 31);
+    return;
+  }
+  auto append = [&](bool in, uint2 key) {
+    const unsigned all = __ballot_sync(0xffffffffu, in);
+    uint32_t at = 0;
+    if (lane == 0 && all) at = atomicAdd(&left->x, (uint32_t)__popc(all));
+    at = (__shfl_sync(0xffffffffu, at, 0) & 0x7fffffffu) + __popc(all & ((1u << lane) - 1u));
+    if (in) list[at] = key;
+  };
+  for (int i0 = threadIdx.x & ~31; i0 < n; i0 += pb::kLocThreads) {
+    const int i = i0 + lane;
+    uint2 key = make_uint2(0u, 0u);
+    bool in = i < n;
+    if (in) {
+      key = v[i];
+      const uint2 e = table_find(T, entries, key.x >> 2);
+      in = e.x >> 31 == 0 && e.y != kMany;
+    }
+    append(in, key);
+  }
+  for (uint32_t i0 = threadIdx.x & ~31; i0 < entries; i0 += pb::kLocThreads) {
+    const uint2 e = i0 + lane < entries ? T[i0 + lane] : make_uint2(kNone, kNone);
+    const bool many = e.x != kNone && (e.x >> 31 || e.y == kMany);
+    const uint2 key = make_uint2((e.x & 0x3fffffffu) << 2, 0u);
+    append(many, key);
+    append(many, key);
+  }
 }
 
 // ---------------------------------------------------- in-bucket sort
@@ -424,31 +561,44 @@ __device__ void pb_pairs(const uint2* v, int n, uint32_t* __restrict__ tab) {
   }
 }
 
+// A bucket sorted in chunks between its region of `buf` (g) and the same region
+// of `alt` (h) in an odd number of passes of up to 6 bits, which leaves it in
+// `alt`, and its runs.
+__device__ __noinline__ void pb_sort(uint2* g, uint2* h, int n, int lbits, int npass, int dbits, LocalSmem& S,
+                                     uint32_t* __restrict__ tab) {
+  const uint32_t mask = (1u << dbits) - 1u;
+  const uint2* src = g;
+  uint2* dst = h;
+  for (int p = 0; p < npass; ++p) {
+    pb_pass_chunked(src, dst, n, p * dbits, mask, lbits, S);
+    uint2* t = (uint2*)src;
+    src = dst;
+    dst = t;
+  }
+  pb_pairs(src, n, tab);  // npass is odd: the sorted bucket is in alt
+}
+
 // Block b finds the unique pairs of bucket b.  A bucket of at most cap
 // (<= kCap) keys is split in shared memory by its top in-bucket bits (up to
 // 9) into at most 512 groups of a few keys each (atomics place a group's keys
 // in any order).  Then one thread per key of A: a key whose mer occurs
 // exactly twice in its group, once per genome, is a pair.  Other buckets, and
-// one with a group of more than kGroupMax keys, are sorted in chunks between
-// their region of `buf` and the same region of `alt` in an odd number of
-// passes of up to 6 bits, which leaves them in `alt`.  Loads and shared-memory
-// round trips bound it: six CTAs per SM (40 registers, spills in the sorting
-// path only) take 0.21 ms for 24 million keys and 0.081 for 9.2, three (80
-// registers) took 0.30 and 0.112.
-__global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(uint2* __restrict__ buf, uint2* __restrict__ alt,
+// one with a group of more than kGroupMax keys, are left to k_pb_repeats.
+// Loads and shared-memory round trips bound it: six CTAs per SM take 0.21 ms for
+// 24 million keys and 0.081 for 9.2, three (80 registers) took 0.30 and 0.112.
+__global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(const uint2* __restrict__ buf,
                                                               const uint32_t* __restrict__ bstart,
-                                                              const uint32_t* __restrict__ bsize, int lbits, int npass,
-                                                              int dbits, int cap, uint32_t* __restrict__ tab) {
+                                                              const uint32_t* __restrict__ bsize, int lbits, int cap,
+                                                              PairPieces P, uint32_t* __restrict__ tab) {
   extern __shared__ __align__(16) uint2 sbuf[];  // kCap elements
-  __shared__ LocalSmem S;
   __shared__ uint32_t gcnt[pb::kGroups], gbeg[pb::kGroups], gcur[pb::kGroups];
   const int tid = threadIdx.x;
   const int b = blockIdx.x;
   const int n = (int)bsize[b];
-  uint2* g = buf + bstart[b];
-  uint2* h = alt + bstart[b];
-  bool sort = n > cap;
-  if (!sort) {
+  const uint2* g = buf + bstart[b];
+  if (n > pb::kPiece) return;  // in pieces
+  bool rest = n > cap;
+  if (!rest) {
     // group bits: mer bits only (never the genome bit), at most 9
     const int hbits = lbits - 1 < 9 ? lbits - 1 : 9, lo = lbits - hbits, ng = 1 << hbits;
     for (int d = tid; d < pb::kGroups; d += pb::kLocThreads) gcnt[d] = 0;
@@ -469,8 +619,8 @@ __global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(uint2* __restri
     const uint32_t st = block_excl_scan256(c0 + c1, nullptr);
     if (d0 < ng) gbeg[d0] = gcur[d0] = st;
     if (d0 + 1 < ng) gbeg[d0 + 1] = gcur[d0 + 1] = st + c0;
-    sort = __syncthreads_or(c0 > (uint32_t)pb::kGroupMax || c1 > (uint32_t)pb::kGroupMax);
-    if (!sort) {
+    rest = __syncthreads_or(c0 > (uint32_t)pb::kGroupMax || c1 > (uint32_t)pb::kGroupMax);
+    if (!rest) {
 #pragma unroll
       for (int k = 0; k < pb::kLocItems; ++k)
         if (k * pb::kLocThreads + tid < n) sbuf[atomicAdd(&gcur[pb_lkey(item[k].x, lbits) >> lo], 1u)] = item[k];
@@ -494,17 +644,46 @@ __global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(uint2* __restri
       }
     }
   }
-  if (sort) {
-    const uint32_t mask = (1u << dbits) - 1u;
-    const uint2* src = g;
-    uint2* dst = h;
-    for (int p = 0; p < npass; ++p) {
-      pb_pass_chunked(src, dst, n, p * dbits, mask, lbits, S);
-      uint2* t = (uint2*)src;
-      src = dst;
-      dst = t;
+  if (rest && tid == 0) {
+    const uint32_t at = atomicAdd(P.count, 1u);
+    P.piece[at] = make_uint4((uint32_t)b, 0u, at, 0u);
+  }
+}
+
+// The buckets in P, a block at a time: whole ones (no pieces), or pieces, of
+// which whoever does a bucket's last looks for the pairs in what they left.
+// (Sorted by one block each, a bucket of 600,000 equal mers took 6 ms, one of
+// the 2 million of a run of N 24.)
+__global__ void __launch_bounds__(pb::kLocThreads) k_pb_repeats(uint2* __restrict__ buf, uint2* __restrict__ alt,
+                                                                const uint32_t* __restrict__ bstart,
+                                                                const uint32_t* __restrict__ bsize, int lbits,
+                                                                int npass, int dbits, int cap, PairPieces P,
+                                                                uint32_t* __restrict__ tab) {
+  extern __shared__ __align__(16) uint2 sbuf[];  // kCap elements
+  __shared__ LocalSmem S;
+  __shared__ uint32_t done;
+  const uint32_t total = *P.count;
+  for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
+    const uint4 piece = P.piece[w];  // bucket, number, the bucket's first, their number
+    const int size = (int)bsize[piece.x];
+    uint2 *const v = buf + bstart[piece.x], *const list = alt + bstart[piece.x];
+    __syncthreads();  // the last round's table is read
+    const uint2* rest = v;
+    int m = size;
+    if (piece.w > 0) {
+      const int at = (int)piece.y * pb::kPiece;
+      uint2* const left = P.left + piece.z;
+      table_thin(sbuf, (uint32_t)cap, v + at, min(pb::kPiece, size - at), list, left);
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) done = atomicAdd(&left->y, 1u);
+      __syncthreads();
+      if (done + 1 < piece.w) continue;
+      __threadfence();  // all pieces are in the list
+      rest = list;
+      m = (int)*(volatile uint32_t*)&left->x;
     }
-    pb_pairs(src, n, tab);  // npass is odd: the sorted bucket is in alt
+    if (m < 0 || !table_pairs(sbuf, (uint32_t)cap, rest, m, tab)) pb_sort(v, list, size, lbits, npass, dbits, S, tab);
   }
 }
 
@@ -521,12 +700,20 @@ int pair_bucket_bufs(Ctx* c, uint64_t n, int bits, PairBucketBufs* b) {
   b->buf = (uint2*)ws.get(c, 31, (size_t)n * 8 + 64);
   // count rows, then the tiles' first slots (ntiles x nbk each)
   b->counts = (uint32_t*)ws.get(c, 32, (size_t)g.ntiles * nbk * 8 + 64);
-  uint32_t* tabs = (uint32_t*)ws.get(c, 33, ((size_t)g.nchunks * nbk + 2 * (size_t)nbk) * 4 + 256);
+  // chunk sums, bucket starts and sizes; the pieces of large buckets (at most
+  // two per kPiece keys) and the buckets k_pb_local leaves: their list, what is
+  // left of the bucket of each, their number
+  const size_t tab_words = ((size_t)g.nchunks * nbk + 2 * (size_t)nbk + 67) & ~(size_t)3;
+  const size_t most = 2 * (n / pb::kPiece) + 2 + nbk;
+  uint32_t* tabs = (uint32_t*)ws.get(c, 33, tab_words * 4 + most * 24 + 16);
   if (!b->alt || !b->buf || !b->counts || !tabs) return report_error(MVG_ERR_NOMEM, "workspace allocation failed");
   b->offs = b->counts + (size_t)g.ntiles * nbk;
   b->csum = tabs;
   b->bstart = tabs + (size_t)g.nchunks * nbk;
   b->bsize = b->bstart + nbk;
+  b->pieces.piece = (uint4*)(tabs + tab_words);
+  b->pieces.left = (uint2*)(b->pieces.piece + most);
+  b->pieces.count = (uint32_t*)(b->pieces.left + most);
   return 0;
 }
 
@@ -534,7 +721,7 @@ void pair_bucket_offsets(Ctx* c, const PairBucketBufs& b) {
   const PairBucketGeom& g = b.g;
   const dim3 grid2((unsigned)((g.nbuckets + 255) / 256), (unsigned)g.nchunks);
   k_pb_csum<<<grid2, 256, 0, c->stream>>>(b.counts, g.ntiles, g.nbuckets, b.csum);
-  k_pb_scan<<<1, 1024, 0, c->stream>>>(b.csum, g.nchunks, g.nbuckets, b.bstart, b.bsize);
+  k_pb_scan<<<1, 1024, 0, c->stream>>>(b.csum, g.nchunks, g.nbuckets, b.bstart, b.bsize, b.pieces);
   k_pb_offsets<<<grid2, 256, 0, c->stream>>>(b.counts, g.ntiles, g.nbuckets, b.csum, b.bstart, b.offs);
   c->launches += 3;
 }
@@ -542,15 +729,23 @@ void pair_bucket_offsets(Ctx* c, const PairBucketBufs& b) {
 void pair_bucket_join(Ctx* c, const PairBucketBufs& b, uint32_t* tab) {
   const PairBucketGeom& g = b.g;
   const int cap = std::min(c->pair_bucket_cap, pb::kCap);
-  k_pb_local<<<(unsigned)g.nbuckets, pb::kLocThreads, pb::kCap * sizeof(uint2), c->stream>>>(
-      b.buf, b.alt, b.bstart, b.bsize, g.lbits, g.npass, g.dbits, cap, tab);
+  const size_t smem = pb::kCap * sizeof(uint2);
+  k_pb_local<<<(unsigned)g.nbuckets, pb::kLocThreads, smem, c->stream>>>(b.buf, b.bstart, b.bsize, g.lbits, cap,
+                                                                         b.pieces, tab);
+  c->launches++;
+}
+
+void pair_bucket_repeats(Ctx* c, const PairBucketBufs& b, uint32_t* tab) {
+  const PairBucketGeom& g = b.g;
+  const int cap = std::min(c->pair_bucket_cap, pb::kCap);
+  k_pb_repeats<<<pb::kRepeatCtas, pb::kLocThreads, pb::kCap * sizeof(uint2), c->stream>>>(
+      b.buf, b.alt, b.bstart, b.bsize, g.lbits, g.npass, g.dbits, cap, b.pieces, tab);
   c->launches++;
 }
 
 template <typename K>
 static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
-                           uint32_t* tab) {
-  PairBucketBufs b;
+                           uint32_t* tab, PairBucketBufs& b) {
   if (int rc = pair_bucket_bufs(c, ca + cb, 2 * s.w, &b)) return rc;
   const PairBucketGeom& g = b.g;
   bool& ready = c->join_ready[sizeof(K) == 8];
@@ -573,9 +768,9 @@ static int pair_buckets_as(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32
 }
 
 int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
-                 uint32_t* tab) {
-  return s.w <= 15 ? pair_buckets_as<uint32_t>(c, ga, ca, gb, cb, s, tab)
-                   : pair_buckets_as<uint64_t>(c, ga, ca, gb, cb, s, tab);
+                 uint32_t* tab, PairBucketBufs* b) {
+  return s.w <= 15 ? pair_buckets_as<uint32_t>(c, ga, ca, gb, cb, s, tab, *b)
+                   : pair_buckets_as<uint64_t>(c, ga, ca, gb, cb, s, tab, *b);
 }
 
 }  // namespace mvg
