@@ -617,8 +617,8 @@ int mvg_set_ring_max_rows(mvg_handle h, int rows);
 int mvg_set_band_whole_full_rows(mvg_handle h, int64_t rows);
 
 /* Full gap-DP passes checkpointed (on = 1, the default): the forward pass
- * keeps every strip's bottom row and, every 128 steps, the strip's state
- * instead of traceback bits (about 0.1 instead of 0.5 bytes per cell), and
+ * keeps every strip's bottom row and, every 64 steps, the strip's state
+ * instead of traceback bits (about 0.17 instead of 0.5 bytes per cell), and
  * the traceback recomputes the bits of only the blocks of the matrix its
  * path crosses, with the same recurrence and tie order; problems of up to
  * 700 columns store the bits all the same.  on = 0 stores the bits (except

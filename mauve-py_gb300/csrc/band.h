@@ -5,8 +5,7 @@
 // strips of `srows` rows, so the kept region is a staircase: strip k spans
 // [lo_k, hi_k], the union over its rows, with strip 0 starting at column 1
 // and the last strip ending at column LB (the path's two end cells).  Both
-// bounds are non-decreasing in k.  The full DP is the same geometry with
-// lo_k = 1 and hi_k = LB for every strip.
+// bounds are non-decreasing in k.
 #pragma once
 #include <stdint.h>
 
@@ -20,7 +19,6 @@ namespace mvg {
 
 struct Band {
   int LA, LB, delta, half, srows, nstrips;
-  bool full;
 };
 
 MVG_HD Band make_band(int LA, int LB, int delta, int half, int srows) {
@@ -31,20 +29,13 @@ MVG_HD Band make_band(int LA, int LB, int delta, int half, int srows) {
   b.half = half < 0 ? 0 : half;
   b.srows = srows;
   b.nstrips = (LA + srows - 1) / srows;
-  b.full = false;
-  return b;
-}
-
-MVG_HD Band make_full(int LA, int LB, int srows) {
-  Band b = make_band(LA, LB, 0, 0, srows);
-  b.full = true;
   return b;
 }
 
 MVG_HD int64_t band_center(const Band& b, int i) { return (int64_t)i * b.LB / b.LA + b.delta; }
 
 MVG_HD int band_lo(const Band& b, int k) {
-  if (k == 0 || b.full) return 1;
+  if (k == 0) return 1;
   int64_t lo = band_center(b, k * b.srows + 1) - b.half;
   if (lo < 1) lo = 1;
   if (lo > b.LB) lo = b.LB;
@@ -52,7 +43,7 @@ MVG_HD int band_lo(const Band& b, int k) {
 }
 
 MVG_HD int band_hi(const Band& b, int k) {
-  if (k == b.nstrips - 1 || b.full) return b.LB;
+  if (k == b.nstrips - 1) return b.LB;
   int last = (k + 1) * b.srows;
   if (last > b.LA) last = b.LA;
   int64_t hi = band_center(b, last) + b.half + 1;
@@ -165,20 +156,6 @@ MVG_HD uint64_t ring_tb_words(const RingBand& b) {
   const int per = ring_steps_per_word(b.R);
   const uint64_t w = per > 1 ? (uint64_t)((b.steps + per - 1) / per) : (uint64_t)b.steps * ring_words_per_step(b.R);
   return w * 32;
-}
-
-// Matrix cells inside the kept region (rows 1..LA, columns 1..LB).
-MVG_HD uint64_t ring_cells(const RingBand& b) {
-  uint64_t cells = 0;
-  for (int g = 0; g < b.G; ++g) {
-    int rows = b.LA - g * b.R;
-    if (rows > b.R) rows = b.R;
-    int lo = ring_lo(b, g), hi = lo + b.W - 1;
-    if (lo < 1) lo = 1;
-    if (hi > b.LB) hi = b.LB;
-    if (hi >= lo) cells += (uint64_t)rows * (uint64_t)(hi - lo + 1);
-  }
-  return cells;
 }
 
 }  // namespace mvg

@@ -13,12 +13,14 @@
 // between two sentinel-derived values (D in row 1, I in column 1) see equal
 // operands exactly as the float code does, so every traceback bit matches.
 //
-// Kernels: k_gapdp_t (gapdp_kernel.cuh) fills the traceback arena;
-// k_traceback walks each problem's bits from (LA, LB) like BitTraceBack
-// (MU/bittraceback.cpp:138-210); k_path_compact moves paths to slot heads.
-// Full-DP passes run checkpointed by default: the forward kernel keeps
-// strip rows and block columns instead of traceback bits, and k_tb_ck
-// (traceback_ck.cuh) recomputes the bits of the blocks each path crosses.
+// Full DP (gapdp_strips.cuh): k_gapdp_strips fills the traceback arena with
+// strip rows and, checkpointed, states or, for problems of few columns, bits;
+// k_strip_walk walks each path from (LA, LB) like BitTraceBack
+// (MU/bittraceback.cpp:138-210), computing again the blocks it crosses, and
+// moves it to its slot's head.  Banded: k_gapdp_ring and k_ring_walk
+// (gapdp_ring.cuh); bands no ring height fits run in k_gapdp_t
+// (gapdp_kernel.cuh), whose bits k_traceback and, for long paths,
+// k_traceback_win (traceback_win.cuh) walk and k_path_compact moves.
 #include <limits.h>
 
 #include <algorithm>
@@ -79,9 +81,6 @@ template __global__ void k_gapdp_t<8>(DpJob);
 static const int kRingRows[] = {4, 6, 8, 12, 16, 24, 32};
 constexpr int kRingHeights = (int)(sizeof(kRingRows) / sizeof(kRingRows[0]));
 
-// Runs f(begin, end, t) over [0, n) in up to 16 contiguous chunks on host
-// threads (one chunk below 20,000 items), chunk t covering items before
-// chunk t + 1's; returns the number of chunks.
 // Indices 0..n-1 ordered by key (ascending, ties in index order): a stable
 // LSD radix sort with 11-bit digits over the key's used bits.
 static std::vector<uint32_t> radix_order(const std::vector<uint64_t>& key) {
@@ -100,6 +99,9 @@ static std::vector<uint32_t> radix_order(const std::vector<uint64_t>& key) {
   return a;
 }
 
+// Runs f(begin, end, t) over [0, n) in up to 16 contiguous chunks on host
+// threads (one chunk below 20,000 items), chunk t covering items before
+// chunk t + 1's; returns the number of chunks.
 template <class F>
 static int host_chunks(int64_t n, F f) {
   int nt = 1;
@@ -245,12 +247,6 @@ struct DpInputs {
   int32_t* env = nullptr;  // optional path envelope output [2 * nprob], full DP only
 };
 
-// Starts the long-path walker for one wave on the aux stream (joined by
-// tb_long_join), beside the thread walker on the main stream.  A warp walks
-// a path about ten times faster than a thread but far fewer warps than
-// threads run at once, so warps take the longest paths only: those with
-// LA + LB >= kTbLongPath, at most one round of the walker's warps, longest
-// first.  *long_path receives the length from which paths go to warps.
 // The streams one DP pass runs on: its own, and the side stream its
 // long-path walker forks to, with the events and workspace slots for that.
 struct TbLanes {
@@ -259,7 +255,11 @@ struct TbLanes {
   int slot_list, slot_ctr;
 };
 
-// Host side of the long-path walker: the slots (of this wave's order) whose
+// The long-path walker runs beside the thread walker.  A warp walks
+// a path about ten times faster than a thread but far fewer warps than
+// threads run at once, so warps take the longest paths only: those with
+// LA + LB >= kTbLongPath, at most one round of the walker's warps, longest
+// first.  Host side: the slots (of this wave's order) whose
 // paths go to warps, longest first, and the length from which they do.
 static int tb_long_plan(Ctx* c, const std::vector<uint32_t>& slot_len, std::vector<uint32_t>* long_slots,
                         int* long_path, int* grid) {
@@ -910,10 +910,6 @@ static int run_ring(Ctx* c, const TbLanes& L, const DpInputs& in, const std::vec
   return 0;
 }
 
-// Whole-matrix problems with at least this many rows run in the full DP's
-// launch (strips of 32 * dp_rows rows), shorter ones in the banded strip
-// launch (32 * band_rows rows).
-
 // Every base code must be 0..3 (the kernels mask to 2 bits; this reports it).
 static int check_codes(Ctx* c, const uint8_t* d_sa, uint64_t na, const uint8_t* d_sb, uint64_t nb) {
   k_check_codes<<<dim3(grid_for(std::max(na, nb) / 16 + 1, 256), 2), 256, 0, c->stream>>>(d_sa, na, d_sb, nb, c->d_err);
@@ -997,11 +993,11 @@ int gapdp_banded_dev(Ctx* c, const uint8_t* d_sa, const uint64_t* d_oa, const ui
   std::vector<int32_t> dv(h_delta, h_delta + nprob), hv(h_half, h_half + nprob);
   uint64_t bc = 0;
   // A band covering at least band_whole (default half) of its matrix saves
-  // little and may still fail its check: such problems are not banded.  They
-  // run in the strip kernel's launch with a band that covers the whole matrix
-  // (no exit cells, so the check always passes and the result is the full
-  // DP's; short strips suit these mostly small problems better than the full
-  // DP's), which spares a second pass for them (status 2).  Other bands run
+  // little and may still fail its check: such problems are not banded (status
+  // 2).  They go to the full DP beside the bands, those below whole_full_rows
+  // (0 by default) to the strip kernel's launch with a band that covers the
+  // whole matrix (no exit cells, so the check always passes and the result is
+  // the full DP's).  Other bands run
   // on the ring schedule with the smallest valid group height, or in the
   // strip kernel when no height is valid (or the ring kernel is switched off).
   std::vector<uint32_t> ids, rids, wids;

@@ -46,7 +46,6 @@ namespace mvg {
 
 constexpr int32_t kNeg = -(1 << 29);
 constexpr int32_t kGap = -200;           // half of gap open -400
-constexpr int32_t kMaxPair = 160;        // max NUC_SP + 60 (C/C, G/G)
 constexpr int kDpThreads = 256;
 constexpr int kDpWarps = kDpThreads / 32;
 constexpr int kCoopMinStrips = 16;       // problems with at least this many strips use a whole CTA

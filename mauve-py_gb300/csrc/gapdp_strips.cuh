@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kStWarps * 32, 5) k_gapdp_strips(StripJob J) {
 // scores fit 32 bits at any length).  A path crosses a strip of 256 rows in
 // about 290 steps, so the kWalkWarps blocks up to the walk's step are
 // computed at once, one per warp, and the first warp walks them: a block is a
-// serial chain of 128 steps, and the longest paths, which end the pass, took
+// serial chain of 64 steps, and the longest paths, which end the pass, took
 // one such chain per block when one warp did everything.
 constexpr int kWalkWarps = 512 / kStBlock;
 struct WalkJob {

@@ -1,7 +1,6 @@
 // Device-side pieces of the seed matcher shared by the genome-pair matcher
 // (match.cu) and the batched gap anchor search (gapsearch.cu): the hash
-// entry, the unique-seed run test, MheCompare / Contains and ExtendMatch's
-// walk.
+// entry, its order, the unique-seed run test and ExtendMatch's walk.
 #pragma once
 #include "mvg_internal.h"
 #include "prim.cuh"
@@ -11,7 +10,7 @@ namespace mvg {
 constexpr int kTableSize = 40000;  // LM/MemHash.h:30 DEFAULT_MEM_TABLE_SIZE
 
 struct Mhe {
-  int64_t s0, s1, len, off;
+  int64_t s0, s1, len;
 };
 
 struct MatchCtx {
@@ -45,19 +44,6 @@ __device__ __forceinline__ bool pair_flag(const K* __restrict__ keys, int64_t n,
 
 // ------------------------------------------------------ hash entries
 
-// LM/MatchHashEntry.cpp:164-200 (Contains), two genomes, both present.
-__device__ __forceinline__ bool mhe_contains(const Mhe& c, const Mhe& m) {
-  if (c.off != m.off) return false;
-  const int64_t diff = m.s0 - c.s0;
-  if (c.s0 == 0) return false;
-  if (diff < 0 || (uint64_t)c.len < (uint64_t)(m.len + diff)) return false;
-  const int64_t diff_rc = m.len - c.len + diff;
-  const int64_t diff_i = m.s1 - c.s1;
-  if (m.s1 == 0 && c.s1 == 0) return true;
-  if (m.s1 < 0 && diff_rc == diff_i) return true;
-  return diff == diff_i;
-}
-
 // LM/MatchHashEntry.cpp:48-67 (strict_start_lessthan_ptr).
 __device__ __forceinline__ bool mhe_strict_lt(const Mhe& a, const Mhe& b, int L) {
   int64_t x = a.s0 < 0 ? -a.s0 + a.len - L : a.s0;
@@ -69,14 +55,8 @@ __device__ __forceinline__ bool mhe_strict_lt(const Mhe& a, const Mhe& b, int L)
   return false;
 }
 
-// LM/MatchHashEntry.h:121-143 (MheCompare) for pairwise entries.
-__device__ __forceinline__ bool mhe_less(const Mhe& a, const Mhe& b, int L) {
-  if (mhe_contains(a, b) || mhe_contains(b, a)) return false;
-  return mhe_strict_lt(a, b, L);
-}
-
-// ExtendMatch (LM/MatchFinder.h:218-374) for two genomes.  The reference cycles through four phases (jump left and right by
-// the seed length until the first mismatching window, then try the L
+// ExtendMatch (LM/MatchFinder.h:218-374) for two genomes.  The reference cycles
+// through four phases (jump left and right by the seed length until the first mismatching window, then try the L
 // single-base offsets left and right and move to the furthest matching one)
 // and restarts while a single-base phase moves.
 //

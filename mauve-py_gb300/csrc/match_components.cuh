@@ -19,7 +19,9 @@
 //  * Where the components of a bucket, in order of their starts in A, end
 //    (with their last seed) before the next one starts, the entries before a
 //    seed x's component start before x and are less, those after it start
-//    behind x and are not less, and its own entry contains it: the comparator
+//    behind x and are not less, and its own entry contains it (MheCompare,
+//    LM/MatchHashEntry.h:121-143, over Contains, LM/MatchHashEntry.cpp:164-200,
+//    where neither is less): the comparator
 //    is monotone for every x and every subset of the entries, lower_bound
 //    finds x's entry iff it is there, and the bucket ends up with its
 //    components in order of their starts, whatever the order of the seeds.
@@ -70,7 +72,6 @@ __device__ __forceinline__ Mhe diag_entry(uint64_t d, uint32_t lo, uint32_t hi, 
   m.s0 = (int64_t)lo + 1;
   m.len = (int64_t)(hi - lo) + L;
   m.s1 = d >> 32 ? -((int64_t)((uint32_t)d - hi) + 1) : (int64_t)((uint32_t)d + lo) + 1;
-  m.off = diag_offset(d, L);
   return m;
 }
 
@@ -359,18 +360,17 @@ struct Components {
 static __global__ void __launch_bounds__(256) k_comp_count(const uint8_t* __restrict__ joined, int64_t n,
                                                     uint32_t* __restrict__ tcount) {
   const int64_t i0 = (int64_t)blockIdx.x * kSegTile + (int64_t)threadIdx.x * 8;
-  uint32_t cnt = 0, total;
+  uint32_t cnt = 0;
   for (int q = 0; q < 8; ++q) {
     const int64_t k = i0 + q;
     cnt += k < n && !(k > 0 && joined[k - 1]);
   }
-  block_excl_scan256(cnt, nullptr);
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   __shared__ uint32_t ws[8];
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = cnt;
   __syncthreads();
   if (threadIdx.x == 0) {
-    total = 0;
+    uint32_t total = 0;
     for (int w = 0; w < 8; ++w) total += ws[w];
     tcount[blockIdx.x] = total;
   }

@@ -54,7 +54,7 @@ struct Ctx {
   int band_ring = 1;          // banded problems on the ring schedule where it is valid
   int band_gate = 0;          // band proposals: divergence gate window threshold (0 = off)
   int pair_bucket_cap = 3072;  // seed-join buckets sorted in shared memory up to this size
-  long long dp_spin_limit = 1ll << 26;  // polls before a whole-CTA gap-DP wait gives up (about a second)
+  long long dp_spin_limit = 1ll << 26;  // polls before a pipelined gap-DP wait gives up (about a second)
   int dp_graph = 1;                      // gap-DP passes launched as one recorded CUDA graph
   int dp_ckpt = 1;                       // full-DP passes keep checkpoints, the traceback recomputes blocks
   int64_t whole_full_rows = 0;           // banded calls: whole-matrix problems from this many rows go to the full DP
@@ -145,7 +145,6 @@ uint8_t* pinned_buf(Ctx* c, int which, size_t need);
 int pack_sequence(Ctx* c, const uint8_t* d_seq, uint64_t n, uint32_t* d_packed);
 int sml_sort(Ctx* c, const uint32_t* d_packed, uint64_t count, const SeedDesc& s, uint32_t* d_pos_out,
              uint64_t* d_mer_out);
-// Both genomes' keys ((seed bits, strand, genome) with A = 0) sorted in one array.
 // The bucketed seed join (pair_buckets.cu) for at most kPairBucketMaxKeys
 // keys: tab[position in A] = position in B | reverse << 31 for every seed
 // unique in both genomes (tab holds ~0 elsewhere).
@@ -182,6 +181,7 @@ int pair_buckets(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, ui
                  uint32_t* tab, PairBucketBufs* b);
 // Exclusive scan of n <= 16384 counts in one launch; *total gets the sum.
 void pair_scan_small(const uint32_t* in, int n, uint32_t* out, uint32_t* total, cudaStream_t st);
+// Both genomes' keys (seed bits, strand, genome: A 0) sorted in one array.
 int pair_sort(Ctx* c, const uint32_t* ga, uint64_t ca, const uint32_t* gb, uint64_t cb, const SeedDesc& s,
               SmlKeys* out);
 int check_device_error(Ctx* c);
