@@ -10,6 +10,8 @@
 // __match_any_sync peer masks and per-warp counts, so equal digits keep their
 // input order and the whole sort is stable.
 #pragma once
+#include <atomic>
+
 #include "mvg_common.cuh"
 
 namespace mvg {
@@ -577,10 +579,13 @@ __global__ void __launch_bounds__(1024) k_small_sort(K* __restrict__ keys, uint3
   }
 }
 
-// false when the device does not give it the shared memory.
+// false when the device does not give it the shared memory.  Static, as its
+// caller: the flags below are this file's kernels', and the local statics of a
+// function with external linkage are one per process, shared with every other
+// copy of the library in it.
 template <typename K>
-bool small_sort_pairs(K* keys, uint32_t* vals, int n, int nbits, cudaStream_t st, uint64_t* launches) {
-  static bool ready[64] = {};  // per device: the opt-in for more than 48 KB
+static bool small_sort_pairs(K* keys, uint32_t* vals, int n, int nbits, cudaStream_t st, uint64_t* launches) {
+  static std::atomic<bool> ready[64];  // per device: the opt-in for more than 48 KB
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
   if (!ready[dev]) {
@@ -607,7 +612,7 @@ inline int64_t sort_scratch_words(int64_t n, int nbits) {
 }
 
 template <typename K>
-int sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n, int nbits, uint32_t* scratch,
+static int sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n, int nbits, uint32_t* scratch,
                cudaStream_t st, uint64_t* launches, uint32_t* err) {
   (void)err;
   if (n <= 0) return 0;

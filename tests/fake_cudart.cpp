@@ -17,6 +17,8 @@ constexpr int kDevices = 4;
 std::mutex mu;
 std::map<std::pair<int, const void*>, size_t> allowed;  // dynamic shared memory, by device and kernel
 size_t refused, largest, free_bytes = (size_t)1 << 40;
+unsigned char reply[64];
+size_t reply_bytes;
 thread_local int device;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct {
@@ -53,8 +55,13 @@ extern "C" {
 size_t fake_refused() { return refused; }
 size_t fake_largest() { return largest; }
 void fake_reset(size_t free_memory) {
-  refused = largest = 0;
+  refused = largest = reply_bytes = 0;
   free_bytes = free_memory;
+}
+// What the next copy of n bytes to the host brings.
+void fake_reply(const void* data, size_t n) {
+  memcpy(reply, data, n);
+  reply_bytes = n;
 }
 
 void** __cudaRegisterFatBinary(void*) {
@@ -137,8 +144,10 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
   *f = *t = free_bytes;
   return cudaSuccess;
 }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind, cudaStream_t) {
-  memcpy(d, s, n);
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind kind, cudaStream_t) {
+  const bool replied = kind == cudaMemcpyDeviceToHost && n == reply_bytes;
+  memcpy(d, replied ? reply : s, n);
+  if (replied) reply_bytes = 0;
   return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {

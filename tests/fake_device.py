@@ -23,6 +23,7 @@ def load(where):
     for name in ("fake_refused", "fake_largest"):
         getattr(lib, name).restype = ctypes.c_size_t
     lib.fake_reset.argtypes = [ctypes.c_size_t]
+    lib.fake_reply.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     lib.mvg_last_error.restype = ctypes.c_char_p
     lib.mvg_get_seed.restype = ctypes.c_uint64
     return lib
