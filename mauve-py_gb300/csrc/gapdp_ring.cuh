@@ -363,7 +363,7 @@ __device__ void ring_solve(const RingJob& J, RingSmem<RMAX>& sm, int w) {
 // Problems of all heights up to RMAX (above the previous launch's), claimed
 // longest first.  One launch for several heights: a launch per height ends in
 // the chain of steps of its longest problem, and those tails added up.
-// 4 and 2 CTAs per SM (117 and 206 registers): 30,011 recoded-pair gaps took
+// 4 and 2 CTAs per SM (128 and 218 registers): 30,011 recoded-pair gaps took
 // 15.8 ms, against 16.6 at 5 and 17.7 at 6 of the low launch.
 template <int RMAX>
 __global__ void __launch_bounds__(kRingThreads, RMAX == 12 ? 4 : 2) k_gapdp_ring(RingJob J) {

@@ -50,7 +50,7 @@ constexpr int kCap = 3072;      // bucket elements sorted in shared memory
 constexpr int kLocItems = kCap / kLocThreads;
 constexpr int kMaxDigit = 64;   // chunked in-bucket passes: digits of at most 6 bits
 constexpr int kGroups = 512;    // groups of a bucket: its top 9 in-bucket bits
-constexpr int kGroupMax = 256;  // larger groups: the bucket goes through the hash table
+constexpr int kGroupMax = 1024;  // larger groups: the bucket goes through the hash table
 constexpr int kPiece = 8192;    // larger buckets: keys of a piece
 constexpr int kRepeatCtas = 608;
 constexpr int kProbes = 512;    // table entries looked at for a mer before the bucket is sorted instead
@@ -582,8 +582,11 @@ __device__ __noinline__ void pb_sort(uint2* g, uint2* h, int n, int lbits, int n
 // (<= kCap) keys is split in shared memory by its top in-bucket bits (up to
 // 9) into at most 512 groups of a few keys each (atomics place a group's keys
 // in any order).  Then one thread per key of A: a key whose mer occurs
-// exactly twice in its group, once per genome, is a pair.  Other buckets, and
-// one with a group of more than kGroupMax keys, are left to k_pb_repeats.
+// exactly twice in its group, once per genome, is a pair.  A repeated mer's keys
+// have seen enough after its third, so a group may hold hundreds of one.  Other
+// buckets, and one with a group of more than kGroupMax keys, are left to
+// k_pb_repeats: that costs the call 40 us, which a bacterial genome should not
+// pay for a mer of 260 positions.
 // Loads and shared-memory round trips bound it: six CTAs per SM take 0.21 ms for
 // 24 million keys and 0.081 for 9.2, three (80 registers) took 0.30 and 0.112.
 __global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(const uint2* __restrict__ buf,
@@ -630,7 +633,7 @@ __global__ void __launch_bounds__(pb::kLocThreads, 6) k_pb_local(const uint2* __
         if (x & 1u) continue;  // the A occurrence of each pair
         const int d = (int)(pb_lkey(x, lbits) >> lo), e0 = (int)gbeg[d], e1 = e0 + (int)gcnt[d];
         int cnt = 0, other = 0;
-        for (int j = e0; j < e1; ++j)
+        for (int j = e0; j < e1 && cnt < 3; ++j)
           if (((sbuf[j].x ^ x) >> 2) == 0) {
             ++cnt;
             if (j != i) other = j;
