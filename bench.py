@@ -953,7 +953,7 @@ def run_gb300(args, world, rank, local):
                        "l2": "flushed between timed steps (256 MiB device write, untimed)",
                        "parallelism": "replicas: one genome pair per GPU"},
             "roofline": {
-                "bound": "hbm", "kernel": "seed path (pack + seed keys + LSD radix sort + unique join), both genomes",
+                "bound": "hbm", "kernel": "seed path (pack + seed keys + bucketed unique join), both genomes",
                 "achieved": round(seed_bytes / (seed_ms / 1e3) / 1e9, 2) if seed_ms else None,
                 "peak": hbm_peak, "unit": "GB/s", "peak_kind": peak_kind,
                 "frac": round(seed_bytes / (seed_ms / 1e3) / 1e9 / hbm_peak, 4) if seed_ms else None,
