@@ -679,6 +679,7 @@ static int gs_device(Ctx* c, const uint8_t* d_a, const uint8_t* d_b, GsChunk& ch
   pair_scan_small(kept, ng, at, sum, c->stream);
   k_gs_out<<<ng, 64, 0, c->stream>>>(d_rows, gap_row, kept, at, d_gaps, d_out);
   c->launches += 4;
+  MVG_CUDA_TRY(cudaGetLastError());
   stage_mark(c, "gs_copy");
   const size_t tab_bytes = ((size_t)ng * 4 + 2) * 4;
   uint32_t* h = (uint32_t*)pinned_buf(c, buf, std::max(tab_bytes, (size_t)r.rows * 24 + 256));

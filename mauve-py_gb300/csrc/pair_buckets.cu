@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(pb::kLocThreads) k_pb_repeats(uint2* __restric
     const uint4 piece = P.piece[w];  // bucket, number, the bucket's first, their number
     const int size = (int)bsize[piece.x];
     uint2 *const v = buf + bstart[piece.x], *const list = alt + bstart[piece.x];
-    __syncthreads();  // the last round's table is read
+    __syncthreads();  // the last bucket's table is read
     const uint2* rest = v;
     int m = size;
     if (piece.w > 0) {

@@ -11,14 +11,15 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 namespace {
 constexpr int kDevices = 4;
 std::mutex mu;
 std::map<std::pair<int, const void*>, size_t> allowed;  // dynamic shared memory, by device and kernel
 size_t refused, largest, free_bytes = (size_t)1 << 40;
-unsigned char reply[64];
-size_t reply_bytes;
+std::map<size_t, std::vector<unsigned char>> replies;  // by size
+long launches, fail_at = -1;
 thread_local int device;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct {
@@ -35,6 +36,7 @@ cudaError_t handle(T* out) {
 
 cudaError_t launch(const void* f, size_t smem) {
   std::lock_guard<std::mutex> lk(mu);
+  if (launches++ == fail_at) return last = cudaErrorLaunchOutOfResources;
   const auto it = allowed.find({device, f});
   if (smem <= std::max<size_t>(48 << 10, it == allowed.end() ? 0 : it->second)) return cudaSuccess;
   ++refused;
@@ -55,14 +57,20 @@ extern "C" {
 size_t fake_refused() { return refused; }
 size_t fake_largest() { return largest; }
 void fake_reset(size_t free_memory) {
-  refused = largest = reply_bytes = 0;
+  refused = largest = 0;
   free_bytes = free_memory;
+  replies.clear();
+  launches = 0;
+  fail_at = -1;
 }
 // What the next copy of n bytes to the host brings.
 void fake_reply(const void* data, size_t n) {
-  memcpy(reply, data, n);
-  reply_bytes = n;
+  const unsigned char* p = (const unsigned char*)data;
+  replies[n].assign(p, p + n);
 }
+// The k-th launch from now (from 0) fails; the launches since the last reset.
+void fake_fail_at(long k) { fail_at = launches + k; }
+long fake_launches() { return launches; }
 
 void** __cudaRegisterFatBinary(void*) {
   static void* h;
@@ -145,9 +153,9 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind kind, cudaStream_t) {
-  const bool replied = kind == cudaMemcpyDeviceToHost && n == reply_bytes;
-  memcpy(d, replied ? reply : s, n);
-  if (replied) reply_bytes = 0;
+  const auto it = kind == cudaMemcpyDeviceToHost ? replies.find(n) : replies.end();
+  memcpy(d, it == replies.end() ? s : it->second.data(), n);
+  if (it != replies.end()) replies.erase(it);
   return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
