@@ -293,34 +293,56 @@ __global__ void k_to_band(const float* __restrict__ o, int64_t n, float alpha, f
 // groups never reach past the allocation.
 static int64_t rows8(int64_t n) { return (n + 7) & ~(int64_t)7; }
 
+template <typename T>
+static void release(T*& p) {
+  cudaFree(p);
+  p = nullptr;
+}
+template <typename T>
+static bool reserve(T*& p, int64_t bytes) {
+  if (cudaMalloc(&p, (size_t)bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  p = nullptr;
+  return false;
+}
+
+static void free_params(MlpState& s) {
+  release(s.w);
+  release(s.g);
+  release(s.m);
+  release(s.v);
+  release(s.wb);
+  release(s.loss);
+}
+static void free_activations(MlpState& s) {
+  s.cap = 0;
+  for (int q = 0; q < 3; ++q) {
+    release(s.z[q]);
+    release(s.h[q]);
+    release(s.dz[q]);
+  }
+  release(s.out);
+}
+
+// After a failure nothing of the group is left, so that the next call tries again.
 static int mlp_alloc(Ctx* c, MlpState& s, int64_t n) {
   if (!s.w) {
-    if (cudaMalloc(&s.w, kNumParams * 4) != cudaSuccess || cudaMalloc(&s.g, kNumParams * 4) != cudaSuccess ||
-        cudaMalloc(&s.m, kNumParams * 4) != cudaSuccess || cudaMalloc(&s.v, kNumParams * 4) != cudaSuccess ||
-        cudaMalloc(&s.wb, kNumParams * 2) != cudaSuccess || cudaMalloc(&s.loss, 64) != cudaSuccess) {
-      cudaGetLastError();
+    if (!reserve(s.w, kNumParams * 4) || !reserve(s.g, kNumParams * 4) || !reserve(s.m, kNumParams * 4) ||
+        !reserve(s.v, kNumParams * 4) || !reserve(s.wb, kNumParams * 2) || !reserve(s.loss, 64)) {
+      free_params(s);
       return report_error(MVG_ERR_NOMEM, "MLP parameter allocation failed");
     }
     MVG_CUDA_TRY(cudaMemsetAsync(s.m, 0, kNumParams * 4, c->stream));
     MVG_CUDA_TRY(cudaMemsetAsync(s.v, 0, kNumParams * 4, c->stream));
   }
   if (n > s.cap) {
-    for (int q = 0; q < 3; ++q) {
-      cudaFree(s.z[q]);
-      cudaFree(s.h[q]);
-    }
-    cudaFree(s.out);
-    for (int q = 0; q < 3; ++q) cudaFree(s.dz[q]);
-    bool ok = true;
-    for (int q = 0; q < 3; ++q) {
-      ok = ok && cudaMalloc(&s.z[q], n * kHid * 4) == cudaSuccess;
-      ok = ok && cudaMalloc(&s.h[q], rows8(n) * kHid * 2) == cudaSuccess;
-      ok = ok && cudaMalloc(&s.dz[q], n * kHid * 2) == cudaSuccess;
-    }
-    ok = ok && cudaMalloc(&s.out, n * kOut * 4) == cudaSuccess;
+    free_activations(s);
+    bool ok = reserve(s.out, n * kOut * 4);
+    for (int q = 0; q < 3; ++q)
+      ok = ok && reserve(s.z[q], n * kHid * 4) && reserve(s.h[q], rows8(n) * kHid * 2) &&
+           reserve(s.dz[q], n * kHid * 2);
     if (!ok) {
-      cudaGetLastError();
-      s.cap = 0;
+      free_activations(s);
       return report_error(MVG_ERR_NOMEM, "MLP activation allocation failed");
     }
     s.cap = n;
@@ -329,19 +351,9 @@ static int mlp_alloc(Ctx* c, MlpState& s, int64_t n) {
 }
 
 static void mlp_free(MlpState& s) {
-  cudaFree(s.w);
-  cudaFree(s.g);
-  cudaFree(s.m);
-  cudaFree(s.v);
-  cudaFree(s.wb);
-  cudaFree(s.loss);
-  for (int q = 0; q < 3; ++q) {
-    cudaFree(s.z[q]);
-    cudaFree(s.h[q]);
-  }
-  for (int q = 0; q < 3; ++q) cudaFree(s.dz[q]);
-  cudaFree(s.out);
-  cudaFree(s.part);
+  free_params(s);
+  free_activations(s);
+  release(s.part);
   s = MlpState();
 }
 
@@ -475,11 +487,8 @@ static int mlp_backward(Ctx* c, MlpState& s, const __nv_bfloat16* X, const float
   cudaStream_t st = c->stream;
   int rc = grad_kernel_ready(c->device);
   if (rc) return rc;
-  if (!s.part && cudaMalloc(&s.part, kPartFloats * 4) != cudaSuccess) {
-    cudaGetLastError();
-    s.part = nullptr;
+  if (!s.part && !reserve(s.part, kPartFloats * 4))
     return report_error(MVG_ERR_NOMEM, "MLP gradient allocation failed");
-  }
   float* part_w[3] = {s.part, s.part + (int64_t)kGradSplits * kHid * kIn,
                       s.part + (int64_t)kGradSplits * kHid * (kIn + kHid)};
   float* part_b[2] = {s.part + kPartW, s.part + kPartW + kPartB};
@@ -569,6 +578,7 @@ int mvg_mlp_set_params(mvg_handle h, const float* params) {
   MVG_CUDA_TRY(cudaMemcpyAsync(s.w, params, kNumParams * 4, cudaMemcpyHostToDevice, c->stream));
   k_to_bf16<<<grid_for(kNumParams, 256), 256, 0, c->stream>>>(s.w, s.wb, kNumParams);
   c->launches++;
+  MVG_CUDA_TRY(cudaGetLastError());
   MVG_CUDA_TRY(cudaMemsetAsync(s.m, 0, kNumParams * 4, c->stream));
   MVG_CUDA_TRY(cudaMemsetAsync(s.v, 0, kNumParams * 4, c->stream));
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));

@@ -19,7 +19,7 @@ std::mutex mu;
 std::map<std::pair<int, const void*>, size_t> allowed;  // dynamic shared memory, by device and kernel
 size_t refused, largest, free_bytes = (size_t)1 << 40;
 std::map<size_t, std::vector<unsigned char>> replies;  // by size
-long launches, fail_at = -1;
+long launches, fail_at = -1, allocations, no_memory_at = -1;
 thread_local int device;
 thread_local cudaError_t last = cudaSuccess;
 thread_local struct {
@@ -43,9 +43,10 @@ cudaError_t launch(const void* f, size_t smem) {
   return last = cudaErrorInvalidValue;
 }
 
-cudaError_t take(void** p, size_t n) {
+cudaError_t take(void** p, size_t n, bool on_device) {
   std::lock_guard<std::mutex> lk(mu);
-  largest = std::max(largest, n);
+  if (allocations++ == no_memory_at) return last = cudaErrorMemoryAllocation;
+  if (on_device) largest = std::max(largest, n);
   *p = calloc(1, n + 64);
   return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }
@@ -60,8 +61,8 @@ void fake_reset(size_t free_memory) {
   refused = largest = 0;
   free_bytes = free_memory;
   replies.clear();
-  launches = 0;
-  fail_at = -1;
+  launches = allocations = 0;
+  fail_at = no_memory_at = -1;
 }
 // What the next copy of n bytes to the host brings.
 void fake_reply(const void* data, size_t n) {
@@ -71,6 +72,9 @@ void fake_reply(const void* data, size_t n) {
 // The k-th launch from now (from 0) fails; the launches since the last reset.
 void fake_fail_at(long k) { fail_at = launches + k; }
 long fake_launches() { return launches; }
+// The same of allocations, on the device or pinned.
+void fake_no_memory_at(long k) { no_memory_at = allocations + k; }
+long fake_allocations() { return allocations; }
 
 void** __cudaRegisterFatBinary(void*) {
   static void* h;
@@ -137,12 +141,9 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
   return cudaErrorNotSupported;
 }
 
-cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n); }
-cudaError_t cudaMallocHost(void** p, size_t n) {
-  *p = calloc(1, n + 64);
-  return cudaSuccess;
-}
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMallocHost(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n, true); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return take(p, n, false); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return take(p, n, false); }
 cudaError_t cudaFree(void* p) {
   free(p);
   return cudaSuccess;

@@ -25,7 +25,9 @@ def load(where):
     lib.fake_reset.argtypes = [ctypes.c_size_t]
     lib.fake_reply.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     lib.fake_fail_at.argtypes = [ctypes.c_long]
-    lib.fake_launches.restype = ctypes.c_long
+    lib.fake_no_memory_at.argtypes = [ctypes.c_long]
+    for name in ("fake_launches", "fake_allocations"):
+        getattr(lib, name).restype = ctypes.c_long
     lib.mvg_last_error.restype = ctypes.c_char_p
     lib.mvg_get_seed.restype = ctypes.c_uint64
     return lib

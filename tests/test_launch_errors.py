@@ -1,6 +1,6 @@
-"""A launch that CUDA refuses makes the call it belongs to fail, whichever of the
-call's launches it is, and leaves nothing for the next call (no GPU:
-fake_device)."""
+"""A launch that CUDA refuses, or an allocation, makes the call it belongs to
+fail, whichever of the call's it is, and leaves nothing for the next call (no
+GPU: fake_device)."""
 import ctypes
 
 import numpy as np
@@ -99,13 +99,32 @@ def _rows(lib, h):
 def _gradient(lib, h):
     lib.mvg_mlp_num_params.restype = ctypes.c_int64
     w = np.zeros(lib.mvg_mlp_num_params(), np.float32)
-    rc = lib.mvg_mlp_set_params(h, _p(w))
+    if rc := lib.mvg_mlp_set_params(h, _p(w)):
+        return rc
     x, t, g, loss = np.zeros(100 * 528, np.uint16), np.zeros(200, np.float32), np.zeros_like(w), ctypes.c_float(0)
-    return rc or lib.mvg_mlp_grad_dev(h, _p(x), _p(t), i64(100), _p(g), ctypes.byref(loss))
+    return lib.mvg_mlp_grad_dev(h, _p(x), _p(t), i64(100), _p(g), ctypes.byref(loss))
 
 
-@pytest.mark.parametrize("call", [_pairwise, _pairwise_sorted, _gap_search, _batch, _banded, _banded_strips, _sml, _lut,
-                                  _xmfa, _rows, _gradient])
+def _train(lib, h):
+    lib.mvg_mlp_num_params.restype = ctypes.c_int64
+    if rc := lib.mvg_mlp_set_params(h, _p(np.zeros(lib.mvg_mlp_num_params(), np.float32))):
+        return rc
+    x, t, loss = np.zeros(100 * 528, np.uint16), np.zeros(200, np.float32), ctypes.c_float(0)
+    return lib.mvg_mlp_train_step_dev(h, _p(x), _p(t), i64(100), ctypes.c_float(0.1), 1, ctypes.byref(loss))
+
+
+def _gapped(lib, h):
+    off, out_off = np.array([0, 3000, N], np.uint64), np.zeros(3, np.uint64)
+    out = [np.zeros(2 * N, np.uint8) for _ in range(2)]
+    return lib.mvg_gapped_alignment(h, _p(SEQ), _p(SEQ), _p(off), i64(2), ctypes.c_double(20000), 3, _p(out[0]),
+                                    _p(out[1]), _p(out_off), u64(2 * N))
+
+
+CALLS = [_pairwise, _pairwise_sorted, _gap_search, _batch, _banded, _banded_strips, _sml, _lut, _xmfa, _rows, _gradient,
+         _train, _gapped]
+
+
+@pytest.mark.parametrize("call", CALLS)
 def test_every_launch(lib, call):
     h = ctypes.c_void_p()
     assert lib.mvg_create(ctypes.byref(h), 0) == 0
@@ -124,3 +143,28 @@ def test_every_launch(lib, call):
         assert rc == 0 or k in silent, (k, lib.mvg_last_error())
     lib.mvg_destroy(h)
     assert not silent, (silent, count)
+
+
+@pytest.mark.parametrize("call", CALLS)
+def test_every_allocation(lib, call):
+    def fresh():
+        h = ctypes.c_void_p()
+        lib.fake_reset(1 << 40)
+        assert lib.mvg_create(ctypes.byref(h), 0) == 0
+        lib.fake_reset(1 << 40)
+        return h
+
+    h = fresh()
+    assert call(lib, h) == 0
+    count = lib.fake_allocations()
+    lib.mvg_destroy(h)
+    assert count >= 1
+    for k in range(count):
+        h = fresh()
+        lib.fake_no_memory_at(k)
+        # the staging and read-back buffers have a way round
+        assert call(lib, h) in ((0, 6) if call in (_batch, _banded, _banded_strips, _xmfa, _gapped) else (6,)), k
+        for _ in range(2):
+            lib.fake_reset(1 << 40)
+            assert call(lib, h) == 0, (k, lib.mvg_last_error())
+        lib.mvg_destroy(h)
