@@ -19,6 +19,7 @@ int report_error(int code, const char* msg) {
 }
 
 int report_cuda(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here, so none of the next call's
   snprintf(g_last_error, sizeof(g_last_error), "%s: %s", what, cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? MVG_ERR_NOMEM : MVG_ERR_CUDA;
 }
@@ -52,6 +53,7 @@ void Workspace::release() {
 }
 
 int check_device_error(Ctx* c) {
+  MVG_CUDA_TRY(cudaGetLastError());  // launches that were refused
   MVG_CUDA_TRY(cudaMemcpyAsync(c->h_err, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream));
   MVG_CUDA_TRY(cudaStreamSynchronize(c->stream));
   switch (*c->h_err) {

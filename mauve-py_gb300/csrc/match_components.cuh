@@ -852,7 +852,6 @@ int match_components(Ctx* c, P& prob, uint32_t* tab, const PairBucketBufs* join,
   k_comp_emit<<<(unsigned)ctiles, 256, 0, c->stream>>>(tab, key, head, last, moved, joined, nseg, coff, C);
   k_comp_out<<<grid_for(nseg, 256), 256, 0, c->stream>>>(prob, C, scal + 3, bflag, flagged, scal + 4);
   c->launches += 6;
-  MVG_CUDA_TRY(cudaGetLastError());
   stage_mark(c, "flagged");
   MVG_CUDA_TRY(cudaMemcpyAsync(c->h_scalars, scal + 3, 8, cudaMemcpyDeviceToHost, c->stream));
   if (int rc = check_device_error(c)) return rc;

@@ -113,6 +113,16 @@ def _train(lib, h):
     return lib.mvg_mlp_train_step_dev(h, _p(x), _p(t), i64(100), ctypes.c_float(0.1), 1, ctypes.byref(loss))
 
 
+def _propose(lib, h):
+    lib.mvg_mlp_num_params.restype = ctypes.c_int64
+    lib.mvg_set_band_gate(h, 20)
+    if rc := lib.mvg_mlp_set_params(h, _p(np.zeros(lib.mvg_mlp_num_params(), np.float32))):
+        return rc
+    delta, half = np.zeros(2, np.int32), np.zeros(2, np.int32)
+    return lib.mvg_band_propose_dev(h, _p(CODES), _p(OFF), _p(CODES), _p(OFF), i64(2), ctypes.c_float(1),
+                                    ctypes.c_float(8), _p(delta), _p(half))
+
+
 def _gapped(lib, h):
     off, out_off = np.array([0, 3000, N], np.uint64), np.zeros(3, np.uint64)
     out = [np.zeros(2 * N, np.uint8) for _ in range(2)]
@@ -120,8 +130,14 @@ def _gapped(lib, h):
                                     _p(out[1]), _p(out_off), u64(2 * N))
 
 
+def _outside_lcbs(lib, h):
+    regions, out, n, w = np.array([1, 4000], np.int64), np.zeros(3000, np.int64), u64(0), ctypes.c_uint32(0)
+    return lib.mvg_search_lcb_gaps(h, _p(SEQ), u64(N), _p(SEQ), u64(N), _p(regions), u64(2), _p(regions), u64(2),
+                                   _p(out), u64(1000), ctypes.byref(n), ctypes.byref(w))
+
+
 CALLS = [_pairwise, _pairwise_sorted, _gap_search, _batch, _banded, _banded_strips, _sml, _lut, _xmfa, _rows, _gradient,
-         _train, _gapped]
+         _train, _propose, _gapped, _outside_lcbs]
 
 
 @pytest.mark.parametrize("call", CALLS)
