@@ -504,32 +504,36 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   const bool few = strips_all <= 4 * c->sms;
   const int max_rows = few ? 4 : c->dp_rows;
   const int min_piped = few ? 2 : c->dp_coop_strips;
-  std::vector<uint64_t> bytes(nwork), cells(nwork), shapes(nwork);
+  std::vector<uint64_t> bytes(nwork), cells(nwork);
   std::vector<char> piped(nwork), direct(nwork);
   std::vector<uint32_t> strips(nwork);
   uint64_t total = 0, most = 0, most_least = 0;
-  auto shape = [&](int64_t w, uint64_t limit) {
-    const uint32_t p = ids[w];
-    const StripShape h = strip_shape_within(strip_shape((int)la[p], (int)lb[p], max_rows, ckpt), limit);
+  auto take = [&](int64_t w, const StripShape& h) {
     bytes[w] = strip_slot_bytes(h);
     strips[w] = (uint32_t)h.n;
     piped[w] = h.n >= min_piped;
     direct[w] = h.direct;
-    shapes[w] = strip_slot(0, h);
     most = std::max(most, bytes[w]);
-    return h;
   };
   for (int64_t w = 0; w < nwork; ++w) {
-    const StripShape h = shape(w, ~0ull);
-    cells[w] = (uint64_t)h.LA * (uint64_t)h.LB;
+    const uint32_t p = ids[w];
+    const StripShape h = strip_shape((int)la[p], (int)lb[p], max_rows, ckpt);
+    take(w, h);
+    cells[w] = (uint64_t)la[p] * (uint64_t)lb[p];
     total += bytes[w];
     most_least = std::max(most_least, std::min(bytes[w], strip_least_bytes(h, c->dp_rows, ckpt)));
   }
   const uint64_t arena = arena_bound(c, kDpSlots.arena, total);
   const bool sparse = most > arena;  // slots cut to fit
+  std::vector<uint64_t> shapes(sparse ? nwork : 0);
   if (sparse) {
     most = 0;
-    for (int64_t w = 0; w < nwork; ++w) shape(w, arena);
+    for (int64_t w = 0; w < nwork; ++w) {
+      const uint32_t p = ids[w];
+      const StripShape h = strip_shape_within(strip_shape((int)la[p], (int)lb[p], max_rows, ckpt), arena);
+      take(w, h);
+      shapes[w] = strip_slot(0, h);
+    }
   }
   if (std::max(most, most_least) > arena)
     return report_error(MVG_ERR_CAPACITY, "one gap-DP problem exceeds the traceback arena");
@@ -537,7 +541,7 @@ static int run_full(Ctx* c, const DpInputs& in, const std::vector<uint32_t>& ids
   const std::vector<uint32_t> idx = largest_first(cells);
   sub.reset(new HostSpan(c, "dp_waves"));
   DpWaves W = deal_waves(idx, piped, bytes, arena);
-  for (int64_t q = 0; q < nwork; ++q) W.off[q] |= shapes[W.item[q]];
+  for (int64_t q = 0; sparse && q < nwork; ++q) W.off[q] |= shapes[W.item[q]];
   const size_t nwaves = W.begin.size() - 1;
   // one upload: the slots' problems, then per wave the pipelined strips in
   // claim order (pairs) and the walk's slots (checkpointed, then direct)

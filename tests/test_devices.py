@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import fake_device
+import test_launch_errors
 
 u64, i64 = ctypes.c_uint64, ctypes.c_int64
 
@@ -55,6 +56,17 @@ def test_second_device(lib, call, arg):
         assert lib.mvg_create(ctypes.byref(h), device) == 0
         lib.fake_reset(1 << 40)
         assert call(lib, h, arg) == 0, lib.mvg_last_error()
+        assert lib.fake_refused() == 0
+        lib.mvg_destroy(h)
+
+
+@pytest.mark.parametrize("call", test_launch_errors.CALLS)
+def test_every_call_on_a_second_device(lib, call):
+    for device in (0, 1):
+        h = ctypes.c_void_p()
+        assert lib.mvg_create(ctypes.byref(h), device) == 0
+        lib.fake_reset(1 << 40)
+        assert call(lib, h) == 0, lib.mvg_last_error()
         assert lib.fake_refused() == 0
         lib.mvg_destroy(h)
 
